@@ -65,7 +65,6 @@ struct Pending {
     std::vector<int> piece;            // case ranges [piece[p], piece[p+1]) of the result copies
     double t_submit = 0.;
     const lmieb_problem *ps = nullptr; // the problems (alive until the call that submitted them returns)
-    int precision = 0;
 };
 
 // One of two buffer sets: a sub-batch is packed into one while the device
@@ -117,7 +116,7 @@ struct Ctx {
     long long redo_ticket = 1LL << 62;   // tickets of the re-solve slot (their own range)
     int submits = 0;                // sub-batches submitted since the counters were reset
     int call_slot[2] = {-1, -1};    // slots of the first two sub-batches since then
-    long long redo = 0;             // INT8 cases solved again in FP64 since then
+    long long redo = 0;             // cases solved again with the FP64 angular kernel since then
     // The FP64 re-solve of INT8 cases takes their coefficient columns and
     // per-radius sums from the INT8 sub-batch's arena (K1 computed them there
     // with the same operations) instead of running K1 again.
@@ -180,6 +179,11 @@ Ctx g_ctx;
 // uneven cases, coarser ones cut the per-item overhead; set by
 // lmieb_set_work_granularity (the autotuner).
 double g_items_per_sm[3] = {64., 2., 2.};
+
+// Work of a sub-batch's angular sums (radii x orders x half-angles x Mie
+// columns) from which LMIEB_PRECISION_FP64 forms them with the seven-digit
+// contraction.
+constexpr double OZ_MIN_SUMS = 2e7;
 
 int prec_slot(int precision) {
     return precision == LMIEB_PRECISION_TF32X3 ? 1 : (precision == LMIEB_PRECISION_INT8 ? 2 : 0);
@@ -352,12 +356,10 @@ struct Plan {
     int tc_seg = 2;             // its segment length (chunks)
     float *bop = nullptr;       // its B operand (tc_layout.cuh)
     size_t bop_bytes = 0;
-    int oz = 0;                 // K3 as the int8 fixed-point contraction (oz_layout.cuh)
+    int oz = 0;                 // K3 as the fixed-point contraction (oz_layout.cuh): digits per value, 0 without
     unsigned char *bop8 = nullptr;   // its B operand digits
     signed char *rowexp = nullptr;   // its row exponents
     int *colexp = nullptr;      // its column exponents
-    long long *rx_start = nullptr;   // (case, half-angle) index space of the row exponents
-    long long n_rx = 0;
     unsigned char *aop = nullptr;    // its A operand digits, every (case, angle tile, chunk)
     long long *a_start = nullptr;    // (case, tile row) index space of the A operand
     long long n_arow = 0;
@@ -570,15 +572,13 @@ int run_accumulate(Plan &L, cudaStream_t s) {
         return 0;
     }
     if (L.save_control != 2) {
-        // int8 K3's row exponents and A operand (the angles only) on the slot's
-        // side stream while K1 runs: K1 keeps 8 warps per SM, so their blocks
+        // the fixed-point K3's A operand (the angles only) on the slot's side stream while K1 runs: K1 keeps 8 warps per SM, so their blocks
         // find room beside it (with per-stage timing: in line, below)
         const bool fork = L.oz && L.n_ang > 0 && L.side && !g_ctx.timing;
         if (fork) {
             LMIEB_CUDA_TRY(cudaEventRecord(L.fork, s));
             LMIEB_CUDA_TRY(cudaStreamWaitEvent(L.side, L.fork, 0));
-            if (launch_oz_operands(L.side, B, L.n_rx, L.rx_start, L.rowexp, L.n_arow, L.a_start, L.aop, 0,
-                                   nullptr, nullptr, nullptr))
+            if (launch_oz_operands(L.side, B, L.oz, L.n_arow, L.a_start, L.rowexp, L.aop, 0, nullptr, nullptr, nullptr))
                 return -1;
             LMIEB_CUDA_TRY(cudaEventRecord(L.join, L.side));
         }
@@ -602,11 +602,11 @@ int run_accumulate(Plan &L, cudaStream_t s) {
             return -1;
         if (L.oz && L.n_ang > 0) {
             if (fork) LMIEB_CUDA_TRY(cudaStreamWaitEvent(s, L.join, 0));
-            if (launch_oz_operands(s, B, fork ? 0 : L.n_rx, L.rx_start, L.rowexp, fork ? 0 : L.n_arow, L.a_start,
-                                   L.aop, L.n_groups, L.coef, L.bop8, L.colexp))
+            if (launch_oz_operands(s, B, L.oz, fork ? 0 : L.n_arow, L.a_start, L.rowexp, L.aop, L.n_groups, L.coef,
+                                   L.bop8, L.colexp))
                 return -1;
             if (g_ctx.timing) LMIEB_CUDA_TRY(cudaEventRecord(g_ctx.k3[0], s));
-            if (launch_angular_oz(s, B, L.n_ang, L.ang, L.bop8, L.part, L.o_trunc + 2 * L.ncase)) return -1;
+            if (launch_angular_oz(s, B, L.oz, L.n_ang, L.ang, L.bop8, L.part, L.o_trunc + 2 * L.ncase)) return -1;
             if (g_ctx.timing) LMIEB_CUDA_TRY(cudaEventRecord(g_ctx.k3[1], s));
         }
         if (n64 > 0) {
@@ -802,12 +802,14 @@ size_t case_bytes(const lmieb_problem &p) {
     b += (size_t) 4 * ncol * p.n_qang * 8 * 8;                        // partials (groups), pf, pfn
     b += (size_t) ncol * 6 * p.n_coef * 8 * (3 + (p.n_qang / 2 + 31) / 32);   // expansion partials + outputs
     b += (size_t) 4 * (p.n_qang / 2) * (p.n_coef / EX_LT + 1) * 16;   // checkpoints
-    if (p.precision == LMIEB_PRECISION_INT8) {
+    if (p.precision == LMIEB_PRECISION_INT8 || p.precision == LMIEB_PRECISION_FP64) {
         // B operand digits (groups padded to whole chunks), row exponents
-        b += (size_t) (tot + (size_t) p.n * OZ_KC) * OZ_BSTAGE / (OZ_KC * oz_rg(std::min(p.nd1, OZ_MAX_NC1)));
-        b += (size_t) (p.n_qang / 2 + 1) * (tot / std::max(p.n, 1) / OZ_KC + 2) * 2;
+        const int digits = p.precision == LMIEB_PRECISION_INT8 ? 6 : 7;
+        b += (size_t) (tot + (size_t) p.n * OZ_KC) * oz_bstage(digits) /
+             (OZ_KC * oz_rg(digits, std::min(p.nd1, OZ_MAX_NC1)));
+        b += (size_t) p.n_qang;
         b += (size_t) p.n * (1 + p.nd1) * 16;                          // exponents K1 tracks
-        b += (size_t) ((p.n_qang / 2 + OZ_HALF - 1) / OZ_HALF) * ((p.n1 + OZ_KC - 1) / OZ_KC) * OZ_ACHUNK;   // A operand
+        b += (size_t) ((p.n_qang / 2 + OZ_HALF - 1) / OZ_HALF) * ((p.n1 + OZ_KC - 1) / OZ_KC) * oz_achunk(digits);   // A operand
     }
     return b;
 }
@@ -923,7 +925,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     // arena: their copy, in pieces of at most GATHER_PIECE doubles (one
     // block each), replaces K1
     std::vector<GatherSeg> gsegs;
-    if (c.gather.on && (int) c.gather.cs.size() == ncase && p0.precision == LMIEB_PRECISION_FP64 &&
+    if (c.gather.on && (int) c.gather.cs.size() == ncase && p0.precision == LMIEB_PRECISION_FP64_SUMS &&
         L.save_control == 0 && L.acc_mode == LMIEB_ACC_WHOLE) {
         constexpr long long GATHER_PIECE = 1 << 15;
         auto add_seg = [&](const double *src, int which, long long dst_off, long long n) {
@@ -1023,13 +1025,22 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     L.tc = p0.precision == LMIEB_PRECISION_TF32X3 && L.save_control == 0 && any_ang && R > 0 &&
            nd1 <= TC_MAX_NC1 && nd2 <= TC_MAX_ND2;
     L.tc_seg = g_tc_seg;
-    L.oz = p0.precision == LMIEB_PRECISION_INT8 && L.save_control == 0 && any_ang && R > 0 &&
-           nd1 <= OZ_MAX_NC1 && nd2 <= OZ_MAX_ND2;
+    if (L.save_control == 0 && any_ang && R > 0 && nd1 <= OZ_MAX_NC1 && nd2 <= OZ_MAX_ND2) {
+        // INT8: six digits.  FP64: seven, for sub-batches whose angular sums
+        // are worth the operand kernels (OZ_MIN_SUMS), of whole solves (the
+        // integrals a group of processes adds up, or a caller takes away, stay
+        // the FP64 kernel's)
+        double sums = 0.;
+        for (int k = 0; k < ncase; ++k) sums += (double) (cs1[k + 1] - cs1[k]) * cs[k].nh * (1. + nd1);
+        const bool whole = L.acc_mode == LMIEB_ACC_WHOLE || (L.acc_mode == LMIEB_ACC_GROUP && g_group.world == 1);
+        if (p0.precision == LMIEB_PRECISION_INT8) L.oz = 6;
+        else if (p0.precision == LMIEB_PRECISION_FP64 && whole && sums >= OZ_MIN_SUMS) L.oz = 7;
+    }
     // with split precision, cases below TC_MIN_N1 orders keep the FP64 K3: their
     // linearised phase matrices cancel strongly on normalisation, and they cost little
     std::vector<char> case_tc(ncase, 0), case_oz(ncase, 0);
     for (int k = 0; k < ncase; ++k) case_tc[k] = L.tc && cs[k].n_qang > 0 && cs[k].n1 >= TC_MIN_N1;
-    // the int8 stage takes the cases of at least OZ_MIN_N1 orders whose radius
+    // the fixed-point stage takes the cases of at least OZ_MIN_N1 orders whose radius
     // groups fit its exact int32 sums (OZ_MAX_NK chunks)
     for (int k = 0; k < ncase; ++k)
         case_oz[k] = L.oz && cs[k].n_qang > 0 && cs[k].n1 >= OZ_MIN_N1 &&
@@ -1150,13 +1161,14 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         }
         largest_first(tmp, ang);
     }
-    // int8 fixed point: radius groups of oz_rg(nd1) radii, each with its B
-    // operand digits; row-exponent tables per case
+    // fixed point: radius groups of oz_rg(digits, nd1) radii, each with its B
+    // operand digits; row exponents and A operand per case
     long long bop8_bytes = 0, rx_bytes = 0, aop_bytes = 0;
     int nkx_all = 0;
-    std::vector<long long> rx_start(ncase + 1, 0), a_start(ncase + 1, 0);
+    std::vector<long long> a_start(ncase + 1, 0);
+    const long long oz_bst = L.oz ? (long long) oz_bstage(L.oz) : 0;
     if (L.oz) {
-        const int RG = oz_rg(nd1);
+        const int RG = oz_rg(L.oz, nd1);
         std::vector<int> cg0(ncase + 1, 0);
         std::vector<long long> cb0(ncase + 1, 0);     // B operand chunks before each case
         std::vector<double> wc(ncase, 0.);
@@ -1187,7 +1199,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             const DevCase &C = cs[k];
             if (!case_oz[k]) return;
             int g = cg0[k];
-            long long o = cb0[k] * OZ_BSTAGE;
+            long long o = cb0[k] * oz_bst;
             for (int r = C.r0; r < C.r0 + C.nr; r += RG, ++g) {
                 const int n = std::min(RG, C.r0 + C.nr - r);
                 int mx = 1;
@@ -1197,33 +1209,32 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
                 tg_n[g] = n;
                 tg_nk[g] = nk;
                 tg_off[g] = o;
-                o += (long long) nk * OZ_BSTAGE;
+                o += nk * oz_bst;
             }
         });
-        bop8_bytes = cb0[ncase] * OZ_BSTAGE;
+        bop8_bytes = cb0[ncase] * oz_bst;
         double W = 0.;
         for (int k = 0; k < ncase; ++k) {
             DevCase &C = cs[k];
-            rx_start[k + 1] = rx_start[k];
             a_start[k + 1] = a_start[k];
             if (!case_oz[k]) continue;
             C.nkx = (cn1max[k] + OZ_KC - 1) / OZ_KC;
             C.rx_off = rx_bytes;
             C.trunc_band = C.accuracy > 0. ? oz_trunc_band(cn1max[k]) : 0.;
-            rx_bytes += (long long) C.nh * C.nkx * 2;
-            rx_start[k + 1] += C.nh;
+            rx_bytes += 2LL * C.nh;
             // the A operand of each angle tile and chunk
             const int ntile = (C.nh + OZ_HALF - 1) / OZ_HALF;
             C.a_off = aop_bytes;
-            aop_bytes += (long long) ntile * C.nkx * OZ_ACHUNK;
+            aop_bytes += (long long) ntile * C.nkx * (long long) oz_achunk(L.oz);
             a_start[k + 1] += (long long) ntile * OZ_M;
             nkx_all = std::max(nkx_all, C.nkx);
             W += wc[k] * ((C.nh + OZ_HALF - 1) / OZ_HALF);
         }
         L.n_groups = (int) tg_r0.size();
-        L.n_rx = rx_start[ncase];
         L.n_arow = a_start[ncase];
-        const double wt = std::max(W / (g_items_per_sm[2] * c.sms), 8.);    // chunks per item
+        // chunks per item (the FP64 setting counts FP64 K3 items: 64 for 2 of these)
+        const double ips = L.oz == 6 ? g_items_per_sm[2] : g_items_per_sm[0] / 32.;
+        const double wt = std::max(W / (ips * c.sms), 8.);
         std::vector<std::pair<double, AngItem>> tmp;
         for (int k = 0; k < ncase; ++k) {
             DevCase &C = cs[k];
@@ -1408,7 +1419,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         } else if (L.save_control != 2) {
             nl += (gsegs.empty() ? (long long) std::max(L.nd1c, 1) : 1) + 1;   // K1 per chunk (or its copy), K2
             if (L.tc) nl += (L.n_ang > 0) + (L.n_ang64 > 0 ? L.n_ang_launch : 0);   // K3
-            else if (L.oz) nl += (L.n_ang > 0 ? 4 : 0) + (L.n_ang64 > 0 ? L.n_ang_launch : 0);   // row exponents, A, B, K3
+            else if (L.oz) nl += (L.n_ang > 0 ? 3 : 0) + (L.n_ang64 > 0 ? L.n_ang_launch : 0);   // A, B, K3
             else nl += L.n_ang > 0 ? L.n_ang_launch : 0;
             if (L.n_ang > 0 || L.n_ang64 > 0) nl += 1;                          // group reduction
         } else {
@@ -1434,11 +1445,11 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         if (!finish) fgsf = fexp = 0.;
         c.work[0] += fang;
         if (L.oz) {
-            // OZ_NPROD products of M x N x K per chunk of every (angle tile, group) pair
+            // the digit products of M x N x K per chunk of every (angle tile, group) pair
             double chunks = 0.;
             for (const AngItem &a : ang)
                 for (int gg = a.rbeg; gg < a.rend; ++gg) chunks += tg_nk[gg];
-            c.tensor_ops += 2. * OZ_NPROD * (double) OZ_M * OZ_NP * OZ_KC * chunks;
+            c.tensor_ops += 2. * oz_nprod(L.oz) * (double) OZ_M * oz_np(L.oz) * OZ_KC * chunks;
         }
         c.work[1] += frec;
         c.work[2] += fgsf;
@@ -1475,7 +1486,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         add(gx.size() * sizeof(ExpItem));
         add(gsegs.size() * sizeof(GatherSeg));
         add(tc_pos.size() * 4); add(tc_roff.size() * 8); add(tg_r0.size() * 4); add(tg_n.size() * 4);
-        add(tg_nk.size() * 4); add(tg_off.size() * 8); add(oz_f2.size() * 8); add(rx_start.size() * 8);
+        add(tg_nk.size() * 4); add(tg_off.size() * 8); add(oz_f2.size() * 8);
         add(a_start.size() * 8);
         for (int q = 0; q < 6; ++q) add((size_t) (ncase + 1) * 8);   // prefix arrays over the cases
         add((size_t) ncase * 4); add((size_t) (ncase + 1) * 8);             // K1 launch order
@@ -1538,7 +1549,6 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     int *h_tgnk = put(hp, ho, tg_nk.data(), tg_nk.size());
     long long *h_tgoff = put(hp, ho, tg_off.data(), tg_off.size());
     double *h_ozf2 = put(hp, ho, oz_f2.data(), oz_f2.size());
-    long long *h_rxs = put(hp, ho, rx_start.data(), rx_start.size());
     long long *h_axs = put(hp, ho, a_start.data(), a_start.size());
     long long *h_pfs = put(hp, ho, pf_start.data(), pf_start.size());
     long long *h_ckg = put(hp, ho, ck_gc.data(), ck_gc.size());
@@ -1587,7 +1597,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             if (L.oz) {
                 add((size_t) bop8_bytes);
                 add((size_t) rx_bytes);
-                add((size_t) L.n_groups * OZ_NP * 4);
+                add((size_t) L.n_groups * oz_np(L.oz) * 4);
                 add((size_t) (1 + nd1) * R * 16);
                 add((size_t) aop_bytes);
             }
@@ -1674,9 +1684,8 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         if (L.oz) {
             L.bop8 = A.take<unsigned char>((size_t) bop8_bytes);
             L.rowexp = A.take<signed char>((size_t) rx_bytes);
-            L.colexp = A.take<int>((size_t) L.n_groups * OZ_NP);
+            L.colexp = A.take<int>((size_t) L.n_groups * oz_np(L.oz));
             B.oz_radexp = A.take<int>((size_t) (1 + nd1) * R * 4);
-            L.rx_start = (long long *) dptr(h_rxs);
             L.aop = A.take<unsigned char>((size_t) aop_bytes);
             L.a_start = (long long *) dptr(h_axs);
             B.oz_aop = L.aop;
@@ -1885,7 +1894,6 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     P.piece.swap(piece);
     P.t_submit = now_ms();
     P.ps = ps;
-    P.precision = p0.precision;
     return 0;
 }
 
@@ -1893,12 +1901,12 @@ long long submit_locked(int n, const lmieb_problem *p, lmieb_result *r);
 int collect_ticket(long long ticket);
 int fit_sub(int n, const lmieb_problem *p);
 
-// INT8 cases whose truncation n_coef is not certain at the contraction's
-// error: some |beta_l| (l up to the truncation) lies within the band of
-// `accuracy` (k_exp_final's band outputs).  They are solved again in FP64 by
-// the caller of collect_slot.
+// Cases of the fixed-point stage (INT8, FP64) whose truncation n_coef could
+// differ from the FP64 angular kernel's: some |beta_l| (l up to the
+// truncation) lies within the band of `accuracy` (k_exp_final's band
+// outputs).  They are solved again with that kernel by collect_slot.
 void uncertain_truncations(const Pending &P, const int *htr, std::vector<int> &out) {
-    if (P.precision != LMIEB_PRECISION_INT8 || !(P.want_gc || P.want_lc)) return;
+    if (!(P.want_gc || P.want_lc)) return;
     const int ncase = P.ncase;
     const int *tr = P.want_lc ? htr + ncase : htr;
     const int *band = htr + 2 * ncase + 1 + (P.want_lc ? 2 * ncase : 0);
@@ -1938,8 +1946,8 @@ int collect_slot(Slot &S) {
             fprintf(stderr, "ERROR: lmie_b200: a tensor-core angular stage timed out waiting for its pipeline\n");
         return -1;
     }
-    // Cases whose truncation the int8 contraction's error could have moved
-    // are solved again in FP64.  They go to the re-solve slot now, so that
+    // Cases whose truncation the fixed-point contraction could have moved are
+    // solved again with the FP64 angular kernel.  They go to the re-solve slot now, so that
     // the device runs them while the host unpacks this sub-batch; their
     // results replace these cases' when they are collected below.
     std::vector<int> redo;
@@ -1951,12 +1959,13 @@ int collect_slot(Slot &S) {
     if (!redo.empty()) {
         for (int k : redo) {
             rq.push_back(P.ps[k]);
-            rq.back().precision = LMIEB_PRECISION_FP64;
+            rq.back().precision = LMIEB_PRECISION_FP64_SUMS;
+            rq.back().acc_mode = LMIEB_ACC_WHOLE;   // (a group of one: the sums are this process's)
             rr.push_back(rs_keep[k]);
         }
         c.redo += (long long) redo.size();
         Slot &R3 = c.slot[2];
-        if (!c.timing && !R3.pend.active) {
+        if (!c.timing && !R3.pend.active && P.acc_mode == LMIEB_ACC_WHOLE) {
             redo_early = fit_sub((int) rq.size(), rq.data());
             if (c.submits < 2) c.call_slot[c.submits] = 2;
             ++c.submits;
@@ -2351,7 +2360,7 @@ extern "C" int lmieb_rerun_device(int reps, int flush_l2, double *ms_total, doub
     std::lock_guard<std::mutex> lock(g_mu);
     Ctx &c = g_ctx;
     // a re-run repeats the resident sub-batches of the last call: exactly one,
-    // or an INT8 sub-batch and the FP64 re-solve of its uncertain cases
+    // or a sub-batch and the FP64 re-solve of its uncertain cases
     const int ns = c.submits;
     bool ok = c.ready && (ns == 1 || (ns == 2 && c.redo > 0 && c.call_slot[0] != c.call_slot[1]));
     for (int i = 0; ok && i < ns; ++i) {
@@ -2553,7 +2562,7 @@ extern "C" int lmieb_oz_selftest_wait(int K, long long wait_cycles, int withhold
         return -1;
     }
     if (ensure_ready()) return -1;
-    const int M = OZ_M, N = OZ_NP;   // one product tile
+    const int M = OZ_M, N = oz_np(6);   // one product tile
     std::vector<double> a((size_t) M * K), b((size_t) N * K), d((size_t) M * N), ref((size_t) M * N, 0.);
     // seeded operands with the growth of the angular products in k: A ~ k^2,
     // B ~ 1/k with a decaying tail, both spanning orders of magnitude over rows

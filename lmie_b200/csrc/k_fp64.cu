@@ -23,6 +23,7 @@
 #include <cstdio>
 
 #include "kernels.h"
+#include "oz_layout.cuh"
 #include "tc_layout.cuh"
 
 namespace {
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, int c0, int write_value,
                              fv4[j - 1] * (re_mulc(alp[k], bp) + re_mulc(ap, blp[k]));
             }
             // expansion coefficients of order j
-            const int ek = 32 - __clz(2 * j - 1);
+            const int ek = oz_ek(j);
             if (write_value) {
                 const cplx cs = (a + b) * f4, cd = (a - b) * f4;
                 if (to_tc) tc_stage<CC>(tcbuf, j, 0, cs.re, cs.im, cd.re, cd.im);

@@ -50,8 +50,8 @@ struct DevCase {
     int scal_off;               // [ncol][4] normalised cross sections and g
     int G;                      // angular radius groups
     int nkx;                    // int8 K3: chunks of OZ_KC orders its row exponents cover
-    long long rx_off;           // int8 K3: its row exponents ([nh][nkx][2] bytes)
-    long long a_off;            // int8 K3: its A operand digits ([tile][nkx][OZ_AROW / 16 pieces][OZ_M rows][16 bytes])
+    long long rx_off;           // int8 K3: its row exponents ([nh][2] bytes)
+    long long a_off;            // int8 K3: its A operand digits ([tile][nkx][AROW / 16 pieces][OZ_M rows][16 bytes])
     double trunc_band;          // > 0: K4 records where |beta_l| comes within trunc_band (2l + 1)
                                 // of `accuracy` (band[2c], band[2c + 1]; see launch_expand)
 };
@@ -89,7 +89,7 @@ struct DevBatch {
     // int8 fixed-point K3 (oz_layout.cuh); null in the other forms
     const double *oz_f2;        // [OZ_KC * max chunks + 2]: (k + 1) / k
     const signed char *oz_rowexp;   // row exponents (DevCase.rx_off)
-    const int *oz_colexp;       // [group][OZ_NP] column exponents
+    const int *oz_colexp;       // [group][NP] column exponents
     const unsigned char *oz_aop;   // A operand digits of every angle tile (DevCase.a_off)
     int *oz_radexp;             // [1 + nd1][R][4]: per radius, coefficient column and component, the
                                 //     largest (biased exponent + e_k) over the orders, 0 if no normal
@@ -131,20 +131,19 @@ int launch_angular_tc(cudaStream_t s, const DevBatch &B, int nitems, const AngIt
                       double *part, int seg, int *err);
 // D[128 x 240] = A[128 x K] B[240 x K]^T through the same tensor-core path
 int launch_tc_selftest(cudaStream_t s, int K, const double *A, const double *Bm, double *D, int *err);
-// K3 as an exact fixed-point contraction on the int8 tensor cores (k_oz.cu):
-// the row exponents (thread per (case, half-angle) of the flat index space
-// row_start), the A operand digits (thread per product row of every angle
-// tile, arow_start) and the B operand digits and column exponents (block per
-// radius group) from K1's FP64 coefficient columns, then the products; items
-// as for launch_angular_tc.
-int launch_oz_operands(cudaStream_t s, const DevBatch &B, long long nrow, const long long *row_start,
-                       signed char *rowexp, long long narow, const long long *arow_start, unsigned char *aop,
-                       int ngroups, const double *coef, unsigned char *bop, int *colexp);
-int launch_angular_oz(cudaStream_t s, const DevBatch &B, int nitems, const AngItem *items, const unsigned char *bop,
-                      double *part, int *err);
-// D[128 x OZ_NP] = A[128 x K] B[OZ_NP x K]^T through the same fixed-point path
+// K3 as an exact fixed-point contraction on the int8 tensor cores (k_oz.cu)
+// with six or seven digits per value: the row exponents and A operand digits
+// (thread per product row of every angle tile, arow_start) and the B operand
+// digits and column exponents (block per radius group) from K1's FP64
+// coefficient columns, then the products; items as for launch_angular_tc.
+int launch_oz_operands(cudaStream_t s, const DevBatch &B, int digits, long long narow, const long long *arow_start,
+                       signed char *rowexp, unsigned char *aop, int ngroups, const double *coef, unsigned char *bop,
+                       int *colexp);
+int launch_angular_oz(cudaStream_t s, const DevBatch &B, int digits, int nitems, const AngItem *items,
+                      const unsigned char *bop, double *part, int *err);
 // *err = 2 if the radius group's failure count *failed is not zero
 int launch_group_flag(cudaStream_t s, const double *failed, int *err);
+// D[128 x 64] = A[128 x K] B[64 x K]^T through the six-digit fixed-point path
 int launch_oz_selftest(cudaStream_t s, int K, const double *A, const double *Bm, double *D, int *err,
                        long long wait_cycles, int withhold);
 // per-case element lists: element e of the flat index space belongs to the

@@ -20,6 +20,11 @@
 extern "C" {
 #endif
 
+/* lmieb_problem.precision beyond LMIEB_PRECISION_* of include/lmie_b200.h: FP64
+ * with the angular sums always in the FP64 kernel (the re-solve of cases at
+ * the truncation threshold). */
+#define LMIEB_PRECISION_FP64_SUMS 3
+
 /* One polydisperse problem, ready for the device.  Derivative slots are in
  * the caller's order kk = 0..nd-1; idx1/idx2 split them like the reference's
  * create_derivs_indexes (src/lmie_interface.c:304-353). */
