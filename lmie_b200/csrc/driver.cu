@@ -125,6 +125,7 @@ struct Ctx {
         const double *coef = nullptr, *rs = nullptr;   // the source sub-batch's K1 outputs
         long long tot = 0;                             // its orders per coefficient column
         int R = 0;                                     // its radii
+        bool hm = false, hx = false, x_own = false;    // its tangent basis
         std::vector<DevCase> cs;                       // its cases, in the order of the re-solve
     } gather;
     cudaEvent_t redo_read = nullptr;   // after a re-solve that reads another slot's arena
@@ -342,7 +343,7 @@ struct Arena {
 struct Plan {
     DevBatch B;
     int ncase = 0;
-    int nd1c = 0, n_ang_launch = 0;
+    int n_ang_launch = 0;
     int want_gc = 0, want_lc = 0, pf_from = 0, save_control = 0, n_qang0 = 0;
     double *ck = nullptr, *coef = nullptr, *rs = nullptr, *sums = nullptr, *part = nullptr;
     double *pfacc = nullptr, *pfn = nullptr, *ckpt = nullptr, *exq = nullptr;
@@ -584,12 +585,8 @@ int run_accumulate(Plan &L, cudaStream_t s) {
         }
         if (L.n_gseg > 0) {
             if (launch_gather(s, L.n_gseg, L.gsegs, L.coef, L.rs)) return -1;
-        } else {
-            for (int ch = 0; ch < (L.nd1c > 0 ? L.nd1c : 1); ++ch) {
-                const int c0 = ch * 4;
-                const int nc = std::max(0, std::min(4, B.nd1 - c0));
-                if (launch_coef(s, B, nc, c0, ch == 0, L.ck, L.coef, L.bop, L.rs)) return -1;
-            }
+        } else if (launch_coef(s, B, L.ck, L.coef, L.bop, L.rs)) {
+            return -1;
         }
         stage(2);
         if (launch_reduce_scalars(s, B, L.rs, L.sums, L.save_control == 1 ? L.o_save1 : nullptr)) return -1;
@@ -797,8 +794,8 @@ size_t case_bytes(const lmieb_problem &p) {
     for (int r = 0; r < p.n; ++r) tot += p.n1r[r] + 1;
     const size_t ncol = 1 + p.nd;
     size_t b = (size_t) tot * 32 * (1 + p.nd1);                        // coef
-    b += (size_t) (tot / K1_B + p.n) * 8 * k1_ck_width(std::min(p.nd1, 4));   // K1 checkpoints
-    b += (size_t) p.n * (64 + 8 * ncol + 40 * (1 + p.nd1));           // per-radius arrays, sums
+    b += (size_t) (tot / K1_B + p.n) * 8 * k1_ck_width(p.nd1 > 0, p.nd1 > 1);   // K1 checkpoints
+    b += (size_t) p.n * (64 + 8 * ncol + 40 * (2 + p.nd1));           // per-radius arrays, sums
     b += (size_t) 4 * ncol * p.n_qang * 8 * 8;                        // partials (groups), pf, pfn
     b += (size_t) ncol * 6 * p.n_coef * 8 * (3 + (p.n_qang / 2 + 31) / 32);   // expansion partials + outputs
     b += (size_t) 4 * (p.n_qang / 2) * (p.n_coef / EX_LT + 1) * 16;   // checkpoints
@@ -806,7 +803,7 @@ size_t case_bytes(const lmieb_problem &p) {
         // B operand digits (groups padded to whole chunks), row exponents
         const int digits = p.precision == LMIEB_PRECISION_INT8 ? 6 : 7;
         b += (size_t) (tot + (size_t) p.n * OZ_KC) * oz_bstage(digits) /
-             (OZ_KC * oz_rg(digits, std::min(p.nd1, OZ_MAX_NC1)));
+             (OZ_KC * oz_rg(digits, std::min(p.nd1, 2)));
         b += (size_t) p.n_qang;
         b += (size_t) p.n * (1 + p.nd1) * 16;                          // exponents K1 tracks
         b += (size_t) ((p.n_qang / 2 + OZ_HALF - 1) / OZ_HALF) * ((p.n1 + OZ_KC - 1) / OZ_KC) * oz_achunk(digits);   // A operand
@@ -834,7 +831,6 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     L.pf_from = p0.n_angles > 0 ? p0.pf_from : 0;
     L.save_control = p0.save_control;
     L.n_qang0 = p0.n_qang;
-    L.nd1c = (nd1 + 3) / 4;
     L.n_ang_launch = std::max(1, std::max((nd1 + 3) / 4, (nd2 + 3) / 4));
     L.acc_mode = p0.acc_mode;
     if (L.acc_mode != LMIEB_ACC_WHOLE && (ncase != 1 || L.save_control != 0)) {
@@ -921,24 +917,44 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         }
     });
     const long long tot = off[R], ckn = ckoff[R];
+    // tangent basis of K1's columns (k_mie.cu)
+    L.tc = p0.precision == LMIEB_PRECISION_TF32X3 && L.save_control == 0 && nqmax > 0 && R > 0 &&
+           nd1 <= TC_MAX_NC1 && nd2 <= TC_MAX_ND2;
+    bool hm = false, hx = false, wl = false;
+    for (int k = 0; k < ncase; ++k) {
+        hm = hm || ps[k].m_tangent;
+        hx = hx || ps[k].x_tangent;
+        wl = wl || ps[k].w_tangent;
+    }
+    bool x_own = nd1 == 1 && hm && hx;
+    if (x_own) hm = false;
+    const bool re_solve = c.gather.on && (int) c.gather.cs.size() == ncase &&
+                          p0.precision == LMIEB_PRECISION_FP64_SUMS && L.save_control == 0 &&
+                          L.acc_mode == LMIEB_ACC_WHOLE;
+    if (re_solve) {
+        hm = c.gather.hm;
+        hx = c.gather.hx;
+        x_own = c.gather.x_own;
+    }
+    const int n_tan = (int) hm + (int) hx;                    // tangent columns of the coefficients
+    const int n_co = 1 + n_tan, n_rs = 1 + 2 * (int) hm + (int) hx, ck_w = k1_ck_width(hm, hx);
     // an FP64 re-solve whose cases' K1 outputs are in an earlier sub-batch's
     // arena: their copy, in pieces of at most GATHER_PIECE doubles (one
     // block each), replaces K1
     std::vector<GatherSeg> gsegs;
-    if (c.gather.on && (int) c.gather.cs.size() == ncase && p0.precision == LMIEB_PRECISION_FP64_SUMS &&
-        L.save_control == 0 && L.acc_mode == LMIEB_ACC_WHOLE) {
+    if (re_solve) {
         constexpr long long GATHER_PIECE = 1 << 15;
         auto add_seg = [&](const double *src, int which, long long dst_off, long long n) {
             for (long long a = 0; a < n; a += GATHER_PIECE)
                 gsegs.push_back(GatherSeg{src + a, dst_off + a, std::min(GATHER_PIECE, n - a), which});
         };
-        const int C1 = 1 + nd1;
         for (int k = 0; k < ncase; ++k) {
             const DevCase &F = c.gather.cs[k], &T = cs[k];
             const long long no = cs1[k + 1] - cs1[k];   // the case's orders (the same radii in both)
-            for (int col = 0; col < C1; ++col) {
+            for (int col = 0; col < n_co; ++col)
                 add_seg(c.gather.coef + ((size_t) col * c.gather.tot + F.o0) * 4, 0, ((long long) col * tot + T.o0) * 4,
                         no * 4);
+            for (int col = 0; col < n_rs; ++col) {
                 for (int q = 0; q < 5; ++q)
                     add_seg(c.gather.rs + (size_t) (col * 5 + q) * c.gather.R + F.r0, 1,
                             (long long) (col * 5 + q) * R + T.r0, T.nr);
@@ -1022,10 +1038,8 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     // ---- angular work items (largest first), partial and pf offsets ----
     bool any_ang = false;
     for (int k = 0; k < ncase; ++k) any_ang |= cs[k].n_qang > 0;
-    L.tc = p0.precision == LMIEB_PRECISION_TF32X3 && L.save_control == 0 && any_ang && R > 0 &&
-           nd1 <= TC_MAX_NC1 && nd2 <= TC_MAX_ND2;
     L.tc_seg = g_tc_seg;
-    if (L.save_control == 0 && any_ang && R > 0 && nd1 <= OZ_MAX_NC1 && nd2 <= OZ_MAX_ND2) {
+    if (L.save_control == 0 && any_ang && R > 0 && nd1 <= OZ_MAX_ND1 && nd2 <= OZ_MAX_ND2) {
         // INT8: six digits.  FP64: seven, for sub-batches whose angular sums
         // are worth the operand kernels (OZ_MIN_SUMS), of whole solves (the
         // integrals a group of processes adds up, or a caller takes away, stay
@@ -1161,14 +1175,14 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         }
         largest_first(tmp, ang);
     }
-    // fixed point: radius groups of oz_rg(digits, nd1) radii, each with its B
+    // fixed point: radius groups of oz_rg(digits, columns) radii, each with its B
     // operand digits; row exponents and A operand per case
     long long bop8_bytes = 0, rx_bytes = 0, aop_bytes = 0;
     int nkx_all = 0;
     std::vector<long long> a_start(ncase + 1, 0);
     const long long oz_bst = L.oz ? (long long) oz_bstage(L.oz) : 0;
     if (L.oz) {
-        const int RG = oz_rg(L.oz, nd1);
+        const int RG = oz_rg(L.oz, n_tan);
         std::vector<int> cg0(ncase + 1, 0);
         std::vector<long long> cb0(ncase + 1, 0);     // B operand chunks before each case
         std::vector<double> wc(ncase, 0.);
@@ -1232,9 +1246,18 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         }
         L.n_groups = (int) tg_r0.size();
         L.n_arow = a_start[ncase];
-        // chunks per item (the FP64 setting counts FP64 K3 items: 64 for 2 of these)
+        // Chunks per item (the FP64 setting counts FP64 K3 items: 64 for 2 of
+        // these).  A block's set-up costs a few chunks' time, so small
+        // sub-batches get the set number of items per SM; where items would be
+        // longer than OZ_ITEM_CHUNKS they are cut, down to a quarter, so that
+        // the SMs' last items end together (x = 5000 alone: 320 items of equal
+        // length on 148 SMs ran as three rounds).
         const double ips = L.oz == 6 ? g_items_per_sm[2] : g_items_per_sm[0] / 32.;
-        const double wt = std::max(W / (ips * c.sms), 8.);
+        constexpr double OZ_ITEM_CHUNKS = 200.;
+        const double w0 = W / (ips * c.sms);
+        const double wt = std::max(std::max(w0 / 4., std::min(w0, OZ_ITEM_CHUNKS)), 8.);
+        int n_fx = 0;
+        for (int k = 0; k < ncase; ++k) n_fx += case_oz[k];
         std::vector<std::pair<double, AngItem>> tmp;
         for (int k = 0; k < ncase; ++k) {
             DevCase &C = cs[k];
@@ -1243,6 +1266,16 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             const int xt = (C.nh + OZ_HALF - 1) / OZ_HALF;
             int G = (int) std::lround(wc[k] / wt);
             G = std::max(1, std::min(G, ng));
+            if (n_fx == 1) {
+                // alone on the device: of the counts up to twice that, the one
+                // whose items fill their last round of SMs best
+                double best = 0.;
+                const int G0 = G;
+                for (int q = G0; q <= std::min(2 * G0, ng); ++q) {
+                    const double r = (double) q * xt / c.sms, f = r / std::ceil(r);
+                    if (f > best + .01) { best = f; G = q; }
+                }
+            }
             std::vector<int> gs(G + 1, cg0[k + 1]);
             gs[0] = cg0[k];
             double run = 0.;
@@ -1257,11 +1290,14 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             C.G = G;
             C.part_off = part_total;
             part_total += (long long) G * Q * C.n_qang;
-            for (int g = 0; g < G; ++g) {
-                double cost = 0.;
-                for (int gg = gs[g]; gg < gs[g + 1]; ++gg) cost += tg_nk[gg] + 1;
-                for (int t = 0; t < xt; ++t) tmp.push_back({cost, AngItem{k, t, g, gs[g], gs[g + 1]}});
-            }
+            // tile by tile: the blocks that run together then share few tiles' A
+            // operands (x = 5000: 4.6 MB each) and read each range's B operand
+            // for several tiles at once, all from L2
+            std::vector<double> cost(G, 0.);
+            for (int g = 0; g < G; ++g)
+                for (int gg = gs[g]; gg < gs[g + 1]; ++gg) cost[g] += tg_nk[gg] + 1;
+            for (int t = 0; t < xt; ++t)
+                for (int g = 0; g < G; ++g) tmp.push_back({cost[g], AngItem{k, t, g, gs[g], gs[g + 1]}});
         }
         largest_first(tmp, ang);
     }
@@ -1282,13 +1318,22 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         }
         // work per block; in a tensor-core batch these are the cases under 16
         // orders (a few half-angles, up to ~2000 radii each), whose blocks
-        // would otherwise walk all their radii one after the other
-        const double wt = std::max(W / (g_items_per_sm[0] * c.sms), (L.tc || L.oz) ? 4096. : 64. * 2 * 64 * 16);
+        // would otherwise walk all their radii one after the other.  Without
+        // one, a block has at least 131072 order-angle products, but no more
+        // than give its case 4 blocks for every SM, down to 4096: a block's
+        // threads walk their radii serially at the latency of the recurrence,
+        // and the 200-radius aerosol solve on 2 blocks took 251 us for 10
+        // MFLOP.  (The case's own work counts, so that a case solved again on
+        // its own is cut as it was in its sub-batch.)
+        const double w_all = W / (g_items_per_sm[0] * c.sms);
         std::vector<std::pair<double, AngItem>> tmp;
         for (int k = 0; k < ncase; ++k) {
             DevCase &C = cs[k];
             if (C.n_qang <= 0 || case_tc[k] || case_oz[k]) continue;
             const int xt = (C.nh + per - 1) / per;
+            const double wt = (L.tc || L.oz) ? std::max(w_all, 4096.)
+                              : w_all > 131072. ? w_all
+                                                : std::min(131072., std::max(wc[k] / (4. * c.sms), 4096.));
             int G = (int) std::lround(wc[k] / (xt * wt));
             G = std::max(1, std::min(G, (L.tc || L.oz) ? std::min(C.nr, 64) : C.nr));
             std::vector<int> gs(G + 1, C.r0 + C.nr);
@@ -1417,7 +1462,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         if (!solve) {
             // integrals uploaded (or zero on an empty share)
         } else if (L.save_control != 2) {
-            nl += (gsegs.empty() ? (long long) std::max(L.nd1c, 1) : 1) + 1;   // K1 per chunk (or its copy), K2
+            nl += 2;                                                             // K1 (or its copy), K2
             if (L.tc) nl += (L.n_ang > 0) + (L.n_ang64 > 0 ? L.n_ang_launch : 0);   // K3
             else if (L.oz) nl += (L.n_ang > 0 ? 3 : 0) + (L.n_ang64 > 0 ? L.n_ang_launch : 0);   // A, B, K3
             else nl += L.n_ang > 0 ? L.n_ang_launch : 0;
@@ -1592,17 +1637,17 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     {
         auto add = [&](size_t b) { dev_bytes += pad(b); };
         if (L.save_control != 2 && L.acc_mode != LMIEB_ACC_FINISH) {
-            add((size_t) ckn * 8 * k1_ck_width(std::min(nd1, 4)));
+            add((size_t) ckn * 8 * ck_w);
             if (L.tc) add((size_t) bop_floats * 4);
             if (L.oz) {
                 add((size_t) bop8_bytes);
                 add((size_t) rx_bytes);
                 add((size_t) L.n_groups * oz_np(L.oz) * 4);
-                add((size_t) (1 + nd1) * R * 16);
+                add((size_t) n_co * R * 16);
                 add((size_t) aop_bytes);
             }
-            add((size_t) (1 + nd1) * (size_t) ctot * 32);
-            add((size_t) (1 + nd1) * 5 * (size_t) R * 8);
+            add((size_t) n_co * (size_t) ctot * 32);
+            add((size_t) n_rs * 5 * (size_t) R * 8);
             add((size_t) part_total * 8);
         }
         add((L.acc_n + 1) * 8);                                  // sums + pfacc + the group's failure count
@@ -1627,6 +1672,12 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     B.R = R;
     B.nd = nd; B.nd1 = nd1; B.nd2 = nd2;
     B.n1max = n1max; B.ncmax = ncmax;
+    B.t_m = hm ? 1 : 0;
+    B.t_x = hx ? 1 + (int) hm : 0;
+    B.x_own = x_own;
+    B.rs_m = 1;
+    B.rs_x = 1 + 2 * (int) hm;
+    B.oz_wl = wl;
     B.pu_lp = g_pu_lp;
     B.cs = (const DevCase *) dptr(h_cs);
     B.idx1 = (const int *) dptr(h_i1);
@@ -1676,7 +1727,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     }
     const bool solve = L.save_control != 2 && L.acc_mode != LMIEB_ACC_FINISH;
     if (solve) {
-        L.ck = A.take<double>((size_t) ckn * k1_ck_width(std::min(nd1, 4)));
+        L.ck = A.take<double>((size_t) ckn * ck_w);
         if (L.tc) {
             L.bop_bytes = (size_t) bop_floats * 4;
             L.bop = A.take<float>((size_t) bop_floats);
@@ -1685,7 +1736,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             L.bop8 = A.take<unsigned char>((size_t) bop8_bytes);
             L.rowexp = A.take<signed char>((size_t) rx_bytes);
             L.colexp = A.take<int>((size_t) L.n_groups * oz_np(L.oz));
-            B.oz_radexp = A.take<int>((size_t) (1 + nd1) * R * 4);
+            B.oz_radexp = A.take<int>((size_t) n_co * R * 4);
             L.aop = A.take<unsigned char>((size_t) aop_bytes);
             L.a_start = (long long *) dptr(h_axs);
             B.oz_aop = L.aop;
@@ -1693,8 +1744,8 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             B.oz_rowexp = L.rowexp;
             B.oz_colexp = L.colexp;
         }
-        L.coef = A.take<double>((size_t) (1 + nd1) * (size_t) ctot * 4);
-        L.rs = A.take<double>((size_t) (1 + nd1) * 5 * (size_t) R);
+        L.coef = A.take<double>((size_t) n_co * (size_t) ctot * 4);
+        L.rs = A.take<double>((size_t) n_rs * 5 * (size_t) R);
         L.part = A.take<double>((size_t) part_total);
     }
     // the integrals in one block, so that a radius group sums them in one call
@@ -1978,6 +2029,9 @@ int collect_slot(Slot &S) {
             c.gather.rs = SL.rs;
             c.gather.tot = SL.B.tot;
             c.gather.R = SL.B.R;
+            c.gather.hm = SL.B.t_m > 0;
+            c.gather.hx = SL.B.t_x > 0;
+            c.gather.x_own = SL.B.x_own != 0;
             c.gather.cs.clear();
             for (int i = 0; i < redo_early; ++i) c.gather.cs.push_back(P.cs[redo[i]]);
             const int rc3 = submit_sub(R3, c.redo_ticket++, redo_early, rq.data(), rr.data());

@@ -327,6 +327,7 @@ typedef struct {
      double *x, *xl, *w, *w2, *mu_user, *dev_out;
      double **rows;             /* the caller's output rows, in device column order */
      int *n1r, *n2r, *idx1, *idx2;
+     int x_tangent, w_tangent;  /* an index1 derivative moves x / the weights (lmieb.h) */
      /* the arrays above (qx .. idx2) come out of one zeroed block (a second
         one holds this process's share of the radii): a case's scratch is
         released with one or two calls, not one per array */
@@ -624,6 +625,8 @@ static int job_prepare(case_job *j) {
                                            j->qx[i] * j->lambda_l[kk] / j->lambda) / j->lambda;
                j->w[(size_t) (1 + kk) * n + i] = j->nr_l[(size_t) i * nd + kk] * j->qw[i] +
                                                  j->nr[i] * j->qw_l[(size_t) i * nd + kk];
+               j->x_tangent |= j->xl[(size_t) k * n + i] != 0.;
+               j->w_tangent |= j->w[(size_t) (1 + kk) * n + i] != 0.;
           }
           for (k = 0; k < nd2; ++k) {
                int kk = j->idx2[k];
@@ -695,6 +698,10 @@ static int job_prepare(case_job *j) {
      j->P.idx1 = j->idx1; j->P.idx2 = j->idx2;
      j->P.lambda = j->lambda; j->P.mr = j->mr; j->P.mi = j->mi;
      j->P.lambda_l = j->lambda_l; j->P.mr_l = j->mr_l; j->P.mi_l = j->mi_l;
+     for (k = 0; k < nd1; ++k)
+          j->P.m_tangent |= j->mr_l[j->idx1[k]] != 0. || j->mi_l[j->idx1[k]] != 0.;
+     j->P.x_tangent = j->x_tangent;
+     j->P.w_tangent = j->w_tangent;
      j->P.x = j->x; j->P.xl = j->xl; j->P.w = j->w; j->P.n1r = j->n1r; j->P.n2r = j->n2r;
      j->P.n1 = n1; j->P.n_qang = n_qang; j->P.n_coef = j->n_coef_all;
      j->P.want_gc = j->gc != NULL; j->P.want_lc = j->lc != NULL;

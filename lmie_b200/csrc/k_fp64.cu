@@ -2,10 +2,6 @@
 // batch of independent cases (one lmie_solution() is a batch of one).
 //
 //   k_gauss          Gauss-Legendre angles on [-1,1]        <- misc/rtutil_math.c:73-129,231-316
-//   k_mie<NC>        per radius: D_n, psi, chi recurrences (checkpointed
-//                    downward sweeps, replayed per block), a_n, b_n, their
-//                    tangent-linear forms, expansion coefficients and the
-//                    per-radius sums                        <- src/lmie_core.c:263-652
 //   k_reduce_scalars radius reduction of Cext/Csca/Cbak/g    <- src/lmie_core.c:537-611,
 //                                                              src/lmie_schedule.c:334-338
 //   k_angular<..>    S1/S2 accumulation over orders and the phase-matrix
@@ -23,8 +19,6 @@
 #include <cstdio>
 
 #include "kernels.h"
-#include "oz_layout.cuh"
-#include "tc_layout.cuh"
 
 namespace {
 
@@ -73,416 +67,6 @@ __global__ void k_gauss(int npairs, const int *__restrict__ pt, const int *__res
 }
 
 // ---------------------------------------------------------------------------
-// K1: one thread per radius.  The downward recurrences -- D_n(mx) from n2 and
-// the psi ratio from n1, each with its tangent-linear columns -- keep only
-// their values at the top of every block of K1_B orders (checkpoints in ck);
-// the ascending pass replays each block from its checkpoint into local
-// arrays (the same operations, so the same values), runs psi and chi upward,
-// forms a_n, b_n and their tangent-linear columns, writes the expansion
-// coefficients fv4 (a +- b) (coef, or the tensor-core B operand) and sums the
-// per-radius cross sections rs[(col*5 + q)*R + r], q: se, ss, Re sb, Im sb, sg,
-// in order.  Follows src/lmie_core.c:298-370 (psi ratio, psi, chi), 386-440
-// (D), 455-510 (a, b and tangents), 515-590 (cross-section and asymmetry
-// sums per radius).
-// ---------------------------------------------------------------------------
-
-// Split-precision operand of K1's radius.  The 8 floats of order j and column
-// slot cc -- e = 0..7: S hi re, S hi im, S lo re, S lo im, D' hi re, D' hi im,
-// D' lo re, D' lo im, with D' = s_j (a - b) fv4 -- are staged in the thread's
-// slot u = (j - 1) % 4 of shared memory, tcbuf[((u * CC + cc) * 8 + e) * T +
-// thread] (a warp's accesses hit consecutive banks); every 4 orders (and after
-// the last) they go out as 16-byte pieces of the K-major core-matrix layout of
-// tc_layout.cuh instead of 4-byte stores per order.
-template <int CC>
-__device__ __forceinline__ void tc_stage(float *tcbuf, int j, int cc, double sre, double sim, double dre,
-                                         double dim) {
-    const int T = blockDim.x, u = (j - 1) & 3;
-    const double sg = (j & 1) ? 1. : -1.;             // s_j of D'
-    float *p = tcbuf + (size_t) ((u * CC + cc) * 8) * T + threadIdx.x;
-    float h, l;
-    tc_split(sre, h, l); p[0] = h; p[2 * T] = l;
-    tc_split(sim, h, l); p[1 * T] = h; p[3 * T] = l;
-    tc_split(sg * dre, h, l); p[4 * T] = h; p[6 * T] = l;
-    tc_split(sg * dim, h, l); p[5 * T] = h; p[7 * T] = l;
-}
-
-// Writes the group of 4 orders that holds order j (orders after j in it are
-// zero) for the column slots this launch produces: slot 0 (the value) when
-// write_value, slots 1.. the tangent-linear columns c0 + 1...
-template <int CC>
-__device__ __forceinline__ void tc_flush(const float *tcbuf, float *__restrict__ rbase, int j, int pos, int c1,
-                                         int c0, int write_value, int gnk) {
-    const int T = blockDim.x, last = (j - 1) & 3, k0 = (j - 1) - last;
-    constexpr int P = TC_BPART / 4;
-    const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int cc = 0; cc < CC; ++cc) {
-        if (cc == 0 && !write_value) continue;
-        const int col = cc == 0 ? 0 : c0 + cc;
-        const int n = (pos * c1 + col) * 2;
-        {
-            const int kc = k0 / TC_KC, kk = k0 - kc * TC_KC;
-            float *base = rbase + (size_t) kc * (TC_BSTAGE / 4);
-            const int i0 = tc_idx(n, kk, TC_NP), d0 = tc_idx(TC_NHALF + n, kk, TC_NP);
-            float v[8][4];
-#pragma unroll
-            for (int e = 0; e < 8; ++e)
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    v[e][u] = u <= last ? tcbuf[(size_t) ((u * CC + cc) * 8 + e) * T + threadIdx.x] : 0.f;
-            *(float4 *) (base + i0) = make_float4(v[0][0], v[0][1], v[0][2], v[0][3]);
-            *(float4 *) (base + i0 + 4) = make_float4(v[1][0], v[1][1], v[1][2], v[1][3]);
-            *(float4 *) (base + P + i0) = make_float4(v[2][0], v[2][1], v[2][2], v[2][3]);
-            *(float4 *) (base + P + i0 + 4) = make_float4(v[3][0], v[3][1], v[3][2], v[3][3]);
-            *(float4 *) (base + d0) = make_float4(v[4][0], v[4][1], v[4][2], v[4][3]);
-            *(float4 *) (base + d0 + 4) = make_float4(v[5][0], v[5][1], v[5][2], v[5][3]);
-            *(float4 *) (base + P + d0) = make_float4(v[6][0], v[6][1], v[6][2], v[6][3]);
-            *(float4 *) (base + P + d0 + 4) = make_float4(v[7][0], v[7][1], v[7][2], v[7][3]);
-        }
-        // after the radius' last order: zeros up to the end of its group's chunks
-        // (the operand buffer is not cleared between solves)
-        for (int k = k0 + 4; k < gnk * TC_KC; k += 4) {
-            const int kc = k / TC_KC, kk = k - kc * TC_KC;
-            float *base = rbase + (size_t) kc * (TC_BSTAGE / 4);
-            const int i0 = tc_idx(n, kk, TC_NP), d0 = tc_idx(TC_NHALF + n, kk, TC_NP);
-            *(float4 *) (base + i0) = z;
-            *(float4 *) (base + i0 + 4) = z;
-            *(float4 *) (base + P + i0) = z;
-            *(float4 *) (base + P + i0 + 4) = z;
-            *(float4 *) (base + d0) = z;
-            *(float4 *) (base + d0 + 4) = z;
-            *(float4 *) (base + P + d0) = z;
-            *(float4 *) (base + P + d0 + 4) = z;
-        }
-    }
-}
-
-// m[c] = max(m[c], biased exponent of component c + ek) over the normal
-// values among (Re cs, Im cs, Re cd, Im cd)
-__device__ __forceinline__ void oz_track(int (&m)[4], cplx cs, cplx cd, int ek) {
-    const double v[4] = {cs.re, cs.im, cd.re, cd.im};
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        const int ex = (__double2hiint(v[c]) >> 20) & 0x7FF;
-        m[c] = max(m[c], ex ? ex + ek : 0);
-    }
-}
-
-template <int NC>
-__global__ void __launch_bounds__(64) k_mie(DevBatch B, int c0, int write_value, double *__restrict__ ck,
-                                            double *__restrict__ coef, float *__restrict__ bop,
-                                            double *__restrict__ rs) {
-    constexpr int CC = 1 + NC;
-    constexpr int CW = k1_ck_width(NC);               // D (2), D_l (2 NC), ratio (1), ratio_l (NC)
-    // thread t takes the radius of rank t in the launch order: cases in the
-    // order k1ord, each from its largest radius down
-    const long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= B.R) return;
-    const int kc = find_case(B.k1pre, B.ncase, t);
-    const int r = [&] {
-        const DevCase &Ck = B.cs[B.k1ord[kc]];
-        return Ck.r0 + Ck.nr - 1 - (int) (t - B.k1pre[kc]);
-    }();
-    const int R = B.R;
-    const DevCase &C = B.cs[B.rcase[r]];
-    const int n1 = B.n1r[r], n2 = B.n2r[r];
-    const double x = B.x[r];
-    const double xinv = 1. / x;
-    const cplx m = C.m, minv = C.minv;
-    const cplx z = mk(m.re * x, m.im * x);
-    const cplx zinv = cinv(z);
-    const int nb = (n1 + K1_B - 1) / K1_B;
-    double *ckr = ck + (size_t) B.ckoff[r] * CW;     // nb blocks of CW doubles
-    const double *fv1 = B.fv, *fv3 = B.fv + 2 * (B.n1max + 2), *fv4 = B.fv + 3 * (B.n1max + 2);
-
-    double xl[NC > 0 ? NC : 1];
-    cplx zl[NC > 0 ? NC : 1], ml[NC > 0 ? NC : 1];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) {
-        const int kk = B.idx1[c0 + k];
-        xl[k] = B.xl[(size_t) (c0 + k) * R + r];
-        ml[k] = B.m_l[C.ml_off + kk];
-        zl[k] = ml[k] * x + m * xl[k];
-    }
-
-    // ---- downward sweeps: checkpoints only ----
-    // Two independent chains: D_n from n2 and the psi ratio from n1 (n2 > n1).
-    // Below n1 they advance in the same loop, so that the dependent steps of
-    // one fill the latency of the other; each chain's arithmetic and order
-    // are those of a sweep of its own.
-    {
-        cplx D = mk(0., 0.), Dl[NC > 0 ? NC : 1];
-        double rn = 0., rl[NC > 0 ? NC : 1];
-#pragma unroll
-        for (int k = 0; k < NC; ++k) {
-            Dl[k] = mk(0., 0.);
-            rl[k] = 0.;
-        }
-        for (int c = 0; c < nb; ++c) {
-            double *q = ckr + (size_t) c * CW;
-            if (c * K1_B + K1_B >= n2) {
-                q[0] = q[1] = 0.;
-#pragma unroll
-                for (int k = 0; k < NC; ++k) q[2 + 2 * k] = q[3 + 2 * k] = 0.;
-            }
-            if (c * K1_B + K1_B >= n1) {
-                q[2 + 2 * NC] = 0.;
-#pragma unroll
-                for (int k = 0; k < NC; ++k) q[3 + 2 * NC + k] = 0.;
-            }
-        }
-        auto d_step = [&](int j) {
-            const cplx c1 = (j + 1.) * zinv;
-            const cplx ic2 = cinv(D + c1);
-            D = c1 - ic2;
-            if (NC > 0) {
-                const cplx c3 = -c1 * zinv;
-                const cplx ic4 = ic2 * ic2;
-#pragma unroll
-                for (int k = 0; k < NC; ++k) {
-                    const cplx c5 = c3 * zl[k];
-                    Dl[k] = c5 + (Dl[k] + c5) * ic4;
-                }
-            }
-            if (j % K1_B == 0 && j / K1_B - 1 < nb) {
-                double *q = ckr + (size_t) (j / K1_B - 1) * CW;
-                q[0] = D.re;
-                q[1] = D.im;
-#pragma unroll
-                for (int k = 0; k < NC; ++k) {
-                    q[2 + 2 * k] = Dl[k].re;
-                    q[3 + 2 * k] = Dl[k].im;
-                }
-            }
-        };
-        auto r_step = [&](int j) {
-            const double a1 = (2. * j + 1.) * xinv;
-            const double rnew = 1. / (a1 - rn);
-            if (NC > 0) {
-                const double a2 = -a1 * xinv, a3 = rnew * rnew;
-#pragma unroll
-                for (int k = 0; k < NC; ++k) rl[k] = -(a2 * xl[k] - rl[k]) * a3;
-            }
-            rn = rnew;
-            if (j % K1_B == 0 && j / K1_B - 1 < nb) {
-                double *q = ckr + (size_t) (j / K1_B - 1) * CW + 2 + 2 * NC;
-                q[0] = rn;
-#pragma unroll
-                for (int k = 0; k < NC; ++k) q[1 + k] = rl[k];
-            }
-        };
-        for (int j = n2 - 1; j >= n1; --j) d_step(j);
-        for (int j = n1 - 1; j >= 1; --j) {
-            d_step(j);
-            r_step(j);
-        }
-    }
-
-    // ---- ascending pass ----
-    double sinx, cosx;
-    sincos(x, &sinx, &cosx);
-    double psi_p = sinx, chi_p = cosx, chi_c = xinv * cosx + sinx;     // psi_0, chi_0, chi_1
-    double psil_p[NC > 0 ? NC : 1], chil_p[NC > 0 ? NC : 1], chil_c[NC > 0 ? NC : 1];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) {
-        psil_p[k] = xl[k] * cosx;
-        chil_p[k] = xl[k] * -sinx;
-        chil_c[k] = (-xinv * xinv) * xl[k] * cosx + xinv * chil_p[k] + xl[k] * cosx;
-    }
-    double acc[5 * CC];
-#pragma unroll
-    for (int q = 0; q < 5 * CC; ++q) acc[q] = 0.;
-    cplx ap = mk(0., 0.), bp = mk(0., 0.), alp[NC > 0 ? NC : 1], blp[NC > 0 ? NC : 1];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) alp[k] = blp[k] = mk(0., 0.);
-    const cplx Dm2f = minv * minv;
-    const size_t tot = (size_t) B.tot, off = (size_t) B.off[r];
-    // split precision: the radii of tensor-core cases write the B operand
-    const int tcode = bop ? B.tc_pos[r] : -1;
-    const bool to_tc = tcode >= 0;
-    const int tpos = tcode & 255, tgnk = tcode >> 8;   // position in the group, the group's chunks
-    const long long troff = to_tc ? B.tc_roff[r] : 0;
-    extern __shared__ float tcbuf[];                  // [4][1 + NC][8][blockDim.x] when bop is set
-    double4 *cf = (double4 *) coef;
-    // int8 form: the largest (biased exponent + e_k) of each column and
-    // component, the column exponents of the fixed-point B operand
-    int *const rx = B.oz_radexp;
-    int mxe[CC][4];
-#pragma unroll
-    for (int q = 0; q < 4 * CC; ++q) mxe[q / 4][q % 4] = 0;
-
-    cplx Dloc[K1_B], Dlloc[NC > 0 ? NC : 1][K1_B];
-    double rloc[K1_B], rlloc[NC > 0 ? NC : 1][K1_B];
-    for (int c = 0; c < nb; ++c) {
-        const int lo = c * K1_B + 1, hi = min(c * K1_B + K1_B, n1);
-        const double *q = ckr + (size_t) c * CW;
-        // replay D, D_l from the block's top (t <= n2) and the psi ratio and
-        // its tangents from hi (t >= hi) down to lo: one loop below hi, as in
-        // the downward sweeps
-        {
-            const int t = min(c * K1_B + K1_B, n2);
-            cplx D = mk(q[0], q[1]), Dl[NC > 0 ? NC : 1];
-#pragma unroll
-            for (int k = 0; k < NC; ++k) Dl[k] = mk(q[2 + 2 * k], q[3 + 2 * k]);
-            if (t <= hi) {
-                Dloc[t - lo] = D;
-#pragma unroll
-                for (int k = 0; k < NC; ++k) Dlloc[k][t - lo] = Dl[k];
-            }
-            const double *qr = q + 2 + 2 * NC;
-            double rn = qr[0], rl[NC > 0 ? NC : 1];
-#pragma unroll
-            for (int k = 0; k < NC; ++k) rl[k] = qr[1 + k];
-            rloc[hi - lo] = rn;
-#pragma unroll
-            for (int k = 0; k < NC; ++k) rlloc[k][hi - lo] = rl[k];
-            auto d_step = [&](int j) {
-                const cplx c1 = (j + 1.) * zinv;
-                const cplx ic2 = cinv(D + c1);
-                D = c1 - ic2;
-                if (NC > 0) {
-                    const cplx c3 = -c1 * zinv;
-                    const cplx ic4 = ic2 * ic2;
-#pragma unroll
-                    for (int k = 0; k < NC; ++k) {
-                        const cplx c5 = c3 * zl[k];
-                        Dl[k] = c5 + (Dl[k] + c5) * ic4;
-                    }
-                }
-                if (j <= hi) {
-                    Dloc[j - lo] = D;
-#pragma unroll
-                    for (int k = 0; k < NC; ++k) Dlloc[k][j - lo] = Dl[k];
-                }
-            };
-            auto r_step = [&](int j) {
-                const double a1 = (2. * j + 1.) * xinv;
-                const double rnew = 1. / (a1 - rn);
-                if (NC > 0) {
-                    const double a2 = -a1 * xinv, a3 = rnew * rnew;
-#pragma unroll
-                    for (int k = 0; k < NC; ++k) rl[k] = -(a2 * xl[k] - rl[k]) * a3;
-                }
-                rn = rnew;
-                rloc[j - lo] = rn;
-#pragma unroll
-                for (int k = 0; k < NC; ++k) rlloc[k][j - lo] = rl[k];
-            };
-            for (int j = t - 1; j >= hi; --j) d_step(j);
-            for (int j = hi - 1; j >= lo; --j) {
-                d_step(j);
-                r_step(j);
-            }
-        }
-        for (int j = lo; j <= hi; ++j) {
-            const double rj = rloc[j - lo];
-            const double psi = rj * psi_p;
-            double psil[NC > 0 ? NC : 1];
-#pragma unroll
-            for (int k = 0; k < NC; ++k) psil[k] = rlloc[k][j - lo] * psi_p + rj * psil_p[k];
-            const cplx D = Dloc[j - lo];
-            const cplx zeta = mk(psi, chi_c), zeta_p = mk(psi_p, chi_p);
-            const double tt = j * xinv;
-            const cplx ca = D * minv + tt;
-            const cplx na = ca * psi - psi_p;
-            const cplx ida = cinv(ca * zeta - zeta_p);
-            const cplx a = na * ida;
-            const cplx cb = m * D + tt;
-            const cplx nbq = cb * psi - psi_p;
-            const cplx idb = cinv(cb * zeta - zeta_p);
-            const cplx b = nbq * idb;
-            cplx al[NC > 0 ? NC : 1], bl[NC > 0 ? NC : 1];
-            if (NC > 0) {
-                const cplx Dm2 = D * Dm2f;
-                const double tx = -tt * xinv;
-#pragma unroll
-                for (int k = 0; k < NC; ++k) {
-                    const cplx Dl = Dlloc[k][j - lo];
-                    const cplx zetal = mk(psil[k], chil_c[k]), zetal_p = mk(psil_p[k], chil_p[k]);
-                    const double tl = tx * xl[k];
-                    const cplx c6 = Dl * minv - Dm2 * ml[k] + tl;
-                    al[k] = (c6 * psi + ca * psil[k] - psil_p[k]) * ida -
-                            na * ((c6 * zeta + ca * zetal - zetal_p) * (ida * ida));
-                    const cplx c4 = ml[k] * D + m * Dl + tl;
-                    bl[k] = (c4 * psi + cb * psil[k] - psil_p[k]) * idb -
-                            nbq * ((c4 * zeta + cb * zetal - zetal_p) * (idb * idb));
-                }
-            }
-            // sums of order j, and the asymmetry term of order j - 1 (it needs a_j, b_j)
-            const double f1 = fv1[j], f4 = fv4[j];
-            const double sgn = (j & 1) ? -1. : 1.;
-            acc[0] += f1 * (a.re + b.re);
-            acc[1] += f1 * (norm2(a) + norm2(b));
-            acc[2] += f1 * sgn * (a.re - b.re);
-            acc[3] += f1 * sgn * (a.im - b.im);
-            if (j >= 2) acc[4] += fv3[j - 1] * (re_mulc(ap, a) + re_mulc(bp, b)) + fv4[j - 1] * re_mulc(ap, bp);
-#pragma unroll
-            for (int k = 0; k < NC; ++k) {
-                double *qq = acc + 5 * (1 + k);
-                qq[0] += f1 * (al[k].re + bl[k].re);
-                qq[1] += f1 * 2. * (re_mulc(a, al[k]) + re_mulc(b, bl[k]));
-                qq[2] += f1 * sgn * (al[k].re - bl[k].re);
-                qq[3] += f1 * sgn * (al[k].im - bl[k].im);
-                if (j >= 2)
-                    qq[4] += fv3[j - 1] * (re_mulc(alp[k], a) + re_mulc(ap, al[k]) + re_mulc(blp[k], b) +
-                                           re_mulc(bp, bl[k])) +
-                             fv4[j - 1] * (re_mulc(alp[k], bp) + re_mulc(ap, blp[k]));
-            }
-            // expansion coefficients of order j
-            const int ek = oz_ek(j);
-            if (write_value) {
-                const cplx cs = (a + b) * f4, cd = (a - b) * f4;
-                if (to_tc) tc_stage<CC>(tcbuf, j, 0, cs.re, cs.im, cd.re, cd.im);
-                else cf[off + j - 1] = make_double4(cs.re, cs.im, cd.re, cd.im);
-                if (rx) oz_track(mxe[0], cs, cd, ek);
-            }
-#pragma unroll
-            for (int k = 0; k < NC; ++k) {
-                const cplx cs = (al[k] + bl[k]) * f4, cd = (al[k] - bl[k]) * f4;
-                if (to_tc) tc_stage<CC>(tcbuf, j, 1 + k, cs.re, cs.im, cd.re, cd.im);
-                else cf[(size_t) (1 + c0 + k) * tot + off + j - 1] = make_double4(cs.re, cs.im, cd.re, cd.im);
-                if (rx) oz_track(mxe[1 + k], cs, cd, ek);
-            }
-            if (to_tc && (((j - 1) & 3) == 3 || j == n1))
-                tc_flush<CC>(tcbuf, bop + troff, j, tpos, 1 + B.nd1, c0, write_value, j == n1 ? tgnk : 0);
-            // upward: chi_{j+1} and its tangents; shift the previous order
-            const double a1 = (2. * j + 1.) * xinv;
-            const double chi_n = a1 * chi_c - chi_p;
-#pragma unroll
-            for (int k = 0; k < NC; ++k) {
-                const double a2l = -a1 * xl[k] * xinv;
-                const double chil_n = a2l * chi_c + a1 * chil_c[k] - chil_p[k];
-                chil_p[k] = chil_c[k];
-                chil_c[k] = chil_n;
-                psil_p[k] = psil[k];
-                alp[k] = al[k];
-                blp[k] = bl[k];
-            }
-            chi_p = chi_c;
-            chi_c = chi_n;
-            psi_p = psi;
-            ap = a;
-            bp = b;
-        }
-    }
-#pragma unroll
-    for (int q = 0; q < 5 * CC; ++q) {
-        const int cc = q / 5, qq = q % 5;
-        if (cc == 0 && !write_value) continue;
-        const size_t col = cc == 0 ? 0 : (size_t) (1 + c0 + cc - 1);
-        rs[(col * 5 + qq) * R + r] = acc[q];
-    }
-    if (rx) {
-#pragma unroll
-        for (int cc = 0; cc < CC; ++cc) {
-            if (cc == 0 && !write_value) continue;
-            const size_t col = cc == 0 ? 0 : (size_t) (1 + c0 + cc - 1);
-            *(int4 *) (rx + (col * R + r) * 4) = make_int4(mxe[cc][0], mxe[cc][1], mxe[cc][2], mxe[cc][3]);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
 // K2: one block per (case, output column); fixed-order block reduction over
 // the case's radii.
 // ---------------------------------------------------------------------------
@@ -514,6 +98,7 @@ __global__ void __launch_bounds__(256) k_reduce_scalars(DevBatch B, const double
             if (B.idx1[k] == kk) { kind = 1; c1 = 1 + k; }
         if (kind == 0) kind = 2;
     }
+    const cplx ml = kind == 1 ? B.m_l[C.ml_off + col - 1] : mk(0., 0.);
     double acc[4] = {0., 0., 0., 0.};
     for (int r = C.r0 + threadIdx.x; r < C.r0 + C.nr; r += blockDim.x) {
         const double f = B.w[r];
@@ -534,11 +119,21 @@ __global__ void __launch_bounds__(256) k_reduce_scalars(DevBatch B, const double
             }
         } else if (kind == 1) {
             const double fl = B.w[(size_t) col * R + r];
-            const double *q = rs + (size_t) c1 * 5 * R;
-            acc[0] += fl * se + f * q[r];
-            acc[1] += fl * ss + f * q[(size_t) R + r];
-            acc[2] += fl * bak + f * 2. * (sbr * q[(size_t) 2 * R + r] + sbi * q[(size_t) 3 * R + r]);
-            acc[3] += fl * sg + f * q[(size_t) 4 * R + r];
+            double q[5];
+            // the derivative from the sums of the tangent basis
+            const double xc = B.t_x ? (B.x_own ? 1. : B.xl[(size_t) (c1 - 1) * R + r]) : 0.;
+#pragma unroll
+            for (int i = 0; i < 5; ++i) {
+                q[i] = 0.;
+                if (B.t_m)
+                    q[i] = ml.re * rs[((size_t) B.rs_m * 5 + i) * R + r] -
+                           ml.im * rs[((size_t) (B.rs_m + 1) * 5 + i) * R + r];
+                if (B.t_x) q[i] += xc * rs[((size_t) B.rs_x * 5 + i) * R + r];
+            }
+            acc[0] += fl * se + f * q[0];
+            acc[1] += fl * ss + f * q[1];
+            acc[2] += fl * bak + f * 2. * (sbr * q[2] + sbi * q[3]);
+            acc[3] += fl * sg + f * q[4];
         } else {
             const double fl = B.w[(size_t) col * R + r];
             acc[0] += fl * se;
@@ -612,15 +207,40 @@ __global__ void __launch_bounds__(ANG_T) k_angular(DevBatch B, int c1base, int c
     constexpr int PF = (ANG_KT * C1 + ANG_T - 1) / ANG_T;
     double4 pre[PF];
     double pre_fv = 0.;
-    auto fetch = [&](size_t off, int n1, int k0) {
+    // the derivatives' refractive-index directions (columns are put together
+    // from the tangent basis as they are fetched)
+    cplx mlc[C1];
+#pragma unroll
+    for (int c = 1; c < C1; ++c) mlc[c] = B.t_m ? B.m_l[C.ml_off + B.idx1[c1base + c - 1]] : mk(0., 0.);
+    auto fetch = [&](int rad, size_t off, int n1, int k0) {
         const int kt = min(ANG_KT, n1 - k0);
 #pragma unroll
         for (int u = 0; u < PF; ++u) {
             const int idx = tid + u * ANG_T;
             if (idx < kt * C1) {
                 const int t = idx / C1, c = idx - t * C1;
-                const size_t col = c == 0 ? 0 : (size_t) (c1base + c);
-                pre[u] = cf[col * tot + off + k0 + t];
+                const double4 *q = cf + off + k0 + t;
+                if (c == 0) {
+                    pre[u] = q[0];
+                } else {
+                    // derivative c1base + c - 1 from the tangent basis
+                    double4 v = make_double4(0., 0., 0., 0.);
+                    if (B.t_m) {
+                        cplx ml = mlc[C1 > 1 ? 1 : 0];
+#pragma unroll
+                        for (int e = 2; e < C1; ++e)
+                            if (c == e) ml = mlc[e];
+                        const double4 a = q[(size_t) B.t_m * tot];
+                        v = make_double4(ml.re * a.x - ml.im * a.y, ml.re * a.y + ml.im * a.x,
+                                         ml.re * a.z - ml.im * a.w, ml.re * a.w + ml.im * a.z);
+                    }
+                    if (B.t_x) {
+                        const double4 a = q[(size_t) B.t_x * tot];
+                        const double xc = B.x_own ? 1. : B.xl[(size_t) (c1base + c - 1) * R + rad];
+                        v = make_double4(v.x + xc * a.x, v.y + xc * a.y, v.z + xc * a.z, v.w + xc * a.w);
+                    }
+                    pre[u] = v;
+                }
             }
         }
         if (tid < kt) pre_fv = fv2[k0 + tid + 1];
@@ -639,7 +259,7 @@ __global__ void __launch_bounds__(ANG_T) k_angular(DevBatch B, int c1base, int c
             for (int c = 0; c < C1; ++c) spA[a][c] = smA[a][c] = spB[a][c] = smB[a][c] = mk(0., 0.);
         }
         double kd = 1.;
-        fetch(off, n1, 0);
+        fetch(r, off, n1, 0);
         for (int k0 = 0; k0 < n1; k0 += ANG_KT) {
             const int kt = min(ANG_KT, n1 - k0);
             __syncthreads();
@@ -650,7 +270,7 @@ __global__ void __launch_bounds__(ANG_T) k_angular(DevBatch B, int c1base, int c
             }
             if (tid < kt) gks[tid] = 1. + pre_fv;
             __syncthreads();
-            if (k0 + ANG_KT < n1) fetch(off, n1, k0 + ANG_KT);
+            if (k0 + ANG_KT < n1) fetch(r, off, n1, k0 + ANG_KT);
             if (!any) continue;
             // orders k = k0 + t + 1: t even <-> k odd <-> mirror sign +1.  With
             // t2 = mu pi_k - pi_{k-1}: tau_k = k t2 - pi_{k-1} and
@@ -1578,29 +1198,6 @@ __global__ void k_group_flag(const double *__restrict__ failed, int *__restrict_
 
 int launch_group_flag(cudaStream_t s, const double *failed, int *err) {
     k_group_flag<<<1, 1, 0, s>>>(failed, err);
-    LMIEB_CUDA_TRY(cudaGetLastError());
-    return 0;
-}
-
-int launch_coef(cudaStream_t s, const DevBatch &B, int nc, int c0, int write_value, double *ck, double *coef,
-                float *bop, double *rs) {
-    const unsigned rb = ceil_div(B.R, 64);
-    switch (nc) {
-#define LMIEB_K1(NC_)                                                                                    \
-    case NC_:                                                                                            \
-        k_mie<NC_><<<rb, 64, bop ? 4 * 8 * (1 + NC_) * 64 * sizeof(float) : 0, s>>>(B, c0, write_value, ck,   \
-                                                                                  coef, bop, rs);        \
-        break;
-    LMIEB_K1(0)
-    LMIEB_K1(1)
-    LMIEB_K1(2)
-    LMIEB_K1(3)
-    LMIEB_K1(4)
-#undef LMIEB_K1
-    default:
-        fprintf(stderr, "ERROR: launch_coef: bad chunk width %d\n", nc);
-        return -1;
-    }
     LMIEB_CUDA_TRY(cudaGetLastError());
     return 0;
 }

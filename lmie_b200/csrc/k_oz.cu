@@ -16,26 +16,46 @@
 //   - k_angular_oz: a block owns one angle tile of one case and a range of its
 //     radius groups; per group, chunks of OZ_KC orders flow through the
 //     pipeline:
-//       * warps 0-3 (one thread per row, the row's tensor-memory lane) load
-//         the chunk's A digit slices of their row -- formed once per (case,
-//         angle tile, chunk) by k_oz_aop -- and store them into the A stage
-//         in tensor memory;
-//       * lane 0 of warp 9 brings the group's B chunks into shared memory with
+//       * warps 0-3 and 4-7 (one thread per row, the row's tensor-memory
+//         lane), alternate chunks each, load the chunk's A digit slices of
+//         their row -- formed once per (case, angle tile, chunk) by k_oz_aop
+//         -- and store them into the A stage in tensor memory;
+//       * lane 0 of warp 14 brings the group's B chunks into shared memory with
 //         bulk copies running ahead of the products;
-//       * lane 0 of warp 8 issues the digit products of a chunk (21 or 28),
+//       * warps 12 and 13 issue the digit products of a chunk (21 or 28),
 //         tcgen05.mma kind::i8 with A in tensor memory and B in shared memory
 //         (M 128, N NP, K 32, int32 accumulation in tensor memory), one
-//         accumulator per digit diagonal;
-//       * after a group's last chunk warps 4-7 (S columns) and 0-3 (D'
+//         accumulator per digit diagonal: one warp the even diagonals, the
+//         other the odd ones.  The tensor pipe queues hardly any products
+//         behind the one it runs, so a single issuing warp leaves it idle
+//         while it waits for and sets up the next chunk (about 280 cycles per
+//         chunk: 33.5 cycles per product of M 128, N 48 instead of 24.5, 43
+//         instead of 32 at N 64); with two, each one's set-up falls into the
+//         other's products (24.3 and 32.2 measured in a loop of this shape);
+//       * during a group's last chunk warps 4-7 (S columns) and 0-3 (D'
 //         columns) read the accumulators of their row (tensor-memory
-//         lane = row), form C exactly (int64 halves, then FP64) into a
-//         shared-memory buffer and hand the accumulators back, so the next
-//         group's products start;
-//       * warps 10-13 form, from the buffer and while the next group's
+//         lane = row) phase by phase -- diagonals 0-2, 3-4, 5 on -- as each
+//         phase's products complete, add them up in int64 and hand the phase's
+//         accumulators back, so the next group's products of that phase start.
+//         The products go out by ascending diagonal, so while one group's
+//         later diagonals run its first ones are read, and while the last ones
+//         are read the next group's first ones run: tensor memory has no room
+//         for a second accumulator set, and reading a whole group between its
+//         last product and the next group's first one left the tensor pipe
+//         idle for 2.2K cycles per group (a chunk's products take 0.7K).  The
+//         sums then go to a shared-memory buffer as doubles;
+//       * warps 8-11 form, from the buffer and while the next group's
 //         products run, the phase-matrix quadratic forms and their
 //         linearisations per radius (reference src/lmie_core.c:723-790; sm of
 //         a row is in its pair row), accumulated over the block's radii in
 //         registers.
+// FP64 arithmetic waits for the products: a DFMA beside a running kind::i8
+// stream completes every 128 cycles (2.5 without one), while integer, FP32 and
+// conversion instructions are not slowed.  So the sums and their scaling are
+// integer arithmetic and one conversion each, and what is left in FP64 is the
+// quadratic forms, kept short: the sums over radii are formed for the complex
+// tangent column (k_mie.cu) with the weight folded into the value's side, and
+// turned into derivatives once at the end.
 // The integer sums are exact, so nothing is drained during a group.
 // Partials go to the same per-group buffer as the FP64 K3.
 //
@@ -55,10 +75,9 @@
 
 namespace {
 
-constexpr int OZ_T = 448;                     // warps 0-3: A stages, D' sums; 4-7: S sums; 8: products;
-                                              // 9: B copies; 10-13: quadratic forms
-constexpr int OZ_MMA_WARP = 8, OZ_COPY_WARP = 9, OZ_QUAD_WARP = 10;
-constexpr int OZ_MAX_NS = 1 + OZ_MAX_NC1 + OZ_MAX_ND2;
+constexpr int OZ_T = 480;                     // warps 0-7: A stages and sums (0-3 D', 4-7 S);
+                                              // 8-11: quadratic forms; 12, 13: products; 14: B copies
+constexpr int OZ_QUAD_WARP = 8, OZ_MMA_WARP = 12, OZ_COPY_WARP = 14;
 constexpr uint32_t OZ_TMEM_COLS = 512;
 
 // sizes and shared-memory offsets of the product kernel
@@ -66,16 +85,16 @@ template <int ND>
 struct OzK : Oz<ND> {
     using F = Oz<ND>;
     static constexpr int MAX_GN = F::NHALF / 2;                        // radii of a group (oz_rg(nd, 0))
+    static constexpr int MAX_W = 128;                                  // weights of a group: one per thread
     static constexpr uint32_t ACOLS = ND * OZ_KC / 4;                  // tensor-memory columns of an A stage
     static constexpr uint32_t ACOL = ND * F::NP;                       // first A stage column
-    // barriers: afull[ASTAGES], adone[ASTAGES], bfull[BSLOTS], bdone[BSLOTS], accfull, accfree,
-    // hready[2], hfree[2], fin
-    static constexpr int NBAR = 2 * F::ASTAGES + 2 * F::BSLOTS + 7;
+    // barriers: afull[BSLOTS], bfull[BSLOTS], done[BSLOTS], accfull[3], accfree[3], hready[2], hfree[2], fin
+    static constexpr int NBAR = 3 * F::BSLOTS + 11;
     static constexpr uint32_t RING = F::BSLOTS * F::BSTAGE;
     static constexpr int HB = F::NP * OZ_M;                            // doubles of one sums buffer
     static constexpr uint32_t HBUF = 2 * HB * 8;                       // two groups' sums, unscaled, [column][row]
-    static constexpr uint32_t WBUF = MAX_GN * OZ_MAX_NS * 8;           // a group's radius weights
-    static constexpr uint32_t CBUF = F::NP * 8;                        // a group's column scales
+    static constexpr uint32_t WBUF = MAX_W * 8;                        // a group's radius weights
+    static constexpr uint32_t CBUF = F::NP * 4;                        // a group's column exponents
     static constexpr uint32_t O_HBUF = RING, O_WBUF = O_HBUF + HBUF, O_CBUF = O_WBUF + WBUF, O_BARS = O_CBUF + CBUF;
     static constexpr uint32_t SMEM = O_BARS + NBAR * 8 + 16;
 
@@ -84,7 +103,9 @@ struct OzK : Oz<ND> {
     static_assert(ACOL + F::ASTAGES * ACOLS <= OZ_TMEM_COLS, "accumulators and A stages in tensor memory");
     static_assert(WBUF % 16 == 0 && CBUF % 16 == 0, "barriers stay 8-byte aligned");
     static_assert(SMEM <= 227 * 1024, "shared memory per block");
-    static_assert(MAX_GN * OZ_MAX_NS <= 128, "one weight per thread of the quadratic-form warps");
+    // weights per radius: value, index2, and with tangent columns index1 (twice with the x column)
+    static_assert(MAX_GN * (1 + OZ_MAX_ND2 + OZ_MAX_ND1) <= MAX_W &&
+                  MAX_GN / 2 * (1 + OZ_MAX_ND2 + 2 * OZ_MAX_ND1) <= MAX_W, "one weight per thread");
     // |V| <= 2^(FRAC - 1) must stay inside the balanced digits (-0x8080.. .. 0x7f7f..)
     static_assert(F::FRAC - 1 <= 8 * ND - 2, "digit weights: the top digit holds at most 64");
 };
@@ -94,25 +115,58 @@ __host__ __device__ constexpr uint32_t idesc_i8(int m, int n) {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (n >> 3) << 17) | ((uint32_t) (m >> 4) << 24);
 }
 
-// true in one lane of a converged warp (the lowest)
-__device__ __forceinline__ bool elect_one() {
+// lane 0's value, which the compiler then knows to be the same in the whole
+// (converged) warp
+template <class T>
+__device__ __forceinline__ T warp_uniform(T v) {
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+
+// 1 in one lane of a converged warp (the lowest), 0 in the others
+__device__ __forceinline__ uint32_t elect_one() {
     uint32_t pred = 0;
     asm volatile(
         "{\n\t.reg .pred P;\n\t"
         "elect.sync _|P, 0xffffffff;\n\t"
         "selp.u32 %0, 1, 0, P;\n\t}"
         : "=r"(pred));
-    return pred != 0;
+    return pred;
 }
 
-// A from tensor memory (column address a), B from shared memory
-__device__ __forceinline__ void mma_i8_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+// A from tensor memory (column address a), B from shared memory; issued by the
+// lane whose `on` is set.  The lane is picked by a guard on the instruction,
+// not by a branch: outside a divergent branch the operands stay in uniform
+// registers, from which the instruction takes them (one warp issues a product
+// every 24 cycles or less this way, every 47 in a branch for one lane).
+__device__ __forceinline__ void mma_i8_ts(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, uint32_t accumulate,
+                                          uint32_t on) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
-        "r"(a), "l"(b), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::i8 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d),
+        "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(on)
         : "memory");
+}
+
+// mma_commit by the lane whose `on` is set
+__device__ __forceinline__ void mma_commit_on(uint32_t bar, uint32_t on) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
+        "r"(on)
+        : "memory");
+}
+
+// 16 bytes that this block reads once: not kept in L1, whose data array the
+// B operand and the sums share
+__device__ __forceinline__ uint4 ld_once(const uint4 *p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                 : "l"(p));
+    return v;
 }
 
 // warp-wide: four consecutive 32-bit columns of this thread's lane
@@ -122,66 +176,125 @@ __device__ __forceinline__ void tmem_st4(uint32_t taddr, uint32_t a, uint32_t b,
                  : "memory");
 }
 
-// The NPROD digit products of one chunk (one thread): a0 the
-// tensor-memory column of the chunk's A stage, b0 the shared address of its
-// B stage, acc the tensor-memory column of diagonal 0; `first`: the chunk
-// opens the group's sums.
+// Read-out phases of the accumulators: diagonals [oz_ph(p), oz_ph(p + 1)).
+constexpr int OZ_NPH = 3;
 template <int ND>
-__device__ __forceinline__ void issue_chunk_i8(uint32_t a0, uint32_t b0, uint32_t acc, bool first) {
+__host__ __device__ constexpr int oz_ph(int p) { return p == 0 ? 0 : (p == 1 ? 3 : (p == 2 ? 5 : ND)); }
+
+// The digit products of diagonals D0, D0 + STEP, ... below D1 of one chunk
+// by the lane with `on` (warp-wide): a0 the tensor-memory column of the
+// chunk's A stage, b0 the shared address of its B stage, acc the
+// tensor-memory column of diagonal 0; `first`: the chunk opens the group's
+// sums.
+template <int ND, int D0, int D1, int STEP>
+__device__ __forceinline__ void issue_products_i8(uint32_t a0, uint32_t b0, uint32_t acc, bool first, uint32_t on) {
     using F = Oz<ND>;
     constexpr uint32_t idesc = idesc_i8(OZ_M, F::NP);
     const uint64_t db = sdesc(b0, F::LBO_B, 128);
 #pragma unroll
-    for (int d = 0; d < ND; ++d)
+    for (int d = D0; d < D1; d += STEP)
 #pragma unroll
         for (int i = 0; i <= d; ++i) {
             const int j = d - i;
             mma_i8_ts(acc + d * F::NP, a0 + i * (OZ_KC / 4), db + (uint64_t) ((j * F::BSLICE) >> 4), idesc,
-                      (first && i == 0) ? 0u : 1u);
+                      (first && i == 0) ? 0u : 1u, on);
         }
 }
 
-// 2^16 sum_d 2^(-8 d) ACC_d of a column's int32 accumulators: U = ACC_0 2^16 +
-// ACC_1 2^8 + ACC_2 and L = ACC_3 2^16 + ACC_4 2^8 + ACC_5 are below 2^46 in
-// magnitude and become doubles exactly (x + 1.5 2^52 read as an integer); a
-// seventh diagonal joins L exactly (ACC_6 2^-8: 54 bits in all at most, the
-// last of them below 2^-32 of U's unit); then U + 2^-24 L with one rounding.
-template <int ND>
-__device__ __forceinline__ double oz_unscaled(const uint32_t (&a)[ND]) {
-    const long long U = (long long) (int) a[0] * 65536 + (long long) (int) a[1] * 256 + (long long) (int) a[2];
-    const long long L = (long long) (int) a[3] * 65536 + (long long) (int) a[4] * 256 + (long long) (int) a[5];
-    const double dU = __longlong_as_double(U + 0x4338000000000000LL) - 6755399441055744.0;
-    double dL = __longlong_as_double(L + 0x4338000000000000LL) - 6755399441055744.0;
-    if (ND == 7) {
-        const double d6 = __hiloint2double(0x43300000, (int) (a[ND - 1] ^ 0x80000000u)) - 4503601774854144.0;   // 2^52 + 2^31
-        dL = fma(d6, 0.00390625, dL);   // 2^-8
+// One issuing warp's products of one chunk: its diagonals (parity PAR) phase by
+// phase.  open: the chunk opens its group's sums; held: the previous group's
+// accumulators of a phase must have been read first (accfree, parity fpar);
+// close: it ends them, and the products of a phase complete the group's sums
+// of it (accfull).  Returns whether a wait gave up (warp-uniform).
+template <int ND, int PAR, int PH>
+__device__ __forceinline__ bool oz_issue_phase(uint32_t a0, uint32_t b0, uint32_t acc, bool open, bool held,
+                                               bool close, uint32_t accfull0, uint32_t accfree0, uint32_t fpar,
+                                               uint32_t done, uint32_t on, const int *err) {
+    constexpr int P0 = oz_ph<ND>(PH), D0 = P0 + ((P0 ^ PAR) & 1);
+    if (held) {
+        if (__any_sync(0xffffffffu, !mbar_wait(accfree0 + 8 * PH, fpar, err))) return true;
+        tc_fence_after();
     }
-    return fma(dL, 5.9604644775390625e-08, dU);   // 2^-24
+    issue_products_i8<ND, D0, oz_ph<ND>(PH + 1), 2>(a0, b0, acc, open, on);
+    if (PH == OZ_NPH - 1) mma_commit_on(done, on);
+    if (close) mma_commit_on(accfull0 + 8 * PH, on);
+    return false;
 }
 
-// The exact sums of `ncol` columns (a multiple of 8) of this thread's lane:
-// ND accumulators per column from tensor memory (taddr: the lane's first
-// column of diagonal 0), eight columns per wait, unscaled values to
-// hb[c OZ_M] (warp-wide).
-template <int ND>
-__device__ __forceinline__ void oz_read_sums(uint32_t taddr, int ncol, double *hb) {
-#pragma unroll 1
-    for (int c = 0; c < ncol; c += 8) {
-        uint32_t a[ND][8];
+template <int ND, int PAR>
+__device__ __forceinline__ bool oz_issue_chunk(uint32_t a0, uint32_t b0, uint32_t acc, bool open, bool held, bool close,
+                                               uint32_t accfull0, uint32_t accfree0, uint32_t fpar, uint32_t done,
+                                               uint32_t on, const int *err) {
+    return oz_issue_phase<ND, PAR, 0>(a0, b0, acc, open, held, close, accfull0, accfree0, fpar, done, on, err) ||
+           oz_issue_phase<ND, PAR, 1>(a0, b0, acc, open, held, close, accfull0, accfree0, fpar, done, on, err) ||
+           oz_issue_phase<ND, PAR, 2>(a0, b0, acc, open, held, close, accfull0, accfree0, fpar, done, on, err);
+}
+
+// Phase PH's part of the sums V[c] (units of 2^-sh of ACC_2's) of one half's
+// columns in this thread's lane, from tensor memory (taddr: the lane's first
+// column of diagonal 0; warp-wide).  The loads of a batch of columns go out
+// before one wait.
+template <int ND, int PH>
+__device__ __forceinline__ void oz_read_phase(uint32_t taddr, int sh, long long (&V)[Oz<ND>::NHALF]) {
+    constexpr int D0 = oz_ph<ND>(PH), NA = oz_ph<ND>(PH + 1) - D0, NHALF = Oz<ND>::NHALF;
+    constexpr int NC = 8;                               // columns per batch
+    static_assert(NHALF % NC == 0, "whole batches");
 #pragma unroll
-        for (int d = 0; d < ND; ++d) tmem_ld8(taddr + d * Oz<ND>::NP + c, a[d]);
+    for (int c = 0; c < NHALF; c += NC) {
+        uint32_t a[NA][NC];
+#pragma unroll
+        for (int d = 0; d < NA; ++d) tmem_ld8(taddr + (D0 + d) * Oz<ND>::NP + c, a[d]);
         tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            uint32_t col[ND];
+        for (int i = 0; i < NC; ++i) {
 #pragma unroll
-            for (int d = 0; d < ND; ++d) {
-                reg_after_wait(a[d][i]);
-                col[d] = a[d][i];
+            for (int d = 0; d < NA; ++d) reg_after_wait(a[d][i]);
+            if (PH == 0) {
+                V[c + i] = ((long long) (int) a[0][i] * 65536 + (long long) (int) a[1][i] * 256 + (int) a[2][i]) << sh;
+            } else if (PH == 1) {
+                V[c + i] += ((long long) (int) a[0][i] * 256 + (int) a[1][i]) << (sh - 16);
+            } else if (ND == 6) {
+                // unit 2^-24: sh is 21 .. 29
+                const long long v = (int) a[0][i];
+                V[c + i] += sh >= 24 ? v << (sh - 24) : (v + (1 << (23 - sh))) >> (24 - sh);
+            } else {
+                // unit 2^-32
+                const long long v = (long long) (int) a[0][i] * 256 + (int) a[NA - 1][i];
+                V[c + i] += (v + (1 << (31 - sh))) >> (32 - sh);
             }
-            hb[(c + i) * OZ_M] = oz_unscaled<ND>(col);
         }
     }
+}
+
+// One thread's part of taking a group's sums out of tensor memory: every phase
+// as its products complete (accfull), handing it back (accfree) for the next
+// group.  Returns whether a wait gave up (warp-uniform: the tensor-memory
+// accesses are warp-wide).
+template <int ND>
+__device__ __forceinline__ bool oz_take(uint32_t taddr, int sh, long long (&V)[Oz<ND>::NHALF], uint32_t accfull0,
+                                        uint32_t accfree0, uint32_t parity, const int *err) {
+    if (__any_sync(0xffffffffu, !mbar_wait(accfull0, parity, err))) return true;
+    tc_fence_after();
+    oz_read_phase<ND, 0>(taddr, sh, V);
+    tc_fence_before();
+    mbar_arrive(accfree0);
+    if (__any_sync(0xffffffffu, !mbar_wait(accfull0 + 8, parity, err))) return true;
+    tc_fence_after();
+    oz_read_phase<ND, 1>(taddr, sh, V);
+    tc_fence_before();
+    mbar_arrive(accfree0 + 8);
+    if (__any_sync(0xffffffffu, !mbar_wait(accfull0 + 16, parity, err))) return true;
+    tc_fence_after();
+    oz_read_phase<ND, 2>(taddr, sh, V);
+    tc_fence_before();
+    mbar_arrive(accfree0 + 16);
+    return false;
+}
+
+// v 2^(e >> 20) for a value v that came from an integer (zero or normal)
+__device__ __forceinline__ double oz_scaled(double v, int e) {
+    const int hi = __double2hiint(v);
+    return __hiloint2double(hi ? hi + e : 0, __double2loint(v));
 }
 
 // ---------------------------------------------------------------------------
@@ -200,7 +313,7 @@ __global__ void __launch_bounds__(OZ_BOP_J * Oz<ND>::NP) k_oz_bop(DevBatch B, co
     constexpr int OZ_NP = Oz<ND>::NP, OZ_NHALF = Oz<ND>::NHALF;
     const int g = blockIdx.x, tid = threadIdx.x;
     const int r0 = B.tg_r0[g], gn = B.tg_n[g], nk = B.tg_nk[g];
-    const int C1 = 1 + B.nd1, P = gn * C1;
+    const int C1 = 1 + (B.t_m > 0) + (B.t_x > 0), P = gn * C1;
     const int n = tid % OZ_NP, j0 = tid / OZ_NP;
     const int rp = (n % OZ_NHALF) >> 1;               // operand column pair (radius, Mie column)
     const int comp = (n >= OZ_NHALF ? 2 : 0) + (n & 1);   // re/im of S, then of D'
@@ -343,32 +456,35 @@ __device__ __forceinline__ int oz_epi_sync_or(int v) {
 // ---------------------------------------------------------------------------
 // The product kernel.
 // ---------------------------------------------------------------------------
-template <int ND, int NC1>
+// TM: the m tangent column; TX: 0 no per-derivative sums, 1 those of index1
+// derivatives that move the weights, 2 those and the x column.
+template <int ND, int TM, int TX>
 __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngItem *__restrict__ items,
                                                         const unsigned char *__restrict__ bop,
                                                         double *__restrict__ part, int *__restrict__ err) {
     using F = OzK<ND>;
-    constexpr int C1 = 1 + NC1, CPR = 2 * C1;
+    constexpr int NT = TM + (TX == 2), CPR = 2 * (1 + NT);   // columns of each half per radius
     constexpr int OZ_NP = F::NP, OZ_NHALF = F::NHALF, OZ_MAX_GN = F::MAX_GN, OZ_HB = F::HB;
     constexpr int OZ_ASTAGES = F::ASTAGES, OZ_BSLOTS = F::BSLOTS, OZ_NBAR = F::NBAR;
     constexpr uint32_t OZ_ACOL = F::ACOL, OZ_ACOLS = F::ACOLS, OZ_BSTAGE = F::BSTAGE, OZ_ACHUNK = F::ACHUNK;
     extern __shared__ __align__(1024) unsigned char smem[];
     double *hbuf = (double *) (smem + F::O_HBUF);            // [2][OZ_NP][OZ_M] sums of a group, unscaled
-    double *wsh = (double *) (smem + F::O_WBUF);             // [OZ_MAX_GN][OZ_MAX_NS] weights
-    double *csh = (double *) (smem + F::O_CBUF);             // [OZ_NP] column scales
+    double *wsh = (double *) (smem + F::O_WBUF);             // [radius][NS] weights
+    int *csh = (int *) (smem + F::O_CBUF);                   // [OZ_NP] column exponents << 20
     uint64_t *bars = (uint64_t *) (smem + F::O_BARS);
     uint32_t *tmem_hold = (uint32_t *) (bars + OZ_NBAR);
     const uint32_t bring = smem_u32(smem);
-    const uint32_t afull0 = smem_u32(bars), adone0 = afull0 + 8 * OZ_ASTAGES;
-    const uint32_t bfull0 = adone0 + 8 * OZ_ASTAGES, bdone0 = bfull0 + 8 * OZ_BSLOTS;
-    const uint32_t accfull = bdone0 + 8 * OZ_BSLOTS, accfree = accfull + 8;
-    const uint32_t hready0 = accfree + 8, hfree0 = hready0 + 16, fin = hfree0 + 16;
+    // chunk q's operands are in place: afull[q % BSLOTS] (the A set's 128 threads), bfull[q % BSLOTS] (the
+    // B copy); its products have completed: done[q % BSLOTS] (both issuing warps)
+    const uint32_t afull0 = smem_u32(bars), bfull0 = afull0 + 8 * OZ_BSLOTS, done0 = bfull0 + 8 * OZ_BSLOTS;
+    const uint32_t accfull0 = done0 + 8 * OZ_BSLOTS, accfree0 = accfull0 + 8 * OZ_NPH;
+    const uint32_t hready0 = accfree0 + 8 * OZ_NPH, hfree0 = hready0 + 16, fin = hfree0 + 16;
 
-    const int tid = threadIdx.x, warp = tid >> 5;
+    const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
     const AngItem it = items[blockIdx.x];
     const DevCase &C = B.cs[it.c];
     const int nh = C.nh, n_qang = C.n_qang, R = B.R;
-    const int nd2 = B.nd2, NS = 1 + NC1 + nd2;
+    const int nd1 = B.nd1, nd2 = B.nd2, NS = 1 + nd2 + (TX > 0 ? nd1 : 0) + (TX == 2 ? nd1 : 0);
 
     // after a failure elsewhere the remaining blocks return at once
     __shared__ int s_skip;
@@ -376,21 +492,20 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
     __syncthreads();
     if (s_skip) return;
     if (tid == 0) {
-        for (int i = 0; i < OZ_ASTAGES; ++i) {
-            mbar_init(afull0 + 8 * i, OZ_M);
-            mbar_init(adone0 + 8 * i, 1);
-        }
         for (int i = 0; i < OZ_BSLOTS; ++i) {
+            mbar_init(afull0 + 8 * i, OZ_M);
             mbar_init(bfull0 + 8 * i, 1);
-            mbar_init(bdone0 + 8 * i, 1);
+            mbar_init(done0 + 8 * i, 2);
         }
-        mbar_init(accfull, 1);
-        mbar_init(accfree, 256);
+        for (int i = 0; i < OZ_NPH; ++i) {
+            mbar_init(accfull0 + 8 * i, 2);
+            mbar_init(accfree0 + 8 * i, 256);
+        }
         for (int i = 0; i < 2; ++i) {
             mbar_init(hready0 + 8 * i, 256);
             mbar_init(hfree0 + 8 * i, 128);
         }
-        mbar_init(fin, 1);
+        mbar_init(fin, 2);
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(smem_u32(tmem_hold), OZ_TMEM_COLS);
@@ -400,73 +515,87 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
     const uint32_t tmem = *tmem_hold;
     int bad = 0;
 
-    if (tid < OZ_M) {
-        // ---------------- warps 0-3: the A digit slices, one row (lane) per thread ----------------
-        const int row = tid;
-        const uint32_t tlane = tmem + ((uint32_t) (warp * 32) << 16);
+    if (warp < OZ_QUAD_WARP) {
+        // ---------------- warps 0-7: A digit slices and the groups' sums, one row (lane) per thread ----------------
+        // Two sets of four warps.  The sets bring alternate chunks of A: a
+        // chunk's loads take 1-2 chunks' time (L2), so one set alone, loading
+        // a chunk while it waits to store it, was what limited the products.
+        // Set 0 takes the D' columns of a group's sums out of tensor memory,
+        // set 1 the S columns.
+        const int set = warp >> 2, row = tid & (OZ_M - 1);
+        const uint32_t tlane = tmem + ((uint32_t) ((warp & 3) * 32) << 16);
+        const int hcol = set == 0 ? OZ_NHALF : 0;            // first column of the set's half
         // this row's A digit slices: piece i of chunk kc of the item's angle
         // tile at arow[kc OZ_ACHUNK / 16 + i OZ_M]
         const uint4 *arow = (const uint4 *) (B.oz_aop + C.a_off + (size_t) it.xt * C.nkx * OZ_ACHUNK) + row;
-        // The digit warps take the D' columns of a group's finished sums out of
-        // tensor memory (warps 4-7 take the S columns): once the quadratic
-        // forms are done with the buffer's previous group, after the group's
-        // last products.  Returns nonzero when a wait gave up.
+        // Takes the set's half of a group's sums out of tensor memory and, once
+        // the quadratic forms are done with the buffer's previous group, into
+        // the buffer.  Returns nonzero when a wait gave up.
         auto take = [&](int gh) -> int {
-            const int g = it.rbeg + gh, ncol = B.tg_n[g] * CPR;
+            long long V[OZ_NHALF];
+            if (oz_take<ND>(tlane + hcol, oz_sum_shift(B.tg_nk[it.rbeg + gh]), V, accfull0, accfree0, gh & 1, err))
+                return 1;
             // the buffer's previous group (gh - 2) has been through the quadratic forms
             const int b = gh & 1;
-            bool ok = gh < 2 || mbar_wait(hfree0 + 8 * b, ((gh >> 1) - 1) & 1, err);
-            ok = ok && mbar_wait(accfull, gh & 1, err);
-            double *hb = hbuf + b * OZ_HB;
-            if (__any_sync(0xffffffffu, !ok)) return 1;
-            tc_fence_after();
-            oz_read_sums<ND>(tlane + OZ_NHALF, (ncol + 7) & ~7, hb + OZ_NHALF * OZ_M + row);
-            tc_fence_before();
-            mbar_arrive(accfree);
+            if (__any_sync(0xffffffffu, gh >= 2 && !mbar_wait(hfree0 + 8 * b, ((gh >> 1) - 1) & 1, err))) return 1;
+            double *hb = hbuf + b * OZ_HB + hcol * OZ_M + row;
+#pragma unroll
+            for (int i = 0; i < OZ_NHALF; ++i) hb[i * OZ_M] = (double) V[i];
             mbar_arrive(hready0 + 8 * b);
             return 0;
         };
         int q = 0, gi = 0, hold_next = 0;
-        int sgrp[OZ_ASTAGES];                              // group of the chunk last written to each stage
+        // groups to be out before a stage is written again: those before its
+        // previous chunk's group, and that group itself when the chunk ended
+        // it.  need[i]: of the chunk i + 1 before this one.
+        int need[OZ_ASTAGES];
 #pragma unroll
-        for (int i = 0; i < OZ_ASTAGES; ++i) sgrp[i] = 0;
+        for (int i = 0; i < OZ_ASTAGES; ++i) need[i] = 0;
         for (int g = it.rbeg; g < it.rend && !bad; ++g, ++gi) {
             const int nk = B.tg_nk[g];
             for (int kc = 0; kc < nk; ++kc, ++q) {
-                const int s = q % OZ_ASTAGES;
-                // the stage's previous chunk must have been consumed by its products,
-                // which reach its group once the sums of every earlier group are out;
-                // warp-uniform decisions: the tensor-memory accesses are warp-wide
-                if (q >= OZ_ASTAGES)
-                    while (!bad && hold_next < sgrp[s]) bad = take(hold_next++);
-                if (bad) break;
-                // the chunk's digit slices of this row, loaded before the wait
-                const uint4 *ac = arow + (size_t) kc * (OZ_ACHUNK / 16);
-                uint4 a[2 * ND];
+                if ((q & 1) == set) {
+                    const int s = q % OZ_ASTAGES;
+                    // the chunk's digit slices of this row, loaded before the waits
+                    const uint4 *ac = arow + (size_t) kc * (OZ_ACHUNK / 16);
+                    uint4 a[2 * ND];
 #pragma unroll
-                for (int i = 0; i < 2 * ND; ++i) a[i] = ac[i * OZ_M];
-                const bool ok = q < OZ_ASTAGES || mbar_wait(adone0 + 8 * s, ((q / OZ_ASTAGES) - 1) & 1, err);
-                if (__any_sync(0xffffffffu, !ok)) {
-                    bad = 1;
-                    break;
-                }
-                tc_fence_after();
-                const uint32_t acol = tlane + OZ_ACOL + s * OZ_ACOLS;
+                    for (int i = 0; i < 2 * ND; ++i) a[i] = ld_once(ac + i * OZ_M);
+                    // The stage's previous chunk must have been consumed by its products,
+                    // which reach its group once the sums of every earlier group are out
+                    // (its own group's sums are taken first when they complete with it, so
+                    // that the next group's products are not kept waiting).  Neither set
+                    // waits for the other: the set with the earlier chunk has taken what
+                    // that chunk's products need, and the other one no less.
+                    // Warp-uniform decisions: the tensor-memory accesses are warp-wide.
+                    while (!bad && hold_next < need[OZ_ASTAGES - 1]) bad = take(hold_next++);
+                    if (bad) break;
+                    const int qp = q - OZ_ASTAGES;
+                    const bool ok = qp < 0 || mbar_wait(done0 + 8 * (qp % OZ_BSLOTS), (qp / OZ_BSLOTS) & 1, err);
+                    if (__any_sync(0xffffffffu, !ok)) {
+                        bad = 1;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t acol = tlane + OZ_ACOL + s * OZ_ACOLS;
 #pragma unroll
-                for (int sl = 0; sl < ND; ++sl) {
-                    tmem_st4(acol + sl * (OZ_KC / 4), a[2 * sl].x, a[2 * sl].y, a[2 * sl].z, a[2 * sl].w);
-                    tmem_st4(acol + sl * (OZ_KC / 4) + 4, a[2 * sl + 1].x, a[2 * sl + 1].y, a[2 * sl + 1].z,
-                             a[2 * sl + 1].w);
+                    for (int sl = 0; sl < ND; ++sl) {
+                        tmem_st4(acol + sl * (OZ_KC / 4), a[2 * sl].x, a[2 * sl].y, a[2 * sl].z, a[2 * sl].w);
+                        tmem_st4(acol + sl * (OZ_KC / 4) + 4, a[2 * sl + 1].x, a[2 * sl + 1].y, a[2 * sl + 1].z,
+                                 a[2 * sl + 1].w);
+                    }
+                    tmem_wait_st();
+                    tc_fence_before();
+                    mbar_arrive(afull0 + 8 * (q % OZ_BSLOTS));
                 }
-                tmem_wait_st();
-                tc_fence_before();
-                sgrp[s] = gi;
-                mbar_arrive(afull0 + 8 * s);
+#pragma unroll
+                for (int i = OZ_ASTAGES - 1; i > 0; --i) need[i] = need[i - 1];
+                need[0] = kc == nk - 1 ? gi + 1 : gi;
             }
         }
         while (!bad && hold_next < it.rend - it.rbeg) bad = take(hold_next++);
-    } else if (warp >= OZ_QUAD_WARP) {
-        // ---------------- warps 10-13: quadratic forms, one row per thread ----------------
+    } else if (warp < OZ_MMA_WARP) {
+        // ---------------- warps 8-11: quadratic forms, one row per thread ----------------
         // A warp whose wait fails keeps taking the barriers of the four warps,
         // which stop together.
         const int t1 = tid - OZ_QUAD_WARP * 32;              // product row
@@ -474,45 +603,55 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
         const int ej = it.xt * OZ_HALF + eh;
         const bool eact = ej < nh;
         const signed char *gtab = B.oz_rowexp + C.rx_off + 2 * (size_t) (eact ? ej : 0) + emir;
-        int slot1[NC1 > 0 ? NC1 : 1];
+        // f-weighted sums over radii: the value's four invariants, those of the
+        // index2 columns, of the index1 derivatives' own weights and x column
+        double rv[4] = {0., 0., 0., 0.}, r2[OZ_MAX_ND2][4], r1[TX ? OZ_MAX_ND1 : 1][4];
 #pragma unroll
-        for (int k = 0; k < NC1; ++k) slot1[k] = 1 + B.idx1[k];
-        // per column set: f-weighted sums over radii of the four invariants
-        double racc[1 + NC1 + OZ_MAX_ND2][4];
+        for (int s = 0; s < OZ_MAX_ND2; ++s)
 #pragma unroll
-        for (int s = 0; s < 1 + NC1 + OZ_MAX_ND2; ++s)
+            for (int e = 0; e < 4; ++e) r2[s][e] = 0.;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) racc[s][e] = 0.;
+        for (int s = 0; s < (TX ? OZ_MAX_ND1 : 1); ++s)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) r1[s][e] = 0.;
+        // with the m column: conj(sp) dsp, conj(sm) dsm, conj(sm) dsp, conj(sp) dsm
+        cplx rm[TM ? 4 : 1];
+#pragma unroll
+        for (int e = 0; e < (TM ? 4 : 1); ++e) rm[e] = mk(0., 0.);
         // the scales of this row and of its pair row (which holds this row's sm)
         const double rsc = oz_pow2(eact ? (int) *gtab : 0);
         const double rsp = __shfl_xor_sync(0xffffffffu, rsc, 1);
-        // A group's radius weights (gn NS <= OZ_MAX_GN OZ_MAX_NS values, at most
-        // one per thread) and column scales (with the row-independent
-        // factor of the combination), fetched into registers one group ahead
-        // so that their loads overlap the previous group's forms.
-        double wnext = 0., cnext = 0.;
+        // A group's radius weights (gn NS <= MAX_W values, at most one per
+        // thread) and column exponents (with the row-independent factor of the
+        // combination), fetched into registers one group ahead so that their
+        // loads overlap the previous group's forms.
+        double wnext = 0.;
+        int cnext = 0;
         auto fetch = [&](int g) {
             const int gn = B.tg_n[g];
             if (t1 < gn * NS && gn <= OZ_MAX_GN) {
-                const int p = t1 / NS, s = t1 - p * NS;
-                const int slot = s == 0 ? 0 : (s <= NC1 ? slot1[s - 1] : 1 + B.idx2[s - 1 - NC1]);
-                wnext = B.w[(size_t) slot * R + B.tg_r0[g] + p];
+                const int p = t1 / NS, s = t1 - p * NS, rad = B.tg_r0[g] + p;
+                if (s <= nd2) {
+                    wnext = B.w[(size_t) (s == 0 ? 0 : 1 + B.idx2[s - 1]) * R + rad];
+                } else if (s <= nd2 + nd1) {
+                    wnext = B.w[(size_t) (1 + B.idx1[s - 1 - nd2]) * R + rad];
+                } else {
+                    wnext = B.x_own ? 1. : B.xl[(size_t) (s - 1 - nd2 - nd1) * R + rad];
+                }
             }
-            if (t1 < OZ_NP) cnext = oz_pow2(B.oz_colexp[(size_t) g * OZ_NP + t1] + F::CSHIFT);
+            if (t1 < OZ_NP)
+                cnext = (B.oz_colexp[(size_t) g * OZ_NP + t1] + F::CSHIFT - oz_sum_shift(B.tg_nk[g])) * (1 << 20);
         };
         if (it.rbeg < it.rend) fetch(it.rbeg);
         int gi = 0;
         for (int g = it.rbeg; g < it.rend; ++g, ++gi) {
             const int gn = B.tg_n[g];
-            // the previous group's weights and scales have been read by all four warps
+            // the previous group's weights and exponents have been read by all four warps
             if (oz_epi_sync_or(bad || gn > OZ_MAX_GN)) {
                 bad = 1;
                 break;
             }
-            if (t1 < gn * NS) {
-                const int p = t1 / NS;
-                wsh[p * OZ_MAX_NS + (t1 - p * NS)] = wnext;
-            }
+            if (t1 < gn * NS) wsh[t1] = wnext;
             if (t1 < OZ_NP) csh[t1] = cnext;
             oz_epi_sync_or(0);
             // the next group's loads, in flight during this group's forms (a
@@ -524,50 +663,67 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
                 bad = 1;
                 continue;
             }
-            // The row scales are left out here: every term of racc[s][0] carries
-            // rsc^2, of racc[s][1] rsp^2 and of racc[s][2..3] rsc rsp (powers of
-            // two, applied once at the end).
+            // The row scales are left out here: every term of an invariant 0
+            // (|sp|^2 and its tangents) carries rsc^2, of an invariant 1 rsp^2
+            // and of the others rsc rsp (powers of two, applied once at the
+            // end).
             for (int p = 0; p < gn; ++p) {
                 // columns of S (i < CPR, this row) and D' (i >= CPR, the pair row: sm)
                 double v[2 * CPR];
 #pragma unroll
                 for (int i = 0; i < CPR; ++i) {
                     const int cs = p * CPR + i, cd = OZ_NHALF + p * CPR + i;
-                    v[i] = hb[cs * OZ_M + t1] * csh[cs];
-                    v[CPR + i] = hb[cd * OZ_M + (t1 ^ 1)] * csh[cd];
+                    v[i] = oz_scaled(hb[cs * OZ_M + t1], csh[cs]);
+                    v[CPR + i] = oz_scaled(hb[cd * OZ_M + (t1 ^ 1)], csh[cd]);
                 }
-                const double *wp = wsh + p * OZ_MAX_NS;
+                const double *wp = wsh + p * NS;
                 const double f = wp[0];
                 // invariants of (sp, sm): |sp|^2, |sm|^2, Re(sp sm*), Im(sm sp*)
                 const double spr = v[0], spi = v[1], smr = v[CPR], smi = v[CPR + 1];
-                const double ia = spr * spr + spi * spi, ib = smr * smr + smi * smi;
-                const double ic = spr * smr + spi * smi, id = smi * spr - smr * spi;
-                racc[0][0] += f * ia;
-                racc[0][1] += f * ib;
-                racc[0][2] += f * ic;
-                racc[0][3] += f * id;
+                const double inv[4] = {spr * spr + spi * spi, smr * smr + smi * smi, spr * smr + spi * smi,
+                                       smi * spr - smr * spi};
 #pragma unroll
-                for (int k = 0; k < NC1; ++k) {
-                    const double fl = wp[1 + k];
-                    const double plr = v[2 + 2 * k], pli = v[3 + 2 * k];
-                    const double mlr = v[CPR + 2 + 2 * k], mli = v[CPR + 3 + 2 * k];
-                    const double da = 2. * (plr * spr + pli * spi), db = 2. * (mlr * smr + mli * smi);
-                    const double dc = plr * smr + pli * smi + spr * mlr + spi * mli;
-                    const double dd = mli * spr - mlr * spi + smi * plr - smr * pli;
-                    racc[1 + k][0] += fl * ia + f * da;
-                    racc[1 + k][1] += fl * ib + f * db;
-                    racc[1 + k][2] += fl * ic + f * dc;
-                    racc[1 + k][3] += fl * id + f * dd;
-                }
+                for (int e = 0; e < 4; ++e) rv[e] += f * inv[e];
 #pragma unroll
-                for (int k = 0; k < OZ_MAX_ND2; ++k) {
+                for (int k = 0; k < OZ_MAX_ND2; ++k)
                     if (k < nd2) {
-                        const double fl = wp[1 + NC1 + k];
-                        racc[1 + NC1 + k][0] += fl * ia;
-                        racc[1 + NC1 + k][1] += fl * ib;
-                        racc[1 + NC1 + k][2] += fl * ic;
-                        racc[1 + NC1 + k][3] += fl * id;
+                        const double fl = wp[1 + k];
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) r2[k][e] += fl * inv[e];
                     }
+                // the weighted value, for the products with its tangents
+                const double gpr = f * spr, gpi = f * spi, gmr = f * smr, gmi = f * smi;
+                if (TM) {
+                    const double dpr = v[2], dpi = v[3], dmr = v[CPR + 2], dmi = v[CPR + 3];
+                    rm[0].re += gpr * dpr;  rm[0].re += gpi * dpi;
+                    rm[0].im += gpr * dpi;  rm[0].im -= gpi * dpr;
+                    rm[1].re += gmr * dmr;  rm[1].re += gmi * dmi;
+                    rm[1].im += gmr * dmi;  rm[1].im -= gmi * dmr;
+                    rm[2].re += gmr * dpr;  rm[2].re += gmi * dpi;
+                    rm[2].im += gmr * dpi;  rm[2].im -= gmi * dpr;
+                    rm[3].re += gpr * dmr;  rm[3].re += gpi * dmi;
+                    rm[3].im += gpr * dmi;  rm[3].im -= gpi * dmr;
+                }
+                if (TX) {
+                    double dx[4] = {0., 0., 0., 0.};
+                    if (TX == 2) {
+                        constexpr int X = 2 + 2 * TM;
+                        const double plr = v[X], pli = v[X + 1], mlr = v[CPR + X], mli = v[CPR + X + 1];
+                        dx[0] = 2. * (plr * gpr + pli * gpi);
+                        dx[1] = 2. * (mlr * gmr + mli * gmi);
+                        dx[2] = plr * gmr + pli * gmi + gpr * mlr + gpi * mli;
+                        dx[3] = mli * gpr - mlr * gpi + gmi * plr - gmr * pli;
+                    }
+#pragma unroll
+                    for (int k = 0; k < OZ_MAX_ND1; ++k)
+                        if (k < nd1) {
+                            const double fl = wp[1 + nd2 + k], xc = TX == 2 ? wp[1 + nd2 + nd1 + k] : 0.;
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) {
+                                r1[k][e] += fl * inv[e];
+                                if (TX == 2) r1[k][e] += xc * dx[e];
+                            }
+                        }
                 }
             }
             // the buffer is free for the group after next
@@ -581,20 +737,38 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
             const int Q = 4 * (1 + B.nd);
             double *pc = part + C.part_off + (size_t) it.g * Q * n_qang;
             const double ss = rsc * rsc, mm = rsp * rsp, sm = rsc * rsp;
-#pragma unroll
-            for (int s = 0; s < 1 + NC1 + OZ_MAX_ND2; ++s) {
-                if (s >= NS) break;
-                const int slot = s == 0 ? 0 : (s <= NC1 ? slot1[s - 1] : 1 + B.idx2[s - 1 - NC1]);
+            auto put = [&](int slot, const double (&q)[4]) {
                 double *o = pc + (size_t) slot * 4 * n_qang + jj;
-                const double a = racc[s][0] * ss, b = racc[s][1] * mm;
+                const double a = q[0] * ss, b = q[1] * mm;
                 o[0] = .25 * (a + b);
                 o[(size_t) n_qang] = .25 * (a - b);
-                o[(size_t) 2 * n_qang] = -.5 * (racc[s][2] * sm);
-                o[(size_t) 3 * n_qang] = .5 * (racc[s][3] * sm);
-            }
+                o[(size_t) 2 * n_qang] = -.5 * (q[2] * sm);
+                o[(size_t) 3 * n_qang] = .5 * (q[3] * sm);
+            };
+            put(0, rv);
+#pragma unroll
+            for (int k = 0; k < OZ_MAX_ND2; ++k)
+                if (k < nd2) put(1 + B.idx2[k], r2[k]);
+#pragma unroll
+            for (int k = 0; k < OZ_MAX_ND1; ++k)
+                if (k < nd1) {
+                    double d[4];
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) d[e] = TX ? r1[TX ? k : 0][e] : 0.;
+                    if (TM) {
+                        // d|sp|^2 = 2 Re(m_l conj(sp) dsp) and so on
+                        const cplx ml = B.m_l[C.ml_off + B.idx1[k]];
+                        const cplx u = rm[TM ? 2 : 0] + rm[TM ? 3 : 0], w = rm[TM ? 2 : 0] - rm[TM ? 3 : 0];
+                        d[0] += 2. * (ml.re * rm[0].re - ml.im * rm[0].im);
+                        d[1] += 2. * (ml.re * rm[TM ? 1 : 0].re - ml.im * rm[TM ? 1 : 0].im);
+                        d[2] += ml.re * u.re - ml.im * u.im;
+                        d[3] -= ml.re * w.im + ml.im * w.re;
+                    }
+                    put(1 + B.idx1[k], d);
+                }
         }
     } else if (warp == OZ_COPY_WARP) {
-        // ---------------- warp 9, lane 0: B copies, up to OZ_BSLOTS chunks ahead ----------------
+        // ---------------- warp 14, lane 0: B copies, up to OZ_BSLOTS chunks ahead ----------------
         if ((tid & 31) == 0) {
             int pq = 0;
             for (int g = it.rbeg; g < it.rend && !bad; ++g) {
@@ -603,7 +777,7 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
                 for (int kc = 0; kc < nk; ++kc, ++pq) {
                     const int ps = pq % OZ_BSLOTS;
                     // the slot's previous chunk pq - OZ_BSLOTS must have been consumed
-                    if (pq >= OZ_BSLOTS && !mbar_wait(bdone0 + 8 * ps, ((pq / OZ_BSLOTS) - 1) & 1, err)) {
+                    if (pq >= OZ_BSLOTS && !mbar_wait(done0 + 8 * ps, ((pq / OZ_BSLOTS) - 1) & 1, err)) {
                         bad = 1;
                         break;
                     }
@@ -616,64 +790,43 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
             const int q0 = pq > OZ_BSLOTS ? pq - OZ_BSLOTS : 0;
             for (int c = q0; c < pq; ++c) mbar_wait(bfull0 + 8 * (c % OZ_BSLOTS), (c / OZ_BSLOTS) & 1, nullptr);
         }
-    } else if (warp == OZ_MMA_WARP) {
-        // ---------------- warp 8: the products ----------------
-        // The whole warp runs the loop (its values stay warp-uniform) and one
-        // elected lane issues; the decisions to stop are warp-uniform.
+    } else {
+        // ---------------- warps 12, 13: the products of the even / odd diagonals ----------------
+        // The whole warp runs the loop and one elected lane issues; the decisions
+        // to stop are warp-uniform, and so is, visibly to the compiler, what
+        // the products' operands are made of: they are taken from uniform
+        // registers, and moving each operand of each product there costs more
+        // than the product takes.
+        const uint32_t tm = warp_uniform(tmem), b0 = warp_uniform(bring);
+        const int rend = warp_uniform(it.rend);
+        const uint32_t on = elect_one();
         int q = 0, gi = 0;
-        for (int g = it.rbeg; g < it.rend && !bad; ++g, ++gi) {
-            const int nk = B.tg_nk[g];
+        for (int g = warp_uniform(it.rbeg); g < rend && !bad; ++g, ++gi) {
+            const int nk = warp_uniform(B.tg_nk[g]);
             for (int kc = 0; kc < nk; ++kc, ++q) {
-                const int s = q % OZ_ASTAGES, sb = q % OZ_BSLOTS;
-                bool ok = mbar_wait(afull0 + 8 * s, (q / OZ_ASTAGES) & 1, err) &&
-                          mbar_wait(bfull0 + 8 * sb, (q / OZ_BSLOTS) & 1, err);
-                // the previous group's accumulators must have been read
-                if (ok && kc == 0 && gi >= 1) ok = mbar_wait(accfree, (gi - 1) & 1, err);
+                const int sb = q % OZ_BSLOTS;
+                const bool ok = mbar_wait(afull0 + 8 * sb, (q / OZ_BSLOTS) & 1, err) &&
+                                mbar_wait(bfull0 + 8 * sb, (q / OZ_BSLOTS) & 1, err);
                 if (__any_sync(0xffffffffu, !ok)) {
                     bad = 1;
                     break;
                 }
                 tc_fence_after();
-                if (elect_one()) {
-                    issue_chunk_i8<ND>(tmem + OZ_ACOL + s * OZ_ACOLS, bring + sb * OZ_BSTAGE, tmem, kc == 0);
-                    mma_commit(adone0 + 8 * s);
-                    mma_commit(bdone0 + 8 * sb);
-                    if (kc == nk - 1) mma_commit(accfull);
+                const uint32_t ac = tm + OZ_ACOL + (q % OZ_ASTAGES) * OZ_ACOLS, bc = b0 + sb * OZ_BSTAGE;
+                const bool open = kc == 0, close = kc == nk - 1, held = open && gi >= 1;
+                const uint32_t fpar = (gi - 1) & 1, done = done0 + 8 * sb;
+                if (warp == OZ_MMA_WARP ? oz_issue_chunk<ND, 0>(ac, bc, tm, open, held, close, accfull0, accfree0, fpar,
+                                                                done, on, err)
+                                        : oz_issue_chunk<ND, 1>(ac, bc, tm, open, held, close, accfull0, accfree0, fpar,
+                                                                done, on, err)) {
+                    bad = 1;
+                    break;
                 }
-                __syncwarp();
             }
         }
         // all products of this warp have completed
-        if (elect_one()) mma_commit(fin);
-        __syncwarp();
+        mma_commit_on(fin, on);
         mbar_wait(fin, 0u, nullptr);
-    } else if (warp >= 4) {
-        // ---------------- warps 4-7: the S sums of each group ----------------
-        const int t1 = tid - 128;                            // product row = tensor-memory lane
-        const uint32_t trow = tmem + ((uint32_t) ((warp - 4) * 32) << 16);
-        int gi = 0;
-        for (int g = it.rbeg; g < it.rend && !bad; ++g, ++gi) {
-            const int ncol = B.tg_n[g] * CPR;                 // used columns of each half
-            // the buffer's previous group has been through the quadratic
-            // forms and this group's products are done (warp-uniform: the
-            // tensor-memory accesses below are warp-wide)
-            const int b = gi & 1;
-            bool ok = gi < 2 || mbar_wait(hfree0 + 8 * b, ((gi >> 1) - 1) & 1, err);
-            ok = ok && mbar_wait(accfull, gi & 1, err);
-            double *hb = hbuf + b * OZ_HB;
-            if (__any_sync(0xffffffffu, !ok)) {
-                bad = 1;
-                break;
-            }
-            tc_fence_after();
-            // the exact sums of the group's used S columns into the buffer
-            // (the digit warps take the D' columns); the accumulators go back
-            // right after
-            oz_read_sums<ND>(trow, (ncol + 7) & ~7, hb + t1);
-            tc_fence_before();
-            mbar_arrive(accfree);
-            mbar_arrive(hready0 + 8 * b);
-        }
     }
     if (bad) atomicExch(err, 1);
     tc_fence_before();
@@ -764,7 +917,7 @@ __global__ void __launch_bounds__(128, 1) k_oz_selftest(int K, const double *__r
         __syncthreads();
         if (tid == 0 && !(withhold && kc == 0)) {
             tc_fence_after();
-            issue_chunk_i8<ND>(tmem + F::ACOL, b0, tmem, kc == 0);
+            issue_products_i8<ND, 0, ND, 1>(tmem + F::ACOL, b0, tmem, kc == 0, 1u);
             mma_commit(done);
         }
         const int lbad = !mbar_wait_for(done, ph, err, wait_cycles);
@@ -779,13 +932,13 @@ __global__ void __launch_bounds__(128, 1) k_oz_selftest(int K, const double *__r
             for (int d = 0; d < ND; ++d) tmem_ld16(trow + d * OZ_NP + c, a[d]);
             tmem_wait_ld();
             for (int i = 0; i < 16; ++i) {
-                uint32_t col[ND];
-                for (int d = 0; d < ND; ++d) {
-                    reg_after_wait(a[d][i]);
-                    col[d] = a[d][i];
-                }
-                D[(size_t) tid * OZ_NP + c + i] =
-                    oz_unscaled<ND>(col) * oz_pow2(gA + fB[c + i] + F::CSHIFT);
+                const int sh = oz_sum_shift(K / OZ_KC);
+                for (int d = 0; d < ND; ++d) reg_after_wait(a[d][i]);
+                long long v = ((long long) (int) a[0][i] * 65536 + (long long) (int) a[1][i] * 256 + (int) a[2][i]) << sh;
+                v += ((long long) (int) a[3][i] * 256 + (int) a[4][i]) << (sh - 16);
+                v += sh >= 24 ? (long long) (int) a[5][i] << (sh - 24)
+                              : ((long long) (int) a[5][i] + (1 << (23 - sh))) >> (24 - sh);
+                D[(size_t) tid * OZ_NP + c + i] = oz_scaled((double) v, (gA + fB[c + i] + F::CSHIFT - sh) * (1 << 20));
             }
         }
     } else if (tid == 0) {
@@ -799,32 +952,37 @@ __global__ void __launch_bounds__(128, 1) k_oz_selftest(int K, const double *__r
     }
 }
 
-template <int ND, int NC1>
+template <int ND, int TM, int TX>
 int launch_oz(cudaStream_t s, const DevBatch &B, int nitems, const AngItem *items, const unsigned char *bop,
               double *part, int *err) {
     constexpr int smem = (int) OzK<ND>::SMEM;
     static bool attr = false;
     if (!attr) {
-        LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_angular_oz<ND, NC1>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_angular_oz<ND, TM, TX>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         attr = true;
     }
-    k_angular_oz<ND, NC1><<<nitems, OZ_T, smem, s>>>(B, items, bop, part, err);
+    k_angular_oz<ND, TM, TX><<<nitems, OZ_T, smem, s>>>(B, items, bop, part, err);
     LMIEB_CUDA_TRY(cudaGetLastError());
     return 0;
 }
 
 template <int ND>
-int launch_oz_nd1(cudaStream_t s, const DevBatch &B, int nitems, const AngItem *items, const unsigned char *bop,
-                  double *part, int *err) {
-    switch (B.nd1) {
-        case 0: return launch_oz<ND, 0>(s, B, nitems, items, bop, part, err);
-        case 1: return launch_oz<ND, 1>(s, B, nitems, items, bop, part, err);
-        case 2: return launch_oz<ND, 2>(s, B, nitems, items, bop, part, err);
-        case 3: return launch_oz<ND, 3>(s, B, nitems, items, bop, part, err);
-        case 4: return launch_oz<ND, 4>(s, B, nitems, items, bop, part, err);
+int launch_oz_basis(cudaStream_t s, const DevBatch &B, int nitems, const AngItem *items, const unsigned char *bop,
+                    double *part, int *err) {
+    if (B.nd1 > OZ_MAX_ND1 || B.nd2 > OZ_MAX_ND2) {
+        fprintf(stderr, "ERROR: lmie_b200: fixed-point angular stage built for at most %d + %d derivatives\n", OZ_MAX_ND1,
+                OZ_MAX_ND2);
+        return -1;
     }
-    fprintf(stderr, "ERROR: lmie_b200: int8 angular stage built for at most %d index1 columns\n", OZ_MAX_NC1);
-    return -1;
+    const int tx = B.t_x ? 2 : (B.oz_wl ? 1 : 0);
+    if (B.t_m) {
+        if (tx == 0) return launch_oz<ND, 1, 0>(s, B, nitems, items, bop, part, err);
+        if (tx == 1) return launch_oz<ND, 1, 1>(s, B, nitems, items, bop, part, err);
+        return launch_oz<ND, 1, 2>(s, B, nitems, items, bop, part, err);
+    }
+    if (tx == 0) return launch_oz<ND, 0, 0>(s, B, nitems, items, bop, part, err);
+    if (tx == 1) return launch_oz<ND, 0, 1>(s, B, nitems, items, bop, part, err);
+    return launch_oz<ND, 0, 2>(s, B, nitems, items, bop, part, err);
 }
 
 template <int ND>
@@ -854,8 +1012,8 @@ int launch_oz_operands(cudaStream_t s, const DevBatch &B, int digits, long long 
 int launch_angular_oz(cudaStream_t s, const DevBatch &B, int digits, int nitems, const AngItem *items,
                       const unsigned char *bop, double *part, int *err) {
     if (nitems <= 0) return 0;
-    return digits == 6 ? launch_oz_nd1<6>(s, B, nitems, items, bop, part, err)
-                       : launch_oz_nd1<7>(s, B, nitems, items, bop, part, err);
+    return digits == 6 ? launch_oz_basis<6>(s, B, nitems, items, bop, part, err)
+                       : launch_oz_basis<7>(s, B, nitems, items, bop, part, err);
 }
 
 int launch_oz_selftest(cudaStream_t s, int K, const double *A, const double *Bm, double *D, int *err,

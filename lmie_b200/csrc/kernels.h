@@ -25,8 +25,8 @@ struct GatherSeg {
 // in L1 at four blocks of 64 threads per SM (16: 3.9 ms of K1 on the
 // 4096-case batch, 8: 3.7 ms, 4: 3.7 ms).
 constexpr int K1_B = 8;
-// doubles per checkpoint block of a chunk of nc tangent-linear columns
-__host__ __device__ constexpr int k1_ck_width(int nc) { return 3 + 3 * nc; }
+// doubles per checkpoint block with the m and / or x column of the tangent basis (k_mie.cu)
+__host__ __device__ constexpr int k1_ck_width(bool hm, bool hx) { return 3 + (hm ? 2 : 0) + (hx ? 3 : 0); }
 
 // One case of a batch (device copy).  Offsets index the batch-wide arrays.
 struct DevCase {
@@ -71,6 +71,12 @@ struct DevBatch {
     const long long *k1pre;     // [ncase + 1] radii of the cases before each in that order
     const double *x;            // [R] size parameters
     const double *xl;           // [nd1][R] d x / d p for index1 slot k
+    // Tangent basis of K1's columns (k_mie.cu): index1 derivative k is
+    // m_l[k] times coefficient column t_m plus xl[k] times column t_x (0: the
+    // basis has no such column; x_own: column t_x is the only derivative's
+    // own), its sums likewise from the columns rs_m (d/dmr; rs_m + 1: d/dmi)
+    // and rs_x.
+    int t_m, t_x, x_own, rs_m, rs_x;
     const double *w;            // [(1 + nd)][R] row 0: f = nr qw; row 1+kk: f_l (index1) or f_l2 (index2)
     const int *n1r, *n2r;       // [R]
     const long long *off;       // [R+1] prefix sums of n1r (coefficient storage)
@@ -87,16 +93,17 @@ struct DevBatch {
     const int *tg_r0, *tg_n, *tg_nk;   // per group: first radius, radii, chunks of TC_KC orders
     const long long *tg_off;    // per group: float offset of its B operand block (int8 K3: byte offset)
     // int8 fixed-point K3 (oz_layout.cuh); null in the other forms
+    int oz_wl;                  // some index1 derivative moves the weights (w rows 1 + idx1 not all zero)
     const double *oz_f2;        // [OZ_KC * max chunks + 2]: (k + 1) / k
     const signed char *oz_rowexp;   // row exponents (DevCase.rx_off)
     const int *oz_colexp;       // [group][NP] column exponents
     const unsigned char *oz_aop;   // A operand digits of every angle tile (DevCase.a_off)
-    int *oz_radexp;             // [1 + nd1][R][4]: per radius, coefficient column and component, the
+    int *oz_radexp;             // [coefficient columns][R][4]: per radius, coefficient column and component, the
                                 //     largest (biased exponent + e_k) over the orders, 0 if no normal
                                 //     value (written by K1)
 };
 
-// Coefficient columns: column 0 = value, column 1+k = index1 slot k.  Entry
+// Coefficient columns: column 0 = value, then the tangent columns.  Entry
 // (col, off[r] + j - 1) holds {Re cs, Im cs, Re cd, Im cd} with
 // cs = fv4_j (a_j + b_j), cd = fv4_j (a_j - b_j).
 // Per-radius sums rs[(col*5 + q)*R + r], q: se, ss, Re sb, Im sb, sg.
@@ -108,11 +115,10 @@ int launch_gauss(cudaStream_t s, int npairs, const int *pt, const int *pi, const
                  const long long *mo, const long long *go, const double *guess, const double *jr,
                  double *pool);
 
-// K1 for one chunk of nc tangent-linear columns starting at index1 slot c0.
-// With bop set, the coefficients go to the tensor-core B operand
-// (tc_layout.cuh) instead of coef.
-int launch_coef(cudaStream_t s, const DevBatch &B, int nc, int c0, int write_value, double *ck, double *coef,
-                float *bop, double *rs);
+// K1 in the tangent basis (k_mie.cu).  With bop set, the derivatives of the
+// split-precision cases go to the tensor-core B operand (tc_layout.cuh)
+// instead of coef.
+int launch_coef(cudaStream_t s, const DevBatch &B, double *ck, double *coef, float *bop, double *rs);
 
 // K2: sums[case][(1+nd)][4] (unnormalised), save1 [4][R] for save_control 1
 int launch_reduce_scalars(cudaStream_t s, const DevBatch &B, const double *rs, double *sums, double *save1);

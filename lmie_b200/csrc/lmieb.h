@@ -44,6 +44,9 @@ typedef struct {
      const double *x;           /* [n]        size parameter 2 pi r / lambda */
      const double *xl;          /* [nd1 * n]  d x / d p for index1 slot k (row k) */
      const double *w;           /* [(1+nd)*n] row 0: f = nr qw; row 1+kk: f_l (index1) or f_l2 (index2) */
+     /* what the index1 derivatives move: some refractive index (mr_l, mi_l),
+        some size parameter (xl), some weight (w row 1 + idx1) not zero */
+     int m_tangent, x_tangent, w_tangent;
      const int *n1r;            /* [n] */
      const int *n2r;            /* [n] */
 

@@ -31,8 +31,9 @@
 //     the largest term each;
 //   - A and B digits are signed bytes; every int32 sum is exact (below
 //     7 * 128 * 128 * 5120 < 2^31 for groups of up to 5120 orders);
-//   - C = 2^(g_r + f_n - 14) sum_d 2^(-8 d) ACC_d, formed exactly in int64
-//     halves and FP64.
+//   - C = 2^(g_r + f_n - 14) sum_d 2^(-8 d) ACC_d, formed in int64 (to 2^-49 of
+//     the largest term of the longest sums, 2^-57 of the shortest) and rounded
+//     once to FP64.
 // Each product then carries ~2^-46 (six digits) or ~2^-54 (seven; FP64: 2^-53
 // and the rounding of every partial sum) of the largest term of its row and
 // column.
@@ -65,8 +66,8 @@
 constexpr int OZ_KC = 32;                            // orders per chunk (the K of one kind::i8 product)
 constexpr int OZ_M = 128;                            // product rows: 64 half-angles and their mirrors
 constexpr int OZ_HALF = OZ_M / 2;
-constexpr int OZ_MAX_NC1 = 4;                        // index1 columns the kernel is built for
-constexpr int OZ_MAX_ND2 = 3;                        // index2 slots the kernel is built for
+constexpr int OZ_MAX_ND1 = 4;                        // index1 derivatives the kernel is built for
+constexpr int OZ_MAX_ND2 = 3;                        // index2 derivatives the kernel is built for
 constexpr int OZ_MAX_NK = 160;                       // chunks per group (5120 orders: int32 sums exact)
 constexpr int OZ_MIN_N1 = 16;                        // smaller cases keep the FP64 angular stage
 
@@ -90,18 +91,28 @@ struct Oz {
     static constexpr int ACHUNK = OZ_M * AROW;            // bytes of one A chunk of an angle tile
     static constexpr int FRAC = 8 * ND - 1;               // fractional bits of the fixed-point values
     // exponent of the combination's row- and column-independent factor:
-    // V_A V_B = 2^(16 (ND - 1)) sum_d 2^(-8 d) ACC_d, and oz_unscaled returns
-    // 2^16 of that sum
+    // V_A V_B = 2^(16 (ND - 1)) sum_d 2^(-8 d) ACC_d, and the sums are kept in
+    // units of 2^-16 of that sum (times 2^oz_sum_shift)
     static constexpr int CSHIFT = 16 * (ND - 1) - 2 * FRAC - 16;
 };
+
+// Bits kept below the unit of ACC_2 in the int64 sums of a group of nk chunks:
+// |ACC_0 2^16 + ACC_1 2^8 + ACC_2| < 1.01 2^33 nk, so the sums stay below 2^63.
+__host__ __device__ inline int oz_sum_shift(int nk) {
+#ifdef __CUDA_ARCH__
+    return 29 - (32 - __clz(nk - 1));
+#else
+    return 29 - (nk > 1 ? 32 - __builtin_clz((unsigned) (nk - 1)) : 0);
+#endif
+}
 
 // the same for code that picks the format at run time
 inline int oz_np(int nd) { return nd == 6 ? Oz<6>::NP : Oz<7>::NP; }
 inline size_t oz_bstage(int nd) { return nd == 6 ? Oz<6>::BSTAGE : Oz<7>::BSTAGE; }
 inline size_t oz_achunk(int nd) { return nd == 6 ? Oz<6>::ACHUNK : Oz<7>::ACHUNK; }
 inline int oz_nprod(int nd) { return nd * (nd + 1) / 2; }
-// radii per group for nd1 index1 columns
-inline int oz_rg(int nd, int nd1) { return oz_np(nd) / 2 / (2 * (1 + nd1)); }
+// radii per group for nt tangent columns (at most 2)
+inline int oz_rg(int nd, int nt) { return oz_np(nd) / 2 / (2 * (1 + nt)); }
 
 // Bound on |beta_l(int8) - beta_l(FP64)| / (2l + 1) of the expansion
 // coefficients near the truncation threshold (|beta_l| within 1e-9 .. 1e-5 of
