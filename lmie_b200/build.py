@@ -29,6 +29,8 @@ CLI = HERE / "calllmie"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ARCH + ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
                      "--expt-relaxed-constexpr", "-diag-suppress", "177"]
+# The Mie recurrences write out their FMAs (csrc/mie_radius.cuh).
+NVCC_FILE_FLAGS = {"k_mie.cu": ["-fmad=false"], "k_noalloc.cu": ["-fmad=false"]}
 CC_FLAGS = ["-O2", "-fPIC", "-std=gnu99", "-Wall", "-Wno-unused-function"]
 
 
@@ -87,7 +89,8 @@ def build(force: bool = False, verbose: bool = False) -> Path:
             if src.suffix == ".c":
                 cmd = ["gcc"] + CC_FLAGS + ["-I", str(INCLUDE), "-c", str(src), "-o", str(obj)]
             else:
-                cmd = [nvcc] + NVCC_FLAGS + ["-I", str(INCLUDE), "-c", str(src), "-o", str(obj)]
+                cmd = ([nvcc] + NVCC_FLAGS + NVCC_FILE_FLAGS.get(src.name, []) +
+                       ["-I", str(INCLUDE), "-c", str(src), "-o", str(obj)])
             jobs.append(cmd)
     if jobs:
         with cf.ThreadPoolExecutor(max_workers=min(len(jobs), os.cpu_count() or 4)) as ex:

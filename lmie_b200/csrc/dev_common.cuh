@@ -18,7 +18,11 @@ __host__ __device__ __forceinline__ cplx operator+(cplx a, cplx b) { return mk(a
 __host__ __device__ __forceinline__ cplx operator-(cplx a, cplx b) { return mk(a.re - b.re, a.im - b.im); }
 __host__ __device__ __forceinline__ cplx operator-(cplx a) { return mk(-a.re, -a.im); }
 __host__ __device__ __forceinline__ cplx operator*(cplx a, cplx b) {
+#ifdef __CUDA_ARCH__
+    return mk(fma(a.re, b.re, -(a.im * b.im)), fma(a.re, b.im, a.im * b.re));
+#else
     return mk(a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re);
+#endif
 }
 __host__ __device__ __forceinline__ cplx operator*(cplx a, double s) { return mk(a.re * s, a.im * s); }
 __host__ __device__ __forceinline__ cplx operator*(double s, cplx a) { return mk(a.re * s, a.im * s); }
@@ -46,7 +50,11 @@ __host__ __device__ __forceinline__ cplx operator/(double s, cplx b) { return mk
 // 1/c = conj(c) / |c|^2 with one real division; for operands whose squared
 // modulus stays inside the double range (all Mie recurrence denominators do).
 __host__ __device__ __forceinline__ cplx cinv(cplx c) {
+#ifdef __CUDA_ARCH__
+    const double d = 1. / fma(c.re, c.re, c.im * c.im);
+#else
     const double d = 1. / (c.re * c.re + c.im * c.im);
+#endif
     return mk(c.re * d, -c.im * d);
 }
 __host__ __device__ __forceinline__ cplx operator/(cplx a, double s) { return mk(a.re / s, a.im / s); }

@@ -26,6 +26,7 @@
 
 #include "host_pool.h"
 #include "kernels.h"
+#include "mie_radius.cuh"
 #include "oz_layout.cuh"
 #include "tc_layout.cuh"
 #include "lmieb.h"
@@ -180,6 +181,19 @@ Ctx g_ctx;
 // uneven cases, coarser ones cut the per-item overhead; set by
 // lmieb_set_work_granularity (the autotuner).
 double g_items_per_sm[3] = {64., 2., 2.};
+
+// Whether K1 runs a block per radius (mie_radius.cuh) or a thread per radius.
+// The threads' time is that of the longest radius, about 1800 cycles an order
+// (900 without derivatives), as long as the radii do not fill the SMs; the
+// blocks' that of their rounds over the SMs, each about 30 cycles an order and
+// 4000 for the rest, at the occupancy their shared memory leaves.
+bool k1_by_block(int R, int n1max, bool hm, bool hx, bool tc, int sms) {
+    const int smem = mie_block_smem(n1max, hx);
+    if (tc || R == 0 || smem > MIE_BLOCK_SMEM) return false;
+    const int per_sm = std::min(2048 / MIE_BLOCK_T, 227 * 1024 / (smem + 1024));
+    const double rounds = std::ceil((double) R / (per_sm * sms));
+    return rounds * (30. * n1max + 4000.) < (hm ? 1800. : 900.) * n1max;
+}
 
 // Work of a sub-batch's angular sums (radii x orders x half-angles x Mie
 // columns) from which LMIEB_PRECISION_FP64 forms them with the seven-digit
@@ -794,7 +808,7 @@ size_t case_bytes(const lmieb_problem &p) {
     for (int r = 0; r < p.n; ++r) tot += p.n1r[r] + 1;
     const size_t ncol = 1 + p.nd;
     size_t b = (size_t) tot * 32 * (1 + p.nd1);                        // coef
-    b += (size_t) (tot / K1_B + p.n) * 8 * k1_ck_width(p.nd1 > 0, p.nd1 > 1);   // K1 checkpoints
+    b += (size_t) (tot / MIE_B + p.n) * 8 * k1_ck_width(p.nd1 > 0);   // K1 checkpoints
     b += (size_t) p.n * (64 + 8 * ncol + 40 * (2 + p.nd1));           // per-radius arrays, sums
     b += (size_t) 4 * ncol * p.n_qang * 8 * 8;                        // partials (groups), pf, pfn
     b += (size_t) ncol * 6 * p.n_coef * 8 * (3 + (p.n_qang / 2 + 31) / 32);   // expansion partials + outputs
@@ -848,7 +862,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         int mx = 1;
         long long a = 0, b = 0, t = 0;
         for (int i = 0; i < p.n; ++i) {
-            t += (p.n1r[i] + K1_B - 1) / K1_B;
+            t += p.n1r[i] / MIE_B + 1;
             a += p.n1r[i];
             b += p.n2r[i];
             mx = std::max(mx, p.n1r[i]);
@@ -912,7 +926,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             n1r[r] = p.n1r[i];
             o += n1r[r];
             off[r + 1] = o;
-            t += (n1r[r] + K1_B - 1) / K1_B;
+            t += n1r[r] / MIE_B + 1;
             ckoff[r + 1] = t;
         }
     });
@@ -937,7 +951,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         x_own = c.gather.x_own;
     }
     const int n_tan = (int) hm + (int) hx;                    // tangent columns of the coefficients
-    const int n_co = 1 + n_tan, n_rs = 1 + 2 * (int) hm + (int) hx, ck_w = k1_ck_width(hm, hx);
+    const int n_co = 1 + n_tan, n_rs = 1 + 2 * (int) hm + (int) hx, ck_w = k1_ck_width(hx);
     // an FP64 re-solve whose cases' K1 outputs are in an earlier sub-batch's
     // arena: their copy, in pieces of at most GATHER_PIECE doubles (one
     // block each), replaces K1
@@ -1678,6 +1692,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     B.rs_m = 1;
     B.rs_x = 1 + 2 * (int) hm;
     B.oz_wl = wl;
+    B.k1_block = k1_by_block(R, n1max, hm, hx, L.tc, c.sms);
     B.pu_lp = g_pu_lp;
     B.cs = (const DevCase *) dptr(h_cs);
     B.idx1 = (const int *) dptr(h_i1);

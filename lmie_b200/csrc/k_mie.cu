@@ -19,14 +19,16 @@
 //     W = psi_{n-1} chi_n - psi_n chi_{n-1}
 // (the quotient rule's difference of two products is this), and likewise for b
 // with c' = d(m D)/dm.  W is formed from the psi and chi at hand: it is 1, but
-// for the last orders, where the psi ratio still feels its start from zero at
-// n1, not to 1e-7, and the derivative of these a and b is wanted.
+// for the last orders, where psi still feels its start from zero at n1, not to
+// 1e-7, and the derivative of these a and b is wanted.  The recurrences and the
+// formulas of an order are in mie_radius.cuh.
 //
 // Reference: src/lmie_core.c:298-370 (psi ratio, psi, chi), 386-440 (D), 455-510
 // (a, b and tangents), 515-590 (cross-section and asymmetry sums per radius).
 #include <cstdio>
 
 #include "kernels.h"
+#include "mie_radius.cuh"
 #include "oz_layout.cuh"
 #include "tc_layout.cuh"
 
@@ -107,145 +109,118 @@ __device__ __forceinline__ void tc_flush(const float *tcbuf, float *__restrict__
     }
 }
 
-// conj(a) b
-__device__ __forceinline__ cplx cmul(cplx a, cplx b) {
-    return mk(a.re * b.re + a.im * b.im, a.re * b.im - a.im * b.re);
+// Where an order's coefficients go: the columns fv4 (a +- b) of coef, with the
+// largest exponents of each (the column exponents of the fixed-point B operand)
+// in mxe when `re` is set.
+template <bool HM, bool HX>
+__device__ __forceinline__ void put_columns(const MieAB &q, double f4, int j, double4 *cf, size_t tot, size_t at,
+                                            bool re, int (&mxe)[1 + HM + HX][4]) {
+    const int ek = oz_ek(j);
+    auto put = [&](int col, cplx va, cplx vb) {
+        const cplx cs = (va + vb) * f4, cd = (va - vb) * f4;
+        cf[(size_t) col * tot + at + j - 1] = make_double4(cs.re, cs.im, cd.re, cd.im);
+        if (re) track(mxe[col], cs, cd, ek);
+    };
+    put(0, q.a, q.b);
+    if (HM) put(1 * HM, q.am, q.bm);
+    if (HX) put((1 + HM) * HX, q.ax, q.bx);
+}
+
+// the radius of rank t in the launch order: cases in the order k1ord, each from
+// its largest radius down
+__device__ __forceinline__ int radius_of(const DevBatch &B, long long t) {
+    const int kc = find_case(B.k1pre, B.ncase, t);
+    const DevCase &C = B.cs[B.k1ord[kc]];
+    return C.r0 + C.nr - 1 - (int) (t - B.k1pre[kc]);
+}
+
+// the x column's direction: x alone, or the single derivative's own
+template <bool HX>
+__device__ __forceinline__ MieRadius<HX> radius_setup(const DevBatch &B, const DevCase &C, int r) {
+    MieRadius<HX> c;
+    double xl = 1.;
+    cplx ml = mk(0., 0.);
+    if (HX && B.x_own) {
+        xl = B.xl[r];
+        ml = B.m_l[C.ml_off + B.idx1[0]];
+    }
+    c.set(B.x[r], C.m, C.minv, xl, ml);
+    return c;
 }
 
 // ---------------------------------------------------------------------------
-// One thread per radius.  The downward recurrences -- D_n(mx) from n2 and the
-// psi ratio from n1, with their tangents -- keep only their values at the top
-// of every block of K1_B orders (checkpoints in ck); the ascending pass replays
-// each block from its checkpoint into local arrays (the same operations, so
-// the same values), runs psi and chi upward, forms a_n, b_n and their tangents,
-// writes the coefficient columns fv4 (a +- b) and sums the per-radius cross
-// sections in order.  HM, HX: with the m, the x column; TC: the split-precision
-// cases' derivatives go to the tensor-core operand instead.  Per-radius sums
-// rs[(col 5 + q) R + r], q: se, ss, Re sb, Im sb, sg, of the columns 0 value,
-// B.rs_m d/dmr, B.rs_m + 1 d/dmi (both from the m column), B.rs_x the x column.
+// One thread per radius.  The downward recurrences keep only their values at
+// the top of every block of MIE_B orders (checkpoints in ck); the ascending
+// pass replays each block from its checkpoint (the same operations, so the same
+// values), forms D_n and the orders' coefficients and tangents, writes the
+// coefficient columns and sums the per-radius cross sections in order.  HM, HX:
+// with the m, the x column; TC: the split-precision cases' derivatives go to the
+// tensor-core operand instead.  Bound by FP64 latency (a thread's chain) where
+// few radii are long, by the FP64 pipe where many fill the SMs.
+// Per-radius sums rs[(col 5 + q) R + r], q: se, ss, Re sb, Im sb, sg, of the
+// columns 0 value, B.rs_m d/dmr, B.rs_m + 1 d/dmi (both from the m column),
+// B.rs_x the x column.
 // ---------------------------------------------------------------------------
 template <bool HM, bool HX, bool TC>
 __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck, double *__restrict__ coef,
                                             float *__restrict__ bop, double *__restrict__ rs) {
-    constexpr int CW = k1_ck_width(HM, HX);       // D (2), D_m (2), ratio (1), D_x (2), ratio_x (1)
-    constexpr int QX = HM ? 5 : 3;
-    // thread t takes the radius of rank t in the launch order: cases in the
-    // order k1ord, each from its largest radius down
+    constexpr int CW = k1_ck_width(HX);              // P (4), u (2), exponent, u's tangent (2)
     const long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= B.R) return;
-    const int kc = find_case(B.k1pre, B.ncase, t);
-    const int r = [&] {
-        const DevCase &Ck = B.cs[B.k1ord[kc]];
-        return Ck.r0 + Ck.nr - 1 - (int) (t - B.k1pre[kc]);
-    }();
+    const int r = radius_of(B, t);
     const int R = B.R;
     const DevCase &C = B.cs[B.rcase[r]];
     const int n1 = B.n1r[r], n2 = B.n2r[r];
-    const double x = B.x[r];
-    const double xinv = 1. / x;
-    const cplx m = C.m, minv = C.minv;
-    const cplx z = mk(m.re * x, m.im * x);
-    const cplx zinv = cinv(z);
-    const int nb = (n1 + K1_B - 1) / K1_B;
+    const MieRadius<HX> c = radius_setup<HX>(B, C, r);
+    const int nb = n1 / MIE_B + 1;
     double *ckr = ck + (size_t) B.ckoff[r] * CW;     // nb blocks of CW doubles
-    const double *fv1 = B.fv, *fv3 = B.fv + 2 * (B.n1max + 2), *fv4 = B.fv + 3 * (B.n1max + 2);
-    // the x column's direction: x alone, or the single derivative's own
-    double xl = 1.;
-    cplx ml = mk(0., 0.), zl = mk(0., 0.);
-    if (HX) {
-        if (B.x_own) {
-            xl = B.xl[r];
-            ml = B.m_l[C.ml_off + B.idx1[0]];
-        }
-        zl = ml * x + m * xl;
-    }
+    const double *fv4 = B.fv + 3 * (B.n1max + 2);
 
-    struct Chain {
-        cplx D, Dm, Dx;
-        double rn, rx;
-    };
-    auto d_step = [&](Chain &c, int j) {
-        const cplx c1 = (j + 1.) * zinv;
-        const cplx ic2 = cinv(c.D + c1);
-        c.D = c1 - ic2;
-        if (HM || HX) {
-            const cplx c3 = -c1 * zinv;
-            const cplx ic4 = ic2 * ic2;
-            if (HM) {
-                const cplx c5 = c3 * x;              // z_m = x
-                c.Dm = c5 + (c.Dm + c5) * ic4;
-            }
-            if (HX) {
-                const cplx c5 = c3 * zl;
-                c.Dx = c5 + (c.Dx + c5) * ic4;
-            }
-        }
-    };
-    auto r_step = [&](Chain &c, int j) {
-        const double a1 = (2. * j + 1.) * xinv;
-        const double rnew = 1. / (a1 - c.rn);
-        if (HX) {
-            const double a2 = -a1 * xinv, a3 = rnew * rnew;
-            c.rx = -(a2 * xl - c.rx) * a3;
-        }
-        c.rn = rnew;
-    };
-    auto put_d = [&](const Chain &c, double *q) {
-        q[0] = c.D.re;
-        q[1] = c.D.im;
-        if (HM) {
-            q[3] = c.Dm.re;
-            q[4] = c.Dm.im;
-        }
-        if (HX) {
-            q[QX] = c.Dx.re;
-            q[QX + 1] = c.Dx.im;
-        }
-    };
-    auto put_r = [&](const Chain &c, double *q) {
-        q[2] = c.rn;
-        if (HX) q[QX + 2] = c.rx;
-    };
-    // ---- downward sweeps: checkpoints only; the two chains (D_n from n2, the
-    // psi ratio from n1 < n2) advance in one loop below n1 ----
+    // ---- downward: P from n2, u from n1 (n2 > n1 + MIE_B), block by block ----
+    double u0, ux0 = 0.;
+    int eu = 0;
     {
-        Chain c;
-        c.D = c.Dm = c.Dx = mk(0., 0.);
-        c.rn = c.rx = 0.;
-        for (int b = 0; b < nb; ++b) {
-            double *q = ckr + (size_t) b * CW;
-            if (b * K1_B + K1_B >= n2) put_d(c, q);
-            if (b * K1_B + K1_B >= n1) put_r(c, q);
+        MieP p;
+        p.hi = mk(1., 0.);                           // P_{n2} = 1, P_{n2 - 1} = n2 / z
+        p.cur = (double) n2 * c.zinv;
+        int n = n2 - 1;
+        for (const int n0 = nb * MIE_B; n >= n0; --n) {
+            p.step(p.next(n, c.zinv));
+            if (n % MIE_B == 0) p.rescale();
         }
-        auto d_down = [&](int j) {
-            d_step(c, j);
-            if (j % K1_B == 0 && j / K1_B - 1 < nb) put_d(c, ckr + (size_t) (j / K1_B - 1) * CW);
-        };
-        for (int j = n2 - 1; j >= n1; --j) d_down(j);
-        for (int j = n1 - 1; j >= 1; --j) {
-            d_down(j);
-            r_step(c, j);
-            if (j % K1_B == 0 && j / K1_B - 1 < nb) put_r(c, ckr + (size_t) (j / K1_B - 1) * CW);
+        MieU<HX> q;
+        q.start();
+        for (int b = nb - 1; b >= 0; --b) {
+            double *w = ckr + (size_t) b * CW;
+            w[0] = p.hi.re; w[1] = p.hi.im; w[2] = p.cur.re; w[3] = p.cur.im;
+            w[4] = q.hi; w[5] = q.cur; w[6] = (double) eu;
+            if (HX) { w[7] = q.xhi; w[CW - 1] = q.xcur; }
+#pragma unroll
+            for (int i = MIE_B - 1; i >= 0; --i) {
+                const int k = b * MIE_B + i;
+                if (b > 0 || i > 0) p.step(p.next(k, c.zinv));
+                if (k <= n1 && (b > 0 || i > 0)) q.step(k, c.xinv);
+            }
+            if (b > 0) {
+                p.rescale();
+                eu += q.rescale();
+            }
         }
+        u0 = q.cur;
+        if (HX) ux0 = q.xcur;
     }
 
     // ---- ascending pass ----
     double sinx, cosx;
-    sincos(x, &sinx, &cosx);
-    double psi_p = sinx, chi_p = cosx, chi_c = xinv * cosx + sinx;     // psi_0, chi_0, chi_1
-    double psix_p = 0., chix_p = 0., chix_c = 0.;
-    if (HX) {
-        psix_p = xl * cosx;
-        chix_p = xl * -sinx;
-        chix_c = (-xinv * xinv) * xl * cosx + xinv * chix_p + xl * cosx;
-    }
-    double acc[5] = {0., 0., 0., 0., 0.};
-    double accr[5] = {0., 0., 0., 0., 0.}, acci[5] = {0., 0., 0., 0., 0.};   // d/dmr, d/dmi
-    double accx[5] = {0., 0., 0., 0., 0.};
-    cplx ap = mk(0., 0.), bp = mk(0., 0.), amp = ap, bmp = ap, axp = ap, bxp = ap;
-    const cplx minv2 = minv * minv;
+    sincos(c.x, &sinx, &cosx);
+    const double spsi = sinx / u0, spsix = HX ? fma(-spsi, ux0, cosx) / u0 : 0.;
+    double chi_p = cosx, chi_c = fma(c.xinv, cosx, sinx);       // chi_0, chi_1
+    double psi_p = spsi * u0, psix_p = HX ? c.xl * fma(spsix, u0, spsi * ux0) : 0.;
+    MieSums<HM, HX> sums;
+    sums.zero();
+    MieAB prev;
+    prev.a = prev.b = prev.am = prev.bm = prev.ax = prev.bx = mk(0., 0.);
     const size_t tot = (size_t) B.tot, off = (size_t) B.off[r];
-    double4 *cf = (double4 *) coef;
     // split precision: the radii of tensor-core cases write the B operand
     const int tcode = TC ? B.tc_pos[r] : -1;
     const bool to_tc = TC && tcode >= 0;
@@ -253,190 +228,141 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     float *const tcb = to_tc ? bop + B.tc_roff[r] : nullptr;
     const int n_tc = 1 + B.nd1;
     extern __shared__ float tcbuf[];                  // [4][1 + nd1][8][blockDim.x] with TC
-    // the largest (biased exponent + e_k) of each column and component, the
-    // column exponents of the fixed-point B operand
     int *const re = B.oz_radexp;
     int mxe[1 + HM + HX][4];
 #pragma unroll
     for (int q = 0; q < 4 * (1 + HM + HX); ++q) mxe[q / 4][q % 4] = 0;
 
-    cplx Dloc[K1_B], Dmloc[HM ? K1_B : 1], Dxloc[HX ? K1_B : 1];
-    double rloc[K1_B], rxloc[HX ? K1_B : 1];
     for (int b = 0; b < nb; ++b) {
-        const int lo = b * K1_B + 1, hi = min(b * K1_B + K1_B, n1);
-        const double *q = ckr + (size_t) b * CW;
-        // replay D from the block's top (top <= n2) and the psi ratio from hi
-        // (top >= hi) down to lo: one loop below hi, as in the downward sweeps
+        const double *w = ckr + (size_t) b * CW;
+        cplx D[MIE_B], Dz[MIE_B];
+        double ub[MIE_B], uxb[HX ? MIE_B : 1];
+        const double su = mb_pow2((int) w[6] - eu);
         {
-            const int top = min(b * K1_B + K1_B, n2);
-            Chain c;
-            c.D = mk(q[0], q[1]);
-            c.rn = q[2];
-            c.Dm = HM ? mk(q[3], q[4]) : mk(0., 0.);
-            c.Dx = HX ? mk(q[QX], q[QX + 1]) : mk(0., 0.);
-            c.rx = HX ? q[QX + 2] : 0.;
-            auto keep_d = [&](int j) {
-                Dloc[j - lo] = c.D;
-                if (HM) Dmloc[j - lo] = c.Dm;
-                if (HX) Dxloc[j - lo] = c.Dx;
-            };
-            auto keep_r = [&](int j) {
-                rloc[j - lo] = c.rn;
-                if (HX) rxloc[j - lo] = c.rx;
-            };
-            if (top <= hi) keep_d(top);
-            keep_r(hi);
-            for (int j = top - 1; j >= hi; --j) {
-                d_step(c, j);
-                if (j <= hi) keep_d(j);
-            }
-            for (int j = hi - 1; j >= lo; --j) {
-                d_step(c, j);
-                keep_d(j);
-                r_step(c, j);
-                keep_r(j);
-            }
-        }
-        for (int j = lo; j <= hi; ++j) {
-            const double rj = rloc[j - lo];
-            const double psi = rj * psi_p;
-            const cplx D = Dloc[j - lo];
-            const cplx zeta = mk(psi, chi_c), zeta_p = mk(psi_p, chi_p);
-            const double tt = j * xinv;
-            const cplx ca = D * minv + tt;
-            const cplx na = ca * psi - psi_p;
-            const cplx ida = cinv(ca * zeta - zeta_p);
-            const cplx a = na * ida;
-            const cplx cb = m * D + tt;
-            const cplx nbq = cb * psi - psi_p;
-            const cplx idb = cinv(cb * zeta - zeta_p);
-            const cplx bb = nbq * idb;
-            const cplx ida2 = ida * ida, idb2 = idb * idb;
-            cplx am = ap, bm = ap, ax = ap, bx = ap;
-            if (HM) {
-                const cplx Dm = Dmloc[j - lo];
-                const cplx da = (Dm * minv - D * minv2) * ida2, db = (D + m * Dm) * idb2;
-                const double W = psi_p * chi_c - psi * chi_p;
-                am = mk(-W * da.im, W * da.re);      // i W da
-                bm = mk(-W * db.im, W * db.re);
-            }
-            double psix = 0.;
-            if (HX) {
-                psix = rxloc[j - lo] * psi_p + rj * psix_p;
-                const cplx Dx = Dxloc[j - lo];
-                const cplx zetal = mk(psix, chix_c), zetal_p = mk(psix_p, chix_p);
-                const double tl = -tt * xinv * xl;
-                const cplx c6 = Dx * minv - D * minv2 * ml + tl;
-                ax = (c6 * psi + ca * psix - psix_p) * ida - na * ((c6 * zeta + ca * zetal - zetal_p) * ida2);
-                const cplx c4 = ml * D + m * Dx + tl;
-                bx = (c4 * psi + cb * psix - psix_p) * idb - nbq * ((c4 * zeta + cb * zetal - zetal_p) * idb2);
-            }
-            // sums of order j, and the asymmetry term of order j - 1 (it needs a_j, b_j)
-            const double f1 = fv1[j], f4 = fv4[j];
-            const double f3p = j >= 2 ? fv3[j - 1] : 0., f4p = j >= 2 ? fv4[j - 1] : 0.;
-            const double sgn = (j & 1) ? -1. : 1.;
-            acc[0] += f1 * (a.re + bb.re);
-            acc[1] += f1 * (norm2(a) + norm2(bb));
-            acc[2] += f1 * sgn * (a.re - bb.re);
-            acc[3] += f1 * sgn * (a.im - bb.im);
-            if (j >= 2) acc[4] += f3p * (re_mulc(ap, a) + re_mulc(bp, bb)) + f4p * re_mulc(ap, bp);
-            if (HM) {
-                // complex derivatives: the real part is d/dmr, the imaginary part d/dmi
-                const cplx s = am + bm, d = am - bm, q2 = cmul(a, am) + cmul(bb, bm);
-                accr[0] += f1 * s.re;
-                acci[0] += f1 * s.im;
-                accr[1] += f1 * 2. * q2.re;
-                acci[1] += f1 * 2. * q2.im;
-                accr[2] += f1 * sgn * d.re;
-                accr[3] += f1 * sgn * d.im;
-                if (j >= 2) {
-                    const cplx g3 = cmul(a, amp) + cmul(ap, am) + cmul(bb, bmp) + cmul(bp, bm);
-                    const cplx g4 = cmul(bp, amp) + cmul(ap, bmp);
-                    accr[4] += f3p * g3.re + f4p * g4.re;
-                    acci[4] += f3p * g3.im + f4p * g4.im;
+            MieP p;
+            p.hi = mk(w[0], w[1]);
+            p.cur = mk(w[2], w[3]);
+            MieU<HX> q;
+            q.hi = w[4];
+            q.cur = w[5];
+            if (HX) { q.xhi = w[7]; q.xcur = w[CW - 1]; }
+#pragma unroll
+            for (int i = MIE_B - 1; i >= 0; --i) {
+                const int k = b * MIE_B + i;
+                ub[i] = q.cur;
+                if (HX) uxb[HX ? i : 0] = q.xcur;
+                if (k > 0) {
+                    const cplx lo = p.next(k, c.zinv);
+                    if (k <= n1) {
+                        mie_d<HM || HX>(c, k, lo, p.cur, p.hi, D[i], Dz[i]);
+                        q.step(k, c.xinv);
+                    }
+                    p.step(lo);
                 }
             }
-            if (HX) {
-                accx[0] += f1 * (ax.re + bx.re);
-                accx[1] += f1 * 2. * (re_mulc(a, ax) + re_mulc(bb, bx));
-                accx[2] += f1 * sgn * (ax.re - bx.re);
-                accx[3] += f1 * sgn * (ax.im - bx.im);
-                if (j >= 2)
-                    accx[4] += f3p * (re_mulc(axp, a) + re_mulc(ap, ax) + re_mulc(bxp, bb) + re_mulc(bp, bx)) +
-                               f4p * (re_mulc(axp, bp) + re_mulc(ap, bxp));
-            }
-            // coefficient columns of order j
-            const int ek = oz_ek(j);
-            auto put = [&](int col, cplx va, cplx vb) {
-                const cplx cs = (va + vb) * f4, cd = (va - vb) * f4;
-                cf[(size_t) col * tot + off + j - 1] = make_double4(cs.re, cs.im, cd.re, cd.im);
-                if (re) track(mxe[col], cs, cd, ek);
-            };
+        }
+#pragma unroll
+        for (int i = 0; i < MIE_B; ++i) {
+            const int j = b * MIE_B + i;
+            if (j < 1 || j > n1) continue;
+            const double psi = spsi * ub[i] * su, psix = HX ? c.xl * (fma(spsix, ub[i], spsi * uxb[HX ? i : 0]) * su) : 0.;
+            const MieAB q = mie_ab<HM, HX>(c, j, D[i], Dz[i], psi, psi_p, chi_c, chi_p, psix, psix_p);
+            sums.add(j, q, prev);
+            const double f4 = fv4[j];
             if (to_tc) {
-                tc_stage(tcbuf, n_tc, j, 0, (a + bb) * f4, (a - bb) * f4);
+                tc_stage(tcbuf, n_tc, j, 0, (q.a + q.b) * f4, (q.a - q.b) * f4);
                 for (int k = 0; k < B.nd1; ++k) {
                     cplx va = mk(0., 0.), vb = va;
                     if (HM) {
-                        const cplx mk_ = B.m_l[C.ml_off + B.idx1[k]];
-                        va = mk_ * am;
-                        vb = mk_ * bm;
+                        const cplx ml = B.m_l[C.ml_off + B.idx1[k]];
+                        va = ml * q.am;
+                        vb = ml * q.bm;
                     }
                     if (HX) {
                         const double xc = B.x_own ? 1. : B.xl[(size_t) k * R + r];
-                        va = va + ax * xc;
-                        vb = vb + bx * xc;
+                        va = cfma(q.ax, xc, va);
+                        vb = cfma(q.bx, xc, vb);
                     }
                     tc_stage(tcbuf, n_tc, j, 1 + k, (va + vb) * f4, (va - vb) * f4);
                 }
                 if (((j - 1) & 3) == 3 || j == n1) tc_flush(tcbuf, tcb, n_tc, j, tpos, j == n1 ? tgnk : 0);
             } else {
-                put(0, a, bb);
-                if (HM) put(1, am, bm);
-                if (HX) put(1 + HM, ax, bx);
+                put_columns<HM, HX>(q, f4, j, (double4 *) coef, tot, off, re != nullptr, mxe);
             }
-            // upward: chi_{j+1} and its tangent; shift the previous order
-            const double a1 = (2. * j + 1.) * xinv;
-            const double chi_n = a1 * chi_c - chi_p;
-            if (HX) {
-                const double a2l = -a1 * xl * xinv;
-                const double chix_n = a2l * chi_c + a1 * chix_c - chix_p;
-                chix_p = chix_c;
-                chix_c = chix_n;
-                psix_p = psix;
-                axp = ax;
-                bxp = bx;
-            }
+            const double chi_n = fma((2. * j + 1.) * c.xinv, chi_c, -chi_p);
             chi_p = chi_c;
             chi_c = chi_n;
             psi_p = psi;
-            ap = a;
-            bp = bb;
-            amp = am;
-            bmp = bm;
+            psix_p = psix;
+            prev = q;
         }
     }
-    auto put_sums = [&](int col, const double (&v)[5]) {
+    sums.close();
 #pragma unroll
-        for (int q = 0; q < 5; ++q) rs[((size_t) col * 5 + q) * R + r] = v[q];
-    };
-    put_sums(0, acc);
-    if (HM) {
-        // sb is complex itself: its derivative w.r.t. mi is -i times the one w.r.t. mr
-        acci[2] = accr[3];
-        acci[3] = -accr[2];
-        put_sums(1, accr);
-        put_sums(2, acci);
-    }
-    if (HX) put_sums(1 + 2 * HM, accx);
+    for (int q = 0; q < MieSums<HM, HX>::N; ++q) rs[(size_t) q * R + r] = sums.v[q];
     if (re) {
 #pragma unroll
-        for (int c = 0; c < 1 + HM + HX; ++c)
-            *(int4 *) (re + ((size_t) c * R + r) * 4) = make_int4(mxe[c][0], mxe[c][1], mxe[c][2], mxe[c][3]);
+        for (int k = 0; k < 1 + HM + HX; ++k)
+            *(int4 *) (re + ((size_t) k * R + r) * 4) = make_int4(mxe[k][0], mxe[k][1], mxe[k][2], mxe[k][3]);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// K1 for few radii: a block per radius.
+// ---------------------------------------------------------------------------
+template <bool HM, bool HX>
+__global__ void __launch_bounds__(MIE_BLOCK_T) k_mie_block(DevBatch B, double *__restrict__ coef,
+                                                           double *__restrict__ rs) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int r = radius_of(B, blockIdx.x), R = B.R;
+    const MieRadius<HX> c = radius_setup<HX>(B, B.cs[B.rcase[r]], r);
+    const double *fv4 = B.fv + 3 * (B.n1max + 2);
+    const size_t tot = (size_t) B.tot, off = (size_t) B.off[r];
+    const bool re = B.oz_radexp != nullptr;
+    constexpr int NC = 1 + HM + HX;
+    int mxe[NC][4];
+#pragma unroll
+    for (int q = 0; q < 4 * NC; ++q) mxe[q / 4][q % 4] = 0;
+    MieSums<HM, HX> sums;
+    mie_block<HM, HX>(smem, c, B.n1r[r], B.n2r[r], B.n1max, sums, [&](int j, const MieAB &q) {
+        put_columns<HM, HX>(q, fv4[j], j, (double4 *) coef, tot, off, re, mxe);
+    });
+    if (threadIdx.x == 0)
+#pragma unroll
+        for (int q = 0; q < MieSums<HM, HX>::N; ++q) rs[(size_t) q * R + r] = sums.v[q];
+    if (re) {
+        // the largest exponents of the block
+        __shared__ int mx[MIE_BLOCK_T / 32][4 * NC];
+#pragma unroll
+        for (int q = 0; q < 4 * NC; ++q) {
+            const int v = __reduce_max_sync(0xffffffffu, mxe[q / 4][q % 4]);
+            if ((threadIdx.x & 31) == 0) mx[threadIdx.x >> 5][q] = v;
+        }
+        __syncthreads();
+        if (threadIdx.x < 4 * NC) {
+            int v = 0;
+            for (int w = 0; w < MIE_BLOCK_T / 32; ++w) v = max(v, mx[w][threadIdx.x]);
+            B.oz_radexp[((size_t) (threadIdx.x / 4) * R + r) * 4 + threadIdx.x % 4] = v;
+        }
     }
 }
 
 template <bool HM, bool HX>
+int launch_block(cudaStream_t s, const DevBatch &B, double *coef, double *rs) {
+    static bool attr = false;
+    if (!attr) {
+        LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_mie_block<HM, HX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            MIE_BLOCK_SMEM));
+        attr = true;
+    }
+    k_mie_block<HM, HX><<<B.R, MIE_BLOCK_T, mie_block_smem(B.n1max, HX), s>>>(B, coef, rs);
+    LMIEB_CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+
+template <bool HM, bool HX>
 int launch(cudaStream_t s, const DevBatch &B, double *ck, double *coef, float *bop, double *rs) {
+    if (B.k1_block) return launch_block<HM, HX>(s, B, coef, rs);
     if (bop)
         k_mie<HM, HX, true><<<ceil_div(B.R, 64), 64, 4 * 8 * (1 + B.nd1) * 64 * sizeof(float), s>>>(B, ck, coef, bop, rs);
     else

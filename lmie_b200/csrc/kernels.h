@@ -20,13 +20,9 @@ struct GatherSeg {
     long long dst_off, n;
     int which;
 };
-// K1 keeps its downward recurrences at the top of every block of K1_B orders
-// and replays a block into per-thread arrays of K1_B entries: with 8 they stay
-// in L1 at four blocks of 64 threads per SM (16: 3.9 ms of K1 on the
-// 4096-case batch, 8: 3.7 ms, 4: 3.7 ms).
-constexpr int K1_B = 8;
-// doubles per checkpoint block with the m and / or x column of the tangent basis (k_mie.cu)
-__host__ __device__ constexpr int k1_ck_width(bool hm, bool hx) { return 3 + (hm ? 2 : 0) + (hx ? 3 : 0); }
+// doubles per K1 checkpoint (k_mie.cu; one per MIE_B orders), hx: with the x
+// column of the tangent basis
+__host__ __device__ constexpr int k1_ck_width(bool hx) { return hx ? 9 : 7; }
 
 // One case of a batch (device copy).  Offsets index the batch-wide arrays.
 struct DevCase {
@@ -77,10 +73,11 @@ struct DevBatch {
     // own), its sums likewise from the columns rs_m (d/dmr; rs_m + 1: d/dmi)
     // and rs_x.
     int t_m, t_x, x_own, rs_m, rs_x;
+    int k1_block;               // K1: a block per radius (mie_radius.cuh) instead of a thread
     const double *w;            // [(1 + nd)][R] row 0: f = nr qw; row 1+kk: f_l (index1) or f_l2 (index2)
     const int *n1r, *n2r;       // [R]
     const long long *off;       // [R+1] prefix sums of n1r (coefficient storage)
-    const long long *ckoff;     // [R+1] prefix sums of ceil(n1r / K1_B) (K1 checkpoint blocks)
+    const long long *ckoff;     // [R+1] prefix sums of n1r / MIE_B + 1 (K1 checkpoint blocks)
     long long tot, ckn;
     const double *fv;           // [4][n1max + 2]: fv1 | fv2 | fv3 | fv4
     const double *rc;           // [8 * ncmax] GSF/Legendre recurrence coefficients per order
