@@ -16,12 +16,18 @@
 //   - k_angular_oz: a block owns one angle tile of one case and a range of its
 //     radius groups; per group, chunks of OZ_KC orders flow through the
 //     pipeline:
-//       * warps 0-3 and 4-7 (one thread per row, the row's tensor-memory
-//         lane), alternate chunks each, load the chunk's A digit slices of
-//         their row -- formed once per (case, angle tile, chunk) by k_oz_aop
-//         -- and store them into the A stage in tensor memory;
-//       * lane 0 of warp 14 brings the group's B chunks into shared memory with
-//         bulk copies running ahead of the products;
+//       * lane 0 of warp 14 brings the chunks' A digit slices -- formed once per
+//         (case, angle tile, chunk) by k_oz_aop -- and the group's B chunks into
+//         shared memory with bulk copies running ahead of the products;
+//       * warps 16-19 (one thread per row, the row's tensor-memory lane) store
+//         A from there into its stage in tensor memory.  (Loads of A by these
+//         threads hold an SM to what they keep in flight: 31 bytes per cycle,
+//         1.6K cycles for a chunk of uneven batches, whose products take 0.7K.
+//         tcgen05.cp from shared memory takes its time from the products, 7 x
+//         34 cycles per chunk; these stores do not.  Six digits, 1000 cases
+//         without index1 derivatives: 1262 us with loads, 987 with
+//         tcgen05.cp, 834 this way; seven digits, 900 cases, one: 3193, 2351,
+//         2006.);
 //       * warps 12 and 13 issue the digit products of a chunk (21 or 28),
 //         tcgen05.mma kind::i8 with A in tensor memory and B in shared memory
 //         (M 128, N NP, K 32, int32 accumulation in tensor memory), one
@@ -75,9 +81,13 @@
 
 namespace {
 
-constexpr int OZ_T = 480;                     // warps 0-7: A stages and sums (0-3 D', 4-7 S);
-                                              // 8-11: quadratic forms; 12, 13: products; 14: B copies
-constexpr int OZ_QUAD_WARP = 8, OZ_MMA_WARP = 12, OZ_COPY_WARP = 14;
+constexpr int OZ_T = 640;                     // warps 0-7: sums (0-3 D', 4-7 S); 8-11: quadratic forms;
+                                              // 12, 13: products; 14: operand copies; 16-19: A stages
+constexpr int OZ_QUAD_WARP = 8, OZ_MMA_WARP = 12, OZ_COPY_WARP = 14, OZ_STAGE_WARP = 16;
+// Registers a thread of each group of four warps: 96 at launch (640 threads),
+// then 2 x 128 + 144 + 2 x 40 = 5 x 96.
+constexpr int OZ_REG_SUMS = 128, OZ_REG_QUAD = 144, OZ_REG_REST = 40;
+static_assert(2 * OZ_REG_SUMS + OZ_REG_QUAD + 2 * OZ_REG_REST <= 5 * 96, "no more registers than at launch");
 constexpr uint32_t OZ_TMEM_COLS = 512;
 
 // sizes and shared-memory offsets of the product kernel
@@ -88,9 +98,10 @@ struct OzK : Oz<ND> {
     static constexpr int MAX_W = 128;                                  // weights of a group: one per thread
     static constexpr uint32_t ACOLS = ND * OZ_KC / 4;                  // tensor-memory columns of an A stage
     static constexpr uint32_t ACOL = ND * F::NP;                       // first A stage column
-    // barriers: afull[BSLOTS], bfull[BSLOTS], done[BSLOTS], accfull[3], accfree[3], hready[2], hfree[2], fin
-    static constexpr int NBAR = 3 * F::BSLOTS + 11;
-    static constexpr uint32_t RING = F::BSLOTS * F::BSTAGE;
+    // barriers: afull[BSLOTS], bfull[BSLOTS], done[BSLOTS], ain[ASLOTS], accfull[3], accfree[3], hready[2],
+    // hfree[2], fin
+    static constexpr int NBAR = 3 * F::BSLOTS + F::ASLOTS + 11;
+    static constexpr uint32_t O_ARING = F::BSLOTS * F::BSTAGE, RING = O_ARING + F::ASLOTS * F::ACHUNK;
     static constexpr int HB = F::NP * OZ_M;                            // doubles of one sums buffer
     static constexpr uint32_t HBUF = 2 * HB * 8;                       // two groups' sums, unscaled, [column][row]
     static constexpr uint32_t WBUF = MAX_W * 8;                        // a group's radius weights
@@ -101,6 +112,7 @@ struct OzK : Oz<ND> {
     static_assert(F::BSTAGE % 128 == 0 && O_HBUF % 128 == 0, "B stages and sums start on 128-byte boundaries");
     static_assert(F::NP % 16 == 0 && F::NP >= 16 && F::NP <= 256, "N of an M=128 kind::i8 product");
     static_assert(ACOL + F::ASTAGES * ACOLS <= OZ_TMEM_COLS, "accumulators and A stages in tensor memory");
+    static_assert(F::ASTAGES <= F::BSLOTS && F::ASLOTS <= F::BSLOTS, "a chunk's barriers outlive its stages");
     static_assert(WBUF % 16 == 0 && CBUF % 16 == 0, "barriers stay 8-byte aligned");
     static_assert(SMEM <= 227 * 1024, "shared memory per block");
     // weights per radius: value, index2, and with tangent columns index1 (twice with the x column)
@@ -113,6 +125,17 @@ struct OzK : Oz<ND> {
 // instruction descriptor of kind::i8: D int32, A and B signed 8-bit, both K-major
 __host__ __device__ constexpr uint32_t idesc_i8(int m, int n) {
     return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t) (n >> 3) << 17) | ((uint32_t) (m >> 4) << 24);
+}
+
+// The registers a thread of the caller's four warps (a multiple of four) may
+// use from here on.
+template <int N>
+__device__ __forceinline__ void reg_inc() {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void reg_dec() {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
 // lane 0's value, which the compiler then knows to be the same in the whole
@@ -157,16 +180,6 @@ __device__ __forceinline__ void mma_commit_on(uint32_t bar, uint32_t on) {
         "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(bar),
         "r"(on)
         : "memory");
-}
-
-// 16 bytes that this block reads once: not kept in L1, whose data array the
-// B operand and the sums share
-__device__ __forceinline__ uint4 ld_once(const uint4 *p) {
-    uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
-                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                 : "l"(p));
-    return v;
 }
 
 // warp-wide: four consecutive 32-bit columns of this thread's lane
@@ -439,7 +452,7 @@ __global__ void __launch_bounds__(128) k_oz_aop(DevBatch B, long long total, con
     }
 }
 
-// barrier 2 over the 128 threads of warps 4-7, OR-reducing v
+// barrier 2 over the 128 threads of warps 8-11, OR-reducing v
 __device__ __forceinline__ int oz_epi_sync_or(int v) {
     uint32_t r;
     asm volatile(
@@ -465,7 +478,7 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
     using F = OzK<ND>;
     constexpr int NT = TM + (TX == 2), CPR = 2 * (1 + NT);   // columns of each half per radius
     constexpr int OZ_NP = F::NP, OZ_NHALF = F::NHALF, OZ_MAX_GN = F::MAX_GN, OZ_HB = F::HB;
-    constexpr int OZ_ASTAGES = F::ASTAGES, OZ_BSLOTS = F::BSLOTS, OZ_NBAR = F::NBAR;
+    constexpr int OZ_ASTAGES = F::ASTAGES, OZ_BSLOTS = F::BSLOTS, OZ_ASLOTS = F::ASLOTS, OZ_NBAR = F::NBAR;
     constexpr uint32_t OZ_ACOL = F::ACOL, OZ_ACOLS = F::ACOLS, OZ_BSTAGE = F::BSTAGE, OZ_ACHUNK = F::ACHUNK;
     extern __shared__ __align__(1024) unsigned char smem[];
     double *hbuf = (double *) (smem + F::O_HBUF);            // [2][OZ_NP][OZ_M] sums of a group, unscaled
@@ -474,10 +487,12 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
     uint64_t *bars = (uint64_t *) (smem + F::O_BARS);
     uint32_t *tmem_hold = (uint32_t *) (bars + OZ_NBAR);
     const uint32_t bring = smem_u32(smem);
-    // chunk q's operands are in place: afull[q % BSLOTS] (the A set's 128 threads), bfull[q % BSLOTS] (the
-    // B copy); its products have completed: done[q % BSLOTS] (both issuing warps)
+    // chunk q: its A digits are in shared memory, ain[q % ASLOTS], and in tensor memory, afull[q % BSLOTS] (the
+    // shared slot is then free again); its B digits are in shared memory, bfull[q % BSLOTS]; its products have
+    // completed, done[q % BSLOTS] (both issuing warps)
     const uint32_t afull0 = smem_u32(bars), bfull0 = afull0 + 8 * OZ_BSLOTS, done0 = bfull0 + 8 * OZ_BSLOTS;
-    const uint32_t accfull0 = done0 + 8 * OZ_BSLOTS, accfree0 = accfull0 + 8 * OZ_NPH;
+    const uint32_t ain0 = done0 + 8 * OZ_BSLOTS;
+    const uint32_t accfull0 = ain0 + 8 * OZ_ASLOTS, accfree0 = accfull0 + 8 * OZ_NPH;
     const uint32_t hready0 = accfree0 + 8 * OZ_NPH, hfree0 = hready0 + 16, fin = hfree0 + 16;
 
     const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
@@ -497,6 +512,7 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
             mbar_init(bfull0 + 8 * i, 1);
             mbar_init(done0 + 8 * i, 2);
         }
+        for (int i = 0; i < OZ_ASLOTS; ++i) mbar_init(ain0 + 8 * i, 1);
         for (int i = 0; i < OZ_NPH; ++i) {
             mbar_init(accfull0 + 8 * i, 2);
             mbar_init(accfree0 + 8 * i, 256);
@@ -516,85 +532,31 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
     int bad = 0;
 
     if (warp < OZ_QUAD_WARP) {
-        // ---------------- warps 0-7: A digit slices and the groups' sums, one row (lane) per thread ----------------
-        // Two sets of four warps.  The sets bring alternate chunks of A: a
-        // chunk's loads take 1-2 chunks' time (L2), so one set alone, loading
-        // a chunk while it waits to store it, was what limited the products.
-        // Set 0 takes the D' columns of a group's sums out of tensor memory,
-        // set 1 the S columns.
+        reg_inc<OZ_REG_SUMS>();
+        // ---------------- warps 0-7: the groups' sums, one row (lane) per thread ----------------
+        // Warps 0-3 take the D' columns of a group's sums out of tensor memory,
+        // warps 4-7 the S columns, and, once the quadratic forms are done with
+        // the buffer's previous group, into the buffer.
         const int set = warp >> 2, row = tid & (OZ_M - 1);
-        const uint32_t tlane = tmem + ((uint32_t) ((warp & 3) * 32) << 16);
         const int hcol = set == 0 ? OZ_NHALF : 0;            // first column of the set's half
-        // this row's A digit slices: piece i of chunk kc of the item's angle
-        // tile at arow[kc OZ_ACHUNK / 16 + i OZ_M]
-        const uint4 *arow = (const uint4 *) (B.oz_aop + C.a_off + (size_t) it.xt * C.nkx * OZ_ACHUNK) + row;
-        // Takes the set's half of a group's sums out of tensor memory and, once
-        // the quadratic forms are done with the buffer's previous group, into
-        // the buffer.  Returns nonzero when a wait gave up.
-        auto take = [&](int gh) -> int {
+        const uint32_t taddr = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + hcol;
+        int nk = it.rbeg < it.rend ? B.tg_nk[it.rbeg] : 1, gi = 0;
+        for (int g = it.rbeg; g < it.rend; ++g, ++gi) {
+            const int sh = oz_sum_shift(nk), b = gi & 1;
+            if (g + 1 < it.rend) nk = B.tg_nk[g + 1];
             long long V[OZ_NHALF];
-            if (oz_take<ND>(tlane + hcol, oz_sum_shift(B.tg_nk[it.rbeg + gh]), V, accfull0, accfree0, gh & 1, err))
-                return 1;
-            // the buffer's previous group (gh - 2) has been through the quadratic forms
-            const int b = gh & 1;
-            if (__any_sync(0xffffffffu, gh >= 2 && !mbar_wait(hfree0 + 8 * b, ((gh >> 1) - 1) & 1, err))) return 1;
+            if (oz_take<ND>(taddr, sh, V, accfull0, accfree0, gi & 1, err) ||
+                __any_sync(0xffffffffu, gi >= 2 && !mbar_wait(hfree0 + 8 * b, ((gi >> 1) - 1) & 1, err))) {
+                bad = 1;
+                break;
+            }
             double *hb = hbuf + b * OZ_HB + hcol * OZ_M + row;
 #pragma unroll
             for (int i = 0; i < OZ_NHALF; ++i) hb[i * OZ_M] = (double) V[i];
             mbar_arrive(hready0 + 8 * b);
-            return 0;
-        };
-        int q = 0, gi = 0, hold_next = 0;
-        // groups to be out before a stage is written again: those before its
-        // previous chunk's group, and that group itself when the chunk ended
-        // it.  need[i]: of the chunk i + 1 before this one.
-        int need[OZ_ASTAGES];
-#pragma unroll
-        for (int i = 0; i < OZ_ASTAGES; ++i) need[i] = 0;
-        for (int g = it.rbeg; g < it.rend && !bad; ++g, ++gi) {
-            const int nk = B.tg_nk[g];
-            for (int kc = 0; kc < nk; ++kc, ++q) {
-                if ((q & 1) == set) {
-                    const int s = q % OZ_ASTAGES;
-                    // the chunk's digit slices of this row, loaded before the waits
-                    const uint4 *ac = arow + (size_t) kc * (OZ_ACHUNK / 16);
-                    uint4 a[2 * ND];
-#pragma unroll
-                    for (int i = 0; i < 2 * ND; ++i) a[i] = ld_once(ac + i * OZ_M);
-                    // The stage's previous chunk must have been consumed by its products,
-                    // which reach its group once the sums of every earlier group are out
-                    // (its own group's sums are taken first when they complete with it, so
-                    // that the next group's products are not kept waiting).  Neither set
-                    // waits for the other: the set with the earlier chunk has taken what
-                    // that chunk's products need, and the other one no less.
-                    // Warp-uniform decisions: the tensor-memory accesses are warp-wide.
-                    while (!bad && hold_next < need[OZ_ASTAGES - 1]) bad = take(hold_next++);
-                    if (bad) break;
-                    const int qp = q - OZ_ASTAGES;
-                    const bool ok = qp < 0 || mbar_wait(done0 + 8 * (qp % OZ_BSLOTS), (qp / OZ_BSLOTS) & 1, err);
-                    if (__any_sync(0xffffffffu, !ok)) {
-                        bad = 1;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t acol = tlane + OZ_ACOL + s * OZ_ACOLS;
-#pragma unroll
-                    for (int sl = 0; sl < ND; ++sl) {
-                        tmem_st4(acol + sl * (OZ_KC / 4), a[2 * sl].x, a[2 * sl].y, a[2 * sl].z, a[2 * sl].w);
-                        tmem_st4(acol + sl * (OZ_KC / 4) + 4, a[2 * sl + 1].x, a[2 * sl + 1].y, a[2 * sl + 1].z,
-                                 a[2 * sl + 1].w);
-                    }
-                    tmem_wait_st();
-                    tc_fence_before();
-                    mbar_arrive(afull0 + 8 * (q % OZ_BSLOTS));
-                }
-#pragma unroll
-                for (int i = OZ_ASTAGES - 1; i > 0; --i) need[i] = need[i - 1];
-                need[0] = kc == nk - 1 ? gi + 1 : gi;
-            }
         }
-        while (!bad && hold_next < it.rend - it.rbeg) bad = take(hold_next++);
     } else if (warp < OZ_MMA_WARP) {
+        reg_inc<OZ_REG_QUAD>();
         // ---------------- warps 8-11: quadratic forms, one row per thread ----------------
         // A warp whose wait fails keeps taking the barriers of the four warps,
         // which stop together.
@@ -667,6 +629,7 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
             // (|sp|^2 and its tangents) carries rsc^2, of an invariant 1 rsp^2
             // and of the others rsc rsp (powers of two, applied once at the
             // end).
+#pragma unroll (TM ? 2 : 4)
             for (int p = 0; p < gn; ++p) {
                 // columns of S (i < CPR, this row) and D' (i >= CPR, the pair row: sm)
                 double v[2 * CPR];
@@ -767,66 +730,110 @@ __global__ void __launch_bounds__(OZ_T, 1) k_angular_oz(DevBatch B, const AngIte
                     put(1 + B.idx1[k], d);
                 }
         }
-    } else if (warp == OZ_COPY_WARP) {
-        // ---------------- warp 14, lane 0: B copies, up to OZ_BSLOTS chunks ahead ----------------
-        if ((tid & 31) == 0) {
-            int pq = 0;
-            for (int g = it.rbeg; g < it.rend && !bad; ++g) {
-                const int nk = B.tg_nk[g];
-                const unsigned char *src = bop + B.tg_off[g];
-                for (int kc = 0; kc < nk; ++kc, ++pq) {
-                    const int ps = pq % OZ_BSLOTS;
-                    // the slot's previous chunk pq - OZ_BSLOTS must have been consumed
-                    if (pq >= OZ_BSLOTS && !mbar_wait(done0 + 8 * ps, ((pq / OZ_BSLOTS) - 1) & 1, err)) {
-                        bad = 1;
-                        break;
-                    }
-                    mbar_expect_tx(bfull0 + 8 * ps, OZ_BSTAGE);
-                    bulk_g2s(bring + ps * OZ_BSTAGE, src, OZ_BSTAGE, bfull0 + 8 * ps);
-                    src += OZ_BSTAGE;
-                }
-            }
-            // the copies in flight land before the block ends
-            const int q0 = pq > OZ_BSLOTS ? pq - OZ_BSLOTS : 0;
-            for (int c = q0; c < pq; ++c) mbar_wait(bfull0 + 8 * (c % OZ_BSLOTS), (c / OZ_BSLOTS) & 1, nullptr);
-        }
-    } else {
-        // ---------------- warps 12, 13: the products of the even / odd diagonals ----------------
-        // The whole warp runs the loop and one elected lane issues; the decisions
-        // to stop are warp-uniform, and so is, visibly to the compiler, what
-        // the products' operands are made of: they are taken from uniform
-        // registers, and moving each operand of each product there costs more
-        // than the product takes.
-        const uint32_t tm = warp_uniform(tmem), b0 = warp_uniform(bring);
-        const int rend = warp_uniform(it.rend);
-        const uint32_t on = elect_one();
-        int q = 0, gi = 0;
-        for (int g = warp_uniform(it.rbeg); g < rend && !bad; ++g, ++gi) {
-            const int nk = warp_uniform(B.tg_nk[g]);
+    } else if (warp >= OZ_STAGE_WARP) {
+        reg_dec<OZ_REG_REST>();
+        // ---------------- warps 16-19: A stages, from shared to tensor memory, one row (lane) per thread ----------------
+        const int row = tid & (OZ_M - 1);
+        const uint32_t taddr = tmem + ((uint32_t) ((warp & 3) * 32) << 16) + OZ_ACOL;
+        const uint4 *aring = (const uint4 *) (smem + F::O_ARING) + row;
+        int q = 0;
+        for (int g = it.rbeg; g < it.rend && !bad; ++g) {
+            const int nk = B.tg_nk[g];
             for (int kc = 0; kc < nk; ++kc, ++q) {
-                const int sb = q % OZ_BSLOTS;
-                const bool ok = mbar_wait(afull0 + 8 * sb, (q / OZ_BSLOTS) & 1, err) &&
-                                mbar_wait(bfull0 + 8 * sb, (q / OZ_BSLOTS) & 1, err);
+                // the digits are there, and the stage's previous chunk has been multiplied
+                const int as = q % OZ_ASLOTS, qp = q - OZ_ASTAGES;
+                const bool ok = mbar_wait(ain0 + 8 * as, (q / OZ_ASLOTS) & 1, err) &&
+                                (qp < 0 || mbar_wait(done0 + 8 * (qp % OZ_BSLOTS), (qp / OZ_BSLOTS) & 1, err));
                 if (__any_sync(0xffffffffu, !ok)) {
                     bad = 1;
                     break;
                 }
                 tc_fence_after();
-                const uint32_t ac = tm + OZ_ACOL + (q % OZ_ASTAGES) * OZ_ACOLS, bc = b0 + sb * OZ_BSTAGE;
-                const bool open = kc == 0, close = kc == nk - 1, held = open && gi >= 1;
-                const uint32_t fpar = (gi - 1) & 1, done = done0 + 8 * sb;
-                if (warp == OZ_MMA_WARP ? oz_issue_chunk<ND, 0>(ac, bc, tm, open, held, close, accfull0, accfree0, fpar,
-                                                                done, on, err)
-                                        : oz_issue_chunk<ND, 1>(ac, bc, tm, open, held, close, accfull0, accfree0, fpar,
-                                                                done, on, err)) {
-                    bad = 1;
-                    break;
+                const uint4 *ac = aring + as * (OZ_ACHUNK / 16);
+                const uint32_t acol = taddr + (q % OZ_ASTAGES) * OZ_ACOLS;
+#pragma unroll
+                for (int i = 0; i < 2 * ND; ++i) {
+                    const uint4 v = ac[i * OZ_M];
+                    tmem_st4(acol + i * (OZ_KC / 8), v.x, v.y, v.z, v.w);
                 }
+                tmem_wait_st();
+                tc_fence_before();
+                mbar_arrive(afull0 + 8 * (q % OZ_BSLOTS));
             }
         }
-        // all products of this warp have completed
-        mma_commit_on(fin, on);
-        mbar_wait(fin, 0u, nullptr);
+    } else {
+        reg_dec<OZ_REG_REST>();
+        if (warp >= OZ_COPY_WARP) {
+            // ---------------- warp 14, lane 0: operand copies, ahead of the products ----------------
+            if (tid == OZ_COPY_WARP * 32) {
+                const unsigned char *asrc = B.oz_aop + C.a_off + (size_t) it.xt * C.nkx * OZ_ACHUNK;
+                int pq = 0, acopied = 0;
+                for (int g = it.rbeg; g < it.rend && !bad; ++g) {
+                    const int nk = B.tg_nk[g];
+                    const unsigned char *src = bop + B.tg_off[g];
+                    for (int kc = 0; kc < nk; ++kc, ++pq) {
+                        const int ps = pq % OZ_BSLOTS, as = pq % OZ_ASLOTS, pa = pq - OZ_ASLOTS;
+                        // the slots' previous chunks must have been copied on and consumed
+                        if (pa >= 0 && !mbar_wait(afull0 + 8 * (pa % OZ_BSLOTS), (pa / OZ_BSLOTS) & 1, err)) {
+                            bad = 1;
+                            break;
+                        }
+                        mbar_expect_tx(ain0 + 8 * as, OZ_ACHUNK);
+                        bulk_g2s(bring + F::O_ARING + as * OZ_ACHUNK, asrc + (size_t) kc * OZ_ACHUNK, OZ_ACHUNK, ain0 + 8 * as);
+                        acopied = pq + 1;
+                        if (pq >= OZ_BSLOTS && !mbar_wait(done0 + 8 * ps, ((pq / OZ_BSLOTS) - 1) & 1, err)) {
+                            bad = 1;
+                            break;
+                        }
+                        mbar_expect_tx(bfull0 + 8 * ps, OZ_BSTAGE);
+                        bulk_g2s(bring + ps * OZ_BSTAGE, src, OZ_BSTAGE, bfull0 + 8 * ps);
+                        src += OZ_BSTAGE;
+                    }
+                }
+                // the copies in flight land before the block ends
+                for (int c = acopied > OZ_ASLOTS ? acopied - OZ_ASLOTS : 0; c < acopied; ++c)
+                    mbar_wait(ain0 + 8 * (c % OZ_ASLOTS), (c / OZ_ASLOTS) & 1, nullptr);
+                for (int c = pq > OZ_BSLOTS ? pq - OZ_BSLOTS : 0; c < pq; ++c)
+                    mbar_wait(bfull0 + 8 * (c % OZ_BSLOTS), (c / OZ_BSLOTS) & 1, nullptr);
+            }
+        } else {
+            // ---------------- warps 12, 13: the products of the even / odd diagonals ----------------
+            // The whole warp runs the loop and one elected lane issues; the decisions
+            // to stop are warp-uniform, and so is, visibly to the compiler, what
+            // the products' operands are made of: they are taken from uniform
+            // registers, and moving each operand of each product there costs more
+            // than the product takes.
+            const uint32_t tm = warp_uniform(tmem), b0 = warp_uniform(bring);
+            const int rend = warp_uniform(it.rend);
+            const uint32_t on = elect_one();
+            int q = 0, gi = 0;
+            for (int g = warp_uniform(it.rbeg); g < rend && !bad; ++g, ++gi) {
+                const int nk = warp_uniform(B.tg_nk[g]);
+                for (int kc = 0; kc < nk; ++kc, ++q) {
+                    const int sb = q % OZ_BSLOTS;
+                    const bool ok = mbar_wait(afull0 + 8 * sb, (q / OZ_BSLOTS) & 1, err) &&
+                                    mbar_wait(bfull0 + 8 * sb, (q / OZ_BSLOTS) & 1, err);
+                    if (__any_sync(0xffffffffu, !ok)) {
+                        bad = 1;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t ac = tm + OZ_ACOL + (q % OZ_ASTAGES) * OZ_ACOLS, bc = b0 + sb * OZ_BSTAGE;
+                    const bool open = kc == 0, close = kc == nk - 1, held = open && gi >= 1;
+                    const uint32_t fpar = (gi - 1) & 1, done = done0 + 8 * sb;
+                    if (warp == OZ_MMA_WARP ? oz_issue_chunk<ND, 0>(ac, bc, tm, open, held, close, accfull0, accfree0, fpar,
+                                                                    done, on, err)
+                                            : oz_issue_chunk<ND, 1>(ac, bc, tm, open, held, close, accfull0, accfree0, fpar,
+                                                                    done, on, err)) {
+                        bad = 1;
+                        break;
+                    }
+                }
+            }
+            // all products of this warp have completed
+            mma_commit_on(fin, on);
+            mbar_wait(fin, 0u, nullptr);
+        }
     }
     if (bad) atomicExch(err, 1);
     tc_fence_before();

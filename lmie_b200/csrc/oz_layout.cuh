@@ -83,7 +83,8 @@ struct Oz {
     static constexpr int NP = ND == 6 ? 64 : 48;          // operand rows (product N) per radius group
     static constexpr int NHALF = NP / 2;                  // rows of S (then D')
     static constexpr int ASTAGES = ND == 6 ? 2 : 3;       // A operand stages (tensor memory)
-    static constexpr int BSLOTS = ND == 6 ? 4 : 6;        // B operand slots (bulk copies)
+    static constexpr int ASLOTS = ND == 6 ? 2 : 3;        // A operand slots in shared memory (bulk copies)
+    static constexpr int BSLOTS = 4;                      // B operand slots (bulk copies)
     static constexpr uint32_t BSLICE = NP * OZ_KC;        // bytes of one B slice of a chunk
     static constexpr uint32_t BSTAGE = ND * BSLICE;       // one B chunk of a group
     static constexpr uint32_t LBO_B = (NP / 8) * 128;     // order-group stride of a B slice
