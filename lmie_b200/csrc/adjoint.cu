@@ -21,10 +21,10 @@
 // transposed angular contraction, from phi; then with the complex derivatives
 // A_n = da_n/dm, B_n = db_n/dm,
 //   dL/dmr = Re sum (conj(a_bar) A + conj(b_bar) B),  dL/dmi = Im sum (...)
-// (m = mr - i mi).  A_n, B_n use dD_n/dz = n(n+1)/z^2 - 1 - D_n^2 (z = m x),
-// so the D_n recurrence is never differentiated; the recurrences are re-run
-// from checkpoints every ADJ_K orders, in both sweeps.
+// (m = mr - i mi).  The coefficients and A_n, B_n come from the recurrences
+// and formulas of the solves (mie_radius.cuh); the reverse sweep reads them.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "dev_common.cuh"
+#include "mie_radius.cuh"
 #include "../../include/lmie_b200.h"
 
 extern "C" int lmieb_calc_n1(double x);
@@ -41,31 +42,29 @@ extern "C" void lmieb_gauss_leg(int n, double x1, double x2, double *x, double *
 
 namespace {
 
-constexpr int ADJ_K = 64;          // orders per checkpoint block
-constexpr int ADJ_T = 128;         // threads of the angular kernels (half-angles)
-constexpr int ADJ_GR = 16;         // radii per block of the forward angular kernel
+constexpr int ADJ_T = 128;         // threads of the angular and the summing kernels
+constexpr int ADJ_GR = 32;         // radii per block of the angular kernel
 
 struct Adj {
     int L, R;                      // wavelengths, radii
     int na, nhu;                   // user angles, half-angles (theta <= 90 deg)
-    int G;                         // radius groups of the forward angular kernel
+    int G;                         // radius groups of the angular kernel
     const double *lam;             // [L]
     const cplx *m;                 // [L]
     const double *W, *q;           // [R]
-    const int *bin;                // [R]
-    const double *x;               // [L*R]
+    const double *rad;             // [R]
     const int *n1, *n2;            // [L*R]
-    const long long *off;          // [L*R+1] per-order offsets (n1 each)
-    const long long *coff;         // [L*R+1] checkpoint offsets (ceil(n1/ADJ_K) each)
-    const double *tab;             // [(n - 1) * nhu + h] -> {pi_n, tau_n}(mu_h), n = 1..n1max
-    const double *tabt;            // [h * n1max + n - 1] -> {pi_n, tau_n}(mu_h) (orders contiguous)
-    int n1max;
-    const double *dw;              // [L][na][2] d11, d12
+    const int *ro;                 // [L*R] orders of the wavelength's radii before this one
+    const long long *ko;           // [L] orders of the wavelengths before this one
+    const double *mu;              // [nhu] cosines of the half-angles
+    int nt;                        // tiles of 8 half-angles (nhu rounded up, zeros there)
+    int nrow;                      // orders in the tables
+    double2 *tabf, *tabb;          // {X_n, Y_n}(mu_h) in the order of the angular kernel's fragments
+    const double2 *dw;             // [L][8 nt][2] {d11, d12} / 2 at the half-angles and their mirrors (zeros: none)
     const double *cw;              // [L][3] c_cext, c_csca, c_g
-    cplx *cs, *cd;                 // per order: fv4 (a +- b)
-    cplx *cbs, *cbd;               // per order: their adjoints (times W dL/dPhi)
-    cplx *ckD;                     // checkpoints of D_n
-    double *ckr;                   // checkpoints of psi_n / psi_{n-1}
+    double4 *c4;                   // per order: fv4 (a + b), fv4 (a - b)
+    double4 *d4;                   // per order: da/dm, db/dm
+    double4 *b4;                   // per order: the adjoints of c4 per W dL/dPhi (before that, K1's checkpoints)
     double *esg;                   // [L*R][4] e, s, g, phi
     double *pfp;                   // [L][G][na][2] partial sums of W F11, W F12
     double *lw;                    // [L][8] dL/dE, dL/dS, dL/dG, dL/dPhi, dL/dN, loss, Cext, Csca
@@ -79,127 +78,117 @@ struct Adj {
 __device__ __forceinline__ double fv3d(int j) { return (j + 2.) * j / (j + 1.); }
 __device__ __forceinline__ double fv4d(int j) { return (2. * j + 1.) / (j * (j + 1.)); }
 
-// D_j for j in [lo, hi] (hi <= n2) by the downward recurrence from the
-// checkpoint value at t (t >= hi): exact replay of the first sweep.
-__device__ __forceinline__ void replay_D(cplx *Dl, int lo, int hi, int t, cplx Dt, cplx z) {
-    cplx D = Dt;
-    if (t <= hi) Dl[t - lo] = D;
-    const cplx zi = cinv(z);
-    for (int j = t - 1; j >= lo; --j) {
-        const cplx u = (j + 1.) * zi;
-        D = u - cinv(D + u);
-        if (j <= hi) Dl[j - lo] = D;
-    }
+__device__ __forceinline__ long long order_offset(const Adj &P, int k, int r) {
+    return P.ko[k] + P.ro[(size_t) k * P.R + r];
 }
 
-__device__ __forceinline__ void replay_r(double *rl, int lo, int hi, int t, double rt, double xinv) {
-    double rr = rt;
-    if (t <= hi) rl[t - lo] = rr;
-    for (int j = t - 1; j >= lo; --j) {
-        rr = 1. / ((2. * j + 1.) * xinv - rr);
-        if (j <= hi) rl[j - lo] = rr;
-    }
+__device__ __forceinline__ void st4(double4 *p, double a, double b, double c, double d) {
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};" ::"l"(p), "d"(a), "d"(b), "d"(c), "d"(d) : "memory");
+}
+__device__ __forceinline__ double4 ld4(const double4 *p) {
+    double4 v;
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+    return v;
 }
 
-// First sweeps of one radius: checkpoints of D (from n2 down) and of the
-// psi ratio (from n1 down); block c covers orders [c ADJ_K + 1, c ADJ_K + ADJ_K]
-// and starts its replay at t_c = min(c ADJ_K + ADJ_K, n2) (D) or n1 (ratio).
-__device__ void checkpoints(int n1, int n2, double x, cplx z, cplx *ckD, double *ckr) {
-    const int nb = (n1 + ADJ_K - 1) / ADJ_K;
-    const cplx zi = cinv(z);
-    cplx D = mk(0., 0.);
-    for (int c = 0; c < nb; ++c)
-        if (c * ADJ_K + ADJ_K >= n2) ckD[c] = D;
-    for (int j = n2 - 1; j >= 1; --j) {
-        const cplx u = (j + 1.) * zi;
-        D = u - cinv(D + u);
-        if (j % ADJ_K == 0 && j / ADJ_K - 1 < nb && j < n2) ckD[j / ADJ_K - 1] = D;
+// ---- forward: coefficients, their derivatives, cross-section sums (thread per (k, r)) ----
+// K1's thread-per-radius form (k_mie.cu), with the checkpoints of a radius in
+// the place of its adjoints: 7 doubles for every 4 orders where those take 16.
+__global__ void __launch_bounds__(64) k_adj_coef(Adj P) {
+    const int nrb = (P.R + 63) / 64, k = blockIdx.x % P.L;
+    const int r = (nrb - 1 - (int) (blockIdx.x / P.L)) * 64 + threadIdx.x;   // large radii first
+    if (r >= P.R) return;
+    const size_t t = (size_t) k * P.R + r;
+    const int n1 = P.n1[t], n2 = P.n2[t];
+    const cplx m = P.m[k];
+    MieRadius<false> c;
+    c.set(2. * LMIEB_PI * P.rad[r] / P.lam[k], m, cinv(m), 0., mk(0., 0.));
+    const long long off = order_offset(P, k, r);
+    double *const ck = (double *) (P.b4 + off);
+    const int nb = n1 / MIE_B + 1;
+    double u0;
+    int eu = 0;
+    {
+        MieP p;
+        p.hi = mk(1., 0.);
+        p.cur = (double) n2 * c.zinv;
+        int n = n2 - 1;
+        for (const int n0 = nb * MIE_B; n >= n0; --n) {
+            p.step(p.next(n, c.zinv));
+            if (n % MIE_B == 0) p.rescale();
+        }
+        MieU<false> q;
+        q.start();
+        for (int b = nb - 1; b >= 0; --b) {
+            double *w = ck + 7 * b;
+            w[0] = p.hi.re; w[1] = p.hi.im; w[2] = p.cur.re; w[3] = p.cur.im;
+            w[4] = q.hi; w[5] = q.cur; w[6] = (double) eu;
+#pragma unroll
+            for (int i = MIE_B - 1; i >= 0; --i) {
+                const int n = b * MIE_B + i;
+                if (b > 0 || i > 0) p.step(p.next(n, c.zinv));
+                if (n <= n1 && (b > 0 || i > 0)) q.step(n, c.xinv);
+            }
+            if (b > 0) {
+                p.rescale();
+                eu += q.rescale();
+            }
+        }
+        u0 = q.cur;
     }
-    const double xinv = 1. / x;
-    double rr = 0.;
-    for (int c = 0; c < nb; ++c)
-        if (c * ADJ_K + ADJ_K >= n1) ckr[c] = 0.;
-    for (int j = n1 - 1; j >= 1; --j) {
-        rr = 1. / ((2. * j + 1.) * xinv - rr);
-        if (j % ADJ_K == 0 && j / ADJ_K - 1 < nb) ckr[j / ADJ_K - 1] = rr;
-    }
-}
-
-// Walks the orders 1..n1 of one radius in ascending order, block by block,
-// calling f(j, psi_j, psi_{j-1}, zeta_j, zeta_{j-1}, D_j).
-template <class F>
-__device__ void ascend(int n1, int n2, double x, cplx z, const cplx *ckD, const double *ckr, F &&f) {
-    cplx Dl[ADJ_K];
-    double rl[ADJ_K];
-    const double xinv = 1. / x;
-    const double sx = sin(x), cx = cos(x);
-    double psi_p = sx, chi_p = cx, chi = cx * xinv + sx;   // psi_0, chi_0, chi_1
-    const int nb = (n1 + ADJ_K - 1) / ADJ_K;
-    for (int c = 0; c < nb; ++c) {
-        const int lo = c * ADJ_K + 1, hi = min(c * ADJ_K + ADJ_K, n1);
-        replay_D(Dl, lo, hi, min(c * ADJ_K + ADJ_K, n2), ckD[c], z);
-        replay_r(rl, lo, hi, min(c * ADJ_K + ADJ_K, n1), ckr[c], xinv);
-        for (int j = lo; j <= hi; ++j) {
-            const double psi = rl[j - lo] * psi_p;
-            const cplx zeta = mk(psi, chi), zeta_p = mk(psi_p, chi_p);
-            f(j, psi, psi_p, zeta, zeta_p, Dl[j - lo]);
-            const double chi_n = (2. * j + 1.) * xinv * chi - chi_p;
-            psi_p = psi;
+    double sinx, cosx;
+    sincos(c.x, &sinx, &cosx);
+    const double spsi = sinx / u0;
+    double chi_p = cosx, chi = fma(c.xinv, cosx, sinx), psi_p = spsi * u0;
+    MieSums<false, false> sums;
+    sums.zero();
+    MieAB prev;
+    prev.a = prev.b = prev.am = prev.bm = prev.ax = prev.bx = mk(0., 0.);
+    for (int b = 0; b < nb; ++b) {
+        const double *w = ck + 7 * b;
+        cplx D[MIE_B], Dz[MIE_B];
+        double ub[MIE_B];
+        const double su = mb_pow2((int) w[6] - eu);
+        MieP p;
+        p.hi = mk(w[0], w[1]);
+        p.cur = mk(w[2], w[3]);
+        MieU<false> u;
+        u.hi = w[4];
+        u.cur = w[5];
+#pragma unroll
+        for (int i = MIE_B - 1; i >= 0; --i) {
+            const int n = b * MIE_B + i;
+            ub[i] = u.cur;
+            if (n > 0) {
+                const cplx lo = p.next(n, c.zinv);
+                if (n <= n1) {
+                    mie_d<true>(c, n, lo, p.cur, p.hi, D[i], Dz[i]);
+                    u.step(n, c.xinv);
+                }
+                p.step(lo);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < MIE_B; ++i) {
+            const int j = b * MIE_B + i;
+            if (j < 1 || j > n1) continue;
+            const double psi = spsi * ub[i] * su, f4 = fv4d(j);
+            const MieAB q = mie_ab<true, false>(c, j, D[i], Dz[i], psi, psi_p, chi, chi_p, 0., 0.);
+            sums.add(j, q, prev);
+            st4(P.c4 + off + j - 1, f4 * (q.a.re + q.b.re), f4 * (q.a.im + q.b.im), f4 * (q.a.re - q.b.re),
+                f4 * (q.a.im - q.b.im));
+            st4(P.d4 + off + j - 1, q.am.re, q.am.im, q.bm.re, q.bm.im);
+            const double chi_n = fma((2. * j + 1.) * c.xinv, chi, -chi_p);
             chi_p = chi;
             chi = chi_n;
+            psi_p = psi;
+            prev = q;
         }
     }
-}
-
-// ---- forward: coefficients, cross-section sums, checkpoints (thread per (k, r)) ----
-__global__ void k_adj_coef(Adj P) {
-    const long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long) P.L * P.R) return;
-    const int k = (int) (t / P.R);
-    const int n1 = P.n1[t], n2 = P.n2[t];
-    const double x = P.x[t];
-    const cplx m = P.m[k], minv = cinv(m), z = m * x;
-    cplx *ckD = P.ckD + P.coff[t];
-    double *ckr = P.ckr + P.coff[t];
-    checkpoints(n1, n2, x, z, ckD, ckr);
-    const double xinv = 1. / x;
-    cplx *cs = P.cs + P.off[t], *cd = P.cd + P.off[t];
-    double e = 0., s = 0., g = 0.;
-    cplx ap = mk(0., 0.), bp = mk(0., 0.);
-    ascend(n1, n2, x, z, ckD, ckr, [&](int j, double psi, double psi_p, cplx zeta, cplx zeta_p, cplx D) {
-        const double tt = j * xinv;
-        const cplx ca = D * minv + tt, cb = m * D + tt;
-        const cplx a = (ca * psi - psi_p) * cinv(ca * zeta - zeta_p);
-        const cplx b = (cb * psi - psi_p) * cinv(cb * zeta - zeta_p);
-        const double f1 = 2. * j + 1., f4 = fv4d(j);
-        e += f1 * (a.re + b.re);
-        s += f1 * (norm2(a) + norm2(b));
-        if (j >= 2) g += fv3d(j - 1) * (re_mulc(ap, a) + re_mulc(bp, b)) + fv4d(j - 1) * re_mulc(ap, bp);
-        cs[j - 1] = (a + b) * f4;
-        cd[j - 1] = (a - b) * f4;
-        ap = a;
-        bp = b;
-    });
-    double *o = P.esg + (size_t) t * 4;
-    o[0] = e;
-    o[1] = s;
-    o[2] = g;
-}
-
-// sp, sm at half-angle h (and its mirror) of one radius from staged coefficients
-__device__ __forceinline__ void angular_sums(const Adj &P, int h, int n1, const cplx *scs, const cplx *scd,
-                                             cplx &spA, cplx &smA, cplx &spB, cplx &smB) {
-    spA = smA = spB = smB = mk(0., 0.);
-    const double *tb = P.tab + 2 * h;
-    for (int n = 1; n <= n1; ++n) {
-        const double pi = tb[(size_t) (n - 1) * 2 * P.nhu], tau = tb[(size_t) (n - 1) * 2 * P.nhu + 1];
-        const double p = pi + tau, q = pi - tau, sg = (n & 1) ? 1. : -1.;
-        const cplx c = scs[n - 1], d = scd[n - 1];
-        spA = spA + c * p;
-        smA = smA + d * q;
-        spB = spB + c * (sg * q);
-        smB = smB + d * (sg * p);
-    }
+    double *o = P.esg + t * 4;
+    o[0] = sums.v[0];
+    o[1] = sums.v[1];
+    o[2] = sums.v[4];
 }
 
 __device__ __forceinline__ double block_sum128(double v, double *sh) {
@@ -214,53 +203,178 @@ __device__ __forceinline__ double block_sum128(double v, double *sh) {
     return s;
 }
 
-// ---- forward: phase matrix at the user angles, phi_r (block per (k, radius group)) ----
-__global__ void __launch_bounds__(ADJ_T) k_adj_fwd(Adj P) {
-    extern __shared__ cplx sco[];                       // [2][n1max]
-    __shared__ double sh[ADJ_T / 32];
-    const int k = blockIdx.x / P.G, grp = blockIdx.x % P.G;
-    const int h = threadIdx.x;
-    const int hm = P.na - 1 - h;                        // mirror angle index
-    const bool act = h < P.nhu, mir = act && hm != h;
-    const double *dw = P.dw + (size_t) k * P.na * 2;
-    double p11A = 0., p12A = 0., p11B = 0., p12B = 0.;
-    for (int r = grp * ADJ_GR; r < min(P.R, grp * ADJ_GR + ADJ_GR); ++r) {
-        const long long t = (long long) k * P.R + r;
-        const int n1 = P.n1[t];
-        cplx *scs = sco, *scd = sco + n1;
-        __syncthreads();
-        for (int i = threadIdx.x; i < n1; i += ADJ_T) {
-            scs[i] = P.cs[P.off[t] + i];
-            scd[i] = P.cd[P.off[t] + i];
-        }
-        __syncthreads();
-        double phi = 0.;
-        if (act) {
-            cplx spA, smA, spB, smB;
-            angular_sums(P, h, n1, scs, scd, spA, smA, spB, smB);
-            const double W = P.W[r];
-            const double f11 = .25 * (norm2(spA) + norm2(smA)), f12 = -.5 * re_mulc(spA, smA);
-            p11A += W * f11;
-            p12A += W * f12;
-            phi = dw[2 * h] * f11 + dw[2 * h + 1] * f12;
-            if (mir) {
-                const double g11 = .25 * (norm2(spB) + norm2(smB)), g12 = -.5 * re_mulc(spB, smB);
-                p11B += W * g11;
-                p12B += W * g12;
-                phi += dw[2 * hm] * g11 + dw[2 * hm + 1] * g12;
+// ---- pi_n, tau_n at the half-angles (thread per half-angle) ----
+// The angular kernel sums over odd and even orders at once.  With sp(mu) =
+// sum c_n (pi_n + tau_n), sm(mu) = sum d_n (pi_n - tau_n) and, at the mirror
+// angle, pi_n -> s_n pi_n, tau_n -> -s_n tau_n (s_n = -(-1)^n),
+//   X_n = pi_n (n odd), tau_n (n even),   Y_n the other one,
+//   x = sum c_n X_n, y = sum c_n Y_n:            sp = x + y, sp(-mu) = x - y,
+//   x = sum s_n d_n X_n, y = sum s_n d_n Y_n:    sm = x - y, sm(-mu) = x + y,
+// half the products of four separate sums; likewise the transposed sums.
+__global__ void k_adj_table(Adj P) {
+    const int h = threadIdx.x;                          // 8 nt threads
+    const double mu = h < P.nhu ? P.mu[h] : 0., on = h < P.nhu ? 1. : 0.;
+    double p0 = 0., p1 = on;
+    for (int n = 0; n < P.nrow; ++n) {                  // order n + 1
+        const double o = n + 1., tau = fma(o * mu, p1, -(o + 1.) * p0);
+        const double2 v = (n & 1) ? make_double2(tau, p1) : make_double2(p1, tau);
+        const int t = h >> 3, c = h & 7;
+        P.tabf[((size_t) (n >> 2) * P.nt + t) * 32 + c * 4 + (n & 3)] = v;
+        P.tabb[(((size_t) (n >> 3) * P.nt + t) * 2 + (c & 1)) * 32 + (n & 7) * 4 + (c >> 1)] = v;
+        const double r = 1. / o, p2 = fma(fma(2., o, 1.) * r * mu, p1, -(o + 1.) * r * p0);
+        p0 = p1;
+        p1 = p2;
+    }
+}
+
+// c += a b: a one element of 8 x 4 (row lane / 4, column lane % 4), b one of
+// 4 x 8 (row lane % 4, column lane / 4), c two of 8 x 8 (row lane / 4, columns
+// 2 (lane % 4) and the next)
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+        : "+d"(c[0]), "+d"(c[1])
+        : "d"(a), "d"(b));
+}
+
+// ---- both angular sweeps (block per (k, group of ADJ_GR radii)) ----
+// Forward: sp, sm at the user angles, the phase matrix sums, phi_r; reverse:
+// the adjoints of the coefficient columns from those of sp, sm.  These are
+// linear in W dL/dPhi, which is known only when all radii have been summed: it
+// is left out here and put in by k_adj_m, so that the sums over orders are
+// formed once and stay in registers between the sweeps.
+//
+// A warp takes two radii at a time as the 8 rows of FP64 m8n8k4 products: row =
+// (radius, {c.re, c.im, s d.re, s d.im}).  Forward, columns = 8 half-angles,
+// K = orders; the sums of all half-angles are the accumulators (4 NT doubles).
+// Reverse, columns = 8 orders, K = half-angles: an accumulator's two columns
+// are half-angles 2 q and 2 q + 1 of its tile, which are taken as the K
+// elements q of two products, so the accumulators are the operands as they are
+// (tabb is laid out for that).  Bound by the FP64 pipe: 16 FMAs per order and
+// half-angle.  256 wavelengths x 2048 radii x 181 angles (17.8 M orders):
+// 3.0 ms (a thread per half-angle, radius by radius, with the forward sums
+// formed again for the reverse sweep: 12.1 ms); the FMAs take 1.5 ms.
+template <int NT>
+__global__ void __launch_bounds__(ADJ_T, NT > 12 ? 2 : 3) k_adj_angles(Adj P) {
+    constexpr int PF = NT > 6 && NT % 2 == 0 ? NT / 2 : NT;   // table entries loaded ahead
+    extern __shared__ double psum[];                    // [4 warps][2 NT][32]: sums of F11, F12 over radii
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int q = lane & 3, row = lane >> 2, comp = row & 3, rr = row >> 2;
+    const int k = blockIdx.x % P.L, grp = P.G - 1 - blockIdx.x / P.L;   // large radii first
+    // Of the two values x + y, x - y of a half-angle, lane bit 2 tells which is
+    // this lane's first: the first values of lanes 0-3 and 4-7 (components 0
+    // and 1) are then those of an angle and of its mirror.  The sign of y does
+    // this, together with sm's (table kernel).
+    const bool b2 = lane & 4, b3 = lane & 8, flip = b2 != (comp >= 2);
+    const double2 *dw = P.dw + (size_t) k * 16 * NT + 4 * q + b2;
+    const int dwo = b2 ? -1 : 1;
+    double *const ps = psum + warp * (2 * NT * 32) + lane;
+#pragma unroll
+    for (int i = 0; i < 2 * NT; ++i) ps[i * 32] = 0.;
+    // This lane's radius of pair p and its coefficients are loaded a pair ahead,
+    // further ones four steps ahead: the coefficients come from DRAM.
+    const int r0 = grp * ADJ_GR + warp * (ADJ_GR / 4) + rr;
+    const long long t0 = (long long) k * P.R;
+    auto orders = [&](int p) { return p < ADJ_GR / 8 && r0 + 2 * p < P.R ? P.n1[t0 + r0 + 2 * p] : 0; };
+    auto offset = [&](int p) { return order_offset(P, k, min(r0 + 2 * p, P.R - 1)); };
+    auto column = [&](long long o) { return (const double *) (P.c4 + o) + comp; };
+    int n1 = orders(0);
+    long long off = offset(0);
+    double a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = 4 * i + q < n1 ? column(off)[4 * (4 * i + q)] : 0.;
+    for (int p = 0; p < ADJ_GR / 8; ++p) {
+        const int r = r0 + 2 * p, n1_next = orders(p + 1);
+        const bool on = r < P.R;
+        const long long t = t0 + (on ? r : 0), off_next = offset(p + 1);
+        const double W = on ? P.W[r] : 0.;
+        const int nmax = max(n1, __shfl_xor_sync(0xffffffffu, n1, 16));
+        if (nmax == 0) break;
+        const double *src = column(off);
+        double X[NT][2], Y[NT][2];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) X[i][0] = X[i][1] = Y[i][0] = Y[i][1] = 0.;
+        {
+            // the next four orders' table entries are loaded as these are used
+            const double2 *tb = P.tabf + lane;
+            double2 b[PF];
+#pragma unroll
+            for (int i = 0; i < PF; ++i) b[i] = tb[i * 32];
+            for (int n0 = 0; n0 < nmax; n0 += 4) {
+                const int nn = n0 + q + 16;
+                const double ax = comp >= 2 && (q & 1) ? -a[0] : a[0], ay = flip ? -ax : ax;
+                a[0] = a[1];
+                a[1] = a[2];
+                a[2] = a[3];
+                a[3] = nn < n1 ? src[4 * nn] : 0.;
+#pragma unroll
+                for (int i = 0; i < NT; ++i) {
+                    dmma(X[i], ax, b[i % PF].x);
+                    dmma(Y[i], ay, b[i % PF].y);
+                    b[i % PF] = tb[(i + PF) * 32];
+                }
+                tb += NT * 32;
             }
         }
-        phi = block_sum128(phi, sh);
-        if (threadIdx.x == 0) P.esg[(size_t) t * 4 + 3] = phi;
-    }
-    double *o = P.pfp + ((size_t) k * P.G + grp) * P.na * 2;
-    if (act) {
-        o[2 * h] = p11A;
-        o[2 * h + 1] = p12A;
-        if (mir) {
-            o[2 * hm] = p11B;
-            o[2 * hm + 1] = p12B;
+        // phase matrix elements and the adjoints of sp, sm: this lane has one
+        // real component of (sp, sm) at an angle (v1) and at its mirror (v2), or
+        // the other way round
+        double phi = 0.;
+#pragma unroll
+        for (int i = 0; i < NT; ++i)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const double v1 = X[i][j] + Y[i][j], v2 = X[i][j] - Y[i][j];
+                // sm's component for sp's and the other way round
+                const double p1 = __shfl_xor_sync(0xffffffffu, v1, 8), p2 = __shfl_xor_sync(0xffffffffu, v2, 8);
+                const double2 w1 = dw[16 * i + 2 * j], w2 = dw[16 * i + 2 * j + dwo];
+                const double s1 = w1.x * v1 - w1.y * p1, s2 = w2.x * v2 - w2.y * p2;
+                phi += v1 * s1 + v2 * s2;
+                X[i][j] = s1 + s2;
+                Y[i][j] = s1 - s2;
+                // sums over the four components, those of F12 twice the same two; of the two radii at the end
+                double f = v1 * v1 + __shfl_xor_sync(0xffffffffu, v2 * v2, 4);
+                const double g = v1 * p1 + __shfl_xor_sync(0xffffffffu, v2 * p2, 4);
+                f += __shfl_xor_sync(0xffffffffu, f, 8);
+                ps[(2 * i + j) * 32] += W * (b3 ? g : f);
+            }
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) phi += __shfl_xor_sync(0xffffffffu, phi, o);
+        if (on && (lane & 15) == 0) P.esg[(size_t) t * 4 + 3] = .5 * phi;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i] = 4 * i + q < n1_next ? column(off_next)[4 * (4 * i + q)] : 0.;
+        // the adjoints of the coefficient columns, 8 orders at a time (this lane: two of them)
+        double *dst = (double *) (P.b4 + off) + comp;
+        const double2 *tb = P.tabb + lane;
+        double2 b[PF];
+#pragma unroll
+        for (int i = 0; i < PF; ++i) b[i] = tb[i * 32];
+        for (int n0 = 0; n0 < nmax; n0 += 8) {
+            double o[4][2] = {};                        // chains of products
+#pragma unroll
+            for (int i = 0; i < 2 * NT; ++i) {
+                dmma(o[i & 1], X[i >> 1][i & 1], b[i % PF].x);
+                dmma(o[2 + (i & 1)], Y[i >> 1][i & 1], b[i % PF].y);
+                b[i % PF] = tb[(i + PF) * 32];
+            }
+            tb += 2 * NT * 32;
+            const int n = n0 + 2 * q;
+            const double y0 = o[2][0] + o[3][0], y1 = o[2][1] + o[3][1];
+            const double v0 = (o[0][0] + o[1][0]) + (flip ? -y0 : y0), v1 = (o[0][1] + o[1][1]) + (flip ? -y1 : y1);
+            if (n < n1) dst[4 * n] = v0;
+            if (n + 1 < n1) dst[4 * n + 4] = comp >= 2 ? -v1 : v1;
         }
+        n1 = n1_next;
+        off = off_next;
+    }
+    __syncthreads();
+    double *o = P.pfp + ((size_t) k * P.G + grp) * P.na * 2;
+    for (int i = threadIdx.x; i < 4 * P.nhu; i += ADJ_T) {
+        const int h = i >> 2, mir = i & 1, el = (i >> 1) & 1, hm = P.na - 1 - h;
+        if (mir && hm == h) continue;
+        const double *v = psum + ((h >> 3) * 2 + (h & 1)) * 32 + ((h & 7) >> 1) + 4 * mir + 8 * el;
+        double sum = 0.;
+        for (int w = 0; w < 4; ++w) sum += v[w * (2 * NT * 32)] + v[w * (2 * NT * 32) + 16];
+        o[2 * (mir ? hm : h) + el] = el ? -.5 * sum : .25 * sum;
     }
 }
 
@@ -313,102 +427,48 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_lambda(Adj P) {
     }
 }
 
-// ---- reverse: adjoints of the coefficient columns (block per (k, r)) ----
-__global__ void __launch_bounds__(ADJ_T) k_adj_back(Adj P) {
-    extern __shared__ cplx sco[];                       // [2][n1] coefficients, then [4][nhu] adjoint sums
-    const long long t = blockIdx.x;
-    const int k = (int) (t / P.R), r = (int) (t % P.R);
-    const int n1 = P.n1[t];
-    cplx *scs = sco, *scd = sco + n1, *sbar = sco + 2 * n1;
-    for (int i = threadIdx.x; i < n1; i += ADJ_T) {
-        scs[i] = P.cs[P.off[t] + i];
-        scd[i] = P.cd[P.off[t] + i];
-    }
-    __syncthreads();
-    const double aphi = P.W[r] * P.lw[(size_t) k * 8 + 3];
-    const double *dw = P.dw + (size_t) k * P.na * 2;
-    const int h = threadIdx.x, hm = P.na - 1 - h;
-    if (h < P.nhu) {
-        cplx spA, smA, spB, smB;
-        angular_sums(P, h, n1, scs, scd, spA, smA, spB, smB);
-        const double a11 = .5 * aphi * dw[2 * h], a12 = .5 * aphi * dw[2 * h + 1];
-        sbar[4 * h] = spA * a11 - smA * a12;            // d phi / d sp (mu_h)
-        sbar[4 * h + 1] = smA * a11 - spA * a12;        // d phi / d sm (mu_h)
-        if (hm != h) {
-            const double b11 = .5 * aphi * dw[2 * hm], b12 = .5 * aphi * dw[2 * hm + 1];
-            sbar[4 * h + 2] = spB * b11 - smB * b12;
-            sbar[4 * h + 3] = smB * b11 - spB * b12;
-        } else {
-            sbar[4 * h + 2] = sbar[4 * h + 3] = mk(0., 0.);
-        }
-    }
-    __syncthreads();
-    // transposed contraction over the angles, one order per thread
-    for (int n = threadIdx.x + 1; n <= n1; n += ADJ_T) {
-        const double2 *tb = (const double2 *) P.tabt + (n - 1);   // consecutive threads, consecutive orders
-        const double sg = (n & 1) ? 1. : -1.;
-        cplx bs = mk(0., 0.), bd = mk(0., 0.);
-        for (int hh = 0; hh < P.nhu; ++hh) {
-            const double2 pt = tb[(size_t) hh * P.n1max];
-            const double pi = pt.x, tau = pt.y;
-            const double p = pi + tau, q = pi - tau;
-            const cplx *sb = sbar + 4 * hh;
-            bs = bs + sb[0] * p + sb[2] * (sg * q);
-            bd = bd + sb[1] * q + sb[3] * (sg * p);
-        }
-        P.cbs[P.off[t] + n - 1] = bs;
-        P.cbd[P.off[t] + n - 1] = bd;
-    }
-}
-
-// ---- reverse: dL/dm of one radius from the checkpoints (thread per (k, r)) ----
-__global__ void k_adj_m(Adj P) {
-    const long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= (long long) P.L * P.R) return;
-    const int k = (int) (t / P.R), r = (int) (t % P.R);
-    const int n1 = P.n1[t], n2 = P.n2[t];
-    const double x = P.x[t];
-    const cplx m = P.m[k], minv = cinv(m), z = m * x;
+// ---- reverse: dL/dm of one radius (eight lanes per (k, r), orders dealt out) ----
+// Bound by memory: 96 bytes per order, read once (the orders before from L1).
+__global__ void __launch_bounds__(256) k_adj_m(Adj P) {
+    const long long t = ((long long) blockIdx.x * blockDim.x + threadIdx.x) >> 3;
+    const int lane = threadIdx.x & 7;
+    const bool on = t < (long long) P.L * P.R;
+    const int k = on ? (int) (t / P.R) : 0, r = on ? (int) (t % P.R) : 0;
+    const int n1 = on ? P.n1[t] : 0;
     const double *lw = P.lw + (size_t) k * 8;
     const double W = P.W[r];
-    const double aE = W * lw[0], aS = W * lw[1], aG = W * lw[2];
-    const double xinv = 1. / x;
-    const cplx zinv = cinv(z), z2inv = zinv * zinv, m2inv = minv * minv;
-    const cplx *cbs = P.cbs + P.off[t], *cbd = P.cbd + P.off[t];
+    const double aE = W * lw[0], aS = W * lw[1], aG = W * lw[2], aP = W * lw[3];
+    const long long off = order_offset(P, k, r);
     cplx Z = mk(0., 0.);
-    cplx ap = mk(0., 0.), bp = mk(0., 0.), Ap = mk(0., 0.), Bp = mk(0., 0.);
-    ascend(n1, n2, x, z, P.ckD + P.coff[t], P.ckr + P.coff[t],
-           [&](int j, double psi, double psi_p, cplx zeta, cplx zeta_p, cplx D) {
-               const double tt = j * xinv;
-               const cplx ca = D * minv + tt, cb = m * D + tt;
-               const cplx ia = cinv(ca * zeta - zeta_p), ib = cinv(cb * zeta - zeta_p);
-               const cplx a = (ca * psi - psi_p) * ia, b = (cb * psi - psi_p) * ib;
-               // dD/dm = x dD/dz,  dD/dz = j (j + 1) / z^2 - 1 - D^2
-               const cplx Dz = z2inv * (j * (j + 1.)) - 1. - D * D;
-               const cplx w = zeta * psi_p - zeta_p * psi;     // (zeta_j psi_{j-1} - psi_j zeta_{j-1})
-               const cplx A = w * (ia * ia) * (Dz * (x * 1.) * minv - D * m2inv);
-               const cplx Bd = w * (ib * ib) * (D + m * Dz * x);
-               const double f1 = 2. * j + 1., f4 = fv4d(j);
-               // adjoints of a_j, b_j except the a_{j+1}, b_{j+1} terms of g
-               cplx abar = mk(aE * f1, 0.) + a * (2. * aS * f1) + (cbs[j - 1] + cbd[j - 1]) * f4;
-               cplx bbar = mk(aE * f1, 0.) + b * (2. * aS * f1) + (cbs[j - 1] - cbd[j - 1]) * f4;
-               if (j < n1) {
-                   abar = abar + b * (aG * f4);
-                   bbar = bbar + a * (aG * f4);
-               }
-               if (j >= 2) {
-                   const double f3 = aG * fv3d(j - 1);
-                   abar = abar + ap * f3;
-                   bbar = bbar + bp * f3;
-                   // the a_j, b_j term of the adjoints of a_{j-1}, b_{j-1}
-                   Z = Z + conjg(a) * Ap * f3 + conjg(b) * Bp * f3;
-               }
-               Z = Z + conjg(abar) * A + conjg(bbar) * Bd;
-               ap = a;
-               bp = b;
-               Ap = A;
-               Bp = Bd;
-           });
+    for (int j = lane + 1; j <= n1; j += 8) {
+        const double4 c = ld4(P.c4 + off + j - 1), d = ld4(P.d4 + off + j - 1), v = ld4(P.b4 + off + j - 1);
+        const double f1 = 2. * j + 1., f4 = fv4d(j), h = .5 / f4;
+        const cplx a = mk(h * (c.x + c.z), h * (c.y + c.w)), b = mk(h * (c.x - c.z), h * (c.y - c.w));
+        const cplx A = mk(d.x, d.y), Bd = mk(d.z, d.w);
+        // adjoints of a_j, b_j except the a_{j+1}, b_{j+1} terms of g
+        const double fp = aP * f4;
+        cplx abar = mk(aE * f1, 0.) + a * (2. * aS * f1) + mk(v.x + v.z, v.y + v.w) * fp;
+        cplx bbar = mk(aE * f1, 0.) + b * (2. * aS * f1) + mk(v.x - v.z, v.y - v.w) * fp;
+        if (j < n1) {
+            abar = abar + b * (aG * f4);
+            bbar = bbar + a * (aG * f4);
+        }
+        if (j >= 2) {
+            const double4 cp = ld4(P.c4 + off + j - 2), dp = ld4(P.d4 + off + j - 2);
+            const double f3 = aG * fv3d(j - 1), hp = .5 / fv4d(j - 1) * f3;
+            abar = abar + mk(hp * (cp.x + cp.z), hp * (cp.y + cp.w));
+            bbar = bbar + mk(hp * (cp.x - cp.z), hp * (cp.y - cp.w));
+            // the a_j, b_j term of the adjoints of a_{j-1}, b_{j-1}
+            Z = Z + conjg(a) * mk(dp.x, dp.y) * f3 + conjg(b) * mk(dp.z, dp.w) * f3;
+        }
+        Z = Z + conjg(abar) * A + conjg(bbar) * Bd;
+    }
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) {
+        Z.re += __shfl_xor_sync(0xffffffffu, Z.re, o);
+        Z.im += __shfl_xor_sync(0xffffffffu, Z.im, o);
+    }
+    if (!on || lane) return;
     double *o = P.zr + (size_t) t * 3;
     o[0] = Z.re;   // dL/dmr of this radius
     o[1] = Z.im;   // dL/dmi
@@ -443,6 +503,30 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_final(Adj P) {
         }
         s = block_sum128(s, sh);
         if (threadIdx.x == 0) P.gout[2 * P.L + bb] = s;
+    }
+}
+
+// The kernels' numbers of half-angle tiles: 181, 91 and 37 angles take 12, 6
+// and 3, up to 255 angles 16.
+constexpr int ADJ_TILES[] = {1, 3, 6, 9, 12, 16};
+
+template <int NT>
+int launch_angles_nt(const Adj &P, cudaStream_t s) {
+    constexpr int SMEM = 4 * 2 * NT * 32 * 8;
+    static_assert(SMEM <= 48 * 1024, "no opt-in needed");
+    k_adj_angles<NT><<<(unsigned) P.L * P.G, ADJ_T, SMEM, s>>>(P);
+    LMIEB_CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+
+int launch_angles(const Adj &P, cudaStream_t s) {
+    switch (P.nt) {
+    case 1: return launch_angles_nt<1>(P, s);
+    case 3: return launch_angles_nt<3>(P, s);
+    case 6: return launch_angles_nt<6>(P, s);
+    case 9: return launch_angles_nt<9>(P, s);
+    case 12: return launch_angles_nt<12>(P, s);
+    default: return launch_angles_nt<16>(P, s);
     }
 }
 
@@ -484,110 +568,23 @@ extern "C" int lmie_solution_adjoint(int n_lambda, const double *lambda, const d
 
     const int L = n_lambda, nb = bins->n_bins, nq = bins->n_quad, R = nb * nq, na = n_angles;
     const int nhu = (na + 1) / 2, G = (R + ADJ_GR - 1) / ADJ_GR;
-    // ---- host tables ----
-    std::vector<double> rad(R), q(R), W(R);
-    std::vector<int> bin(R), bstart(nb + 1);
-    for (int b = 0; b < nb; ++b) {
-        bstart[b] = b * nq;
-        lmieb_gauss_leg(nq, bins->edges[b], bins->edges[b + 1], &rad[(size_t) b * nq], &q[(size_t) b * nq]);
-        for (int i = 0; i < nq; ++i) {
-            bin[b * nq + i] = b;
-            W[b * nq + i] = bins->weight[b] * q[b * nq + i];
-        }
-    }
-    bstart[nb] = R;
-    const size_t LR = (size_t) L * R;
-    std::vector<double> x(LR);
-    std::vector<int> n1(LR), n2(LR);
-    std::vector<long long> off(LR + 1), coff(LR + 1);
-    std::vector<cplx> mm(L);
-    off[0] = coff[0] = 0;
-    int n1max = 1;
-    // size parameters and truncations, one wavelength per task on the host's threads
-    struct XJob { const double *rad, *lambda, *mr, *mi; double *x; int *n1, *n2; int R; } xj{
-        rad.data(), lambda, mr, mi, x.data(), n1.data(), n2.data(), R};
-    lmieb_host_parallel(L, 64, [](void *arg, int k) {
-        const XJob &j = *(const XJob *) arg;
-        for (int r = 0; r < j.R; ++r) {
-            const size_t t = (size_t) k * j.R + r;
-            j.x[t] = 2. * LMIEB_PI * j.rad[r] / j.lambda[k];
-            j.n1[t] = lmieb_calc_n1(j.x[t]);
-            j.n2[t] = lmieb_calc_n2(j.n1[t], j.mr[k] * j.x[t], -j.mi[k] * j.x[t]);
-        }
-    }, &xj);
-    for (int k = 0; k < L; ++k) {
-        mm[k] = mk(mr[k], -mi[k]);
-        for (int r = 0; r < R; ++r) {
-            const size_t t = (size_t) k * R + r;
-            n1max = std::max(n1max, n1[t]);
-            off[t + 1] = off[t] + n1[t];
-            coff[t + 1] = coff[t] + (n1[t] + ADJ_K - 1) / ADJ_K;
-        }
-    }
-    const size_t smem_back = (size_t) 2 * n1max * sizeof(cplx) + (size_t) 4 * nhu * sizeof(cplx);
-    if (smem_back > 200 * 1024) {
-        fprintf(stderr, "ERROR: lmie_solution_adjoint(): size parameters up to %.0f exceed this build's limit\n",
-                *std::max_element(x.begin(), x.end()));
-        return -1;
-    }
-    // pi_n, tau_n at the half-angles theta_h = h 180 / (na - 1), h < nhu
-    std::vector<double> tab((size_t) n1max * nhu * 2);
-    for (int h = 0; h < nhu; ++h) {
-        const double mu = cos(h * LMIEB_PI / (na - 1));
-        double p0 = 0., p1 = 1.;
-        for (int n = 1; n <= n1max; ++n) {
-            tab[((size_t) (n - 1) * nhu + h) * 2] = p1;
-            tab[((size_t) (n - 1) * nhu + h) * 2 + 1] = n * mu * p1 - (n + 1.) * p0;
-            const double p2 = ((2. * n + 1.) * mu * p1 - (n + 1.) * p0) / n;
-            p0 = p1;
-            p1 = p2;
-        }
-    }
-    std::vector<double> tabt(tab.size());
-    for (int n = 1; n <= n1max; ++n)
-        for (int h = 0; h < nhu; ++h) {
-            tabt[((size_t) h * n1max + n - 1) * 2] = tab[((size_t) (n - 1) * nhu + h) * 2];
-            tabt[((size_t) h * n1max + n - 1) * 2 + 1] = tab[((size_t) (n - 1) * nhu + h) * 2 + 1];
-        }
-    std::vector<double> dw((size_t) L * na * 2, 0.), cw((size_t) L * 3);
-    for (int k = 0; k < L; ++k) {
-        cw[(size_t) k * 3] = weights[k].c_cext;
-        cw[(size_t) k * 3 + 1] = weights[k].c_csca;
-        cw[(size_t) k * 3 + 2] = weights[k].c_g;
-        for (int i = 0; i < na; ++i) {
-            dw[((size_t) k * na + i) * 2] = weights[k].d_p11 ? weights[k].d_p11[i] : 0.;
-            dw[((size_t) k * na + i) * 2 + 1] = weights[k].d_p12 ? weights[k].d_p12[i] : 0.;
-        }
-    }
-    const long long tot = off[LR], ctot = coff[LR];
-
-    // ---- staging: inputs in one pinned block, outputs in another ----
-    struct Piece { const void *src; size_t bytes; size_t at; };
-    std::vector<Piece> in;
+    // ---- inputs, in one pinned block; outputs in another part of it ----
     size_t in_bytes = 0;
-    auto add = [&](const void *p, size_t b) { in.push_back({p, b, in_bytes}); in_bytes += pad256(b); return in.size() - 1; };
-    const size_t i_lam = add(lambda, (size_t) L * 8), i_m = add(mm.data(), (size_t) L * 16);
-    const size_t i_W = add(W.data(), (size_t) R * 8), i_q = add(q.data(), (size_t) R * 8);
-    const size_t i_bin = add(bin.data(), (size_t) R * 4), i_bs = add(bstart.data(), (size_t) (nb + 1) * 4);
-    const size_t i_x = add(x.data(), LR * 8), i_n1 = add(n1.data(), LR * 4), i_n2 = add(n2.data(), LR * 4);
-    const size_t i_off = add(off.data(), (LR + 1) * 8), i_coff = add(coff.data(), (LR + 1) * 8);
-    const size_t i_tab = add(tab.data(), tab.size() * 8), i_dw = add(dw.data(), dw.size() * 8);
-    const size_t i_tabt = add(tabt.data(), tabt.size() * 8);
-    const size_t i_cw = add(cw.data(), cw.size() * 8);
+    auto take = [&](size_t bytes) { const size_t at = in_bytes; in_bytes += pad256(bytes); return at; };
+    int nt = (nhu + 7) / 8;                             // tiles of 8 half-angles, as many as there is a kernel for
+    for (int c : ADJ_TILES)
+        if (c >= nt) {
+            nt = c;
+            break;
+        }
+    const size_t LR = (size_t) L * R;
+    const size_t i_lam = take((size_t) L * 8), i_m = take((size_t) L * 16), i_W = take((size_t) R * 8);
+    const size_t i_q = take((size_t) R * 8), i_rad = take((size_t) R * 8), i_bs = take((size_t) (nb + 1) * 4);
+    const size_t i_n1 = take(LR * 4), i_n2 = take(LR * 4), i_ro = take(LR * 4), i_ko = take((size_t) L * 8);
+    const size_t i_mu = take((size_t) nhu * 8), i_dw = take((size_t) L * 8 * nt * 32), i_cw = take((size_t) L * 3 * 8);
     const size_t out_vals = (size_t) L * (3 + 2 * na) * 8, out_lw = (size_t) L * 8 * 8;
     const size_t out_g = (size_t) (2 * L + nb) * 8;
     const size_t out_bytes = pad256(out_vals) + pad256(out_lw) + pad256(out_g);
-    size_t dev_bytes = in_bytes + out_bytes;
-    const size_t b_cs = pad256((size_t) tot * 16), b_ck = pad256((size_t) ctot * 16), b_ckr = pad256((size_t) ctot * 8);
-    const size_t b_esg = pad256(LR * 4 * 8), b_pfp = pad256((size_t) L * G * na * 2 * 8), b_zr = pad256(LR * 3 * 8);
-    dev_bytes += 4 * b_cs + b_ck + b_ckr + b_esg + b_pfp + b_zr;
-    if (dev_bytes > g_dcap) {
-        if (g_dbuf) cudaFree(g_dbuf);
-        g_dbuf = nullptr;
-        g_dcap = 0;
-        LMIEB_CUDA_TRY(cudaMalloc((void **) &g_dbuf, dev_bytes));
-        g_dcap = dev_bytes;
-    }
     if (in_bytes + out_bytes > g_hcap) {
         if (g_hbuf) cudaFreeHost(g_hbuf);
         g_hbuf = nullptr;
@@ -595,60 +592,132 @@ extern "C" int lmie_solution_adjoint(int n_lambda, const double *lambda, const d
         LMIEB_CUDA_TRY(cudaMallocHost((void **) &g_hbuf, in_bytes + out_bytes));
         g_hcap = in_bytes + out_bytes;
     }
-    struct CopyJob { const Piece *in; char *dst; } cj{in.data(), g_hbuf};
-    lmieb_host_parallel((int) in.size(), 16, [](void *arg, int i) {
-        const CopyJob &j = *(const CopyJob *) arg;
-        memcpy(j.dst + j.in[i].at, j.in[i].src, j.in[i].bytes);
-    }, &cj);
+    char *const hb = g_hbuf;
+    double *rad = (double *) (hb + i_rad), *q = (double *) (hb + i_q), *W = (double *) (hb + i_W);
+    int *bstart = (int *) (hb + i_bs);
+    for (int b = 0; b < nb; ++b) {
+        bstart[b] = b * nq;
+        lmieb_gauss_leg(nq, bins->edges[b], bins->edges[b + 1], rad + (size_t) b * nq, q + (size_t) b * nq);
+        for (int i = 0; i < nq; ++i) W[b * nq + i] = bins->weight[b] * q[b * nq + i];
+    }
+    bstart[nb] = R;
+    // the half-angles theta_h = h 180 / (na - 1), h < nhu
+    double *mu = (double *) (hb + i_mu);
+    for (int h = 0; h < nhu; ++h) mu[h] = cos(h * LMIEB_PI / (na - 1));
+    // truncations and weights, one wavelength per task on the host's threads
+    std::vector<long long> orders(L);
+    std::vector<int> top(L);
+    struct XJob {
+        const double *rad, *lambda, *mr, *mi;
+        const lmie_loss_weights *weights;
+        double *lam;
+        cplx *m;
+        double *dw, *cw;
+        int *n1, *n2, *ro;
+        long long *orders;
+        int *top;
+        int R, na, nhu, nt;
+    } xj{rad, lambda, mr, mi, weights, (double *) (hb + i_lam), (cplx *) (hb + i_m), (double *) (hb + i_dw),
+         (double *) (hb + i_cw), (int *) (hb + i_n1), (int *) (hb + i_n2), (int *) (hb + i_ro), orders.data(), top.data(),
+         R, na, nhu, nt};
+    lmieb_host_parallel(L, 64, [](void *arg, int k) {
+        const XJob &j = *(const XJob *) arg;
+        const size_t t0 = (size_t) k * j.R;
+        long long sum = 0;
+        int top = 1;
+        for (int r = 0; r < j.R; ++r) {
+            const double x = 2. * LMIEB_PI * j.rad[r] / j.lambda[k];
+            const int n1 = lmieb_calc_n1(x);
+            j.n1[t0 + r] = n1;
+            j.n2[t0 + r] = lmieb_calc_n2(n1, j.mr[k] * x, -j.mi[k] * x);
+            j.ro[t0 + r] = (int) sum;
+            sum += n1;
+            top = std::max(top, n1);
+        }
+        j.orders[k] = sum;
+        j.top[k] = top;
+        j.lam[k] = j.lambda[k];
+        j.m[k] = mk(j.mr[k], -j.mi[k]);
+        const lmie_loss_weights &w = j.weights[k];
+        j.cw[(size_t) k * 3] = w.c_cext;
+        j.cw[(size_t) k * 3 + 1] = w.c_csca;
+        j.cw[(size_t) k * 3 + 2] = w.c_g;
+        double *dw = j.dw + (size_t) k * 8 * j.nt * 4;
+        memset(dw, 0, (size_t) 8 * j.nt * 32);
+        for (int i = 0; i < j.na; ++i) {
+            double *o = dw + (i < j.nhu ? 4 * i : 4 * (j.na - 1 - i) + 2);
+            o[0] = w.d_p11 ? .5 * w.d_p11[i] : 0.;
+            o[1] = w.d_p12 ? .5 * w.d_p12[i] : 0.;
+        }
+    }, &xj);
+    long long *ko = (long long *) (hb + i_ko), tot = 0;
+    int n1max = 1, k_top = 0;
+    for (int k = 0; k < L; ++k) {
+        ko[k] = tot;
+        tot += orders[k];
+        if (top[k] > n1max) {
+            n1max = top[k];
+            k_top = k;
+        }
+        if (orders[k] > INT_MAX) {
+            fprintf(stderr, "ERROR: lmie_solution_adjoint(): %lld orders of wavelength %d\n", orders[k], k);
+            return -1;
+        }
+    }
+    // the longest radii this solve accepts
+    if ((size_t) 2 * n1max * sizeof(cplx) + (size_t) 4 * nhu * sizeof(cplx) > 200 * 1024) {
+        fprintf(stderr, "ERROR: lmie_solution_adjoint(): size parameters up to %.0f exceed this build's limit\n",
+                2. * LMIEB_PI * *std::max_element(rad, rad + R) / lambda[k_top]);
+        return -1;
+    }
+    const int nrow = ((n1max + 7) & ~7) + 8;              // the kernel loads 8 orders ahead
+
+    size_t dev_bytes = in_bytes + out_bytes;
+    const size_t b_c = pad256((size_t) tot * 32), b_tab = pad256((size_t) nrow * nt * 8 * 16);
+    const size_t b_esg = pad256(LR * 4 * 8), b_pfp = pad256((size_t) L * G * na * 2 * 8), b_zr = pad256(LR * 3 * 8);
+    dev_bytes += 2 * b_tab + 3 * b_c + b_esg + b_pfp + b_zr;
+    if (dev_bytes > g_dcap) {
+        if (g_dbuf) cudaFree(g_dbuf);
+        g_dbuf = nullptr;
+        g_dcap = 0;
+        LMIEB_CUDA_TRY(cudaMalloc((void **) &g_dbuf, dev_bytes));
+        g_dcap = dev_bytes;
+    }
     char *d = g_dbuf;
-    auto dp = [&](size_t i) { return (void *) (d + in[i].at); };
+    auto dp = [&](size_t at) { return (void *) (d + at); };
     Adj P;
     memset(&P, 0, sizeof(P));
     P.L = L; P.R = R; P.na = na; P.nhu = nhu; P.G = G; P.n_bins = nb;
     P.lam = (const double *) dp(i_lam); P.m = (const cplx *) dp(i_m);
-    P.W = (const double *) dp(i_W); P.q = (const double *) dp(i_q); P.bin = (const int *) dp(i_bin);
+    P.W = (const double *) dp(i_W); P.q = (const double *) dp(i_q); P.rad = (const double *) dp(i_rad);
     P.bstart = (const int *) dp(i_bs);
-    P.x = (const double *) dp(i_x); P.n1 = (const int *) dp(i_n1); P.n2 = (const int *) dp(i_n2);
-    P.off = (const long long *) dp(i_off); P.coff = (const long long *) dp(i_coff);
-    P.tabt = (const double *) dp(i_tabt);
-    P.n1max = n1max;
-    P.tab = (const double *) dp(i_tab); P.dw = (const double *) dp(i_dw); P.cw = (const double *) dp(i_cw);
+    P.n1 = (const int *) dp(i_n1); P.n2 = (const int *) dp(i_n2);
+    P.ro = (const int *) dp(i_ro); P.ko = (const long long *) dp(i_ko);
+    P.mu = (const double *) dp(i_mu); P.nt = nt; P.nrow = nrow;
+    P.dw = (const double2 *) dp(i_dw); P.cw = (const double *) dp(i_cw);
     char *o = d + in_bytes;
     P.vals = (double *) o; o += pad256(out_vals);
     P.lw = (double *) o; o += pad256(out_lw);
     P.gout = (double *) o; o += pad256(out_g);
-    P.cs = (cplx *) o; o += b_cs;
-    P.cd = (cplx *) o; o += b_cs;
-    P.cbs = (cplx *) o; o += b_cs;
-    P.cbd = (cplx *) o; o += b_cs;
-    P.ckD = (cplx *) o; o += b_ck;
-    P.ckr = (double *) o; o += b_ckr;
+    P.c4 = (double4 *) o; o += b_c;
+    P.d4 = (double4 *) o; o += b_c;
+    P.b4 = (double4 *) o; o += b_c;
     P.esg = (double *) o; o += b_esg;
     P.pfp = (double *) o; o += b_pfp;
     P.zr = (double *) o; o += b_zr;
+    P.tabf = (double2 *) o; o += b_tab;
+    P.tabb = (double2 *) o; o += b_tab;
 
     // ---- run ----
     LMIEB_CUDA_TRY(cudaMemcpyAsync(d, g_hbuf, in_bytes, cudaMemcpyHostToDevice, s));
-    const size_t smem_fwd = (size_t) 2 * n1max * sizeof(cplx);
-    static size_t attr_fwd = 0, attr_back = 0;
-    if (smem_fwd > 48 * 1024 && smem_fwd > attr_fwd) {
-        LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_adj_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_fwd));
-        attr_fwd = smem_fwd;
-    }
-    if (smem_back > 48 * 1024 && smem_back > attr_back) {
-        LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_adj_back, cudaFuncAttributeMaxDynamicSharedMemorySize, (int) smem_back));
-        attr_back = smem_back;
-    }
-    const unsigned nthr = 64, nblk = ceil_div(LR, nthr);
-    k_adj_coef<<<nblk, nthr, 0, s>>>(P);
+    k_adj_coef<<<(unsigned) L * ((R + 63) / 64), 64, 0, s>>>(P);
     LMIEB_CUDA_TRY(cudaGetLastError());
-    k_adj_fwd<<<(unsigned) L * G, ADJ_T, smem_fwd, s>>>(P);
+    k_adj_table<<<1, 8 * nt, 0, s>>>(P);
     LMIEB_CUDA_TRY(cudaGetLastError());
+    if (launch_angles(P, s)) return -1;
     k_adj_lambda<<<L, ADJ_T, 0, s>>>(P);
     LMIEB_CUDA_TRY(cudaGetLastError());
-    k_adj_back<<<(unsigned) LR, ADJ_T, smem_back, s>>>(P);
-    LMIEB_CUDA_TRY(cudaGetLastError());
-    k_adj_m<<<nblk, nthr, 0, s>>>(P);
+    k_adj_m<<<ceil_div(8 * LR, 256), 256, 0, s>>>(P);
     LMIEB_CUDA_TRY(cudaGetLastError());
     k_adj_final<<<L + nb, ADJ_T, 0, s>>>(P);
     LMIEB_CUDA_TRY(cudaGetLastError());

@@ -20,10 +20,10 @@
 // u's recurrence, since u is not exactly psi (it starts from zero at n1) and the
 // reference differentiates what it computes.
 //
-// Files that include this are compiled without FMA contraction: every FMA is
-// written out, so a radius' coefficients are the same bits whichever kernel
-// forms them (derivatives near resonances carry a rounding of a recurrence to
-// 1e-12 of a case's cross section).
+// Every FMA is written out, and K1's and the cross sections' files are compiled
+// without FMA contraction, so a radius' coefficients are the same bits
+// whichever of them forms them (derivatives near resonances carry a rounding
+// of a recurrence to 1e-12 of a case's cross section).
 #pragma once
 
 #include "dev_common.cuh"
