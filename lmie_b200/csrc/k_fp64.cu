@@ -394,41 +394,81 @@ __global__ void k_reduce_pf(DevBatch B, long long total, const long long *__rest
 }
 
 // save_control 2 (single case): re-weight stored per-radius kernels
-// (src/lmie_schedule.c:1087-1124)
-__global__ void k_save_reweight_pf(DevBatch B, int n_qang, const double *__restrict__ save2,
-                                   const double *__restrict__ w2, double *__restrict__ pfacc) {
-    const size_t i = (size_t) blockIdx.x * blockDim.x + threadIdx.x;   // e*n_qang + jj
-    if (i >= (size_t) 4 * n_qang) return;
-    const int e = (int) (i / n_qang), jj = (int) (i % n_qang);
-    const int n = B.R;
-    double s = 0.;
-    for (int r = 0; r < n; ++r) s += save2[((size_t) e * n + r) * n_qang + jj] * B.w[r];
-    pfacc[(size_t) e * n_qang + jj] = s;
-    for (int k = 0; k < B.nd; ++k) {
-        double v = 0.;
-        bool idx2 = false;
-        for (int q = 0; q < B.nd2; ++q) idx2 |= B.idx2[q] == k;
-        if (idx2)
-            for (int r = 0; r < n; ++r) v += save2[((size_t) e * n + r) * n_qang + jj] * w2[(size_t) k * n + r];
-        pfacc[((size_t) (1 + k) * 4 + e) * n_qang + jj] = v;
+// (src/lmie_schedule.c:1087-1124).  Column 0 carries the weights, the columns
+// of the index2 derivatives theirs (w2), the others zero.
+__device__ __forceinline__ bool rw_has_column(const DevBatch &B, int col) {
+    bool on = col == 0;
+    for (int q = 0; q < B.nd2; ++q) on |= B.idx2[q] == col - 1;
+    return on;
+}
+
+// Bound by memory: the kernels [4][R][n_qang] are read once for RW_COLS columns.
+// A block takes RW_J angles of one element, its half-warps every 32nd radius
+// each, which keeps 32 KB in flight; their sums meet in shared memory.  2000
+// radii x 957 angles (61 MB), value and two derivatives: 45 us (a thread per
+// angle and element, column after column: 1190 us).
+constexpr int RW_T = 512, RW_J = 16, RW_COLS = 4;
+__global__ void __launch_bounds__(RW_T) k_save_reweight_pf(DevBatch B, int n_qang, const double *__restrict__ save2,
+                                                           const double *__restrict__ w2,
+                                                           double *__restrict__ pfacc) {
+    __shared__ double sh[RW_T / RW_J][RW_COLS][RW_J];
+    const int e = blockIdx.y, lj = threadIdx.x % RW_J, row = threadIdx.x / RW_J, n = B.R;
+    const int jj = blockIdx.x * RW_J + lj;
+    const double *src = save2 + (size_t) e * n * n_qang + min(jj, n_qang - 1);
+    for (int c0 = 0; c0 <= B.nd; c0 += RW_COLS) {
+        const double *w[RW_COLS];
+#pragma unroll
+        for (int c = 0; c < RW_COLS; ++c) {
+            const int col = c0 + c;
+            w[c] = col > B.nd || !rw_has_column(B, col) ? nullptr : (col == 0 ? B.w : w2 + (size_t) (col - 1) * n);
+        }
+        double s[RW_COLS] = {};
+#pragma unroll 8
+        for (int r = row; r < n; r += RW_T / RW_J) {
+            const double v = src[(size_t) r * n_qang];
+#pragma unroll
+            for (int c = 0; c < RW_COLS; ++c)
+                if (w[c]) s[c] += v * w[c][r];
+        }
+#pragma unroll
+        for (int c = 0; c < RW_COLS; ++c) sh[row][c][lj] = s[c];
+        __syncthreads();
+        if (row < RW_COLS && c0 + row <= B.nd && jj < n_qang) {
+            double v = 0.;
+            for (int k = 0; k < RW_T / RW_J; ++k) v += sh[k][row][lj];
+            pfacc[((size_t) (c0 + row) * 4 + e) * n_qang + jj] = v;
+        }
+        __syncthreads();
     }
 }
 
-__global__ void k_save_reweight_scal(DevBatch B, const double *__restrict__ save1, const double *__restrict__ w2,
-                                     double *__restrict__ sums) {
-    const int col = threadIdx.x;    // 0..nd
-    if (col > B.nd) return;
-    const int n = B.R;
+// A block per column (one warp of one block summing all: 316 us at 2000 radii).
+__global__ void __launch_bounds__(256) k_save_reweight_scal(DevBatch B, const double *__restrict__ save1,
+                                                            const double *__restrict__ w2,
+                                                            double *__restrict__ sums) {
+    __shared__ double sh[8][4];
+    const int col = blockIdx.x, n = B.R;
     double acc[4] = {0., 0., 0., 0.};
-    bool on = col == 0;
-    if (col > 0)
-        for (int q = 0; q < B.nd2; ++q) on |= B.idx2[q] == col - 1;
-    if (on)
-        for (int r = 0; r < n; ++r) {
-            const double a = col == 0 ? B.w[r] : w2[(size_t) (col - 1) * n + r];
+    if (rw_has_column(B, col)) {
+        const double *w = col == 0 ? B.w : w2 + (size_t) (col - 1) * n;
+        for (int r = threadIdx.x; r < n; r += 256) {
+            const double a = w[r];
+#pragma unroll
             for (int q = 0; q < 4; ++q) acc[q] += save1[(size_t) q * n + r] * a;
         }
-    for (int q = 0; q < 4; ++q) sums[col * 4 + q] = acc[q];
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+        if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5][q] = acc[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double v = 0.;
+        for (int k = 0; k < 8; ++k) v += sh[k][threadIdx.x];
+        sums[col * 4 + threadIdx.x] = v;
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1251,10 +1291,10 @@ int launch_reduce_pf(cudaStream_t s, const DevBatch &B, long long total, const l
 
 int launch_save_reweight(cudaStream_t s, const DevBatch &B, int n_qang, const double *save1, const double *save2,
                          const double *w2, double *sums, double *pfacc) {
-    k_save_reweight_scal<<<1, 32 * ceil_div(1 + B.nd, 32), 0, s>>>(B, save1, w2, sums);
+    k_save_reweight_scal<<<1 + B.nd, 256, 0, s>>>(B, save1, w2, sums);
     LMIEB_CUDA_TRY(cudaGetLastError());
     if (n_qang > 0) {
-        k_save_reweight_pf<<<ceil_div((size_t) 4 * n_qang, 128), 128, 0, s>>>(B, n_qang, save2, w2, pfacc);
+        k_save_reweight_pf<<<dim3(ceil_div(n_qang, RW_J), 4), RW_T, 0, s>>>(B, n_qang, save2, w2, pfacc);
         LMIEB_CUDA_TRY(cudaGetLastError());
     }
     return 0;
