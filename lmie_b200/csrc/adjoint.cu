@@ -102,7 +102,8 @@ __global__ void __launch_bounds__(64) k_adj_coef(Adj P) {
     const int n1 = P.n1[t], n2 = P.n2[t];
     const cplx m = P.m[k];
     MieRadius<false> c;
-    c.set(2. * LMIEB_PI * P.rad[r] / P.lam[k], m, cinv(m), 0., mk(0., 0.));
+    c.set_m(m, cinv(m), mk(0., 0.));
+    c.set_x(2. * LMIEB_PI * P.rad[r] / P.lam[k], 0.);
     const long long off = order_offset(P, k, r);
     double *const ck = (double *) (P.b4 + off);
     const int nb = n1 / MIE_B + 1;
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(64) k_adj_coef(Adj P) {
     sums.zero();
     MieAB prev;
     prev.a = prev.b = prev.am = prev.bm = prev.ax = prev.bx = mk(0., 0.);
+    double f4p = 0.;                                  // fv4 of the order before
     for (int b = 0; b < nb; ++b) {
         const double *w = ck + 7 * b;
         cplx D[MIE_B], Dz[MIE_B];
@@ -172,9 +174,9 @@ __global__ void __launch_bounds__(64) k_adj_coef(Adj P) {
         for (int i = 0; i < MIE_B; ++i) {
             const int j = b * MIE_B + i;
             if (j < 1 || j > n1) continue;
-            const double psi = spsi * ub[i] * su, f4 = fv4d(j);
+            const double psi = spsi * ub[i] * su, f4 = fv4d(j), f3 = (double) (j - 1) * (j + 1) / j;
             const MieAB q = mie_ab<true, false>(c, j, D[i], Dz[i], psi, psi_p, chi, chi_p, 0., 0.);
-            sums.add(j, q, prev);
+            sums.add(j, q, prev, f3, f4p);
             st4(P.c4 + off + j - 1, f4 * (q.a.re + q.b.re), f4 * (q.a.im + q.b.im), f4 * (q.a.re - q.b.re),
                 f4 * (q.a.im - q.b.im));
             st4(P.d4 + off + j - 1, q.am.re, q.am.im, q.bm.re, q.bm.im);
@@ -183,6 +185,7 @@ __global__ void __launch_bounds__(64) k_adj_coef(Adj P) {
             chi = chi_n;
             psi_p = psi;
             prev = q;
+            f4p = f4;
         }
     }
     double *o = P.esg + t * 4;

@@ -182,19 +182,6 @@ Ctx g_ctx;
 // lmieb_set_work_granularity (the autotuner).
 double g_items_per_sm[3] = {64., 2., 2.};
 
-// Whether K1 runs a block per radius (mie_radius.cuh) or a thread per radius.
-// The threads' time is that of the longest radius, about 1800 cycles an order
-// (900 without derivatives), as long as the radii do not fill the SMs; the
-// blocks' that of their rounds over the SMs, each about 30 cycles an order and
-// 4000 for the rest, at the occupancy their shared memory leaves.
-bool k1_by_block(int R, int n1max, bool hm, bool hx, bool tc, int sms) {
-    const int smem = mie_block_smem(n1max, hx);
-    if (tc || R == 0 || smem > MIE_BLOCK_SMEM) return false;
-    const int per_sm = std::min(2048 / MIE_BLOCK_T, 227 * 1024 / (smem + 1024));
-    const double rounds = std::ceil((double) R / (per_sm * sms));
-    return rounds * (30. * n1max + 4000.) < (hm ? 1800. : 900.) * n1max;
-}
-
 // Work of a sub-batch's angular sums (radii x orders x half-angles x Mie
 // columns) from which LMIEB_PRECISION_FP64 forms them with the seven-digit
 // contraction.
@@ -299,6 +286,45 @@ extern "C" void lmieb_host_parallel(int n, int n_threads, void (*fn)(void *, int
     host_pool().run(nt, body);
 }
 
+// K1's blocks (mie_radius.cuh): each has radii of one case, cases in the order
+// ord (first radius and number of radii of case c: rad(c)), n1(c, i): the
+// orders of its i-th radius from the largest down.  Returns the shared-memory
+// rows of a block, 0 for a thread per radius.  A radius to a block while that
+// makes no more than four blocks per SM, else as many as K1_ROWS rows hold (1000
+// rows: 729 instead of 596 us for 766 uneven cases).  A thread per radius, whose
+// time is that of the longest radius (0.8 us an order with derivatives,
+// 0.65 without), is as fast where the rows of the longest radii leave one or two
+// blocks to an SM and there are more than 36 rounds of them: x = 5000, 3000
+// radii 1.8 ms by blocks and 3.1 by threads, 8000 radii 4.7 and 3.8.
+template <class Orders>
+int k1_blocks(const std::vector<int> &ord, const std::vector<DevCase> &cs, int R, int n1max, bool hx, bool tc, int sms,
+              std::vector<int4> &blk, Orders &&n1) {
+    constexpr int K1_ROWS = 1500;
+    blk.clear();
+    const int rows = std::max(mie_block_rows(n1max), R > 4 * sms ? K1_ROWS : 0);
+    if (tc || R == 0 || mie_block_smem(rows, hx) > MIE_BLOCK_SMEM) return 0;
+    const int per_sm = std::min(8, 227 * 1024 / (mie_block_smem(rows, hx) + 1024));
+    const int most = R <= 4 * sms ? 1 : std::min(MIE_BLOCK_MAX, std::max(4, (R + 4 * sms - 1) / (4 * sms)));
+    if (per_sm < 3 && R > 36 * per_sm * sms) return 0;
+    // a case's blocks; counted first
+    auto cut = [&](int c, int4 *out) {
+        int nb = 0;
+        for (int i = 0; i < cs[c].nr; ++nb) {
+            const int n = std::min(std::min(most, cs[c].nr - i), std::max(1, rows / mie_block_rows(n1(c, i))));
+            if (out) out[nb] = make_int4(cs[c].r0 + cs[c].nr - 1 - i, n, c, 0);
+            i += n;
+        }
+        return nb;
+    };
+    const int ncase = (int) ord.size();
+    std::vector<int> at(ncase + 1, 0);
+    parallel_for(ncase, 64, [&](int k) { at[k + 1] = cut(ord[k], nullptr); });
+    for (int k = 0; k < ncase; ++k) at[k + 1] += at[k];
+    blk.resize(at[ncase]);
+    parallel_for(ncase, 64, [&](int k) { cut(ord[k], blk.data() + at[k]); });
+    return rows;
+}
+
 // memcpy of a large block on one host thread per core
 void par_memcpy(void *dst, const void *src, size_t bytes) {
     const size_t chunk = std::max((size_t) 256 << 10, (bytes / 16 + 4095) & ~(size_t) 4095);
@@ -381,8 +407,9 @@ struct Plan {
     int n_groups = 0;
     ExpItem *ex = nullptr;
     int n_ex = 0;
-    ExpItem *gx = nullptr;      // (case, 0, angle tile) of the GSF expansion runs, longest first
+    ExpItem *gx = nullptr;      // (case, first order tile, angle tile) of the GSF expansion runs, longest first
     int n_gx = 0;
+    int ex_run = 1, pu_lp = PU_LP;    // orders tiles per GSF run, orders per K5 block
     GatherSeg *gsegs = nullptr; // K1's outputs copied from an earlier sub-batch instead of computed
     int n_gseg = 0;
     long long *pf_start = nullptr, *ck_gc = nullptr, *ck_lc = nullptr, *fin_start = nullptr, *pu_start = nullptr;
@@ -982,6 +1009,10 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     for (int k = 0; k < ncase; ++k) k1ord[k] = k;
     std::stable_sort(k1ord.begin(), k1ord.end(), [&](int a, int b) { return cn1max[a] > cn1max[b]; });
     for (int k = 0; k < ncase; ++k) k1pre[k + 1] = k1pre[k] + ps[k1ord[k]].n;
+    std::vector<int4> k1_blk;
+    const int k1_rows = re_solve ? 0 : k1_blocks(k1ord, cs, R, n1max, hx, L.tc, c.sms, k1_blk, [&](int k, int i) {
+        return ps[k].n1r[ps[k].n - 1 - i];
+    });
 
     // ---- order tables ----
     std::vector<double> fv((size_t) 4 * (n1max + 2), 0.);
@@ -1405,18 +1436,38 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         for (int lt = 0; lt < nlt; ++lt)
             for (int at = 0; at < nat; ++at) *e++ = ExpItem{k, lt, at};
     });
-    // the GSF expansion runs one block per (case, angle tile) over all the
-    // case's orders: cases with the most orders first
+    // The GSF expansion runs one block per (case, angle tile) over all the
+    // case's orders: cases with the most orders first.  Where that leaves the
+    // device with fewer than EX_RUN_BLOCKS blocks per SM (three of them run on one
+    // at a time), the orders are cut into runs of ex_run tiles, as few of them
+    // as fill that: 950 orders and 479 half-angles took 97 us in 15 blocks and
+    // 30 us in 450; 1531 cases (2264 blocks a part) would only repeat the
+    // recurrences.
+    constexpr long long EX_RUN_BLOCKS = 6;
     static std::vector<ExpItem> gx;
     gx.clear();
+    L.ex_run = 1 << 20;
     if (L.want_gc) {
         std::vector<int> byn(ncase);
-        for (int k = 0; k < ncase; ++k) byn[k] = k;
+        int nlt, nat, nlt_max = 0;
+        for (int k = 0; k < ncase; ++k) {
+            byn[k] = k;
+            if (ex_tiles(cs[k], nlt, nat)) nlt_max = std::max(nlt_max, nlt);
+        }
+        for (int parts = 1; parts <= nlt_max; ++parts) {
+            const int run = (nlt_max + parts - 1) / parts;
+            long long blocks = 0;
+            for (int k = 0; k < ncase && blocks <= EX_RUN_BLOCKS * c.sms; ++k)
+                if (ex_tiles(cs[k], nlt, nat)) blocks += (long long) nat * ((nlt + run - 1) / run);
+            if (parts > 1 && blocks > EX_RUN_BLOCKS * c.sms) break;
+            if (parts > 1) L.ex_run = run;
+            if (blocks > EX_RUN_BLOCKS * c.sms) break;
+        }
         std::stable_sort(byn.begin(), byn.end(), [&](int a, int b) { return cs[a].n_coef > cs[b].n_coef; });
         for (int k : byn) {
-            int nlt, nat;
             if (!ex_tiles(cs[k], nlt, nat) || nlt == 0) continue;
-            for (int at = 0; at < nat; ++at) gx.push_back(ExpItem{k, 0, at});
+            for (int lt = 0; lt < nlt; lt += L.ex_run)
+                for (int at = 0; at < nat; ++at) gx.push_back(ExpItem{k, lt, at});
         }
     }
     L.nck_gc = ck_gc[ncase];
@@ -1432,6 +1483,19 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     std::vector<double> mu_user;
     std::unordered_map<int, long long> mu_at;
     size_t o_scal = 0, o_gc = 0, o_lc = 0, o_pf = 0;
+    // Orders per K5 block: as set; unset, PU_LP, or fewer where that leaves the
+    // device with fewer than PU_BLOCKS blocks per SM (950 orders, 181
+    // angles: 130 us in 12 blocks, 23 in 45).
+    constexpr long long PU_BLOCKS = 2;
+    L.pu_lp = g_pu_lp;
+    for (bool more = g_pu_lp == PU_LP; more && L.pu_lp > PU_T;) {
+        const int lp = L.pu_lp / 2;
+        long long blocks = 0;
+        for (int k = 0; k < ncase && blocks <= PU_BLOCKS * c.sms; ++k)
+            blocks += (long long) ((cs[k].n_angles + PU_T - 1) / PU_T) * ((cs[k].n_coef + lp - 1) / lp);
+        more = blocks <= PU_BLOCKS * c.sms;
+        if (more) L.pu_lp = lp;
+    }
     for (int k = 0; k < ncase; ++k) {
         DevCase &C = cs[k];
         if (C.n_angles > 0) {
@@ -1445,7 +1509,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             }
         }
         // K5: parts of PU_LP orders; the partial sums of a case of several
-        C.pu_parts = (L.pf_from && C.n_angles > 0) ? std::max(1, (C.n_coef + g_pu_lp - 1) / g_pu_lp) : 0;
+        C.pu_parts = (L.pf_from && C.n_angles > 0) ? std::max(1, (C.n_coef + L.pu_lp - 1) / L.pu_lp) : 0;
         C.pu_scr_off = pu_scr_total;
         const long long pu_n = (long long) ncol * 6 * C.n_angles;
         if (C.pu_parts > 1) pu_scr_total += C.pu_parts * pu_n;
@@ -1548,7 +1612,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         add(tg_nk.size() * 4); add(tg_off.size() * 8); add(oz_f2.size() * 8);
         add(a_start.size() * 8);
         for (int q = 0; q < 6; ++q) add((size_t) (ncase + 1) * 8);   // prefix arrays over the cases
-        add((size_t) ncase * 4); add((size_t) (ncase + 1) * 8);             // K1 launch order
+        add((size_t) ncase * 4); add((size_t) (ncase + 1) * 8); add(k1_blk.size() * sizeof(int4));   // K1 launch order and blocks
         add(gl_ns.size() * 4); add(gl_mo.size() * 8); add(gl_go.size() * 8); add(gl_pt.size() * 4);
         add(gl_pi.size() * 4); add(gl_guess.size() * 8); add(gl_jr.size() * 8);
         if (L.save_control == 2) {
@@ -1586,6 +1650,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         for (int i = 0; i < p.n; ++i) h_rcase[r0 + i] = k;
     }, host_cores());
     int *h_k1ord = put(hp, ho, k1ord.data(), (size_t) ncase);
+    int4 *h_k1blk = put(hp, ho, k1_blk.data(), k1_blk.size());
     long long *h_k1pre = put(hp, ho, k1pre.data(), (size_t) ncase + 1);
     long long *h_off = put(hp, ho, coff.data(), (size_t) R + 1);
     long long *h_ckoff = put(hp, ho, ckoff.data(), (size_t) R + 1);
@@ -1692,8 +1757,11 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     B.rs_m = 1;
     B.rs_x = 1 + 2 * (int) hm;
     B.oz_wl = wl;
-    B.k1_block = k1_by_block(R, n1max, hm, hx, L.tc, c.sms);
-    B.pu_lp = g_pu_lp;
+    B.k1_nblk = (int) k1_blk.size();
+    B.k1_rows = k1_rows;
+    B.k1_blk = (const int4 *) dptr(h_k1blk);
+    B.pu_lp = L.pu_lp;
+    B.ex_run = L.ex_run;
     B.cs = (const DevCase *) dptr(h_cs);
     B.idx1 = (const int *) dptr(h_i1);
     B.idx2 = (const int *) dptr(h_i2);

@@ -570,52 +570,81 @@ __device__ __forceinline__ double basis_next(int f, int l, const double *rc, dou
 // recurrence over all orders and checkpoints (p_{l-2}, p_{l-1}) at the start
 // of every EX_LT-order tile.
 // ---------------------------------------------------------------------------
-// one chain: function F of the set at node x over all n_coef orders
+// n orders of function F from order l on, their recurrence coefficients in rc
+// (shared memory); fully unrolled for whole tiles, so that the coefficients'
+// loads go ahead of the dependent steps
 template <int KIND, int F>
-__device__ __forceinline__ void ckpt_chain(const DevCase &C, int i, double x, const double *__restrict__ rc,
-                                           double *__restrict__ ck) {
-    constexpr int NF = KIND == 0 ? 4 : 1;
+__device__ __forceinline__ void chain_tile(int l, int n, double x, const double *rc, double &prev, double &cur) {
     constexpr int first = KIND == 1 ? 2 : 3;
-    double prev = 0., cur = 0.;
-    for (int lb = 0; lb < C.n_coef; lb += EX_LT) {
-        const size_t o = (((size_t) (lb / EX_LT) * NF + F) * C.nh + i) * 2;
-        ck[o] = prev;
-        ck[o + 1] = cur;
-        const int le = min(C.n_coef, lb + EX_LT);
-        int l = lb;
-        for (; l < le && l < first; ++l) {
-            const double v = basis_first<KIND>(F, l, x);
+    if (l >= first && n == EX_LT) {
+#pragma unroll
+        for (int u = 0; u < EX_LT; ++u) {
+            const double v = basis_step<KIND>(F, rc + 8 * u, x, cur, prev);
             prev = cur;
             cur = v;
         }
-        // the recurrence coefficients do not depend on the chain: unrolled,
-        // with the function fixed, their loads are issued ahead of the
-        // dependent steps
-#pragma unroll 8
-        for (; l < le; ++l) {
-            const double v = basis_step<KIND>(F, rc + 8 * (size_t) l, x, cur, prev);
-            prev = cur;
-            cur = v;
-        }
+        return;
+    }
+    for (int u = 0; u < n; ++u) {
+        const double v = l + u < first ? basis_first<KIND>(F, l + u, x) : basis_step<KIND>(F, rc + 8 * u, x, cur, prev);
+        prev = cur;
+        cur = v;
     }
 }
-
 template <int KIND>
-__global__ void k_exp_ckpt(DevBatch B, long long total, const long long *__restrict__ start,
-                           double *__restrict__ ckpt) {
-    const long long e = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= total) return;
-    const int c = find_case(start, B.ncase, e);
+__device__ __forceinline__ void chain_tile(int f, int l, int n, double x, const double *rc, double &prev, double &cur) {
+    if (KIND == 1 || f == 0) chain_tile<KIND, 0>(l, n, x, rc, prev, cur);
+    else if (f == 1) chain_tile<KIND, 1>(l, n, x, rc, prev, cur);
+    else if (f == 2) chain_tile<KIND, 2>(l, n, x, rc, prev, cur);
+    else chain_tile<KIND, 3>(l, n, x, rc, prev, cur);
+}
+
+// Bound by the latency of the chain (Legendre: three dependent operations of 9
+// cycles per order).  The coefficients come through shared memory, the next
+// tile's while this one's are used: loaded by each thread as it needed them,
+// an order took 200 cycles (30 bands of 161 radius sizes up to x = 162: 44 us,
+// now 11).
+constexpr int EX_CT = 128;
+template <int KIND>
+__global__ void __launch_bounds__(EX_CT) k_exp_ckpt(DevBatch B, long long total, const long long *__restrict__ start,
+                                                    double *__restrict__ ckpt) {
+    __shared__ double rcs[2][8 * EX_LT];
+    __shared__ int sh_max;
+    constexpr int NF = KIND == 0 ? 4 : 1, PER = 8 * EX_LT / EX_CT;
+    const long long e = (long long) blockIdx.x * EX_CT + threadIdx.x;
+    const int c = find_case(start, B.ncase, min(e, total - 1));
     const DevCase &C = B.cs[c];
+    const int ncf = e < total ? C.n_coef : 0;
+    if (threadIdx.x == 0) sh_max = 0;
+    __syncthreads();
+    atomicMax(&sh_max, ncf);
+    __syncthreads();
+    const int nmax = sh_max;
     const long long local = e - start[c];
-    const int f = (int) (local / C.nh), i = (int) (local % C.nh);
-    const double x = B.mu_pool[C.mu_off + C.nh + i];
-    double *ck = ckpt + C.ck_off;
-    if (KIND == 1) ckpt_chain<KIND, 0>(C, i, x, B.rc, ck);
-    else if (f == 0) ckpt_chain<KIND, 0>(C, i, x, B.rc, ck);
-    else if (f == 1) ckpt_chain<KIND, 1>(C, i, x, B.rc, ck);
-    else if (f == 2) ckpt_chain<KIND, 2>(C, i, x, B.rc, ck);
-    else ckpt_chain<KIND, 3>(C, i, x, B.rc, ck);
+    const int f = ncf ? (int) (local / C.nh) : 0, i = ncf ? (int) (local % C.nh) : 0;
+    const double x = ncf ? B.mu_pool[C.mu_off + C.nh + i] : 0.;
+    double *ck = ckpt + C.ck_off + ((size_t) f * C.nh + i) * 2;
+    double prev = 0., cur = 0., r[PER];
+    auto load = [&](int lb) {
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int t = q * EX_CT + threadIdx.x;
+            r[q] = t < 8 * (nmax - lb) ? B.rc[8 * (size_t) lb + t] : 0.;
+        }
+    };
+    load(0);
+    for (int lb = 0, p = 0; lb < nmax; lb += EX_LT, p ^= 1) {
+#pragma unroll
+        for (int q = 0; q < PER; ++q) rcs[p][q * EX_CT + threadIdx.x] = r[q];
+        __syncthreads();
+        if (lb + EX_LT < nmax) load(lb + EX_LT);
+        if (lb < ncf) {
+            double *o = ck + (size_t) (lb / EX_LT) * NF * C.nh * 2;
+            o[0] = prev;
+            o[1] = cur;
+            chain_tile<KIND>(f, lb, min(EX_LT, ncf - lb), x, rcs[p], prev, cur);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -639,8 +668,10 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
 
 // ---------------------------------------------------------------------------
 // K4 of the GSF expansion on the FP64 tensor cores (k_exp_gsf): one block of
-// 4 warps per (case, angle tile) runs over all the case's orders, a tile of
-// EX_LT orders at a time.  Thread (function f, node pair ia) continues its
+// 4 warps per (case, angle tile, B.ex_run order tiles) runs over these orders, a
+// tile of EX_LT at a time; where there are few blocks the orders are cut into
+// several runs, and a run's block first advances its recurrences from order 0
+// (9 cycles an order and function, a tile's products 3 us).  Thread (function f, node pair ia) continues its
 // basis recurrence from tile to tile in registers (no checkpoints), writing
 // the tile's values into shared memory; the weighted phase-matrix moments of
 // the block's node pairs are staged once; the recurrence coefficients of the
@@ -654,11 +685,13 @@ __device__ __forceinline__ void dmma(double &d0, double &d1, double a, double b)
 // ---------------------------------------------------------------------------
 constexpr int EX_NB = 4;                 // n-blocks of 8 outputs: up to 16 columns
 constexpr int EX_KS = EX_AT / 4;         // k-steps of 4 node pairs
+constexpr int EX_SKIP = 8;               // order tiles whose coefficients are staged at once before a run
 // one fragment (32 lanes) every EX_SEG doubles: a warp's fragment load reads
 // 32 consecutive doubles, and the staging stores of a warp (4 lanes of each
 // of 8 k-steps) fall on distinct bank pairs
 constexpr int EX_SEG = 36;
 constexpr int EX_AF = 4 * 2 * 2 * EX_KS * EX_SEG;   // basis fragments: [f][parity][m-block][k-step]
+static_assert(2 * EX_SKIP * 8 * EX_LT <= EX_AF, "two stages of coefficients in the fragments' place");
 
 // GSF function F of one node pair over the orders of a tile (u < lt, zeros
 // after), into its fragment positions (order u = par + 2 m: block par,
@@ -696,6 +729,8 @@ constexpr int EX_BSEG = 32;
 
 __host__ __device__ inline int ex_bf_run_size(int ncol) { return 2 * 4 * ((2 * ncol + 7) / 8) * EX_KS * EX_BSEG; }
 
+// RUNS: the orders are cut (its skipping of orders, compiled in, slowed whole runs by a fifth)
+template <bool RUNS>
 __global__ void __launch_bounds__(128) k_exp_gsf(DevBatch B, const ExpItem *__restrict__ items,
                                                 const double *__restrict__ pfn, double *__restrict__ exq) {
     extern __shared__ double sm[];
@@ -749,8 +784,9 @@ __global__ void __launch_bounds__(128) k_exp_gsf(DevBatch B, const ExpItem *__re
     const double x = i < nh ? mup[nh + i] : 0.;
     double prev = 0., cur = 0.;
     // the first tile's recurrence coefficients
-    const int nlt = (ncf + EX_LT - 1) / EX_LT;
-    for (int t = threadIdx.x; t < 8 * min(EX_LT, ncf); t += blockDim.x) rcs[t] = B.rc[t];
+    const int nlt = (ncf + EX_LT - 1) / EX_LT, lt0 = RUNS ? it.lt : 0;
+    for (int t = threadIdx.x; t < 8 * min(EX_LT, ncf - lt0 * EX_LT); t += blockDim.x)
+        rcs[(lt0 & 1) * 8 * EX_LT + t] = B.rc[8 * (size_t) lt0 * EX_LT + t];
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int par = warp & 1, mb = warp >> 1;
@@ -759,11 +795,37 @@ __global__ void __launch_bounds__(128) k_exp_gsf(DevBatch B, const ExpItem *__re
     const double *b0 = Bf + (size_t) par * 4 * nbn * EX_KS * EX_BSEG + lane;
     const int BS = nbn * EX_KS * EX_BSEG;                                         // stride of a slot
     double *out = exq + C.ex_off + (size_t) it.at * ncol * 6 * ncf;
-    for (int lt = 0; lt < nlt; ++lt) {
+    const int lte = RUNS ? min(nlt, it.lt + B.ex_run) : nlt;
+    if (RUNS && it.lt > 0) {
+        // up to the run's first tile, the coefficients of EX_SKIP tiles at a time
+        // in the basis fragments' place, the next ones' loads under way
+        constexpr int PER = EX_SKIP * 8 * EX_LT / 128;
+        double r[PER];
+        const int nskip = it.lt * EX_LT;
+        auto load = [&](int lb) {
+#pragma unroll
+            for (int q = 0; q < PER; ++q) {
+                const int t = q * 128 + threadIdx.x;
+                r[q] = t < 8 * (nskip - lb) ? B.rc[8 * (size_t) lb + t] : 0.;
+            }
+        };
+        load(0);
+        for (int lb = 0, p = 0; lb < nskip; lb += EX_SKIP * EX_LT, p ^= 1) {
+            double *sk = Af + p * (EX_SKIP * 8 * EX_LT);
+#pragma unroll
+            for (int q = 0; q < PER; ++q) sk[q * 128 + threadIdx.x] = r[q];
+            __syncthreads();
+            if (lb + EX_SKIP * EX_LT < nskip) load(lb + EX_SKIP * EX_LT);
+            for (int u = 0; u < EX_SKIP && lb + u * EX_LT < nskip; ++u)
+                chain_tile<0>(f, lb + u * EX_LT, EX_LT, x, sk + u * 8 * EX_LT, prev, cur);
+        }
+        __syncthreads();
+    }
+    for (int lt = lt0; lt < lte; ++lt) {
         const int l0 = lt * EX_LT, lc = min(EX_LT, ncf - l0);
         const double *rc = rcs + (lt & 1) * 8 * EX_LT;
         // the next tile's coefficients, loaded now and stored after the chain
-        const int l1 = l0 + EX_LT, lc1 = min(EX_LT, ncf - l1);
+        const int l1 = l0 + EX_LT, lc1 = lt + 1 < lte ? min(EX_LT, ncf - l1) : 0;
         const int t0 = threadIdx.x, t1 = threadIdx.x + 128;
         double r0 = 0., r1 = 0.;
         if (lc1 > 0) {
@@ -970,6 +1032,7 @@ __global__ void k_exp_final(DevBatch B, long long total, const long long *__rest
     const int col = (int) (local / ncf), l = (int) (local % ncf);
     const int nat = (C.nh + EX_AT - 1) / EX_AT;
     double v[6] = {0., 0., 0., 0., 0., 0.};
+#pragma unroll 4
     for (int at = 0; at < nat; ++at) {
         const double *q = exq + C.ex_off + ((size_t) at * ncol + col) * 6 * ncf + l;
 #pragma unroll
@@ -1001,23 +1064,53 @@ __global__ void k_exp_final(DevBatch B, long long total, const long long *__rest
 
 // ---------------------------------------------------------------------------
 // K5: phase matrix at the user's angles from the truncated expansion; one
-// block per (case, tile of PU_T user angles, part of B.pu_lp orders), one
-// thread per angle, cases with the most orders first.  A block runs the basis
-// recurrences from order 0 and sums the terms of its part's orders, so that a
-// case with many orders is spread over several blocks instead of one long
-// chain; a case of several parts writes their sums to scr, added up in order
+// block per (case, tile of PU_T user angles, part of B.pu_lp orders), cases
+// with the most orders first.  Four threads per angle: GSF, one for each basis
+// function with the outputs that it feeds; Legendre, one for each of four
+// groups of outputs, with a recurrence each.  A block runs its recurrences
+// from order 0 and sums the terms of its part's orders, so that a case with
+// many orders is spread over several blocks instead of one long chain (9
+// cycles an order before the part, GSF; a term's sums take several times
+// that); a case of several parts writes their sums to scr, added up in order
 // by k_phase_user_sum.  The basis functions of an order are generated once
 // per angle and used by up to CG columns at a time; the expansion
-// coefficients of those columns (GSF: with the a2 +- a3 pair combined) and the
-// recurrence coefficients of PU_T orders at a time are staged in shared
-// memory, which all threads read.
+// coefficients of those columns (GSF: with the a2 +- a3 pair combined) are
+// staged in shared memory, the recurrence coefficients of PU_T orders at a
+// time too, those of the next PU_T loaded while they are used.  950 orders,
+// 181 angles, five columns: 23 us (one thread per angle with all four
+// functions, parts of 256 orders: 130 us).
 // ---------------------------------------------------------------------------
+constexpr int PU_BT = 4 * PU_T;            // threads of a K5 block
+template <int KIND, int F, int CG, bool SUM>
+__device__ __forceinline__ void pu_orders(int l0, int lt, double x, const double *rc, const double (&cfs)[CG][6][PU_T],
+                                          double &prev, double &cur, double (&s)[CG][2]) {
+    // the outputs of function F (GSF: 1 and 2 are the sum's and the difference's pair), of group F
+    constexpr int EA = KIND == 0 ? (F == 0 ? 0 : F == 1 ? 4 : F - 1) : (F == 0 ? 0 : F == 1 ? 2 : F + 2);
+    constexpr int EB = F == 0 ? (KIND == 0 ? 3 : 1) : F == 1 ? (KIND == 0 ? 5 : 3) : -1;
+    constexpr int first = KIND == 1 ? 2 : 3;
+    auto order = [&](int u, double v) {
+        prev = cur;
+        cur = v;
+        if (SUM) {
+#pragma unroll
+            for (int g = 0; g < CG; ++g) {
+                s[g][0] += cfs[g][EA][u] * v;
+                if (EB >= 0) s[g][1] += cfs[g][EB < 0 ? 0 : EB][u] * v;
+            }
+        }
+    };
+    int u = 0;
+    for (; u < lt && l0 + u < first; ++u) order(u, basis_first<KIND>(F, l0 + u, x));
+#pragma unroll 8
+    for (; u < lt; ++u) order(u, basis_step<KIND>(F, rc + 8 * u, x, cur, prev));
+}
+
 template <int KIND, int CG>
-__global__ void __launch_bounds__(PU_T) k_phase_user(DevBatch B, const long long *__restrict__ start,
-                                                     const double *__restrict__ coefs,
-                                                     const int *__restrict__ trunc, double *__restrict__ out,
-                                                     double *__restrict__ scr) {
-    __shared__ double cfs[CG][6][PU_T], rcs[8 * PU_T];
+__global__ void __launch_bounds__(PU_BT) k_phase_user(DevBatch B, const long long *__restrict__ start,
+                                                      const double *__restrict__ coefs,
+                                                      const int *__restrict__ trunc, double *__restrict__ out,
+                                                      double *__restrict__ scr) {
+    __shared__ double cfs[CG][6][PU_T], rcs[2][8 * PU_T], pair[CG][PU_T];
     const int kr = find_case(start, B.ncase, blockIdx.x);
     const int c = B.k1ord[kr];
     const DevCase &C = B.cs[c];
@@ -1025,7 +1118,7 @@ __global__ void __launch_bounds__(PU_T) k_phase_user(DevBatch B, const long long
     const int ntile = (na + PU_T - 1) / PU_T;
     const int local = (int) (blockIdx.x - start[kr]);
     const int part = local / ntile, tile = local - part * ntile;
-    const int a = tile * PU_T + threadIdx.x;
+    const int f = threadIdx.x / PU_T, ta = threadIdx.x % PU_T, a = tile * PU_T + ta;
     const bool act = a < na;
     const int nt = trunc[c] > 0 ? ncf - trunc[c] + 1 : ncf;
     // this block's orders [lbeg, lend); the tiles of PU_T orders before lbeg
@@ -1035,87 +1128,77 @@ __global__ void __launch_bounds__(PU_T) k_phase_user(DevBatch B, const long long
     const double *cf0 = coefs + (KIND == 0 ? C.gc_off : C.lc_off);
     for (int g0 = 0; g0 < ncol; g0 += CG) {
         const int ng = min(CG, ncol - g0);
-        double s[CG][6];
+        double s[CG][2];
 #pragma unroll
-        for (int g = 0; g < CG; ++g)
+        for (int g = 0; g < CG; ++g) s[g][0] = s[g][1] = 0.;
+        double prev = 0., cur = 0., r[2];
+        auto load = [&](int l0) {
 #pragma unroll
-            for (int e = 0; e < 6; ++e) s[g][e] = 0.;
-        double q[4] = {0., 0., 0., 0.}, p[4] = {0., 0., 0., 0.};
-        for (int l0 = 0; l0 < lend; l0 += PU_T) {
+            for (int q = 0; q < 2; ++q) {
+                const int t = q * PU_BT + threadIdx.x;
+                r[q] = t < 8 * (lend - l0) ? B.rc[8 * (size_t) l0 + t] : 0.;
+            }
+        };
+        if (lbeg < lend) load(0);
+        for (int l0 = 0, p = 0; lbeg < lend && l0 < lend; l0 += PU_T, p ^= 1) {
             const int lt = min(PU_T, lend - l0);
             const bool sum = l0 >= lbeg;
-            __syncthreads();
-            for (int t = threadIdx.x; sum && t < ng * PU_T; t += PU_T) {
-                const int g = t / PU_T, u = t % PU_T;
-                const double *cf = cf0 + (size_t) (g0 + g) * 6 * ncf + l0 + u;
-                double v[6] = {0., 0., 0., 0., 0., 0.};
-                if (u < lt)
 #pragma unroll
-                    for (int e = 0; e < 6; ++e) v[e] = cf[(size_t) e * ncf];
-                if (KIND == 0) {
-                    const double a2 = v[1], a3 = v[2];
-                    v[1] = a2 + a3;
-                    v[2] = a2 - a3;
+            for (int q = 0; q < 2; ++q) rcs[p][q * PU_BT + threadIdx.x] = r[q];
+            if (sum) {
+                __syncthreads();          // the previous orders' coefficients have been used
+                for (int t = threadIdx.x; t < ng * PU_T; t += PU_BT) {
+                    const int g = t / PU_T, u = t % PU_T;
+                    const double *cf = cf0 + (size_t) (g0 + g) * 6 * ncf + l0 + u;
+                    double v[6] = {0., 0., 0., 0., 0., 0.};
+                    if (u < lt)
+#pragma unroll
+                        for (int e = 0; e < 6; ++e) v[e] = cf[(size_t) e * ncf];
+                    if (KIND == 0) {
+                        const double a2 = v[1], a3 = v[2];
+                        v[1] = a2 + a3;
+                        v[2] = a2 - a3;
+                    }
+#pragma unroll
+                    for (int e = 0; e < 6; ++e) cfs[g][e][u] = v[e];
                 }
-#pragma unroll
-                for (int e = 0; e < 6; ++e) cfs[g][e][u] = v[e];
             }
-            for (int t = threadIdx.x; t < 8 * lt; t += PU_T) rcs[t] = B.rc[8 * (size_t) l0 + t];
             __syncthreads();
-            for (int u = 0; u < lt; ++u) {
-                const int l = l0 + u;
-                const double *rl = rcs + 8 * u;                       // recurrence coefficients of order l
-                if (KIND == 0) {
-#pragma unroll
-                    for (int f = 0; f < 4; ++f) {
-                        const double v = l < 3 ? basis_first<0>(f, l, x) : basis_step<0>(f, rl, x, p[f], q[f]);
-                        q[f] = p[f];
-                        p[f] = v;
-                    }
-                    if (!sum) continue;
-#pragma unroll
-                    for (int g = 0; g < CG; ++g) {
-                        s[g][0] += cfs[g][0][u] * p[0];
-                        s[g][3] += cfs[g][3][u] * p[0];
-                        if (l >= 2) {
-                            s[g][4] += cfs[g][4][u] * p[1];
-                            s[g][5] += cfs[g][5][u] * p[1];
-                            s[g][1] += cfs[g][1][u] * p[2];
-                            s[g][2] += cfs[g][2][u] * p[3];
-                        }
-                    }
-                } else {
-                    const double v = l < 2 ? basis_first<1>(0, l, x) : basis_step<1>(0, rl, x, p[0], q[0]);
-                    q[0] = p[0];
-                    p[0] = v;
-                    if (!sum) continue;
-#pragma unroll
-                    for (int g = 0; g < CG; ++g)
-#pragma unroll
-                        for (int e = 0; e < 6; ++e) s[g][e] += cfs[g][e][u] * v;
-                }
+            if (l0 + PU_T < lend) load(l0 + PU_T);
+            const double *rc = rcs[p];
+            if (sum) {
+                if (f == 0) pu_orders<KIND, 0, CG, true>(l0, lt, x, rc, cfs, prev, cur, s);
+                else if (f == 1) pu_orders<KIND, 1, CG, true>(l0, lt, x, rc, cfs, prev, cur, s);
+                else if (f == 2) pu_orders<KIND, 2, CG, true>(l0, lt, x, rc, cfs, prev, cur, s);
+                else pu_orders<KIND, 3, CG, true>(l0, lt, x, rc, cfs, prev, cur, s);
+            } else {
+                if (f == 0) pu_orders<KIND, 0, CG, false>(l0, lt, x, rc, cfs, prev, cur, s);
+                else if (f == 1) pu_orders<KIND, 1, CG, false>(l0, lt, x, rc, cfs, prev, cur, s);
+                else if (f == 2) pu_orders<KIND, 2, CG, false>(l0, lt, x, rc, cfs, prev, cur, s);
+                else pu_orders<KIND, 3, CG, false>(l0, lt, x, rc, cfs, prev, cur, s);
             }
         }
+        __syncthreads();
+        if (KIND == 0 && f == 3)
+#pragma unroll
+            for (int g = 0; g < CG; ++g) pair[g][ta] = s[g][0];
+        __syncthreads();
         if (act) {
 #pragma unroll
             for (int g = 0; g < CG; ++g) {
                 if (g >= ng) break;
                 double *o = (C.pu_parts > 1 ? scr + C.pu_scr_off + (size_t) part * ncol * 6 * na
-                                            : out + C.pf_out_off) + (size_t) (g0 + g) * 6 * na;
-                if (KIND == 0) {
-                    o[a] = s[g][0];
-                    o[(size_t) 3 * na + a] = s[g][3];
-                    o[(size_t) 4 * na + a] = s[g][4];
-                    o[(size_t) 5 * na + a] = s[g][5];
-                    o[(size_t) 1 * na + a] = (s[g][1] + s[g][2]) / 2.;
-                    o[(size_t) 2 * na + a] = (s[g][1] - s[g][2]) / 2.;
+                                            : out + C.pf_out_off) + (size_t) (g0 + g) * 6 * na + a;
+                if (f < 2) {
+                    o[(size_t) (KIND == 0 ? 4 * f : 2 * f) * na] = s[g][0];
+                    o[(size_t) (KIND == 0 ? 3 + 2 * f : 2 * f + 1) * na] = s[g][1];
+                } else if (KIND == 0) {
+                    if (f == 2) {
+                        o[(size_t) 1 * na] = (s[g][0] + pair[g][ta]) / 2.;
+                        o[(size_t) 2 * na] = (s[g][0] - pair[g][ta]) / 2.;
+                    }
                 } else {
-                    o[a] = s[g][0];
-                    o[(size_t) 1 * na + a] = s[g][1];
-                    o[(size_t) 2 * na + a] = s[g][2];
-                    o[(size_t) 3 * na + a] = s[g][3];
-                    o[(size_t) 4 * na + a] = s[g][4];
-                    o[(size_t) 5 * na + a] = -s[g][5];
+                    o[(size_t) (2 + f) * na] = f == 3 ? -s[g][0] : s[g][0];
                 }
             }
         }
@@ -1200,12 +1283,14 @@ int run_expand(cudaStream_t s, const DevBatch &B, long long nck, const long long
         const size_t smm = sizeof(double) * ((size_t) EX_AF + ex_bf_run_size(ncol) + (size_t) 2 * 8 * EX_LT);
         static bool attr_mma = false;
         if (!attr_mma) {
-            LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_exp_gsf, cudaFuncAttributeMaxDynamicSharedMemorySize, SMAX));
+            LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_exp_gsf<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMAX));
+            LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_exp_gsf<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMAX));
             attr_mma = true;
         }
-        if (nruns > 0) k_exp_gsf<<<nruns, 128, smm, s>>>(B, runs, pfn, exq);
+        if (nruns > 0 && B.ex_run < 1 << 20) k_exp_gsf<true><<<nruns, 128, smm, s>>>(B, runs, pfn, exq);
+        else if (nruns > 0) k_exp_gsf<false><<<nruns, 128, smm, s>>>(B, runs, pfn, exq);
     } else {
-        k_exp_ckpt<KIND><<<ceil_div(nck, 128), 128, 0, s>>>(B, nck, ck_start, ckpt);
+        k_exp_ckpt<KIND><<<ceil_div(nck, EX_CT), EX_CT, 0, s>>>(B, nck, ck_start, ckpt);
         LMIEB_CUDA_TRY(cudaGetLastError());
         const int nt = std::min(EX_TMAX, std::max(128, (ncol * EX_LT + 31) / 32 * 32));
         k_exp_tile<KIND><<<nitems, nt, sm, s>>>(B, items, pfn, ckpt, exq);
@@ -1332,13 +1417,13 @@ int launch_phase_user(cudaStream_t s, const DevBatch &B, int kind, long long tot
     const int ncol = 1 + B.nd;
     const unsigned nb = (unsigned) total;
     if (kind == 0) {
-        if (ncol == 1) k_phase_user<0, 1><<<nb, PU_T, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
-        else if (ncol <= 3) k_phase_user<0, 3><<<nb, PU_T, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
-        else k_phase_user<0, 5><<<nb, PU_T, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
+        if (ncol == 1) k_phase_user<0, 1><<<nb, PU_BT, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
+        else if (ncol <= 3) k_phase_user<0, 3><<<nb, PU_BT, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
+        else k_phase_user<0, 5><<<nb, PU_BT, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
     } else {
-        if (ncol == 1) k_phase_user<1, 1><<<nb, PU_T, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
-        else if (ncol <= 3) k_phase_user<1, 3><<<nb, PU_T, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
-        else k_phase_user<1, 5><<<nb, PU_T, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
+        if (ncol == 1) k_phase_user<1, 1><<<nb, PU_BT, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
+        else if (ncol <= 3) k_phase_user<1, 3><<<nb, PU_BT, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
+        else k_phase_user<1, 5><<<nb, PU_BT, 0, s>>>(B, start, coefs, trunc, pf_out, scr);
     }
     LMIEB_CUDA_TRY(cudaGetLastError());
     if (nred > 0) {

@@ -138,13 +138,8 @@ __device__ __forceinline__ int radius_of(const DevBatch &B, long long t) {
 template <bool HX>
 __device__ __forceinline__ MieRadius<HX> radius_setup(const DevBatch &B, const DevCase &C, int r) {
     MieRadius<HX> c;
-    double xl = 1.;
-    cplx ml = mk(0., 0.);
-    if (HX && B.x_own) {
-        xl = B.xl[r];
-        ml = B.m_l[C.ml_off + B.idx1[0]];
-    }
-    c.set(B.x[r], C.m, C.minv, xl, ml);
+    c.set_m(C.m, C.minv, HX && B.x_own ? B.m_l[C.ml_off + B.idx1[0]] : mk(0., 0.));
+    c.set_x(B.x[r], HX && B.x_own ? B.xl[r] : 1.);
     return c;
 }
 
@@ -174,7 +169,7 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     const MieRadius<HX> c = radius_setup<HX>(B, C, r);
     const int nb = n1 / MIE_B + 1;
     double *ckr = ck + (size_t) B.ckoff[r] * CW;     // nb blocks of CW doubles
-    const double *fv4 = B.fv + 3 * (B.n1max + 2);
+    const double *fv4 = B.fv + 3 * (B.n1max + 2), *fv3 = fv4 - (B.n1max + 2);
 
     // ---- downward: P from n2, u from n1 (n2 > n1 + MIE_B), block by block ----
     double u0, ux0 = 0.;
@@ -267,7 +262,7 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
             if (j < 1 || j > n1) continue;
             const double psi = spsi * ub[i] * su, psix = HX ? c.xl * (fma(spsix, ub[i], spsi * uxb[HX ? i : 0]) * su) : 0.;
             const MieAB q = mie_ab<HM, HX>(c, j, D[i], Dz[i], psi, psi_p, chi_c, chi_p, psix, psix_p);
-            sums.add(j, q, prev);
+            sums.add(j, q, prev, fv3[j - 1], fv4[j - 1]);
             const double f4 = fv4[j];
             if (to_tc) {
                 tc_stage(tcbuf, n_tc, j, 0, (q.a + q.b) * f4, (q.a - q.b) * f4);
@@ -308,61 +303,98 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
 }
 
 // ---------------------------------------------------------------------------
-// K1 for few radii: a block per radius.
+// K1 by blocks: block i's B.k1_blk[i].y radii are of case .z, from radius .x
+// down.  Bound by instruction issue (half of it taken, a third of the FP64
+// pipe's) where the blocks are many, by the chains' latency where they are few.
+// 107 thousand radii, 777 cases, values only: 303 us (a thread per radius: 789);
+// 109 thousand, 766 cases, with the m column: 596 us (915); the cloud
+// droplet's 2000 radii up to x = 436: 41 us (a thread per radius 380).
 // ---------------------------------------------------------------------------
-template <bool HM, bool HX>
-__global__ void __launch_bounds__(MIE_BLOCK_T) k_mie_block(DevBatch B, double *__restrict__ coef,
+template <bool HM, bool HX, int TEAM>
+__global__ void __launch_bounds__(MIE_BLOCK_T, HX ? 2 : 4) k_mie_block(DevBatch B, double *__restrict__ coef,
                                                            double *__restrict__ rs) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int r = radius_of(B, blockIdx.x), R = B.R;
-    const MieRadius<HX> c = radius_setup<HX>(B, B.cs[B.rcase[r]], r);
-    const double *fv4 = B.fv + 3 * (B.n1max + 2);
-    const size_t tot = (size_t) B.tot, off = (size_t) B.off[r];
-    const bool re = B.oz_radexp != nullptr;
     constexpr int NC = 1 + HM + HX;
+    const int4 blk = B.k1_blk[blockIdx.x];
+    const DevCase &C = B.cs[blk.z];
+    const int R = B.R;
+    const double *fv4 = B.fv + 3 * (B.n1max + 2), *fv3 = fv4 - (B.n1max + 2);
+    const size_t tot = (size_t) B.tot;
+    const bool re = B.oz_radexp != nullptr;
     int mxe[NC][4];
 #pragma unroll
     for (int q = 0; q < 4 * NC; ++q) mxe[q / 4][q % 4] = 0;
-    MieSums<HM, HX> sums;
-    mie_block<HM, HX>(smem, c, B.n1r[r], B.n2r[r], B.n1max, sums, [&](int j, const MieAB &q) {
-        put_columns<HM, HX>(q, fv4[j], j, (double4 *) coef, tot, off, re, mxe);
-    });
-    if (threadIdx.x == 0)
+    int r = 0;                                        // the team's radius and its first order
+    size_t off = 0;
+    mie_block<HM, HX, TEAM>(
+        smem, B.k1_rows, blk.y,
+        [&](MieRadius<HX> &c) {
+            c.set_m(C.m, C.minv, HX && B.x_own ? B.m_l[C.ml_off + B.idx1[0]] : mk(0., 0.));
+        },
+        [&](int g, MieRadius<HX> &c, int &n1, int &n2) {
+            const int q = blk.x - g;
+            c.set_x(B.x[q], HX && B.x_own ? B.xl[q] : 1.);
+            n1 = B.n1r[q];
+            n2 = B.n2r[q];
+        },
+        [&](int n, double &f3, double &f4) {
+            f3 = fv3[n - 1];
+            f4 = fv4[n - 1];
+        },
+        [&](int g) {
+            r = blk.x - g;
+            off = (size_t) B.off[r];
+        },
+        [&](int j, const MieAB &q) { put_columns<HM, HX>(q, fv4[j], j, (double4 *) coef, tot, off, re, mxe); },
+        [&](const MieSums<HM, HX> &sums) {
+            if ((TEAM == 32 ? threadIdx.x & 31 : threadIdx.x) == 0)
 #pragma unroll
-        for (int q = 0; q < MieSums<HM, HX>::N; ++q) rs[(size_t) q * R + r] = sums.v[q];
-    if (re) {
-        // the largest exponents of the block
-        __shared__ int mx[MIE_BLOCK_T / 32][4 * NC];
+                for (int q = 0; q < MieSums<HM, HX>::N; ++q) rs[(size_t) q * R + r] = sums.v[q];
+            if (re) {
+                // the largest exponents of the team
+                __shared__ int mx[MIE_BLOCK_T / 32][4 * NC];
 #pragma unroll
-        for (int q = 0; q < 4 * NC; ++q) {
-            const int v = __reduce_max_sync(0xffffffffu, mxe[q / 4][q % 4]);
-            if ((threadIdx.x & 31) == 0) mx[threadIdx.x >> 5][q] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < 4 * NC) {
-            int v = 0;
-            for (int w = 0; w < MIE_BLOCK_T / 32; ++w) v = max(v, mx[w][threadIdx.x]);
-            B.oz_radexp[((size_t) (threadIdx.x / 4) * R + r) * 4 + threadIdx.x % 4] = v;
-        }
-    }
+                for (int q = 0; q < 4 * NC; ++q) {
+                    const int v = __reduce_max_sync(0xffffffffu, mxe[q / 4][q % 4]);
+                    mxe[q / 4][q % 4] = 0;
+                    if ((threadIdx.x & 31) == 0) mx[threadIdx.x >> 5][q] = v;
+                }
+                if (TEAM == 32) __syncwarp();
+                else __syncthreads();
+                const int l = TEAM == 32 ? threadIdx.x & 31 : threadIdx.x;
+                if (l < 4 * NC) {
+                    int v = 0;
+                    if (TEAM == 32) v = mx[threadIdx.x >> 5][l];
+                    else
+                        for (int w = 0; w < MIE_BLOCK_T / 32; ++w) v = max(v, mx[w][l]);
+                    B.oz_radexp[((size_t) (l / 4) * R + r) * 4 + l % 4] = v;
+                }
+                if (TEAM == 32) __syncwarp();
+            }
+        });
 }
 
-template <bool HM, bool HX>
+template <bool HM, bool HX, int TEAM>
 int launch_block(cudaStream_t s, const DevBatch &B, double *coef, double *rs) {
     static bool attr = false;
     if (!attr) {
-        LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_mie_block<HM, HX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_mie_block<HM, HX, TEAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             MIE_BLOCK_SMEM));
         attr = true;
     }
-    k_mie_block<HM, HX><<<B.R, MIE_BLOCK_T, mie_block_smem(B.n1max, HX), s>>>(B, coef, rs);
+    k_mie_block<HM, HX, TEAM><<<B.k1_nblk, MIE_BLOCK_T, mie_block_smem(B.k1_rows, HX), s>>>(B, coef, rs);
     LMIEB_CUDA_TRY(cudaGetLastError());
     return 0;
 }
 
 template <bool HM, bool HX>
 int launch(cudaStream_t s, const DevBatch &B, double *ck, double *coef, float *bop, double *rs) {
-    if (B.k1_block) return launch_block<HM, HX>(s, B, coef, rs);
+    // the orders of a radius by the whole block where it has one, or where they
+    // are many: means of 700 and 250 orders took 520 and 125 us that way, 667 and
+    // 112 us with a warp per radius
+    if (B.k1_nblk && (B.k1_nblk == B.R || B.tot >= 400LL * B.R))
+        return launch_block<HM, HX, MIE_BLOCK_T>(s, B, coef, rs);
+    if (B.k1_nblk) return launch_block<HM, HX, 32>(s, B, coef, rs);
     if (bop)
         k_mie<HM, HX, true><<<ceil_div(B.R, 64), 64, 4 * 8 * (1 + B.nd1) * 64 * sizeof(float), s>>>(B, ck, coef, bop, rs);
     else

@@ -38,13 +38,13 @@ constexpr double NA_MAX_X = 900.;
 struct Trunc {
     int2 n[NA_MAX_RADII];
 };
-static_assert(mie_block_smem(NA_MAX_ORDER, false) <= 48 * 1024, "shared memory of a block");
+static_assert(mie_block_smem(mie_block_rows(NA_MAX_ORDER), false) <= 48 * 1024, "shared memory of a block");
 
 // Bound by FP64 latency: the three chains of the largest radius (n1 dependent
 // pairs of FMAs), then n1 / 128 rounds of orders.  1000 radii up to x = 880: 66 us, the
 // whole call: 130 us (a thread per radius with D and psi in device memory: 1795).
 __global__ void __launch_bounds__(MIE_BLOCK_T) k_cross_sections(int n, const double *__restrict__ radius,
-                                                                double lambda, cplx m, cplx minv, int n1max,
+                                                                double lambda, cplx m, cplx minv, int rows,
                                                                 const __grid_constant__ Trunc trunc,
                                                                 double *__restrict__ out) {
     extern __shared__ __align__(16) unsigned char smem[];
@@ -55,17 +55,28 @@ __global__ void __launch_bounds__(MIE_BLOCK_T) k_cross_sections(int n, const dou
         if (threadIdx.x < 4) out[(size_t) threadIdx.x * n + i] = __longlong_as_double(0x7ff8000000000000LL);
         return;
     }
-    MieRadius<false> c;
-    c.set(2. * LMIEB_PI * radius[i] / lambda, m, minv, 0., mk(0., 0.));
-    MieSums<false, false> sums;
-    mie_block<false, false>(smem, c, nn.x, nn.y, n1max, sums, [](int, const MieAB &) {});
-    if (threadIdx.x == 0) {
-        const double lam2 = lambda * lambda / (2. * LMIEB_PI);
-        out[i] = sums.v[0] * lam2;
-        out[(size_t) n + i] = sums.v[1] * lam2;
-        out[(size_t) 2 * n + i] = norm2(mk(sums.v[2], sums.v[3])) * lam2 / (2. * 4. * LMIEB_PI);
-        out[(size_t) 3 * n + i] = sums.v[4] / sums.v[1] * 2.;
-    }
+    mie_block<false, false, MIE_BLOCK_T>(
+        smem, rows, 1,
+        [&](MieRadius<false> &c) { c.set_m(m, minv, mk(0., 0.)); },
+        [&](int, MieRadius<false> &c, int &n1, int &n2) {
+            c.set_x(2. * LMIEB_PI * radius[i] / lambda, 0.);
+            n1 = nn.x;
+            n2 = nn.y;
+        },
+        [](int n, double &f3, double &f4) {
+            f3 = (double) (n - 1) * (n + 1) / n;
+            f4 = n >= 2 ? (2. * n - 1.) / ((double) n * (n - 1)) : 0.;
+        },
+        [](int) {}, [](int, const MieAB &) {},
+        [&](const MieSums<false, false> &sums) {
+            if (threadIdx.x == 0) {
+                const double lam2 = lambda * lambda / (2. * LMIEB_PI);
+                out[i] = sums.v[0] * lam2;
+                out[(size_t) n + i] = sums.v[1] * lam2;
+                out[(size_t) 2 * n + i] = norm2(mk(sums.v[2], sums.v[3])) * lam2 / (2. * 4. * LMIEB_PI);
+                out[(size_t) 3 * n + i] = sums.v[4] / sums.v[1] * 2.;
+            }
+        });
 }
 
 }  // namespace
@@ -108,8 +119,9 @@ extern "C" int lmie_cross_sections_noalloc(int n_radii, const double *radius, do
         trunc.n[i] = make_int2(n1, n2);
         n1max = n1 > n1max ? n1 : n1max;
     }
-    k_cross_sections<<<n_radii, MIE_BLOCK_T, mie_block_smem(n1max, false), s>>>(n_radii, radius, lambda, m, 1. / m,
-                                                                                n1max, trunc, out);
+    const int rows = mie_block_rows(n1max);
+    k_cross_sections<<<n_radii, MIE_BLOCK_T, mie_block_smem(rows, false), s>>>(n_radii, radius, lambda, m, 1. / m, rows,
+                                                                               trunc, out);
     LMIEB_CUDA_TRY(cudaGetLastError());
     LMIEB_CUDA_TRY(cudaStreamSynchronize(s));
     if (bad) {

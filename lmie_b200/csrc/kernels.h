@@ -58,6 +58,7 @@ struct DevBatch {
     int nd, nd1, nd2;           // derivative layout (uniform over the batch)
     int n1max, ncmax;           // largest n1 and n_coef (table lengths)
     int pu_lp;                  // K5: orders per block (a multiple of PU_T)
+    int ex_run;                 // K4, GSF: order tiles per block
     const DevCase *cs;          // [ncase]
     const int *idx1, *idx2;     // [nd1], [nd2]
     const cplx *m_l;            // [ncase * nd]
@@ -73,7 +74,8 @@ struct DevBatch {
     // own), its sums likewise from the columns rs_m (d/dmr; rs_m + 1: d/dmi)
     // and rs_x.
     int t_m, t_x, x_own, rs_m, rs_x;
-    int k1_block;               // K1: a block per radius (mie_radius.cuh) instead of a thread
+    int k1_nblk, k1_rows;       // K1: blocks (0: a thread per radius) and the shared-memory rows of one
+    const int4 *k1_blk;         // [k1_nblk] blocks (mie_radius.cuh): largest radius, radii, case
     const double *w;            // [(1 + nd)][R] row 0: f = nr qw; row 1+kk: f_l (index1) or f_l2 (index2)
     const int *n1r, *n2r;       // [R]
     const long long *off;       // [R+1] prefix sums of n1r (coefficient storage)
@@ -173,9 +175,10 @@ struct ExpItem {
 };
 // ck_start: flat (case, half-angle, function) checkpoint-thread index space;
 // fin_start: flat (case, column, order) index space of the finalisation.
-// runs: (case, 0, angle tile) items of the GSF expansion on the FP64 tensor
-// cores, one block each over all the case's orders (used with kind 0 when the
-// columns fit it, see expand_gsf_launches; else the items and checkpoints).
+// runs: (case, first order tile, angle tile) items of the GSF expansion on the
+// FP64 tensor cores, one block each over B.ex_run order tiles (used with kind 0
+// when the columns fit it, see expand_gsf_launches; else the items and
+// checkpoints).
 // K1's outputs (coefficient columns, per-radius sums) copied in instead of
 // computed: one block per segment
 int launch_gather(cudaStream_t s, int nseg, const GatherSeg *segs, double *coef, double *rs);

@@ -30,19 +30,22 @@
 
 constexpr int MIE_B = 4;                              // orders per block of the recurrences (a power of two)
 
-// A block per radius: with a thread per radius a solve of few radii lasts as
-// long as its largest radius' recurrences and orders one after the other.
-// Three warps' first lanes run the three chains of the radius at the same time
-// into shared memory, and then all threads form the orders side by side.
+// A block's team for one radius or several: with a thread per radius a solve of
+// few radii lasts as long as its largest radius' recurrences and orders one
+// after the other, and one of many is held by the latency of an order (some 1800
+// cycles with derivatives).  Here three warps run the three chains of the
+// block's radii, a lane each, into shared memory, and then the orders are formed
+// side by side: by all threads for one radius (TEAM 128), a warp per radius
+// (TEAM 32) for several.
 constexpr int MIE_BLOCK_T = 128;
+constexpr int MIE_BLOCK_MAX = 32;                     // radii of a block
 constexpr int MIE_BLOCK_SMEM = 220 * 1024;            // what a block may take
 
-// bytes for radii of up to n1 orders: P, u, chi (and u's tangent), two exponents per MIE_B orders, the
-// coefficients passed from one round of orders to the next, reduction space
+// rows of shared memory of a radius of n1 orders; bytes of a block of that many rows: P, u, chi (and u's
+// tangent), two exponents per MIE_B orders, reduction space, what the team needs to know of each radius
 __host__ __device__ constexpr int mie_block_rows(int n1) { return (n1 + 2 * MIE_B) & ~(MIE_B - 1); }
-__host__ __device__ constexpr int mie_block_smem(int n1, bool hx) {
-    return mie_block_rows(n1) * (16 + 8 + 8 + (hx ? 8 : 0)) + mie_block_rows(n1) / MIE_B * 8 +
-           (MIE_BLOCK_T + 1) * (hx ? 96 : 64) + 20 * (MIE_BLOCK_T / 32) * 8;
+__host__ __device__ constexpr int mie_block_smem(int rows, bool hx) {
+    return rows * (16 + 8 + 8 + (hx ? 8 : 0)) + rows / MIE_B * 8 + (4 * 12 + 20 * 4) * 8 + MIE_BLOCK_MAX * 72;
 }
 
 #ifdef __CUDACC__
@@ -83,16 +86,19 @@ struct MieRadius {
     cplx m, minv, minv2, zinv, zinv2;
     double xl;                  // HX: the x column's direction (x_l, m_l)
     cplx ml;
-    __device__ __forceinline__ void set(double x_, cplx m_, cplx minv_, double xl_, cplx ml_) {
-        x = x_;
-        xinv = 1. / x;
+    // the refractive index (and its part of the x column's direction)
+    __device__ __forceinline__ void set_m(cplx m_, cplx minv_, cplx ml_) {
         m = m_;
         minv = minv_;
         minv2 = minv * minv;
+        ml = ml_;
+    }
+    __device__ __forceinline__ void set_x(double x_, double xl_) {
+        x = x_;
+        xinv = 1. / x;
         zinv = cinv(mk(m.re * x, m.im * x));
         zinv2 = zinv * zinv;
         xl = xl_;
-        ml = ml_;
     }
 };
 
@@ -107,10 +113,10 @@ struct MieP {
         hi = cur;
         cur = nx;
     }
-    // at the end of a block of orders; returns the exponent taken out
+    // at the end of a block of orders; returns the exponent taken out (of the
+    // older value: it is there while the newer one is still being formed)
     __device__ __forceinline__ int rescale() {
-        const int g = mb_exp(cur.re, cur.im);
-        if (g <= 40 && g >= -40) return 0;
+        const int e = mb_exp(hi.re, hi.im), g = e <= 40 && e >= -40 ? 0 : e;
         const double sc = mb_pow2(-g);
         cur = cur * sc;
         hi = hi * sc;
@@ -138,8 +144,7 @@ struct MieU {
         cur = nx;
     }
     __device__ __forceinline__ int rescale() {
-        const int g = mb_exp(cur, hi);
-        if (g <= 40 && g >= -40) return 0;
+        const int e = mb_exp(hi, hi), g = e <= 40 && e >= -40 ? 0 : e;
         const double sc = mb_pow2(-g);
         cur *= sc;
         hi *= sc;
@@ -211,11 +216,10 @@ struct MieSums {
 #pragma unroll
         for (int q = 0; q < N; ++q) v[q] = 0.;
     }
-    // order n, p the coefficients of order n - 1 (zeros for n = 1)
-    __device__ __forceinline__ void add(int n, const MieAB &q, const MieAB &p) {
+    // order n, p the coefficients of order n - 1 (zeros for n = 1); the asymmetry
+    // factors of order n - 1: f3 = (n^2 - 1) / n, f4 = (2n - 1) / (n (n - 1)) (n = 1: any finite ones)
+    __device__ __forceinline__ void add(int n, const MieAB &q, const MieAB &p, double f3, double f4) {
         const double f1 = 2. * n + 1., sgn = (n & 1) ? -f1 : f1;
-        // the asymmetry factors of order n - 1: (n^2 - 1) / n, (2n - 1) / (n (n - 1))
-        const double f3 = (double) (n - 1) * (n + 1) / n, f4 = n >= 2 ? (2. * n - 1.) / ((double) n * (n - 1)) : 0.;
         v[0] = fma(f1, q.a.re + q.b.re, v[0]);
         v[1] = fma(f1, rfmac(q.a, q.a, rmulc(q.b, q.b)), v[1]);
         v[2] = fma(sgn, q.a.re - q.b.re, v[2]);
@@ -253,136 +257,213 @@ struct MieSums {
     }
 };
 
-// The block's radius: n1 orders (the shared memory laid out for n1max), D_n
-// from n2.  store(n, ab) is called once per order, by one thread each; all
-// threads return with the sums.
-template <bool HM, bool HX, class Store>
-__device__ __forceinline__ void mie_block(unsigned char *smem, const MieRadius<HX> &c, int n1, int n2, int n1max,
-                                          MieSums<HM, HX> &sums, Store &&store) {
-    constexpr int T = MIE_BLOCK_T, NP = HX ? 12 : 8, NS = MieSums<HM, HX>::N;
-    const int rows = mie_block_rows(n1max), tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    double2 *P = (double2 *) smem;                    // [n1 + 2]
+// The block's radii, G of them (TEAM 128: one), of one refractive index, in
+// shared memory laid out for `rows`.  common(c) sets up what the radii share,
+// radius(g, c, n1, n2) radius g; factors(n, f3, f4) gives MieSums::add's;
+// begin(g) is called by a radius' team, then store(n, ab) once per order, by one
+// thread each, and sum(sums) by all its threads.
+template <bool HM, bool HX, int TEAM, class Common, class Radius, class Factors, class Begin, class Store, class Sum>
+__device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, Common &&common, Radius &&radius,
+                                          Factors &&factors, Begin &&begin, Store &&store, Sum &&sum) {
+    constexpr int T = MIE_BLOCK_T, W = T / 32, NP = HX ? 12 : 8, NS = MieSums<HM, HX>::N;
+    static_assert(TEAM == T || TEAM == 32, "the block or a warp");
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    double2 *P = (double2 *) smem;
     double *u = (double *) (P + rows), *chi = u + rows, *ux = chi + rows;
-    double *pass = chi + rows + (HX ? rows : 0);      // [T + 1][NP] coefficients of the round (entry 0: the order before)
-    double *red = pass + (T + 1) * NP;                // [20][T / 32]
-    int *eP = (int *) (red + 20 * (T / 32)), *eU = eP + rows / MIE_B;
-    __shared__ double sh_psi, sh_psix;                // psi_n = sh_psi u_n 2^(eU[n / MIE_B] - sh_eu)
-    __shared__ int sh_eu;
+    double *pass = chi + rows + (HX ? rows : 0);      // [W][12] last coefficients of a warp
+    double *red = pass + W * 12;                      // [20][W]
+    // psi_n = spsi u_n 2^(eU[n / MIE_B] - eu)
+    double *sh_psi = red + 20 * W, *sh_psix = sh_psi + MIE_BLOCK_MAX;
+    double *sh_x = sh_psix + MIE_BLOCK_MAX, *sh_xinv = sh_x + MIE_BLOCK_MAX, *sh_zr = sh_xinv + MIE_BLOCK_MAX;
+    double *sh_zi = sh_zr + MIE_BLOCK_MAX, *sh_xl = sh_zi + MIE_BLOCK_MAX;
+    int *sh_eu = (int *) (sh_xl + MIE_BLOCK_MAX), *sh_row = sh_eu + MIE_BLOCK_MAX, *sh_n1 = sh_row + MIE_BLOCK_MAX;
+    int *eP = sh_n1 + 2 * MIE_BLOCK_MAX, *eU = eP + rows / MIE_B;
 
-    if (warp == 0) {
-        if (lane == 0) {
+    MieRadius<HX> c;
+    common(c);
+    if (warp < 3) {
+        int n1 = 0, n2 = 0;
+        if (lane < G) radius(lane, c, n1, n2);
+        // first row: the rows of the radii before
+        const int own = lane < G ? mie_block_rows(n1) : 0;
+        int row = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, row, o);
+            if (lane >= o) row += v;
+        }
+        row -= own;
+        // The lanes' chains go block by block of MIE_B orders together, each at
+        // its own order; a chain's first block is entered at its order.
+        if (lane >= G) {
+        } else if (warp == 0) {
+            sh_row[lane] = row;
+            sh_n1[lane] = n1;
+            sh_x[lane] = c.x;
+            sh_xinv[lane] = c.xinv;
+            sh_zr[lane] = c.zinv.re;
+            sh_zi[lane] = c.zinv.im;
+            if (HX) sh_xl[lane] = c.xl;
             MieP p;
             p.hi = mk(1., 0.);                        // P_{n2} = 1, P_{n2 - 1} = n2 / z
             p.cur = (double) n2 * c.zinv;
-            for (int n = n2 - 1, e = 0; n >= 0;) {
-                const int b = n / MIE_B, n0 = b * MIE_B;
-                if (n0 <= n1 + 1) eP[b] = e;
-#pragma unroll 4
-                for (; n >= n0; --n) {
-                    if (n <= n1 + 1) P[n] = make_double2(p.cur.re, p.cur.im);
-                    p.step(p.next(n, c.zinv));
+            double2 *Pr = P + row;
+            int *er = eP + row / MIE_B, b = (n2 - 1) / MIE_B, e = 0;
+            for (int n = n2 - 1; n >= b * MIE_B; --n) p.step(p.next(n, c.zinv));   // n2 > n1 + 2 MIE_B
+            e += p.rescale();
+            for (--b; b * MIE_B > n1 + 1; --b) {
+#pragma unroll
+                for (int i = MIE_B - 1; i >= 0; --i) p.step(p.next(b * MIE_B + i, c.zinv));
+                e += p.rescale();
+            }
+            for (; b >= 0; --b) {
+                er[b] = e;
+#pragma unroll
+                for (int i = MIE_B - 1; i >= 0; --i) {
+                    Pr[b * MIE_B + i] = make_double2(p.cur.re, p.cur.im);
+                    p.step(p.next(b * MIE_B + i, c.zinv));
                 }
                 e += p.rescale();
             }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
+        } else if (warp == 1) {
             MieU<HX> q;
             q.start();
-            int e = 0;
-            for (int n = n1; n >= 0;) {
-                const int b = n / MIE_B, n0 = b * MIE_B;
-                eU[b] = e;
-#pragma unroll 4
-                for (; n >= n0; --n) {
-                    u[n] = q.cur;
-                    if (HX) ux[n] = q.xcur;
-                    q.step(n, c.xinv);
-                }
-                if (n >= 0) e += q.rescale();
+            double *ur = u + row, *uxr = ux + row;
+            int *er = eU + row / MIE_B, b = n1 / MIE_B, e = 0;
+            er[b] = 0;
+            for (int n = n1; n >= b * MIE_B; --n) {
+                ur[n] = q.cur;
+                if (HX) uxr[n] = q.xcur;
+                if (n > 0) q.step(n, c.xinv);
             }
-            sh_psi = sin(c.x) / u[0];
-            if (HX) sh_psix = fma(-sh_psi, ux[0], cos(c.x)) / u[0];
-            sh_eu = e;
-        }
-    } else if (warp == 2) {
-        if (lane == 0) {
+            for (--b; b >= 0; --b) {
+                e += q.rescale();
+                er[b] = e;
+#pragma unroll
+                for (int i = MIE_B - 1; i >= 0; --i) {
+                    ur[b * MIE_B + i] = q.cur;
+                    if (HX) uxr[b * MIE_B + i] = q.xcur;
+                    if (b + i > 0) q.step(b * MIE_B + i, c.xinv);
+                }
+            }
+            const double spsi = sin(c.x) / q.cur;
+            sh_psi[lane] = spsi;
+            if (HX) sh_psix[lane] = fma(-spsi, q.xcur, cos(c.x)) / q.cur;
+            sh_eu[lane] = e;
+        } else {
             double sinx, cosx;
             sincos(c.x, &sinx, &cosx);
             double lo = cosx, cur = fma(c.xinv, cosx, sinx);
-            chi[0] = lo;
+            double *cr = chi + row;
+            cr[0] = lo;
 #pragma unroll 4
             for (int n = 1; n <= n1; ++n) {
-                chi[n] = cur;
+                cr[n] = cur;
                 const double nx = fma((2. * n + 1.) * c.xinv, cur, -lo);
                 lo = cur;
                 cur = nx;
             }
         }
     }
-    if (tid < NP) pass[tid] = 0.;                     // order 0
     __syncthreads();
 
-    const double spsi = sh_psi, spsix = HX ? sh_psix : 0.;
-    const int eu0 = sh_eu;
-    sums.zero();
-    for (int j0 = 0; j0 < n1; j0 += T) {
-        const int j = j0 + tid + 1;
-        const bool on = j <= n1;
-        MieAB q;
-        q.a = q.b = q.am = q.bm = q.ax = q.bx = mk(0., 0.);
-        if (on) {
-            const double2 p1 = P[j], p0 = P[j - 1], p2 = P[j + 1];
-            const int e1 = eP[j / MIE_B];
-            cplx lo = mk(p0.x, p0.y), hi = mk(p2.x, p2.y), D, Dz;
-            if (j % MIE_B == 0) lo = lo * mb_pow2(eP[j / MIE_B - 1] - e1);
-            if (j % MIE_B == MIE_B - 1) hi = hi * mb_pow2(eP[j / MIE_B + 1] - e1);
-            mie_d<HM || HX>(c, j, lo, mk(p1.x, p1.y), hi, D, Dz);
-            const double s1 = mb_pow2(eU[j / MIE_B] - eu0), s0 = mb_pow2(eU[(j - 1) / MIE_B] - eu0);
-            const double psi = spsi * u[j] * s1, psi_p = spsi * u[j - 1] * s0;
-            double psix = 0., psix_p = 0.;
-            if (HX) {
-                psix = c.xl * (fma(spsix, u[j], spsi * ux[j]) * s1);
-                psix_p = c.xl * (fma(spsix, u[j - 1], spsi * ux[j - 1]) * s0);
+    for (int g = TEAM == 32 ? warp : 0; g < G; g += TEAM == 32 ? W : 1) {
+        begin(g);
+        const int n1 = sh_n1[g];
+        c.x = sh_x[g];
+        c.xinv = sh_xinv[g];
+        c.zinv = mk(sh_zr[g], sh_zi[g]);
+        c.zinv2 = c.zinv * c.zinv;
+        if (HX) c.xl = sh_xl[g];
+        const double spsi = sh_psi[g], spsix = HX ? sh_psix[g] : 0.;
+        const int eu0 = sh_eu[g], row = sh_row[g];
+        const double2 *Pr = P + row;
+        const double *ur = u + row, *uxr = ux + row, *cr = chi + row;
+        const int *er = eP + row / MIE_B, *eur = eU + row / MIE_B;
+        MieSums<HM, HX> sums;
+        sums.zero();
+        // the coefficients of the order before: from the lane before, for lane 0 from lane 31 of the warp before
+        // (order 0: zeros) or of the round before, kept in `last`
+        double last[NP];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) last[q] = 0.;
+        for (int j0 = 0; j0 < n1; j0 += TEAM) {
+            const int j = j0 + (TEAM == 32 ? lane : tid) + 1;
+            const bool on = j <= n1;
+            MieAB q;
+            q.a = q.b = q.am = q.bm = q.ax = q.bx = mk(0., 0.);
+            if (on) {
+                const double2 p1 = Pr[j], p0 = Pr[j - 1], p2 = Pr[j + 1];
+                const int e1 = er[j / MIE_B];
+                cplx lo = mk(p0.x, p0.y), hi = mk(p2.x, p2.y), D, Dz;
+                if (j % MIE_B == 0) lo = lo * mb_pow2(er[j / MIE_B - 1] - e1);
+                if (j % MIE_B == MIE_B - 1) hi = hi * mb_pow2(er[j / MIE_B + 1] - e1);
+                mie_d<HM || HX>(c, j, lo, mk(p1.x, p1.y), hi, D, Dz);
+                const double s1 = mb_pow2(eur[j / MIE_B] - eu0), s0 = mb_pow2(eur[(j - 1) / MIE_B] - eu0);
+                const double psi = spsi * ur[j] * s1, psi_p = spsi * ur[j - 1] * s0;
+                double psix = 0., psix_p = 0.;
+                if (HX) {
+                    psix = c.xl * (fma(spsix, ur[j], spsi * uxr[j]) * s1);
+                    psix_p = c.xl * (fma(spsix, ur[j - 1], spsi * uxr[j - 1]) * s0);
+                }
+                q = mie_ab<HM, HX>(c, j, D, Dz, psi, psi_p, cr[j], cr[j - 1], psix, psix_p);
+                store(j, q);
             }
-            q = mie_ab<HM, HX>(c, j, D, Dz, psi, psi_p, chi[j], chi[j - 1], psix, psix_p);
-            store(j, q);
-        }
-        double *ps = pass + (size_t) (tid + 1) * NP;
-        ps[0] = q.a.re; ps[1] = q.a.im; ps[2] = q.b.re; ps[3] = q.b.im;
-        if (HM) { ps[4] = q.am.re; ps[5] = q.am.im; ps[6] = q.bm.re; ps[7] = q.bm.im; }
-        if (HX) { ps[NP - 4] = q.ax.re; ps[NP - 3] = q.ax.im; ps[NP - 2] = q.bx.re; ps[NP - 1] = q.bx.im; }
-        __syncthreads();
-        if (on) {
-            const double *pv = pass + (size_t) tid * NP;
+            double v[12] = {q.a.re, q.a.im, q.b.re, q.b.im};
+            if (HM) { v[4] = q.am.re; v[5] = q.am.im; v[6] = q.bm.re; v[7] = q.bm.im; }
+            if (HX) { v[NP - 4] = q.ax.re; v[NP - 3] = q.ax.im; v[NP - 2] = q.bx.re; v[NP - 1] = q.bx.im; }
+            constexpr int NV = 4 * (1 + HM + HX);
+            if (TEAM != 32) {
+                if (lane == 31)
+#pragma unroll
+                    for (int k = 0; k < NP; ++k) pass[warp * 12 + k] = v[k];
+                __syncthreads();
+            }
             MieAB p;
-            p.a = mk(pv[0], pv[1]);
-            p.b = mk(pv[2], pv[3]);
             p.am = p.bm = p.ax = p.bx = mk(0., 0.);
-            if (HM) { p.am = mk(pv[4], pv[5]); p.bm = mk(pv[6], pv[7]); }
-            if (HX) { p.ax = mk(pv[NP - 4], pv[NP - 3]); p.bx = mk(pv[NP - 2], pv[NP - 1]); }
-            sums.add(j, q, p);
+            double w[12];
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                if (k >= NV && !(HX && k >= NP - 4)) continue;
+                w[k] = __shfl_sync(0xffffffffu, TEAM == 32 && lane == 31 ? last[k] : v[k], (lane + 31) & 31);
+                if (TEAM == 32) {
+                    last[k] = v[k];
+                } else {
+                    if (lane == 0) w[k] = warp == 0 ? last[k] : pass[(warp - 1) * 12 + k];
+                    last[k] = pass[(W - 1) * 12 + k];
+                }
+            }
+            p.a = mk(w[0], w[1]);
+            p.b = mk(w[2], w[3]);
+            if (HM) { p.am = mk(w[4], w[5]); p.bm = mk(w[6], w[7]); }
+            if (HX) { p.ax = mk(w[NP - 4], w[NP - 3]); p.bx = mk(w[NP - 2], w[NP - 1]); }
+            if (on) {
+                double f3, f4;
+                factors(j, f3, f4);
+                sums.add(j, q, p, f3, f4);
+            }
+            if (TEAM != 32) __syncthreads();
         }
-        __syncthreads();
-        // the round's last order for the next one
-        if (tid < NP) pass[tid] = pass[(size_t) T * NP + tid];
-        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < NS; ++q) {
+            double v = sums.v[q];
+#pragma unroll
+            for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            sums.v[q] = v;
+            if (TEAM != 32 && lane == 0) red[q * W + warp] = v;
+        }
+        if (TEAM != 32) {
+            __syncthreads();
+#pragma unroll
+            for (int q = 0; q < NS; ++q) {
+                sums.v[q] = red[q * W];
+#pragma unroll
+                for (int w = 1; w < W; ++w) sums.v[q] += red[q * W + w];
+            }
+        }
+        sums.close();
+        sum(sums);
     }
-#pragma unroll
-    for (int q = 0; q < NS; ++q) {
-        double v = sums.v[q];
-#pragma unroll
-        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (lane == 0) red[q * (T / 32) + warp] = v;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < NS; ++q) {
-        sums.v[q] = red[q * (T / 32)];
-#pragma unroll
-        for (int w = 1; w < T / 32; ++w) sums.v[q] += red[q * (T / 32) + w];
-    }
-    sums.close();
 }
 
 }  // namespace
