@@ -1279,7 +1279,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             if (!case_oz[k]) continue;
             C.nkx = (cn1max[k] + OZ_KC - 1) / OZ_KC;
             C.rx_off = rx_bytes;
-            C.trunc_band = C.accuracy > 0. ? oz_trunc_band(cn1max[k]) : 0.;
+            C.trunc_band = C.accuracy > 0. ? oz_trunc_band(cn1max[k], C.nr) : 0.;
             rx_bytes += 2LL * C.nh;
             // the A operand of each angle tile and chunk
             const int ntile = (C.nh + OZ_HALF - 1) / OZ_HALF;
