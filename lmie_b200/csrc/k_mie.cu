@@ -126,6 +126,43 @@ __device__ __forceinline__ void put_columns(const MieAB &q, double f4, int j, do
     if (HX) put((1 + HM) * HX, q.ax, q.bx);
 }
 
+// The columns of a split-precision case's order j in its operand (see tc_stage):
+// put(col, a + b, a - b), times fv4, of the value and the index1 derivatives.
+template <bool HM, bool HX, class Put>
+__device__ __forceinline__ void tc_columns(const DevBatch &B, const DevCase &C, int r, const MieAB &q, double f4,
+                                           Put &&put) {
+    put(0, (q.a + q.b) * f4, (q.a - q.b) * f4);
+    for (int k = 0; k < B.nd1; ++k) {
+        cplx va = mk(0., 0.), vb = va;
+        if (HM) {
+            const cplx ml = B.m_l[C.ml_off + B.idx1[k]];
+            va = ml * q.am;
+            vb = ml * q.bm;
+        }
+        if (HX) {
+            const double xc = B.x_own ? 1. : B.xl[(size_t) k * B.R + r];
+            va = cfma(q.ax, xc, va);
+            vb = cfma(q.bx, xc, vb);
+        }
+        put(1 + k, (va + vb) * f4, (va - vb) * f4);
+    }
+}
+
+// order j of column cc of the radius at position pos of its group, CC columns
+// in all (four lanes of consecutive orders write 16 bytes of each value)
+__device__ __forceinline__ void tc_put(float *__restrict__ rbase, int CC, int pos, int j, int cc, cplx cs, cplx cd) {
+    constexpr int P = TC_BPART / 4;
+    const int kc = (j - 1) / TC_KC, kk = (j - 1) - kc * TC_KC, n = (pos * CC + cc) * 2;
+    float *base = rbase + (size_t) kc * (TC_BSTAGE / 4);
+    const int i0 = tc_idx(n, kk, TC_NP), d0 = tc_idx(TC_NHALF + n, kk, TC_NP);
+    const double sg = (j & 1) ? 1. : -1.;             // s_j of D'
+    float h, l;
+    tc_split(cs.re, h, l); base[i0] = h; base[P + i0] = l;
+    tc_split(cs.im, h, l); base[i0 + 4] = h; base[P + i0 + 4] = l;
+    tc_split(sg * cd.re, h, l); base[d0] = h; base[P + d0] = l;
+    tc_split(sg * cd.im, h, l); base[d0 + 4] = h; base[P + d0 + 4] = l;
+}
+
 // the radius of rank t in the launch order: cases in the order k1ord, each from
 // its largest radius down
 __device__ __forceinline__ int radius_of(const DevBatch &B, long long t) {
@@ -265,21 +302,7 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
             sums.add(j, q, prev, fv3[j - 1], fv4[j - 1]);
             const double f4 = fv4[j];
             if (to_tc) {
-                tc_stage(tcbuf, n_tc, j, 0, (q.a + q.b) * f4, (q.a - q.b) * f4);
-                for (int k = 0; k < B.nd1; ++k) {
-                    cplx va = mk(0., 0.), vb = va;
-                    if (HM) {
-                        const cplx ml = B.m_l[C.ml_off + B.idx1[k]];
-                        va = ml * q.am;
-                        vb = ml * q.bm;
-                    }
-                    if (HX) {
-                        const double xc = B.x_own ? 1. : B.xl[(size_t) k * R + r];
-                        va = cfma(q.ax, xc, va);
-                        vb = cfma(q.bx, xc, vb);
-                    }
-                    tc_stage(tcbuf, n_tc, j, 1 + k, (va + vb) * f4, (va - vb) * f4);
-                }
+                tc_columns<HM, HX>(B, C, r, q, f4, [&](int cc, cplx cs, cplx cd) { tc_stage(tcbuf, n_tc, j, cc, cs, cd); });
                 if (((j - 1) & 3) == 3 || j == n1) tc_flush(tcbuf, tcb, n_tc, j, tpos, j == n1 ? tgnk : 0);
             } else {
                 put_columns<HM, HX>(q, f4, j, (double4 *) coef, tot, off, re != nullptr, mxe);
@@ -310,9 +333,10 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
 // 109 thousand, 766 cases, with the m column: 596 us (915); the cloud
 // droplet's 2000 radii up to x = 436: 41 us (a thread per radius 380).
 // ---------------------------------------------------------------------------
-template <bool HM, bool HX, int TEAM>
+template <bool HM, bool HX, bool TC, int TEAM>
 __global__ void __launch_bounds__(MIE_BLOCK_T, HX ? 2 : 4) k_mie_block(DevBatch B, double *__restrict__ coef,
-                                                           double *__restrict__ rs) {
+                                                                       float *__restrict__ bop,
+                                                                       double *__restrict__ rs) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int NC = 1 + HM + HX;
     const int4 blk = B.k1_blk[blockIdx.x];
@@ -324,8 +348,11 @@ __global__ void __launch_bounds__(MIE_BLOCK_T, HX ? 2 : 4) k_mie_block(DevBatch 
     int mxe[NC][4];
 #pragma unroll
     for (int q = 0; q < 4 * NC; ++q) mxe[q / 4][q % 4] = 0;
-    int r = 0;                                        // the team's radius and its first order
+    int r = 0, tcode = -1;                            // the team's radius, its operand position, its first order
     size_t off = 0;
+    float *tcb = nullptr;
+    constexpr int TS = TEAM == 32 ? 32 : MIE_BLOCK_T;
+    const int tl = threadIdx.x % TS;
     mie_block<HM, HX, TEAM>(
         smem, B.k1_rows, blk.y,
         [&](MieRadius<HX> &c) {
@@ -344,12 +371,27 @@ __global__ void __launch_bounds__(MIE_BLOCK_T, HX ? 2 : 4) k_mie_block(DevBatch 
         [&](int g) {
             r = blk.x - g;
             off = (size_t) B.off[r];
+            if (TC) {
+                tcode = B.tc_pos[r];
+                tcb = bop + B.tc_roff[r];
+            }
         },
-        [&](int j, const MieAB &q) { put_columns<HM, HX>(q, fv4[j], j, (double4 *) coef, tot, off, re, mxe); },
+        [&](int j, const MieAB &q) {
+            if (TC && tcode >= 0)
+                tc_columns<HM, HX>(B, C, r, q, fv4[j], [&](int cc, cplx cs, cplx cd) {
+                    tc_put(tcb, 1 + B.nd1, tcode & 255, j, cc, cs, cd);
+                });
+            else put_columns<HM, HX>(q, fv4[j], j, (double4 *) coef, tot, off, re, mxe);
+        },
         [&](const MieSums<HM, HX> &sums) {
             if ((TEAM == 32 ? threadIdx.x & 31 : threadIdx.x) == 0)
 #pragma unroll
                 for (int q = 0; q < MieSums<HM, HX>::N; ++q) rs[(size_t) q * R + r] = sums.v[q];
+            if (TC && tcode >= 0)
+                // zeros up to the end of the group's chunks (the operand buffer is not cleared between solves)
+                for (int j = B.n1r[r] + 1 + tl; j <= (tcode >> 8) * TC_KC; j += TS)
+                    for (int cc = 0; cc <= B.nd1; ++cc)
+                        tc_put(tcb, 1 + B.nd1, tcode & 255, j, cc, mk(0., 0.), mk(0., 0.));
             if (re) {
                 // the largest exponents of the team
                 __shared__ int mx[MIE_BLOCK_T / 32][4 * NC];
@@ -374,15 +416,15 @@ __global__ void __launch_bounds__(MIE_BLOCK_T, HX ? 2 : 4) k_mie_block(DevBatch 
         });
 }
 
-template <bool HM, bool HX, int TEAM>
-int launch_block(cudaStream_t s, const DevBatch &B, double *coef, double *rs) {
+template <bool HM, bool HX, bool TC, int TEAM>
+int launch_block(cudaStream_t s, const DevBatch &B, double *coef, float *bop, double *rs) {
     static bool attr = false;
     if (!attr) {
-        LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_mie_block<HM, HX, TEAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        LMIEB_CUDA_TRY(cudaFuncSetAttribute(k_mie_block<HM, HX, TC, TEAM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             MIE_BLOCK_SMEM));
         attr = true;
     }
-    k_mie_block<HM, HX, TEAM><<<B.k1_nblk, MIE_BLOCK_T, mie_block_smem(B.k1_rows, HX), s>>>(B, coef, rs);
+    k_mie_block<HM, HX, TC, TEAM><<<B.k1_nblk, MIE_BLOCK_T, mie_block_smem(B.k1_rows, HX), s>>>(B, coef, bop, rs);
     LMIEB_CUDA_TRY(cudaGetLastError());
     return 0;
 }
@@ -393,8 +435,11 @@ int launch(cudaStream_t s, const DevBatch &B, double *ck, double *coef, float *b
     // are many: means of 700 and 250 orders took 520 and 125 us that way, 667 and
     // 112 us with a warp per radius
     if (B.k1_nblk && (B.k1_nblk == B.R || B.tot >= 400LL * B.R))
-        return launch_block<HM, HX, MIE_BLOCK_T>(s, B, coef, rs);
-    if (B.k1_nblk) return launch_block<HM, HX, 32>(s, B, coef, rs);
+        return bop ? launch_block<HM, HX, true, MIE_BLOCK_T>(s, B, coef, bop, rs)
+                   : launch_block<HM, HX, false, MIE_BLOCK_T>(s, B, coef, bop, rs);
+    if (B.k1_nblk)
+        return bop ? launch_block<HM, HX, true, 32>(s, B, coef, bop, rs)
+                   : launch_block<HM, HX, false, 32>(s, B, coef, bop, rs);
     if (bop)
         k_mie<HM, HX, true><<<ceil_div(B.R, 64), 64, 4 * 8 * (1 + B.nd1) * 64 * sizeof(float), s>>>(B, ck, coef, bop, rs);
     else
