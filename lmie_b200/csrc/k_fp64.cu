@@ -66,27 +66,10 @@ __global__ void k_gauss(int npairs, const int *__restrict__ pt, const int *__res
     w[n - 1 - i] = w[i];
 }
 
-// ---------------------------------------------------------------------------
-// K2: one block per (case, output column); fixed-order block reduction over
-// the case's radii.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ double block_sum(double v, double *sh) {
-    const int t = threadIdx.x;
-    sh[t] = v;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (t < s) sh[t] += sh[t + s];
-        __syncthreads();
-    }
-    double r = sh[0];
-    __syncthreads();
-    return r;
-}
-
 __global__ void __launch_bounds__(256) k_reduce_scalars(DevBatch B, const double *__restrict__ rs,
                                                         double *__restrict__ sums,
                                                         double *__restrict__ save1) {
-    __shared__ double sh[256];
+    __shared__ double sh[4][8];
     const int cidx = blockIdx.x;
     const int col = blockIdx.y;           // 0 = value, 1+kk = slot kk
     const DevCase &C = B.cs[cidx];
@@ -100,7 +83,8 @@ __global__ void __launch_bounds__(256) k_reduce_scalars(DevBatch B, const double
     }
     const cplx ml = kind == 1 ? B.m_l[C.ml_off + col - 1] : mk(0., 0.);
     double acc[4] = {0., 0., 0., 0.};
-    for (int r = C.r0 + threadIdx.x; r < C.r0 + C.nr; r += blockDim.x) {
+#pragma unroll 4
+    for (int r = C.r0 + threadIdx.x; r < C.r0 + C.nr; r += 256) {
         const double f = B.w[r];
         const double se = rs[r], ss = rs[(size_t) R + r];
         const double sbr = rs[(size_t) 2 * R + r], sbi = rs[(size_t) 3 * R + r];
@@ -143,9 +127,17 @@ __global__ void __launch_bounds__(256) k_reduce_scalars(DevBatch B, const double
         }
     }
     const int ncol = 1 + B.nd;
+#pragma unroll
     for (int q = 0; q < 4; ++q) {
-        double v = block_sum(acc[q], sh);
-        if (threadIdx.x == 0) sums[((size_t) cidx * ncol + col) * 4 + q] = v;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], o);
+        if ((threadIdx.x & 31) == 0) sh[q][threadIdx.x >> 5] = acc[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double v = 0.;
+        for (int w = 0; w < 8; ++w) v += sh[threadIdx.x][w];
+        sums[((size_t) cidx * ncol + col) * 4 + threadIdx.x] = v;
     }
 }
 
