@@ -29,8 +29,11 @@ int lmie_solution_batch(int n_cases, lmie_in_data *in, lmie_out_data *out, int a
                         int verbose, int n_threads);
 
 /* Arithmetic of the batched solve.
- * LMIEB_PRECISION_FP64: every stage in FP64, the reference's arithmetic
- *   (within 1e-10 of it); lmie_solution and lmie_solution_batch use it.
+ * LMIEB_PRECISION_FP64: the reference's arithmetic (within 1e-10 of it);
+ *   lmie_solution and lmie_solution_batch use it.  Every stage runs in FP64 but
+ *   the angular S1/S2 sums of sub-batches with 2e7 products and more, which are
+ *   formed as LMIEB_PRECISION_INT8 does with seven digits (2^-53 of the largest
+ *   term of a row and column), closer to 64-bit truth than the FP64 kernel's.
  * LMIEB_PRECISION_TF32X3: the angular S1/S2 contraction runs on the tensor
  *   cores with each operand split into two TF32 terms (lo*hi + hi*lo + hi*hi):
  *   the hi*hi products accumulate in FP32 over segments of 32 orders
@@ -48,7 +51,7 @@ int lmie_solution_batch(int n_cases, lmie_in_data *in, lmie_out_data *out, int a
  *   bits and split into six signed 8-bit digits; the 21 digit products that
  *   carry the result are summed exactly in int32 and combined in FP64.  Each
  *   product carries about 2^-46 of the largest term of its row and column
- *   (FP64: 2^-53); everything else is the FP64 form's arithmetic.  A case
+ *   (FP64: 2^-53 of itself); everything else is the FP64 form's arithmetic.  A case
  *   whose truncation n_coef could depend on that difference -- some
  *   |beta_l| (l < n_coef) within the contraction's error bound of `accuracy`
  *   -- is solved again in FP64 within the same call, so n_coef is always the
@@ -83,7 +86,8 @@ int lmieb_get_split_segment(void);
 /* Orders per block of the phase matrix at the user angles (its tiles: 64 user
  * angles by this many orders; a case with more orders is spread over several
  * blocks whose sums are added in order): a multiple of 64 from 64 to 4096,
- * default 256; results differ only in the order of partial sums.  Returns 0
+ * default 256, which becomes 128 or 64 where that leaves the device with fewer
+ * than two blocks per SM; results differ only in the order of partial sums.  Returns 0
  * or -1. */
 int lmieb_set_user_angle_part(int orders);
 int lmieb_get_user_angle_part(void);
@@ -290,13 +294,11 @@ int lmieb_fp64_peak(double *tflops);
  * larger requests return -1 with an ERROR line (out-of-range radii get NaN).
  * The truncation orders n1, n2 of every radius are computed on the host with
  * the same formulas and libm as in lmie_solution (the radii are copied to the
- * host, the orders back into the static array below).
- * The work uses a fixed 24 MiB scratch array compiled into the library, which
- * every GPU that loads the library keeps until the process exits; no call
- * allocates or frees device memory.  All calls on a device share that array:
- * calls that overlap on the GPU (other threads, other streams) race on it.
- * The first call on a device looks up the array's device address; every call
- * copies the radii to the host and waits for `stream`.  Runs on the calling thread's current device on
+ * host, the orders go back with the kernel's arguments).
+ * The work uses shared memory only: no call allocates, frees or keeps device
+ * memory, and calls that overlap on the GPU (other threads, other streams)
+ * share nothing.  Every call copies the radii to the host and waits for
+ * `stream`.  Runs on the calling thread's current device on
  * `stream` (a cudaStream_t; NULL for the default stream) and returns after
  * the results are in `out`.  Returns 0 or -1. */
 int lmie_cross_sections_noalloc(int n_radii, const double *radius, double lambda,
