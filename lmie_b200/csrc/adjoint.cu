@@ -93,7 +93,7 @@ __device__ __forceinline__ double4 ld4(const double4 *p) {
 
 // ---- forward: coefficients, their derivatives, cross-section sums (thread per (k, r)) ----
 // K1's thread-per-radius form (k_mie.cu), with the checkpoints of a radius in
-// the place of its adjoints: 7 doubles for every 4 orders where those take 16.
+// the place of its adjoints: 5 doubles for every 4 orders where those take 16.
 __global__ void __launch_bounds__(64) k_adj_coef(Adj P) {
     const int nrb = (P.R + 63) / 64, k = blockIdx.x % P.L;
     const int r = (nrb - 1 - (int) (blockIdx.x / P.L)) * 64 + threadIdx.x;   // large radii first
@@ -110,30 +110,21 @@ __global__ void __launch_bounds__(64) k_adj_coef(Adj P) {
     double u0;
     int eu = 0;
     {
-        MieP p;
-        p.hi = mk(1., 0.);
-        p.cur = (double) n2 * c.zinv;
-        int n = n2 - 1;
-        for (const int n0 = nb * MIE_B; n >= n0; --n) {
-            p.step(p.next(n, c.zinv));
-            if (n % MIE_B == 0) p.rescale();
-        }
+        MieD p;
+        p.start();                                   // D_{n2} = 0, n2 > n1 + MIE_B
+        for (int n = n2 - 1; n >= nb * MIE_B; --n) p.step(n, c.zinv);
         MieU<false> q;
         q.start();
         for (int b = nb - 1; b >= 0; --b) {
-            double *w = ck + 7 * b;
-            w[0] = p.hi.re; w[1] = p.hi.im; w[2] = p.cur.re; w[3] = p.cur.im;
-            w[4] = q.hi; w[5] = q.cur; w[6] = (double) eu;
+            double *w = ck + 5 * b;
+            w[0] = p.cur.re; w[1] = p.cur.im; w[2] = q.hi; w[3] = q.cur; w[4] = (double) eu;
 #pragma unroll
             for (int i = MIE_B - 1; i >= 0; --i) {
                 const int n = b * MIE_B + i;
-                if (b > 0 || i > 0) p.step(p.next(n, c.zinv));
+                if (b > 0 || i > 0) p.step(n, c.zinv);
                 if (n <= n1 && (b > 0 || i > 0)) q.step(n, c.xinv);
             }
-            if (b > 0) {
-                p.rescale();
-                eu += q.rescale();
-            }
+            if (b > 0) eu += q.rescale();
         }
         u0 = q.cur;
     }
@@ -147,27 +138,26 @@ __global__ void __launch_bounds__(64) k_adj_coef(Adj P) {
     prev.a = prev.b = prev.am = prev.bm = prev.ax = prev.bx = mk(0., 0.);
     double f4p = 0.;                                  // fv4 of the order before
     for (int b = 0; b < nb; ++b) {
-        const double *w = ck + 7 * b;
+        const double *w = ck + 5 * b;
         cplx D[MIE_B], Dz[MIE_B];
         double ub[MIE_B];
-        const double su = mb_pow2((int) w[6] - eu);
-        MieP p;
-        p.hi = mk(w[0], w[1]);
-        p.cur = mk(w[2], w[3]);
+        const double su = mb_pow2((int) w[4] - eu);
+        MieD p;
+        p.cur = mk(w[0], w[1]);
         MieU<false> u;
-        u.hi = w[4];
-        u.cur = w[5];
+        u.hi = w[2];
+        u.cur = w[3];
 #pragma unroll
         for (int i = MIE_B - 1; i >= 0; --i) {
             const int n = b * MIE_B + i;
             ub[i] = u.cur;
             if (n > 0) {
-                const cplx lo = p.next(n, c.zinv);
+                p.step(n, c.zinv);
                 if (n <= n1) {
-                    mie_d<true>(c, n, lo, p.cur, p.hi, D[i], Dz[i]);
+                    D[i] = p.cur;
+                    Dz[i] = mie_dz(c, n, p.cur);
                     u.step(n, c.xinv);
                 }
-                p.step(lo);
             }
         }
 #pragma unroll

@@ -291,21 +291,23 @@ extern "C" void lmieb_host_parallel(int n, int n_threads, void (*fn)(void *, int
 // orders of its i-th radius from the largest down.  Returns the shared-memory
 // rows of a block, 0 for a thread per radius.  A radius to a block while that
 // makes no more than four blocks per SM, else as many as K1_ROWS rows hold (1000
-// rows: 729 instead of 596 us for 766 uneven cases).  A thread per radius, whose
-// time is that of the longest radius (0.8 us an order with derivatives,
-// 0.65 without), is as fast where the rows of the longest radii leave one or two
-// blocks to an SM and there are more than 36 rounds of them: x = 5000, 3000
-// radii 1.8 ms by blocks and 3.1 by threads, 8000 radii 4.7 and 3.8.
+// rows took a fifth more for 766 uneven cases).  A thread per radius, whose time
+// is that of the longest radius (0.8 us an order with derivatives, 0.65 without),
+// is the faster form where the rows of the longest radii leave one or two blocks
+// to an SM and there are many rounds of them, of 105 cycles an order with
+// derivatives and 18 without (mie_radius.cuh): x = 5000 without, 3000 radii 1.8 ms
+// by blocks and 3.1 by threads, 8000 radii 4.7 and 3.8; with, 1000 radii about 2
+// and 3.7 ms, 8000 radii 24 and 4.2.
 template <class Orders>
-int k1_blocks(const std::vector<int> &ord, const std::vector<DevCase> &cs, int R, int n1max, bool hx, int sms,
-              std::vector<int4> &blk, Orders &&n1) {
+int k1_blocks(const std::vector<int> &ord, const std::vector<DevCase> &cs, int R, int n1max, bool hm, bool hx,
+              int sms, std::vector<int4> &blk, Orders &&n1) {
     constexpr int K1_ROWS = 1500;
     blk.clear();
     const int rows = std::max(mie_block_rows(n1max), R > 4 * sms ? K1_ROWS : 0);
     if (R == 0 || mie_block_smem(rows, hx) > MIE_BLOCK_SMEM) return 0;
     const int per_sm = std::min(8, 227 * 1024 / (mie_block_smem(rows, hx) + 1024));
     const int most = R <= 4 * sms ? 1 : std::min(MIE_BLOCK_MAX, std::max(4, (R + 4 * sms - 1) / (4 * sms)));
-    if (per_sm < 3 && R > 36 * per_sm * sms) return 0;
+    if (per_sm < 3 && R > (hm || hx ? 8 : 36) * per_sm * sms) return 0;
     // a case's blocks; counted first
     auto cut = [&](int c, int4 *out) {
         int nb = 0;
@@ -1010,7 +1012,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     std::stable_sort(k1ord.begin(), k1ord.end(), [&](int a, int b) { return cn1max[a] > cn1max[b]; });
     for (int k = 0; k < ncase; ++k) k1pre[k + 1] = k1pre[k] + ps[k1ord[k]].n;
     std::vector<int4> k1_blk;
-    const int k1_rows = re_solve ? 0 : k1_blocks(k1ord, cs, R, n1max, hx, c.sms, k1_blk, [&](int k, int i) {
+    const int k1_rows = re_solve ? 0 : k1_blocks(k1ord, cs, R, n1max, hm, hx, c.sms, k1_blk, [&](int k, int i) {
         return ps[k].n1r[ps[k].n - 1 - i];
     });
 

@@ -196,7 +196,7 @@ __device__ __forceinline__ MieRadius<HX> radius_setup(const DevBatch &B, const D
 template <bool HM, bool HX, bool TC>
 __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck, double *__restrict__ coef,
                                             float *__restrict__ bop, double *__restrict__ rs) {
-    constexpr int CW = k1_ck_width(HX);              // P (4), u (2), exponent, u's tangent (2)
+    constexpr int CW = k1_ck_width(HX);              // D (2), u (2), exponent, u's tangent (2)
     const long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= B.R) return;
     const int r = radius_of(B, t);
@@ -212,31 +212,22 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     double u0, ux0 = 0.;
     int eu = 0;
     {
-        MieP p;
-        p.hi = mk(1., 0.);                           // P_{n2} = 1, P_{n2 - 1} = n2 / z
-        p.cur = (double) n2 * c.zinv;
-        int n = n2 - 1;
-        for (const int n0 = nb * MIE_B; n >= n0; --n) {
-            p.step(p.next(n, c.zinv));
-            if (n % MIE_B == 0) p.rescale();
-        }
+        MieD p;
+        p.start();                                   // D_{n2} = 0, n2 > n1 + MIE_B
+        for (int n = n2 - 1; n >= nb * MIE_B; --n) p.step(n, c.zinv);
         MieU<HX> q;
         q.start();
         for (int b = nb - 1; b >= 0; --b) {
             double *w = ckr + (size_t) b * CW;
-            w[0] = p.hi.re; w[1] = p.hi.im; w[2] = p.cur.re; w[3] = p.cur.im;
-            w[4] = q.hi; w[5] = q.cur; w[6] = (double) eu;
-            if (HX) { w[7] = q.xhi; w[CW - 1] = q.xcur; }
+            w[0] = p.cur.re; w[1] = p.cur.im; w[2] = q.hi; w[3] = q.cur; w[4] = (double) eu;
+            if (HX) { w[5] = q.xhi; w[CW - 1] = q.xcur; }
 #pragma unroll
             for (int i = MIE_B - 1; i >= 0; --i) {
                 const int k = b * MIE_B + i;
-                if (b > 0 || i > 0) p.step(p.next(k, c.zinv));
+                if (b > 0 || i > 0) p.step(k, c.zinv);
                 if (k <= n1 && (b > 0 || i > 0)) q.step(k, c.xinv);
             }
-            if (b > 0) {
-                p.rescale();
-                eu += q.rescale();
-            }
+            if (b > 0) eu += q.rescale();
         }
         u0 = q.cur;
         if (HX) ux0 = q.xcur;
@@ -269,27 +260,26 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
         const double *w = ckr + (size_t) b * CW;
         cplx D[MIE_B], Dz[MIE_B];
         double ub[MIE_B], uxb[HX ? MIE_B : 1];
-        const double su = mb_pow2((int) w[6] - eu);
+        const double su = mb_pow2((int) w[4] - eu);
         {
-            MieP p;
-            p.hi = mk(w[0], w[1]);
-            p.cur = mk(w[2], w[3]);
+            MieD p;
+            p.cur = mk(w[0], w[1]);
             MieU<HX> q;
-            q.hi = w[4];
-            q.cur = w[5];
-            if (HX) { q.xhi = w[7]; q.xcur = w[CW - 1]; }
+            q.hi = w[2];
+            q.cur = w[3];
+            if (HX) { q.xhi = w[5]; q.xcur = w[CW - 1]; }
 #pragma unroll
             for (int i = MIE_B - 1; i >= 0; --i) {
                 const int k = b * MIE_B + i;
                 ub[i] = q.cur;
                 if (HX) uxb[HX ? i : 0] = q.xcur;
                 if (k > 0) {
-                    const cplx lo = p.next(k, c.zinv);
+                    p.step(k, c.zinv);
                     if (k <= n1) {
-                        mie_d<HM || HX>(c, k, lo, p.cur, p.hi, D[i], Dz[i]);
+                        D[i] = p.cur;
+                        if (HM || HX) Dz[i] = mie_dz(c, k, p.cur);
                         q.step(k, c.xinv);
                     }
-                    p.step(lo);
                 }
             }
         }
@@ -330,8 +320,8 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
 // down.  Bound by instruction issue (half of it taken, a third of the FP64
 // pipe's) where the blocks are many, by the chains' latency where they are few.
 // 107 thousand radii, 777 cases, values only: 303 us (a thread per radius: 789);
-// 109 thousand, 766 cases, with the m column: 596 us (915); the cloud
-// droplet's 2000 radii up to x = 436: 41 us (a thread per radius 380).
+// 109 thousand, 766 cases, with the m column: 766 us (915); the cloud
+// droplet's 2000 radii up to x = 436: 69 us (a thread per radius 380).
 // ---------------------------------------------------------------------------
 template <bool HM, bool HX, bool TC, int TEAM>
 __global__ void __launch_bounds__(MIE_BLOCK_T, HX ? 2 : 4) k_mie_block(DevBatch B, double *__restrict__ coef,

@@ -22,7 +22,7 @@ struct GatherSeg {
 };
 // doubles per K1 checkpoint (k_mie.cu; one per MIE_B orders), hx: with the x
 // column of the tangent basis
-__host__ __device__ constexpr int k1_ck_width(bool hx) { return hx ? 9 : 7; }
+__host__ __device__ constexpr int k1_ck_width(bool hx) { return hx ? 7 : 5; }
 
 // One case of a batch (device copy).  Offsets index the batch-wide arrays.
 struct DevCase {

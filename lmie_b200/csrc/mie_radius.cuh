@@ -2,23 +2,27 @@
 // formulas of an order, shared by K1's two forms (k_mie.cu: a thread per radius,
 // a block per radius) and the device cross sections (k_noalloc.cu).
 //
-// The recurrences are run in their three-term forms,
-//     P_{n-1} = (2n + 1)/z P_n - P_{n+1}        downward from D_{n2} = 0 (D_n = P_{n-1}/P_n - n/z),
-//     u_{n-1} = (2n + 1)/x u_n - u_{n+1}        downward from psi_{n1} = 0 (psi_n = sin x u_n/u_0),
-//     chi_{n+1} = (2n + 1)/x chi_n - chi_{n-1}  upward,
-// with the starting values of the reference's ratio recurrences
-// (src/lmie_core.c:298-440), from which they differ by rounding only.  An order
-// costs two dependent FMAs of latency; the ratio forms wait for a reciprocal
-// (a division takes more than 100 cycles from operand to result), and the
-// reciprocal of P_n, from which D_n and dD/dz follow, is off the chain.  P and u
-// grow by many orders of magnitude, so both are brought back to order 1 at the
-// ends of blocks of MIE_B orders, by a power of two (exact).
+// The recurrences
+//     D_n = (n + 1)/z - 1 / (D_{n+1} + (n + 1)/z)   downward from D_{n2} = 0,
+//     u_{n-1} = (2n + 1)/x u_n - u_{n+1}            downward from psi_{n1} = 0 (psi_n = sin x u_n/u_0),
+//     chi_{n+1} = (2n + 1)/x chi_n - chi_{n-1}      upward,
+// have the starting values of the reference's (src/lmie_core.c:298-440), whose
+// psi runs in ratios: an order of u costs one dependent FMA, a ratio waits for a
+// reciprocal (60 cycles).  u grows by many orders of magnitude, so it is brought
+// back to order 1 at the ends of blocks of MIE_B orders, by a power of two
+// (exact).  Where only values are wanted, the blocks run D in a three-term form
+// too, P_{n-1} = (2n + 1)/z P_n - P_{n+1}, D_n = P_{n-1}/P_n - n/z: 18 cycles an
+// order instead of 105 (107 thousand radii 308 us instead of 495).  Its rounding
+// is another one, which values show by 1e-11 at most; derivatives at the
+// resonances of weakly absorbing spheres carry a rounding of D up to 1e-7 of
+// their value, as far as the reference's own, so with derivatives D is rounded as
+// it always was here.
 //
-// Derivatives: dD/dz = -1 + n/z^2 + rho (tau - 1/z), rho = P_{n-1}/P_n, tau =
-// P_{n+1}/P_n -- the Riccati equation without its difference of large terms, no
-// recurrence of its own; chi' = chi_{n-1} - n/x chi_n; psi' from the tangent of
-// u's recurrence, since u is not exactly psi (it starts from zero at n1) and the
-// reference differentiates what it computes.
+// Derivatives: dD/dz = n/z^2 - 1 + (n/z - D)(n/z + D), the Riccati equation with
+// its difference of large terms in factors, no recurrence of its own; chi' =
+// chi_{n-1} - n/x chi_n; psi' from the tangent of u's recurrence, since u is not
+// exactly psi (it starts from zero at n1) and the reference differentiates what
+// it computes.
 //
 // Every FMA is written out, and K1's and the cross sections' files are compiled
 // without FMA contraction, so a radius' coefficients are the same bits
@@ -41,7 +45,7 @@ constexpr int MIE_BLOCK_T = 128;
 constexpr int MIE_BLOCK_MAX = 32;                     // radii of a block
 constexpr int MIE_BLOCK_SMEM = 220 * 1024;            // what a block may take
 
-// rows of shared memory of a radius of n1 orders; bytes of a block of that many rows: P, u, chi (and u's
+// rows of shared memory of a radius of n1 orders; bytes of a block of that many rows: D, u, chi (and u's
 // tangent), two exponents per MIE_B orders, reduction space, what the team needs to know of each radius
 __host__ __device__ constexpr int mie_block_rows(int n1) { return (n1 + 2 * MIE_B) & ~(MIE_B - 1); }
 __host__ __device__ constexpr int mie_block_smem(int rows, bool hx) {
@@ -102,7 +106,8 @@ struct MieRadius {
     }
 };
 
-// The chain of P: cur = P_n, hi = P_{n+1}.
+// The chain of P, whose ratios are D (values only): P_{n-1} = (2n + 1)/z P_n - P_{n+1}, D_n = P_{n-1}/P_n - n/z;
+// cur = P_n, hi = P_{n+1}.
 struct MieP {
     cplx hi, cur;
     __device__ __forceinline__ cplx next(int n, cplx zinv) const {
@@ -121,6 +126,20 @@ struct MieP {
         cur = cur * sc;
         hi = hi * sc;
         return g;
+    }
+};
+
+// The chain of D_n (cur), from D_{n2} = 0.
+struct MieD {
+    cplx cur;
+    __device__ __forceinline__ void start() { cur = mk(0., 0.); }
+    // from D_{n + 1} to D_n
+    __device__ __forceinline__ void step(int n, cplx zinv) {
+        const double s = n + 1.;
+        const cplx g = mk(__dmul_rn(s, zinv.re), __dmul_rn(s, zinv.im));
+        const cplx e = mk(__dadd_rn(cur.re, g.re), __dadd_rn(cur.im, g.im));
+        const double d = 1. / fma(e.re, e.re, e.im * e.im);
+        cur = mk(__dsub_rn(g.re, __dmul_rn(e.re, d)), __dadd_rn(g.im, __dmul_rn(e.im, d)));
     }
 };
 
@@ -156,12 +175,11 @@ struct MieU {
     }
 };
 
-// D_n and, with TAN, dD/dz from P_{n-1}, P_n, P_{n+1} (scaled alike)
-template <bool TAN, bool HX>
-__device__ __forceinline__ void mie_d(const MieRadius<HX> &c, int n, cplx lo, cplx cur, cplx hi, cplx &D, cplx &Dz) {
-    const cplx inv = cinv(cur), rho = lo * inv, nz = (double) n * c.zinv;
-    D = rho - nz;
-    if (TAN) Dz = cfma(rho, cfma(hi, inv, -c.zinv), cfma(c.zinv2, (double) n, mk(-1., 0.)));
+// dD/dz of D_n
+template <bool HX>
+__device__ __forceinline__ cplx mie_dz(const MieRadius<HX> &c, int n, cplx D) {
+    const cplx nz = (double) n * c.zinv;
+    return cfma(nz - D, nz + D, cfma(c.zinv2, (double) n, mk(-1., 0.)));
 }
 
 // The coefficients of order n and their tangents: a, b; am, bm w.r.t. m; ax, bx
@@ -268,8 +286,8 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
     constexpr int T = MIE_BLOCK_T, W = T / 32, NP = HX ? 12 : 8, NS = MieSums<HM, HX>::N;
     static_assert(TEAM == T || TEAM == 32, "the block or a warp");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    double2 *P = (double2 *) smem;
-    double *u = (double *) (P + rows), *chi = u + rows, *ux = chi + rows;
+    double2 *Ds = (double2 *) smem;
+    double *u = (double *) (Ds + rows), *chi = u + rows, *ux = chi + rows;
     double *pass = chi + rows + (HX ? rows : 0);      // [W][12] last coefficients of a warp
     double *red = pass + W * 12;                      // [20][W]
     // psi_n = spsi u_n 2^(eU[n / MIE_B] - eu)
@@ -277,7 +295,8 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
     double *sh_x = sh_psix + MIE_BLOCK_MAX, *sh_xinv = sh_x + MIE_BLOCK_MAX, *sh_zr = sh_xinv + MIE_BLOCK_MAX;
     double *sh_zi = sh_zr + MIE_BLOCK_MAX, *sh_xl = sh_zi + MIE_BLOCK_MAX;
     int *sh_eu = (int *) (sh_xl + MIE_BLOCK_MAX), *sh_row = sh_eu + MIE_BLOCK_MAX, *sh_n1 = sh_row + MIE_BLOCK_MAX;
-    int *eP = sh_n1 + 2 * MIE_BLOCK_MAX, *eU = eP + rows / MIE_B;
+    int *eU = sh_n1 + 2 * MIE_BLOCK_MAX, *eP = eU + rows / MIE_B;
+    constexpr bool DER = HM || HX;                    // D itself in Ds, or P
 
     MieRadius<HX> c;
     common(c);
@@ -304,26 +323,36 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
             sh_zr[lane] = c.zinv.re;
             sh_zi[lane] = c.zinv.im;
             if (HX) sh_xl[lane] = c.xl;
-            MieP p;
-            p.hi = mk(1., 0.);                        // P_{n2} = 1, P_{n2 - 1} = n2 / z
-            p.cur = (double) n2 * c.zinv;
-            double2 *Pr = P + row;
-            int *er = eP + row / MIE_B, b = (n2 - 1) / MIE_B, e = 0;
-            for (int n = n2 - 1; n >= b * MIE_B; --n) p.step(p.next(n, c.zinv));   // n2 > n1 + 2 MIE_B
-            e += p.rescale();
-            for (--b; b * MIE_B > n1 + 1; --b) {
-#pragma unroll
-                for (int i = MIE_B - 1; i >= 0; --i) p.step(p.next(b * MIE_B + i, c.zinv));
-                e += p.rescale();
-            }
-            for (; b >= 0; --b) {
-                er[b] = e;
-#pragma unroll
-                for (int i = MIE_B - 1; i >= 0; --i) {
-                    Pr[b * MIE_B + i] = make_double2(p.cur.re, p.cur.im);
-                    p.step(p.next(b * MIE_B + i, c.zinv));
+            double2 *Dr = Ds + row;
+            if (DER) {
+                MieD p;
+                p.start();
+                for (int n = n2 - 1; n > n1; --n) p.step(n, c.zinv);
+                for (int n = n1; n >= 1; --n) {       // n2 > n1
+                    p.step(n, c.zinv);
+                    Dr[n] = make_double2(p.cur.re, p.cur.im);
                 }
+            } else {
+                MieP p;
+                p.hi = mk(1., 0.);                    // P_{n2} = 1, P_{n2 - 1} = n2 / z
+                p.cur = (double) n2 * c.zinv;
+                int *er = eP + row / MIE_B, b = (n2 - 1) / MIE_B, e = 0;
+                for (int n = n2 - 1; n >= b * MIE_B; --n) p.step(p.next(n, c.zinv));   // n2 > n1 + 2 MIE_B
                 e += p.rescale();
+                for (--b; b * MIE_B > n1; --b) {
+#pragma unroll
+                    for (int i = MIE_B - 1; i >= 0; --i) p.step(p.next(b * MIE_B + i, c.zinv));
+                    e += p.rescale();
+                }
+                for (; b >= 0; --b) {
+                    er[b] = e;
+#pragma unroll
+                    for (int i = MIE_B - 1; i >= 0; --i) {
+                        Dr[b * MIE_B + i] = make_double2(p.cur.re, p.cur.im);
+                        p.step(p.next(b * MIE_B + i, c.zinv));
+                    }
+                    e += p.rescale();
+                }
             }
         } else if (warp == 1) {
             MieU<HX> q;
@@ -377,9 +406,9 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
         if (HX) c.xl = sh_xl[g];
         const double spsi = sh_psi[g], spsix = HX ? sh_psix[g] : 0.;
         const int eu0 = sh_eu[g], row = sh_row[g];
-        const double2 *Pr = P + row;
+        const double2 *Dr = Ds + row;
         const double *ur = u + row, *uxr = ux + row, *cr = chi + row;
-        const int *er = eP + row / MIE_B, *eur = eU + row / MIE_B;
+        const int *eur = eU + row / MIE_B;
         MieSums<HM, HX> sums;
         sums.zero();
         // the coefficients of the order before: from the lane before, for lane 0 from lane 31 of the warp before
@@ -393,12 +422,16 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
             MieAB q;
             q.a = q.b = q.am = q.bm = q.ax = q.bx = mk(0., 0.);
             if (on) {
-                const double2 p1 = Pr[j], p0 = Pr[j - 1], p2 = Pr[j + 1];
-                const int e1 = er[j / MIE_B];
-                cplx lo = mk(p0.x, p0.y), hi = mk(p2.x, p2.y), D, Dz;
-                if (j % MIE_B == 0) lo = lo * mb_pow2(er[j / MIE_B - 1] - e1);
-                if (j % MIE_B == MIE_B - 1) hi = hi * mb_pow2(er[j / MIE_B + 1] - e1);
-                mie_d<HM || HX>(c, j, lo, mk(p1.x, p1.y), hi, D, Dz);
+                const double2 dj = Dr[j];
+                cplx D = mk(dj.x, dj.y), Dz = mk(0., 0.);
+                if (DER) {
+                    Dz = mie_dz(c, j, D);
+                } else {
+                    const double2 lo = Dr[j - 1];
+                    const int *er = eP + row / MIE_B;
+                    const double sc = j % MIE_B == 0 ? mb_pow2(er[j / MIE_B - 1] - er[j / MIE_B]) : 1.;
+                    D = mk(lo.x * sc, lo.y * sc) * cinv(D) - (double) j * c.zinv;
+                }
                 const double s1 = mb_pow2(eur[j / MIE_B] - eu0), s0 = mb_pow2(eur[(j - 1) / MIE_B] - eu0);
                 const double psi = spsi * ur[j] * s1, psi_p = spsi * ur[j - 1] * s0;
                 double psix = 0., psix_p = 0.;
