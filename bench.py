@@ -72,12 +72,12 @@ from lmie_b200 import abi, shard, workloads  # noqa: E402
 METRIC = "polydisperse solves/s (+Jacobian)"
 UNIT = "solves/s"
 N_CASES = 4096
-# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_angular /
-# k_angular_tc / k_angular_oz launch on this workload: measured with ncu on a
-# 256-case batch of the same generator and scaled by the ratio of angular work
-# (13.33; 13.0 in chunks of the int8 product: 317.6 MB -> 4.13 GB, about the
-# B operand digits read once).
-ANGULAR_TRAFFIC = {"fp64": 12.21e9, "tf32x3": 5.15e9, "int8": 4.13e9}
+# DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of one k_angular_oz
+# (seven and six digits) / k_angular_tc launch on this workload, measured with
+# ncu on smaller batches of the same generator and scaled: 1531 cases 1.82 GB,
+# 1000 cases 0.943 GB (about the B operand digits read once), both by the cases;
+# 256 cases by the ratio of angular work (13.33).
+ANGULAR_TRAFFIC = {"fp64": 4.87e9, "tf32x3": 5.15e9, "int8": 3.86e9}
 WORKLOAD = ("batched uneven: 4096 seeded cases (r_eff 0.05-20 um, v_eff 0.02-0.3, lambda 0.34-2.1 um, "
             "mr 1.33-1.60, mi 1e-8-0.1, gamma/log-normal, 100-2000 radii, x_max 0.2-1063), "
             "4 derivatives each (mr, mi, a1, a2), GSF + 181-angle phase matrix")
@@ -655,14 +655,17 @@ def run_b200(args) -> int:
         "fp64_equivalent_note": "algorithmic S1/S2 flops (8 per angle, order, radius, Mie column) per second "
                                 "of this kernel, against the FP64 FMA peak below",
         "fp64_fma_peak_tflops": fp64_peak.value}
-    ang64 = m64["stage_ms"]["angular"]
     fp64 = {k: m64[k] for k in ("value", "e2e", "unit", "ms_per_step", "stage_ms", "host_ms", "autotuned")}
+    k64_ms = m64["int8_kernel_ms"]
+    tops64 = m64["int8_ops"] / (k64_ms * 1e-3) / 1e12 if k64_ms > 0 else None
     fp64["roofline"] = {
-        "kernel": "k_angular (S1/S2 accumulation + phase-matrix forms, FP64)", "bound": "fp64",
-        "achieved": m64["flops"][0] / (ang64 * 1e-3) / 1e12 if ang64 > 0 else None, "peak": fp64_peak.value,
-        "unit": "TFLOP/s", "traffic": ANGULAR_TRAFFIC["fp64"],
-        "frac": (m64["flops"][0] / (ang64 * 1e-3) / 1e12 / fp64_peak.value) if ang64 > 0 else None,
-        "peak_source": "live FP64 FMA microbenchmark (lmieb_fp64_peak)"}
+        "kernel": "k_angular_oz, seven digits (the large S1/S2 sums of the FP64 form: 28 digit products per chunk of "
+                  "32 orders)",
+        "bound": "tensor", "achieved": tops64, "peak": int8_peak, "unit": "TOPS",
+        "frac": (tops64 / int8_peak) if (tops64 and int8_peak) else None, "traffic": ANGULAR_TRAFFIC["fp64"],
+        "peak_source": "dense int8 = 2x the measured bf16 burst in MEASURED_PEAKS.json (of measured)",
+        "ops_per_launch": m64["int8_ops"], "ms_per_launch": k64_ms,
+        "fp64_equivalent_tflops": m64["flops"][0] / (k64_ms * 1e-3) / 1e12 if k64_ms > 0 else None}
 
     single = split = plain = adj = stress = reweight = errs8 = None
     if rank == 0:
