@@ -31,7 +31,7 @@ int lmie_solution_batch(int n_cases, lmie_in_data *in, lmie_out_data *out, int a
 /* Arithmetic of the batched solve.
  * LMIEB_PRECISION_FP64: the reference's arithmetic (within 1e-10 of it);
  *   lmie_solution and lmie_solution_batch use it.  Every stage runs in FP64 but
- *   the angular S1/S2 sums of sub-batches with 2e7 products and more, which are
+ *   the angular S1/S2 sums of sub-batches with 2e6 products and more, which are
  *   formed as LMIEB_PRECISION_INT8 does with seven digits (2^-53 of the largest
  *   term of a row and column), closer to 64-bit truth than the FP64 kernel's.
  * LMIEB_PRECISION_TF32X3: the angular S1/S2 contraction runs on the tensor
