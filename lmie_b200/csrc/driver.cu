@@ -25,6 +25,7 @@
 #include <unistd.h>
 
 #include "host_pool.h"
+#include "k1_blocks.h"
 #include "kernels.h"
 #include "mie_radius.cuh"
 #include "oz_layout.cuh"
@@ -289,9 +290,9 @@ extern "C" void lmieb_host_parallel(int n, int n_threads, void (*fn)(void *, int
 }
 
 // K1's blocks (mie_radius.cuh): each has radii of one case, cases in the order
-// ord (first radius and number of radii of case c: rad(c)), n1(c, i): the
-// orders of its i-th radius from the largest down.  Returns the shared-memory
-// rows of a block, 0 for a thread per radius.  A radius to a block while that
+// ord, n1(c, i): the orders of case c's i-th radius from the last one back (the
+// largest first where the radii ascend).  Returns the shared-memory rows of a
+// block, 0 for a thread per radius.  A radius to a block while that
 // makes no more than four blocks per SM, else as many as K1_ROWS rows hold (1000
 // rows took a fifth more for 766 uneven cases).  A thread per radius, whose time
 // is that of the longest radius (0.8 us an order with derivatives, 0.65 without),
@@ -312,13 +313,9 @@ int k1_blocks(const std::vector<int> &ord, const std::vector<DevCase> &cs, int R
     if (per_sm < 3 && R > (hm || hx ? 8 : 36) * per_sm * sms) return 0;
     // a case's blocks; counted first
     auto cut = [&](int c, int4 *out) {
-        int nb = 0;
-        for (int i = 0; i < cs[c].nr; ++nb) {
-            const int n = std::min(std::min(most, cs[c].nr - i), std::max(1, rows / mie_block_rows(n1(c, i))));
-            if (out) out[nb] = make_int4(cs[c].r0 + cs[c].nr - 1 - i, n, c, 0);
-            i += n;
-        }
-        return nb;
+        return k1_cut(cs[c].nr, rows, most, [&](int i) { return mie_block_rows(n1(c, i)); }, [&](int i, int n) {
+            if (out) *out++ = make_int4(cs[c].r0 + cs[c].nr - 1 - i, n, c, 0);
+        });
     };
     const int ncase = (int) ord.size();
     std::vector<int> at(ncase + 1, 0);
