@@ -208,7 +208,7 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     double *ckr = ck + (size_t) B.ckoff[r] * CW;     // nb blocks of CW doubles
     const double *fv4 = B.fv + 3 * (B.n1max + 2), *fv3 = fv4 - (B.n1max + 2);
 
-    // ---- downward: P from n2, u from n1 (n2 > n1 + MIE_B), block by block ----
+    // ---- downward: D from n2, u from n1 (n2 > n1 + MIE_B), block by block ----
     double u0, ux0 = 0.;
     int eu = 0;
     {

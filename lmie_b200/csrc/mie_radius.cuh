@@ -10,13 +10,15 @@
 // psi runs in ratios: an order of u costs one dependent FMA, a ratio waits for a
 // reciprocal (60 cycles).  u grows by many orders of magnitude, so it is brought
 // back to order 1 at the ends of blocks of MIE_B orders, by a power of two
-// (exact).  Where only values are wanted, the blocks run D in a three-term form
-// too, P_{n-1} = (2n + 1)/z P_n - P_{n+1}, D_n = P_{n-1}/P_n - n/z: 18 cycles an
-// order instead of 105 (107 thousand radii 308 us instead of 495).  Its rounding
-// is another one, which values show by 1e-11 at most; derivatives at the
-// resonances of weakly absorbing spheres carry a rounding of D up to 1e-7 of
-// their value, as far as the reference's own, so with derivatives D is rounded as
-// it always was here.
+// (exact).  Where only values are wanted, the block form runs D of radii with
+// MIE_P_MIN orders and more in a three-term form too, P_{n-1} = (2n + 1)/z P_n -
+// P_{n+1}, D_n = P_{n-1}/P_n - n/z: 18 cycles an order instead of 105 (107
+// thousand radii 308 us instead of 495).  Its rounding is another one, which
+// values show by 1e-11 at most; derivatives at the resonances of weakly absorbing
+// spheres carry a rounding of D up to 1e-7 of their value, as far as the
+// reference's own, so with derivatives D is rounded as it always was here.  Nor
+// do small spheres take it: the difference of P_{n-1}/P_n and n/z takes bits from
+// Im D, which is all of a small absorbing sphere's extinction (see MIE_P_MIN).
 //
 // Derivatives: dD/dz = n/z^2 - 1 + (n/z - D)(n/z + D), the Riccati equation with
 // its difference of large terms in factors, no recurrence of its own; chi' =
@@ -25,9 +27,11 @@
 // it computes.
 //
 // Every FMA is written out, and K1's and the cross sections' files are compiled
-// without FMA contraction, so a radius' coefficients are the same bits
-// whichever of them forms them (derivatives near resonances carry a rounding
-// of a recurrence to 1e-12 of a case's cross section).
+// without FMA contraction, so with derivatives a radius' coefficients are the
+// same bits whichever of them forms them (derivatives near resonances carry a
+// rounding of a recurrence to 1e-12 of a case's cross section).  Without, the
+// thread-per-radius form keeps the chain of D where a block runs P, and its
+// values differ by that rounding.
 #pragma once
 
 #include "dev_common.cuh"
@@ -44,6 +48,13 @@ constexpr int MIE_B = 4;                              // orders per block of the
 constexpr int MIE_BLOCK_T = 128;
 constexpr int MIE_BLOCK_MAX = 32;                     // radii of a block
 constexpr int MIE_BLOCK_SMEM = 220 * 1024;            // what a block may take
+// Orders from which a block runs D as ratios of P where only values are wanted.
+// Largest relative errors against 113-bit arithmetic, 200 spheres of mi 1e-5 ..
+// 0.1 each, chain of D / ratios of P: Cext at x 0.001 .. 0.1 (8 and 9 orders)
+// 1.1e-15 / 1.2e-14, x 0.3 .. 1 2.4e-15 / 5.4e-15, x 1 .. 2 2.9e-15 / 3.7e-15; from
+// x = 2 (15 orders) to 900 equal for Cext, Csca, Cbak, g and Cext - Csca.  A
+// chain of D from below 32 orders takes at most 3 us.
+constexpr int MIE_P_MIN = 32;
 
 // rows of shared memory of a radius of n1 orders; bytes of a block of that many rows: D, u, chi (and u's
 // tangent), two exponents per MIE_B orders, reduction space, what the team needs to know of each radius
@@ -106,7 +117,7 @@ struct MieRadius {
     }
 };
 
-// The chain of P, whose ratios are D (values only): P_{n-1} = (2n + 1)/z P_n - P_{n+1}, D_n = P_{n-1}/P_n - n/z;
+// The chain of P, whose ratios are D (values only, MIE_P_MIN): P_{n-1} = (2n + 1)/z P_n - P_{n+1}, D_n = P_{n-1}/P_n - n/z;
 // cur = P_n, hi = P_{n+1}.
 struct MieP {
     cplx hi, cur;
@@ -296,7 +307,8 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
     double *sh_zi = sh_zr + MIE_BLOCK_MAX, *sh_xl = sh_zi + MIE_BLOCK_MAX;
     int *sh_eu = (int *) (sh_xl + MIE_BLOCK_MAX), *sh_row = sh_eu + MIE_BLOCK_MAX, *sh_n1 = sh_row + MIE_BLOCK_MAX;
     int *eU = sh_n1 + 2 * MIE_BLOCK_MAX, *eP = eU + rows / MIE_B;
-    constexpr bool DER = HM || HX;                    // D itself in Ds, or P
+    constexpr bool DER = HM || HX;
+    auto chain_d = [](int n1) { return DER || n1 < MIE_P_MIN; };   // D itself in Ds, or P
 
     MieRadius<HX> c;
     common(c);
@@ -324,7 +336,7 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
             sh_zi[lane] = c.zinv.im;
             if (HX) sh_xl[lane] = c.xl;
             double2 *Dr = Ds + row;
-            if (DER) {
+            if (chain_d(n1)) {
                 MieD p;
                 p.start();
                 for (int n = n2 - 1; n > n1; --n) p.step(n, c.zinv);
@@ -424,9 +436,8 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
             if (on) {
                 const double2 dj = Dr[j];
                 cplx D = mk(dj.x, dj.y), Dz = mk(0., 0.);
-                if (DER) {
-                    Dz = mie_dz(c, j, D);
-                } else {
+                if (DER) Dz = mie_dz(c, j, D);
+                if (!chain_d(n1)) {
                     const double2 lo = Dr[j - 1];
                     const int *er = eP + row / MIE_B;
                     const double sc = j % MIE_B == 0 ? mb_pow2(er[j / MIE_B - 1] - er[j / MIE_B]) : 1.;
