@@ -1085,13 +1085,19 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     bool any_ang = false;
     for (int k = 0; k < ncase; ++k) any_ang |= cs[k].n_qang > 0;
     L.tc_seg = g_tc_seg;
+    // the fixed-point stage takes the cases of at least OZ_MIN_N1 orders whose radius
+    // groups fit its exact int32 sums (OZ_MAX_NK chunks)
+    auto oz_takes = [&](int k) {
+        return cs[k].n_qang > 0 && cs[k].n1 >= OZ_MIN_N1 && (cn1max[k] + OZ_KC - 1) / OZ_KC <= OZ_MAX_NK;
+    };
     if (L.save_control == 0 && any_ang && R > 0 && nd1 <= OZ_MAX_ND1 && nd2 <= OZ_MAX_ND2) {
         // INT8: six digits.  FP64: seven, for sub-batches whose angular sums
-        // are worth the operand kernels (OZ_MIN_SUMS), of whole solves (the
+        // in this form are worth the operand kernels (OZ_MIN_SUMS), of whole solves (the
         // integrals a group of processes adds up, or a caller takes away, stay
         // the FP64 kernel's)
         double sums = 0.;
-        for (int k = 0; k < ncase; ++k) sums += (double) (cs1[k + 1] - cs1[k]) * cs[k].nh * (1. + nd1);
+        for (int k = 0; k < ncase; ++k)
+            if (oz_takes(k)) sums += (double) (cs1[k + 1] - cs1[k]) * cs[k].nh * (1. + nd1);
         const bool whole = L.acc_mode == LMIEB_ACC_WHOLE || (L.acc_mode == LMIEB_ACC_GROUP && g_group.world == 1);
         if (p0.precision == LMIEB_PRECISION_INT8) L.oz = 6;
         else if (p0.precision == LMIEB_PRECISION_FP64 && whole && sums >= OZ_MIN_SUMS) L.oz = 7;
@@ -1100,11 +1106,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     // linearised phase matrices cancel strongly on normalisation, and they cost little
     std::vector<char> case_tc(ncase, 0), case_oz(ncase, 0);
     for (int k = 0; k < ncase; ++k) case_tc[k] = L.tc && cs[k].n_qang > 0 && cs[k].n1 >= TC_MIN_N1;
-    // the fixed-point stage takes the cases of at least OZ_MIN_N1 orders whose radius
-    // groups fit its exact int32 sums (OZ_MAX_NK chunks)
-    for (int k = 0; k < ncase; ++k)
-        case_oz[k] = L.oz && cs[k].n_qang > 0 && cs[k].n1 >= OZ_MIN_N1 &&
-                     (cn1max[k] + OZ_KC - 1) / OZ_KC <= OZ_MAX_NK;
+    for (int k = 0; k < ncase; ++k) case_oz[k] = L.oz && oz_takes(k);
     std::vector<AngItem> ang, ang64;
     std::vector<long long> pf_start(ncase + 1, 0);
     for (int k = 0; k < ncase; ++k) {
@@ -1362,10 +1364,10 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             wc[k] = (double) (cs1[k + 1] - cs1[k]) * cs[k].nh;
             W += wc[k];
         }
-        // work per block; in a tensor-core batch these are the cases under 16
-        // orders (a few half-angles, up to ~2000 radii each), whose blocks
+        // work per block; in a tensor-core batch the cases under 16
+        // orders (a few half-angles, up to ~2000 radii each) have blocks that
         // would otherwise walk all their radii one after the other.  Without
-        // one, a block has at least 131072 order-angle products, but no more
+        // one, and for cases too long for the fixed-point sums, a block has at least 131072 order-angle products, but no more
         // than give its case 4 blocks for every SM, down to 4096: a block's
         // threads walk their radii serially at the latency of the recurrence,
         // and the 200-radius aerosol solve on 2 blocks took 251 us for 10
@@ -1377,11 +1379,12 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             DevCase &C = cs[k];
             if (C.n_qang <= 0 || case_tc[k] || case_oz[k]) continue;
             const int xt = (C.nh + per - 1) / per;
-            const double wt = (L.tc || L.oz) ? std::max(w_all, 4096.)
+            const bool tail = L.tc || (L.oz && C.n1 < OZ_MIN_N1);
+            const double wt = tail ? std::max(w_all, 4096.)
                               : w_all > 131072. ? w_all
                                                 : std::min(131072., std::max(wc[k] / (4. * c.sms), 4096.));
             int G = (int) std::lround(wc[k] / (xt * wt));
-            G = std::max(1, std::min(G, (L.tc || L.oz) ? std::min(C.nr, 64) : C.nr));
+            G = std::max(1, std::min(G, tail ? std::min(C.nr, 64) : C.nr));
             std::vector<int> gs(G + 1, C.r0 + C.nr);
             gs[0] = C.r0;
             const long long o0 = off[C.r0], ot = off[C.r0 + C.nr] - o0;
