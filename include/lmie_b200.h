@@ -262,10 +262,17 @@ int lmieb_rerun_device(int reps, int flush_l2, double *ms_total, double *ms_stag
  * pointer may be NULL. */
 int lmieb_last_work(double *flops, long long *launches, size_t *h2d, size_t *d2h);
 
-/* Cases of the last batch call that LMIEB_PRECISION_INT8 solved again in
- * FP64 because their truncation n_coef was not certain at the fixed-point
- * contraction's error.  Returns 0. */
+/* Cases of the last call whose angular sums took the fixed-point form (all of
+ * LMIEB_PRECISION_INT8, the large ones of LMIEB_PRECISION_FP64) and that were
+ * solved again with the FP64 angular kernel because their truncation n_coef
+ * was not certain at that form's error.  Returns 0. */
 int lmieb_last_redo(long long *cases);
+
+/* The bound on that error: |beta_l(fixed point) - beta_l(FP64 kernel)| / (2l + 1)
+ * near the truncation threshold, for a case whose radii reach `orders` orders.  A
+ * case with some |beta_l| (l up to the truncation) within this times 2l + 1 of
+ * `accuracy` is solved again. */
+double lmieb_truncation_band(int orders);
 
 /* The LMIEB_PRECISION_INT8 product kernel of the last solve: the
  * tensor-core operations it runs (2 per 8-bit multiply-add) and, after

@@ -1282,7 +1282,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             if (!case_oz[k]) continue;
             C.nkx = (cn1max[k] + OZ_KC - 1) / OZ_KC;
             C.rx_off = rx_bytes;
-            C.trunc_band = C.accuracy > 0. ? oz_trunc_band(cn1max[k], C.nr) : 0.;
+            C.trunc_band = C.accuracy > 0. ? oz_trunc_band(cn1max[k]) : 0.;
             rx_bytes += 2LL * C.nh;
             // the A operand of each angle tile and chunk
             const int ntile = (C.nh + OZ_HALF - 1) / OZ_HALF;
@@ -2773,6 +2773,8 @@ extern "C" int lmieb_last_host_timing(double *ms, int n) {
     for (int i = 0; i < n && i < LMIEB_N_HOST; ++i) ms[i] = g_ctx.host_ms[i];
     return LMIEB_N_HOST;
 }
+
+extern "C" double lmieb_truncation_band(int orders) { return oz_trunc_band(orders); }
 
 extern "C" int lmieb_set_work_granularity(int precision, double items_per_sm) {
     std::lock_guard<std::mutex> lock(g_mu);

@@ -117,16 +117,17 @@ inline int oz_rg(int nd, int nt) { return oz_np(nd) / 2 / (2 * (1 + nt)); }
 
 // Bound on |beta_l(fixed point) - beta_l(FP64)| / (2l + 1) of the expansion
 // coefficients near the truncation threshold (|beta_l| within 1e-9 .. 1e-5 of
-// 2l + 1), for a case of nr radii reaching n1 orders.  Measured at most, with
-// seven digits and with six: up to 1152 orders 8.4e-15 and 1.1e-14 (8192 uneven
-// cases of 100 radii and more), 2.6e-14 and 9.1e-14 (600 cases of 1 to 30
-// radii); beyond, 1.3e-13 (x from 1100 to 5000, 1 to 8000 radii).  A case with
-// some |beta_l| within oz_trunc_band (2l + 1) of `accuracy` before its
+// 2l + 1), for a case reaching n1 orders.  Measured at most, with seven digits
+// and with six: up to 1152 orders 7.3e-14 and 9.8e-14 (2000 single radii, 4600
+// cases of 2 to 2000 radii in narrow and in broad ranges, 9000 distributions of
+// every width); beyond, 1.4e-13 (880 cases of x from 1120 to 5000, 1 to 300 radii).
+// Averaging over many radii does not lower it -- the largest values with seven
+// digits belong to 500 radii over x up to 980, and most of them are the FP64
+// kernel's -- although it is small (8.4e-15, 1.1e-14) in 8192 uneven cases.  A
+// case with some |beta_l| within oz_trunc_band (2l + 1) of `accuracy` before its
 // truncation point is solved again in FP64, which costs a batch the time of its
-// largest such case: 3 of 1531 cases 2.0 ms at 2.5e-13.
-__host__ __device__ inline double oz_trunc_band(int n1, int nr) {
-    return n1 > 1152 ? 5e-13 : nr < 100 ? 2.5e-13 : 4e-14;
-}
+// largest such case: 3 of 1531 cases 2.0 ms.
+__host__ __device__ inline double oz_trunc_band(int n1) { return n1 > 1152 ? 5e-13 : 2.5e-13; }
 // 1.5 * 2^52 + 0x808080808080: see oz_digits
 constexpr double OZ_MAGIC = 6896688841130112.0;
 
