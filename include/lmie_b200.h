@@ -183,9 +183,10 @@ typedef struct {
  * One forward sweep (Mie recurrences, coefficients, the phase matrix at the
  * n_angles angles) and one reverse sweep in FP64: the derivative of the
  * logarithmic derivative D_n(z) is taken in closed form (dD_n/dz =
- * n(n+1)/z^2 - 1 - D_n^2, from the Riccati-Bessel equation), and the reverse
- * sweep re-runs the recurrences from checkpoints stored every 64 orders
- * instead of per-order arrays.  This entry point has no counterpart in the
+ * n(n+1)/z^2 - 1 - D_n^2, from the Riccati-Bessel equation).  The coefficients,
+ * their derivatives and their adjoints take 96 bytes of device memory for every
+ * order of every radius and wavelength; where there is no room for them all, the
+ * wavelengths go through in passes, with the same results.  This entry point has no counterpart in the
  * reference.  Returns 0 or -1. */
 int lmie_solution_adjoint(int n_lambda, const double *lambda, const double *mr, const double *mi,
                           const lmie_bins *bins, int n_angles, const lmie_loss_weights *weights,

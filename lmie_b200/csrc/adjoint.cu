@@ -55,7 +55,7 @@ struct Adj {
     const double *rad;             // [R]
     const int *n1, *n2;            // [L*R]
     const int *ro;                 // [L*R] orders of the wavelength's radii before this one
-    const long long *ko;           // [L] orders of the wavelengths before this one
+    const long long *ko;           // [L] orders of the pass' wavelengths before this one
     const double *mu;              // [nhu] cosines of the half-angles
     int nt;                        // tiles of 8 half-angles (nhu rounded up, zeros there)
     int nrow;                      // orders in the tables
@@ -527,12 +527,21 @@ int launch_angles(const Adj &P, cudaStream_t s) {
 std::mutex g_amu;
 char *g_dbuf = nullptr, *g_hbuf = nullptr;
 size_t g_dcap = 0, g_hcap = 0;
+bool g_dshort = false;             // the device had no room for all orders of that solve
+
+// The columns of the orders (c4, d4, b4) are most of what a solve holds on the
+// device, 96 bytes for every order of every radius and wavelength.  Where the
+// device has no room for them all, the wavelengths go through in passes, as many
+// at a time as fit ADJ_PASS_BYTES (still some 5 times the benchmark's 17.8 M
+// orders, enough to fill the device) or the largest of them.
+constexpr size_t ADJ_ORDER_BYTES = 3 * sizeof(double4), ADJ_PASS_BYTES = (size_t) 8 << 30;
 
 size_t pad256(size_t b) { return (b + 255) & ~(size_t) 255; }
 
 }  // namespace
 
 extern "C" int lmieb_stream(void **stream);
+extern "C" int lmieb_fault_injected(const char *site);
 
 extern "C" int lmie_solution_adjoint(int n_lambda, const double *lambda, const double *mr, const double *mi,
                                      const lmie_bins *bins, int n_angles, const lmie_loss_weights *weights,
@@ -643,11 +652,11 @@ extern "C" int lmie_solution_adjoint(int n_lambda, const double *lambda, const d
             o[1] = w.d_p12 ? .5 * w.d_p12[i] : 0.;
         }
     }, &xj);
-    long long *ko = (long long *) (hb + i_ko), tot = 0;
+    long long tot = 0, most = 0;                          // orders of all wavelengths, of the longest
     int n1max = 1, k_top = 0;
     for (int k = 0; k < L; ++k) {
-        ko[k] = tot;
         tot += orders[k];
+        most = std::max(most, orders[k]);
         if (top[k] > n1max) {
             n1max = top[k];
             k_top = k;
@@ -665,17 +674,51 @@ extern "C" int lmie_solution_adjoint(int n_lambda, const double *lambda, const d
     }
     const int nrow = ((n1max + 7) & ~7) + 8;              // the kernel loads 8 orders ahead
 
-    size_t dev_bytes = in_bytes + out_bytes;
-    const size_t b_c = pad256((size_t) tot * 32), b_tab = pad256((size_t) nrow * nt * 8 * 16);
+    const size_t b_tab = pad256((size_t) nrow * nt * 8 * 16);
     const size_t b_esg = pad256(LR * 4 * 8), b_pfp = pad256((size_t) L * G * na * 2 * 8), b_zr = pad256(LR * 3 * 8);
-    dev_bytes += 2 * b_tab + 3 * b_c + b_esg + b_pfp + b_zr;
-    if (dev_bytes > g_dcap) {
+    const size_t fixed = in_bytes + out_bytes + 2 * b_tab + b_esg + b_pfp + b_zr + 3 * 256;
+    auto room = [&](long long n) { return fixed + (size_t) n * ADJ_ORDER_BYTES; };
+    long long cap = tot;                                  // orders of a pass
+    const long long pass_most = std::min(tot, std::max(most, (long long) (ADJ_PASS_BYTES / ADJ_ORDER_BYTES)));
+    const bool fail = lmieb_fault_injected("adjoint");
+    if (fail || (room(tot) > g_dcap && !(g_dshort && room(pass_most) <= g_dcap))) {
         if (g_dbuf) cudaFree(g_dbuf);
         g_dbuf = nullptr;
         g_dcap = 0;
-        LMIEB_CUDA_TRY(cudaMalloc((void **) &g_dbuf, dev_bytes));
-        g_dcap = dev_bytes;
+        cudaError_t e = fail ? cudaErrorMemoryAllocation : cudaMalloc((void **) &g_dbuf, room(tot));
+        g_dshort = e == cudaErrorMemoryAllocation;
+        if (g_dshort) {
+            cudaGetLastError();
+            // what is there, but for a tenth
+            size_t fr = 0, all = 0;
+            LMIEB_CUDA_TRY(cudaMemGetInfo(&fr, &all));
+            const size_t use = fail ? 0 : fr / 10 * 9;
+            cap = use > fixed ? (long long) ((use - fixed) / ADJ_ORDER_BYTES) : 0;
+            cap = std::max(most, std::min(cap, pass_most));
+            e = cudaMalloc((void **) &g_dbuf, room(cap));
+            if (e == cudaErrorMemoryAllocation && cap > most) {
+                cudaGetLastError();
+                cap = most;
+                e = cudaMalloc((void **) &g_dbuf, room(cap));
+            }
+        }
+        LMIEB_CUDA_TRY(e);
+        g_dcap = room(cap);
+    } else if (room(tot) > g_dcap) {
+        cap = (long long) ((g_dcap - fixed) / ADJ_ORDER_BYTES);
     }
+    const size_t b_c = pad256((size_t) cap * sizeof(double4));
+    long long *ko = (long long *) (hb + i_ko);
+    std::vector<int> pass{0};                             // first wavelengths of the passes
+    for (long long k = 0, n = 0; k < L; ++k) {
+        if (n + orders[k] > cap) {
+            pass.push_back((int) k);
+            n = 0;
+        }
+        ko[k] = n;
+        n += orders[k];
+    }
+    pass.push_back(L);
     char *d = g_dbuf;
     auto dp = [&](size_t at) { return (void *) (d + at); };
     Adj P;
@@ -703,15 +746,29 @@ extern "C" int lmie_solution_adjoint(int n_lambda, const double *lambda, const d
 
     // ---- run ----
     LMIEB_CUDA_TRY(cudaMemcpyAsync(d, g_hbuf, in_bytes, cudaMemcpyHostToDevice, s));
-    k_adj_coef<<<(unsigned) L * ((R + 63) / 64), 64, 0, s>>>(P);
-    LMIEB_CUDA_TRY(cudaGetLastError());
-    k_adj_table<<<1, 8 * nt, 0, s>>>(P);
-    LMIEB_CUDA_TRY(cudaGetLastError());
-    if (launch_angles(P, s)) return -1;
-    k_adj_lambda<<<L, ADJ_T, 0, s>>>(P);
-    LMIEB_CUDA_TRY(cudaGetLastError());
-    k_adj_m<<<ceil_div(8 * LR, 256), 256, 0, s>>>(P);
-    LMIEB_CUDA_TRY(cudaGetLastError());
+    for (size_t i = 0; i + 1 < pass.size(); ++i) {
+        // the pass' wavelengths: their part of everything but the orders' columns and the tables
+        const int k0 = pass[i], n = pass[i + 1] - k0;
+        const size_t r0 = (size_t) k0 * R;
+        Adj Q = P;
+        Q.L = n;
+        Q.lam += k0; Q.m += k0; Q.ko += k0;
+        Q.n1 += r0; Q.n2 += r0; Q.ro += r0;
+        Q.dw += (size_t) k0 * 16 * nt; Q.cw += (size_t) k0 * 3;
+        Q.esg += r0 * 4; Q.zr += r0 * 3; Q.pfp += (size_t) k0 * G * na * 2;
+        Q.lw += (size_t) k0 * 8; Q.vals += (size_t) k0 * (3 + 2 * na);
+        k_adj_coef<<<(unsigned) n * ((R + 63) / 64), 64, 0, s>>>(Q);
+        LMIEB_CUDA_TRY(cudaGetLastError());
+        if (i == 0) {
+            k_adj_table<<<1, 8 * nt, 0, s>>>(Q);
+            LMIEB_CUDA_TRY(cudaGetLastError());
+        }
+        if (launch_angles(Q, s)) return -1;
+        k_adj_lambda<<<n, ADJ_T, 0, s>>>(Q);
+        LMIEB_CUDA_TRY(cudaGetLastError());
+        k_adj_m<<<ceil_div(8 * (size_t) n * R, 256), 256, 0, s>>>(Q);
+        LMIEB_CUDA_TRY(cudaGetLastError());
+    }
     k_adj_final<<<L + nb, ADJ_T, 0, s>>>(P);
     LMIEB_CUDA_TRY(cudaGetLastError());
     char *ho = g_hbuf + in_bytes;

@@ -492,7 +492,9 @@ int ensure_ready() {
 // sub-batch's input upload) or "graph" (instantiating a captured kernel
 // sequence), several separated by commas -- that step fails as its CUDA call
 // would (the arena and the staging buffer are released first, as when a
-// larger one cannot be had), and the error propagates as -1.
+// larger one cannot be had), and the error propagates as -1.  ("adjoint", in
+// adjoint.cu, fails the allocation of all of a gradient's orders, which then
+// goes through in passes.)
 bool fault_injected(const char *site);
 }  // namespace
 
