@@ -1045,7 +1045,20 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     if (ncmax > 2) rc[(size_t) 8 * 2 + 1] = 1. / 2.;   // Legendre at l = 2
 
     // ---- Gauss angles: pool entries, new orders computed on the device ----
+    // (a sub-batch that fails before their computation is queued takes its
+    // entries with it)
     std::vector<int> gl_ns, gl_pt, gl_pi;
+    struct NewEntries {
+        Ctx &c;
+        const std::vector<int> &ns;
+        const size_t used;
+        bool queued;
+        ~NewEntries() {
+            if (queued) return;
+            for (int n : ns) c.gl_map.erase(n);
+            c.gl_used = used;
+        }
+    } gl_new{c, gl_ns, c.gl_used, false};
     std::vector<long long> gl_mo, gl_go;
     std::vector<double> gl_guess, gl_jr((size_t) std::max(nqmax, 1), 0.);
     for (int j = 0; j < nqmax; ++j) gl_jr[j] = j / (j + 1.);
@@ -1912,6 +1925,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         LMIEB_CUDA_TRY(cudaEventRecord(c.gl_ready, s));
         c.gl_pending = true;
     }
+    gl_new.queued = true;
     // A sub-batch whose kernel sequence the slot ran recently (the same
     // structure of radii, orders and angles in the same arena: retrieval loops
     // that change the refractive index or the weights, the parts of repeated
