@@ -107,6 +107,13 @@ struct Slot {
     Pending pend;
 };
 
+// counted while a call's sub-batches are laid out
+struct Work {
+    double flops[4] = {};           // algorithmic flops of the last solve (see lmieb_last_work)
+    double tensor_ops = 0.;         // tensor-core operations (2 per multiply-add) its int8 products run
+    long long launches = 0;         // kernel launches of one device run of the last solve
+};
+
 struct Ctx {
     bool ready = false;
     int device = -1;
@@ -137,11 +144,9 @@ struct Ctx {
     cudaEvent_t ev[NSTAGE + 1] = {};
     bool timing = false;
     double stage_ms[NSTAGE] = {};
-    double work[4] = {};            // algorithmic flops of the last solve (see lmieb_last_work)
-    double tensor_ops = 0.;         // tensor-core operations (2 per multiply-add) its int8 products run
+    Work work;
     cudaEvent_t k3[2] = {};         // with timing: around the int8 product kernel
     double k3_ms = 0.;
-    long long launches = 0;         // kernel launches of one device run of the last solve
     size_t h2d = 0, d2h = 0;        // bytes copied by the last solve
     long long graph_captures = 0, graph_replays = 0;   // kernel sequences captured / replayed (all calls)
     // radius groups: whether this process's solve has entered the group's
@@ -492,9 +497,10 @@ int ensure_ready() {
 // sub-batch's input upload) or "graph" (instantiating a captured kernel
 // sequence), several separated by commas -- that step fails as its CUDA call
 // would (the arena and the staging buffer are released first, as when a
-// larger one cannot be had), and the error propagates as -1.  ("adjoint", in
-// adjoint.cu, fails the allocation of all of a gradient's orders, which then
-// goes through in passes.)
+// larger one cannot be had), and the error propagates as -1.  Two sites stand
+// for a device without room for the faster form: "operands" (the arena of a
+// sub-batch with FP64's fixed-point sums, which then takes the FP64 kernel's) and
+// "adjoint" (all of a gradient's orders, which then go through in passes).
 bool fault_injected(const char *site);
 }  // namespace
 
@@ -551,8 +557,12 @@ bool seen_plan(Slot &S, unsigned long long sig) {
     return hit;
 }
 
-int ensure_device(Slot &S, size_t bytes) {
-    const bool fail = fault_injected("alloc");
+constexpr int SUB_NO_ROOM = -2;
+
+// The slot's arena with at least `bytes`; SUB_NO_ROOM if the device has no such
+// block.  operands: those of FP64's fixed-point sums are part of it.
+int ensure_device(Slot &S, size_t bytes, bool operands) {
+    const bool fail = fault_injected("alloc") || (operands && fault_injected("operands"));
     if (bytes <= S.dcap && !fail) return 0;
     S.have_plan = false;
     drop_graph(S);
@@ -560,7 +570,12 @@ int ensure_device(Slot &S, size_t bytes) {
     S.dbuf = nullptr;
     S.dcap = 0;
     size_t want = bytes + bytes / 4;
-    LMIEB_CUDA_TRY(fail ? cudaErrorMemoryAllocation : cudaMalloc((void **) &S.dbuf, want));
+    const cudaError_t e = fail ? cudaErrorMemoryAllocation : cudaMalloc((void **) &S.dbuf, want);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        return SUB_NO_ROOM;
+    }
+    LMIEB_CUDA_TRY(e);
     S.dcap = want;
     return 0;
 }
@@ -843,7 +858,8 @@ size_t case_bytes(const lmieb_problem &p) {
     b += (size_t) 4 * ncol * p.n_qang * 8 * 8;                        // partials (groups), pf, pfn
     b += (size_t) ncol * 6 * p.n_coef * 8 * (3 + (p.n_qang / 2 + 31) / 32);   // expansion partials + outputs
     b += (size_t) 4 * (p.n_qang / 2) * (p.n_coef / EX_LT + 1) * 16;   // checkpoints
-    if (p.precision == LMIEB_PRECISION_INT8 || p.precision == LMIEB_PRECISION_FP64) {
+    if ((p.precision == LMIEB_PRECISION_INT8 || p.precision == LMIEB_PRECISION_FP64) && p.save_control == 0 &&
+        p.n_qang > 0 && p.nd1 <= OZ_MAX_ND1 && p.nd2 <= OZ_MAX_ND2 && oz_takes_orders(p.n1, p.n1)) {
         // B operand digits (groups padded to whole chunks), row exponents
         const int digits = p.precision == LMIEB_PRECISION_INT8 ? 6 : 7;
         b += (size_t) (tot + (size_t) p.n * OZ_KC) * oz_bstage(digits) /
@@ -856,8 +872,10 @@ size_t case_bytes(const lmieb_problem &p) {
 }
 
 // Packs one sub-batch ps[0..n) into slot S and queues its device work and the
-// download of its outputs; collect_slot() unpacks them.
-int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lmieb_result *rs_out) {
+// download of its outputs; collect_slot() unpacks them.  fp64_sums:
+// LMIEB_PRECISION_FP64 with the FP64 angular kernel whatever the size.  Returns
+// SUB_NO_ROOM, without an ERROR line, if the device has no room for the arena.
+int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lmieb_result *rs_out, bool fp64_sums) {
     Ctx &c = g_ctx;
     const double t_pack = now_ms();
     S.have_plan = false;        // the slot's graph is kept while the plan repeats (below)
@@ -1013,9 +1031,11 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     std::stable_sort(k1ord.begin(), k1ord.end(), [&](int a, int b) { return cn1max[a] > cn1max[b]; });
     for (int k = 0; k < ncase; ++k) k1pre[k + 1] = k1pre[k] + ps[k1ord[k]].n;
     std::vector<int4> k1_blk;
+    // (K1's checkpoints are the thread-per-radius form's only)
     const int k1_rows = re_solve ? 0 : k1_blocks(k1ord, cs, R, n1max, hm, hx, c.sms, k1_blk, [&](int k, int i) {
         return ps[k].n1r[ps[k].n - 1 - i];
     });
+    const size_t ck_used = k1_rows > 0 ? 0 : (size_t) ckn * ck_w;
 
     // ---- order tables ----
     std::vector<double> fv((size_t) 4 * (n1max + 2), 0.);
@@ -1100,11 +1120,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     bool any_ang = false;
     for (int k = 0; k < ncase; ++k) any_ang |= cs[k].n_qang > 0;
     L.tc_seg = g_tc_seg;
-    // the fixed-point stage takes the cases of at least OZ_MIN_N1 orders whose radius
-    // groups fit its exact int32 sums (OZ_MAX_NK chunks)
-    auto oz_takes = [&](int k) {
-        return cs[k].n_qang > 0 && cs[k].n1 >= OZ_MIN_N1 && (cn1max[k] + OZ_KC - 1) / OZ_KC <= OZ_MAX_NK;
-    };
+    auto oz_takes = [&](int k) { return cs[k].n_qang > 0 && oz_takes_orders(cs[k].n1, cn1max[k]); };
     if (L.save_control == 0 && any_ang && R > 0 && nd1 <= OZ_MAX_ND1 && nd2 <= OZ_MAX_ND2) {
         // INT8: six digits.  FP64: seven, for sub-batches whose angular sums
         // in this form are worth the operand kernels (OZ_MIN_SUMS), of whole solves (the
@@ -1115,7 +1131,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
             if (oz_takes(k)) sums += (double) (cs1[k + 1] - cs1[k]) * cs[k].nh * (1. + nd1);
         const bool whole = L.acc_mode == LMIEB_ACC_WHOLE || (L.acc_mode == LMIEB_ACC_GROUP && g_group.world == 1);
         if (p0.precision == LMIEB_PRECISION_INT8) L.oz = 6;
-        else if (p0.precision == LMIEB_PRECISION_FP64 && whole && sums >= OZ_MIN_SUMS) L.oz = 7;
+        else if (p0.precision == LMIEB_PRECISION_FP64 && whole && !fp64_sums && sums >= OZ_MIN_SUMS) L.oz = 7;
     }
     // with split precision, cases below TC_MIN_N1 orders keep the FP64 K3: their
     // linearised phase matrices cancel strongly on normalisation, and they cost little
@@ -1585,18 +1601,18 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         }
         if (L.save_control == 2 || !solve) fang = frec = 0.;
         if (!finish) fgsf = fexp = 0.;
-        c.work[0] += fang;
+        c.work.flops[0] += fang;
         if (L.oz) {
             // the digit products of M x N x K per chunk of every (angle tile, group) pair
             double chunks = 0.;
             for (const AngItem &a : ang)
                 for (int gg = a.rbeg; gg < a.rend; ++gg) chunks += tg_nk[gg];
-            c.tensor_ops += 2. * oz_nprod(L.oz) * (double) OZ_M * oz_np(L.oz) * OZ_KC * chunks;
+            c.work.tensor_ops += 2. * oz_nprod(L.oz) * (double) OZ_M * oz_np(L.oz) * OZ_KC * chunks;
         }
-        c.work[1] += frec;
-        c.work[2] += fgsf;
-        c.work[3] += fexp;
-        c.launches += nl + (gl_pt.empty() ? 0 : 1);
+        c.work.flops[1] += frec;
+        c.work.flops[2] += fgsf;
+        c.work.flops[3] += fexp;
+        c.work.launches += nl + (gl_pt.empty() ? 0 : 1);
     }
 
     // ---- host staging: inputs then outputs ----
@@ -1735,7 +1751,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     {
         auto add = [&](size_t b) { dev_bytes += pad(b); };
         if (L.save_control != 2 && L.acc_mode != LMIEB_ACC_FINISH) {
-            add((size_t) ckn * 8 * ck_w);
+            add(ck_used * 8);
             if (L.tc) add((size_t) bop_floats * 4);
             if (L.oz) {
                 add((size_t) bop8_bytes);
@@ -1754,7 +1770,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
         add((size_t) ex_total * 8);
         add((size_t) pu_scr_total * 8);
     }
-    if (ensure_device(S, dev_bytes)) return -1;
+    if (const int rc = ensure_device(S, dev_bytes, L.oz == 7)) return rc;
     Arena A{S.dbuf, 0, S.dcap};
     char *d_in = A.take<char>(h_in_end);
     char *d_out = A.take<char>(out_bytes);
@@ -1829,7 +1845,7 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     }
     const bool solve = L.save_control != 2 && L.acc_mode != LMIEB_ACC_FINISH;
     if (solve) {
-        L.ck = A.take<double>((size_t) ckn * ck_w);
+        L.ck = A.take<double>(ck_used);
         if (L.tc) {
             L.bop_bytes = (size_t) bop_floats * 4;
             L.bop = A.take<float>((size_t) bop_floats);
@@ -2051,6 +2067,44 @@ int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lm
     return 0;
 }
 
+// Gives the arenas of the other slots back, as far as nothing uses them.
+void release_idle(Slot &S) {
+    Ctx &c = g_ctx;
+    if (c.slot[2].pend.active) return;          // (it may be reading another slot's arena)
+    for (Slot &T : c.slot) {
+        if (&T == &S || T.pend.active || !T.dbuf) continue;
+        if (cudaStreamSynchronize(T.stream) != cudaSuccess) continue;
+        T.have_plan = false;
+        drop_graph(T);
+        cudaFree(T.dbuf);
+        T.dbuf = nullptr;
+        T.dcap = 0;
+    }
+}
+
+// submit_sub_as() with what the device has room for: the operands of FP64's
+// fixed-point sums can take as much again as all the rest of an arena, so
+// without room for them their sub-batch takes the FP64 angular kernel; and idle
+// slots give up their arenas.  keep_idle: they must not (SUB_NO_ROOM instead).
+int submit_sub(Slot &S, long long ticket, int ncase, const lmieb_problem *ps, lmieb_result *rs_out,
+               bool keep_idle = false) {
+    Ctx &c = g_ctx;
+    const Work before = c.work;
+    int rc = submit_sub_as(S, ticket, ncase, ps, rs_out, false);
+    for (int again = 0; rc == SUB_NO_ROOM && again < (keep_idle ? 1 : 2); ++again) {
+        if (again == 0 && S.plan->oz != 7) continue;
+        if (again == 1) release_idle(S);
+        c.work = before;
+        rc = submit_sub_as(S, ticket, ncase, ps, rs_out, true);
+    }
+    if (rc == SUB_NO_ROOM && !keep_idle) {
+        fprintf(stderr, "ERROR: lmie_b200: the device has no room for the arena of %d cases: %s\n", ncase,
+                cudaGetErrorString(cudaErrorMemoryAllocation));
+        rc = -1;
+    }
+    return rc;
+}
+
 long long submit_locked(int n, const lmieb_problem *p, lmieb_result *r);
 int collect_ticket(long long ticket);
 int fit_sub(int n, const lmieb_problem *p);
@@ -2137,14 +2191,19 @@ int collect_slot(Slot &S) {
             c.gather.x_own = SL.B.x_own != 0;
             c.gather.cs.clear();
             for (int i = 0; i < redo_early; ++i) c.gather.cs.push_back(P.cs[redo[i]]);
-            const int rc3 = submit_sub(R3, c.redo_ticket++, redo_early, rq.data(), rr.data());
+            const int rc3 = submit_sub(R3, c.redo_ticket++, redo_early, rq.data(), rr.data(), true);
             c.gather.on = false;
-            if (rc3) {
-                R3.pend.active = false;
+            if (rc3) R3.pend.active = false;
+            if (rc3 == SUB_NO_ROOM) {
+                // no room for it beside this slot: when the slot has been unpacked
+                redo_early = 0;
+                if (--c.submits < 2) c.call_slot[c.submits] = -1;
+            } else if (rc3) {
                 return -1;
+            } else {
+                LMIEB_CUDA_TRY(cudaEventRecord(c.redo_read, R3.stream));
+                c.redo_src = (int) (&S - c.slot);
             }
-            LMIEB_CUDA_TRY(cudaEventRecord(c.redo_read, R3.stream));
-            c.redo_src = (int) (&S - c.slot);
         }
     }
     for (size_t p = 0; p + 1 < P.piece.size(); ++p) {
@@ -2289,13 +2348,11 @@ void reset_counters() {
     for (int i = 0; i < NSTAGE; ++i) c.stage_ms[i] = 0.;
     for (int i = 1; i < 4; ++i) c.host_ms[i] = 0.;
     c.host_ms[5] = c.host_ms[6] = 0.;
-    for (int i = 0; i < 4; ++i) c.work[i] = 0.;
-    c.launches = 0;
+    c.work = Work();
     c.h2d = c.d2h = 0;
     c.submits = 0;
     c.call_slot[0] = c.call_slot[1] = -1;
     c.redo = 0;
-    c.tensor_ops = 0.;
 }
 
 // submits p[0..n) (one sub-batch); returns its ticket or -1
@@ -2586,7 +2643,7 @@ extern "C" int lmieb_last_redo(long long *cases) {
 
 extern "C" int lmieb_last_int8_kernel(double *tensor_ops, double *ms) {
     std::lock_guard<std::mutex> lock(g_mu);
-    if (tensor_ops) *tensor_ops = g_ctx.tensor_ops;
+    if (tensor_ops) *tensor_ops = g_ctx.work.tensor_ops;
     if (ms) *ms = g_ctx.k3_ms;
     return 0;
 }
@@ -2595,8 +2652,8 @@ extern "C" int lmieb_last_work(double *flops, long long *launches, size_t *h2d, 
     std::lock_guard<std::mutex> lock(g_mu);
     Ctx &c = g_ctx;
     if (flops)
-        for (int i = 0; i < 4; ++i) flops[i] = c.work[i];
-    if (launches) *launches = c.launches;
+        for (int i = 0; i < 4; ++i) flops[i] = c.work.flops[i];
+    if (launches) *launches = c.work.launches;
     if (h2d) *h2d = c.h2d;
     if (d2h) *d2h = c.d2h;
     return 0;

@@ -71,6 +71,12 @@ constexpr int OZ_MAX_ND2 = 3;                        // index2 derivatives the k
 constexpr int OZ_MAX_NK = 160;                       // chunks per group (5120 orders: int32 sums exact)
 constexpr int OZ_MIN_N1 = 16;                        // smaller cases keep the FP64 angular stage
 
+// whether the stage takes a case of truncation n1 whose radii reach n1max orders: at least OZ_MIN_N1, and
+// radius groups that fit its exact int32 sums
+inline bool oz_takes_orders(int n1, int n1max) {
+    return n1 >= OZ_MIN_N1 && (n1max + OZ_KC - 1) / OZ_KC <= OZ_MAX_NK;
+}
+
 // The sizes of the two formats.  Tensor memory holds ND accumulators of NP
 // columns and the A stages of 8 ND columns (512 in all): six digits leave
 // room for 64 columns and two stages, seven for 48 columns (M 128, N 48 runs
