@@ -499,9 +499,10 @@ __global__ void __launch_bounds__(ADJ_T) k_adj_final(Adj P) {
     }
 }
 
-// The kernels' numbers of half-angle tiles: 181, 91 and 37 angles take 12, 6
-// and 3, up to 255 angles 16.
-constexpr int ADJ_TILES[] = {1, 3, 6, 9, 12, 16};
+// Tiles of 8 half-angles of the most angles that the entry point takes; there is
+// a kernel for every number of them (the accumulators of all tiles stay in
+// registers, and a tile too many costs as much as a used one).
+constexpr int ADJ_MAX_TILES = (ADJ_T + 7) / 8;
 
 template <int NT>
 int launch_angles_nt(const Adj &P, cudaStream_t s) {
@@ -512,14 +513,15 @@ int launch_angles_nt(const Adj &P, cudaStream_t s) {
     return 0;
 }
 
+// the kernel of P.nt tiles
+template <int NT = ADJ_MAX_TILES>
 int launch_angles(const Adj &P, cudaStream_t s) {
-    switch (P.nt) {
-    case 1: return launch_angles_nt<1>(P, s);
-    case 3: return launch_angles_nt<3>(P, s);
-    case 6: return launch_angles_nt<6>(P, s);
-    case 9: return launch_angles_nt<9>(P, s);
-    case 12: return launch_angles_nt<12>(P, s);
-    default: return launch_angles_nt<16>(P, s);
+    if (P.nt == NT) return launch_angles_nt<NT>(P, s);
+    if constexpr (NT > 1) {
+        return launch_angles<NT - 1>(P, s);
+    } else {
+        fprintf(stderr, "ERROR: lmie_solution_adjoint(): %d tiles of half-angles\n", P.nt);
+        return -1;
     }
 }
 
@@ -573,12 +575,7 @@ extern "C" int lmie_solution_adjoint(int n_lambda, const double *lambda, const d
     // ---- inputs, in one pinned block; outputs in another part of it ----
     size_t in_bytes = 0;
     auto take = [&](size_t bytes) { const size_t at = in_bytes; in_bytes += pad256(bytes); return at; };
-    int nt = (nhu + 7) / 8;                             // tiles of 8 half-angles, as many as there is a kernel for
-    for (int c : ADJ_TILES)
-        if (c >= nt) {
-            nt = c;
-            break;
-        }
+    const int nt = (nhu + 7) / 8;                       // tiles of 8 half-angles
     const size_t LR = (size_t) L * R;
     const size_t i_lam = take((size_t) L * 8), i_m = take((size_t) L * 16), i_W = take((size_t) R * 8);
     const size_t i_q = take((size_t) R * 8), i_rad = take((size_t) R * 8), i_bs = take((size_t) (nb + 1) * 4);
