@@ -1,8 +1,8 @@
 // k1_blocks.h -- how K1's blocks of several radii (mie_radius.cuh) take the
 // radii of one case: a block's shared memory is laid out for a fixed number of
-// rows, so its radii's rows must not add up to more, in whatever order the case
-// has its radii (an integration range given from the larger end downwards
-// brings them largest first).  Host code without CUDA, so that the rule can be
+// rows, so its radii's rows must not add up to more.  The host layer refuses
+// radii of more orders than r2 has, so the orders of the radii it accepts ascend;
+// the cut does not lean on that.  Host code without CUDA, so that the rule can be
 // checked by itself.
 #pragma once
 
