@@ -296,8 +296,8 @@ extern "C" void lmieb_host_parallel(int n, int n_threads, void (*fn)(void *, int
 
 // K1's blocks (mie_radius.cuh): each has radii of one case, cases in the order
 // ord, n1(c, i): the orders of case c's i-th radius from the last one back (the
-// largest first where the radii ascend).  Returns the shared-memory rows of a
-// block, 0 for a thread per radius.  A radius to a block while that
+// largest first where the radii ascend), dz[c]: some radius of the case takes
+// dD/dz from D's recurrence.  Returns false for a thread per radius.  A radius to a block while that
 // makes no more than four blocks per SM, else as many as K1_ROWS rows hold (1000
 // rows took a fifth more for 766 uneven cases).  A thread per radius, whose time
 // is that of the longest radius (0.8 us an order with derivatives, 0.65 without),
@@ -306,29 +306,50 @@ extern "C" void lmieb_host_parallel(int n, int n_threads, void (*fn)(void *, int
 // derivatives and 18 without (mie_radius.cuh): x = 5000 without, 3000 radii 1.8 ms
 // by blocks and 3.1 by threads, 8000 radii 4.7 and 3.8; with, 1000 radii about 2
 // and 3.7 ms, 8000 radii 24 and 4.2.
+struct K1Blocks {
+    std::vector<int4> blk;
+    int smem = 0, rows = 0, rows_dz = 0;   // of a block; its rows, without and with dD/dz
+};
 template <class Orders>
-int k1_blocks(const std::vector<int> &ord, const std::vector<DevCase> &cs, int R, int n1max, bool hm, bool hx,
-              int sms, std::vector<int4> &blk, Orders &&n1) {
+bool k1_blocks(const std::vector<int> &ord, const std::vector<DevCase> &cs, const std::vector<int> &cn1max,
+               const std::vector<char> &dz, int R, bool hm, bool hx, int sms, K1Blocks &K, Orders &&n1) {
     constexpr int K1_ROWS = 1500;
-    blk.clear();
-    const int rows = std::max(mie_block_rows(n1max), R > 4 * sms ? K1_ROWS : 0);
-    if (R == 0 || mie_block_smem(rows, hx) > MIE_BLOCK_SMEM) return 0;
-    const int per_sm = std::min(8, 227 * 1024 / (mie_block_smem(rows, hx) + 1024));
-    const int most = R <= 4 * sms ? 1 : std::min(MIE_BLOCK_MAX, std::max(4, (R + 4 * sms - 1) / (4 * sms)));
-    if (per_sm < 3 && R > (hm || hx ? 8 : 36) * per_sm * sms) return 0;
-    // a case's blocks; counted first
-    auto cut = [&](int c, int4 *out) {
-        return k1_cut(cs[c].nr, rows, most, [&](int i) { return mie_block_rows(n1(c, i)); }, [&](int i, int n) {
-            if (out) *out++ = make_int4(cs[c].r0 + cs[c].nr - 1 - i, n, c, 0);
-        });
-    };
+    std::vector<int4> &blk = K.blk;
     const int ncase = (int) ord.size();
-    std::vector<int> at(ncase + 1, 0);
-    parallel_for(ncase, 64, [&](int k) { at[k + 1] = cut(ord[k], nullptr); });
-    for (int k = 0; k < ncase; ++k) at[k + 1] += at[k];
-    blk.resize(at[ncase]);
-    parallel_for(ncase, 64, [&](int k) { cut(ord[k], blk.data() + at[k]); });
-    return rows;
+    int top = 0, top_dz = 0;               // orders of the longest radius, and of the cases with dD/dz
+    for (int k = 0; k < ncase; ++k) {
+        top = std::max(top, cn1max[k]);
+        if (dz[k]) top_dz = std::max(top_dz, cn1max[k]);
+    }
+    const int rows = std::max(mie_block_rows(top), R > 4 * sms ? K1_ROWS : 0);
+    const int smem = std::max(mie_block_smem(rows, hx, false), top_dz ? mie_block_smem(mie_block_rows(top_dz), hx, true) : 0);
+    if (R == 0 || smem > MIE_BLOCK_SMEM) return false;
+    int rows_dz = rows;
+    while (mie_block_smem(rows_dz, hx, true) > smem) rows_dz -= MIE_B;
+    const int per_sm = std::min(8, 227 * 1024 / (smem + 1024));
+    const int most = R <= 4 * sms ? 1 : std::min(MIE_BLOCK_MAX, std::max(4, (R + 4 * sms - 1) / (4 * sms)));
+    if (per_sm < 3 && R > (hm || hx ? 8 : 36) * per_sm * sms) return false;
+    // a case's blocks; counted first, but for a case alone
+    auto cut = [&](int c, int4 *out) {
+        return k1_cut(cs[c].nr, dz[c] ? rows_dz : rows, most, [&](int i) { return mie_block_rows(n1(c, i)); },
+                      [&](int i, int n) {
+                          if (out) *out++ = make_int4(cs[c].r0 + cs[c].nr - 1 - i, n, c, dz[c]);
+                      });
+    };
+    if (ncase == 1) {
+        blk.resize(R);
+        blk.resize(cut(ord[0], blk.data()));
+    } else {
+        std::vector<int> at(ncase + 1, 0);
+        parallel_for(ncase, 64, [&](int k) { at[k + 1] = cut(ord[k], nullptr); });
+        for (int k = 0; k < ncase; ++k) at[k + 1] += at[k];
+        blk.resize(at[ncase]);
+        parallel_for(ncase, 64, [&](int k) { cut(ord[k], blk.data() + at[k]); });
+    }
+    K.smem = smem;
+    K.rows = rows;
+    K.rows_dz = rows_dz;
+    return true;
 }
 
 // memcpy of a large block on one host thread per core
@@ -853,7 +874,7 @@ size_t case_bytes(const lmieb_problem &p) {
     for (int r = 0; r < p.n; ++r) tot += p.n1r[r] + 1;
     const size_t ncol = 1 + p.nd;
     size_t b = (size_t) tot * 32 * (1 + p.nd1);                        // coef
-    b += (size_t) (tot / MIE_B + p.n) * 8 * k1_ck_width(p.nd1 > 0);   // K1 checkpoints
+    b += (size_t) (tot / MIE_B + p.n) * 8 * k1_ck_width(p.nd1 > 0, p.nd1 > 0);   // K1 checkpoints
     b += (size_t) p.n * (64 + 8 * ncol + 40 * (2 + p.nd1));           // per-radius arrays, sums
     b += (size_t) 4 * ncol * p.n_qang * 8 * 8;                        // partials (groups), pf, pfn
     b += (size_t) ncol * 6 * p.n_coef * 8 * (3 + (p.n_qang / 2 + 31) / 32);   // expansion partials + outputs
@@ -999,7 +1020,7 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
         x_own = c.gather.x_own;
     }
     const int n_tan = (int) hm + (int) hx;                    // tangent columns of the coefficients
-    const int n_co = 1 + n_tan, n_rs = 1 + 2 * (int) hm + (int) hx, ck_w = k1_ck_width(hx);
+    const int n_co = 1 + n_tan, n_rs = 1 + 2 * (int) hm + (int) hx, ck_w = k1_ck_width(hm, hx);
     // an FP64 re-solve whose cases' K1 outputs are in an earlier sub-batch's
     // arena: their copy, in pieces of at most GATHER_PIECE doubles (one
     // block each), replaces K1
@@ -1030,12 +1051,16 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
     for (int k = 0; k < ncase; ++k) k1ord[k] = k;
     std::stable_sort(k1ord.begin(), k1ord.end(), [&](int a, int b) { return cn1max[a] > cn1max[b]; });
     for (int k = 0; k < ncase; ++k) k1pre[k + 1] = k1pre[k] + ps[k1ord[k]].n;
-    std::vector<int4> k1_blk;
-    // (K1's checkpoints are the thread-per-radius form's only)
-    const int k1_rows = re_solve ? 0 : k1_blocks(k1ord, cs, R, n1max, hm, hx, c.sms, k1_blk, [&](int k, int i) {
+    std::vector<char> case_dz(ncase, 0);
+    if (hm || x_own)
+        for (int k = 0; k < ncase; ++k)   // (the radii ascend: the host layer refuses others)
+            case_dz[k] = ps[k].n > 0 && mie_dz_chain(cs[k].m, ps[k].x[ps[k].n - 1]);
+    K1Blocks k1;
+    const bool k1_block = !re_solve && k1_blocks(k1ord, cs, cn1max, case_dz, R, hm, hx, c.sms, k1, [&](int k, int i) {
         return ps[k].n1r[ps[k].n - 1 - i];
     });
-    const size_t ck_used = k1_rows > 0 ? 0 : (size_t) ckn * ck_w;
+    // (K1's checkpoints are the thread-per-radius form's only)
+    const size_t ck_used = k1_block ? 0 : (size_t) ckn * ck_w;
 
     // ---- order tables ----
     std::vector<double> fv((size_t) 4 * (n1max + 2), 0.);
@@ -1647,7 +1672,7 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
         add(tg_nk.size() * 4); add(tg_off.size() * 8); add(oz_f2.size() * 8);
         add(a_start.size() * 8);
         for (int q = 0; q < 6; ++q) add((size_t) (ncase + 1) * 8);   // prefix arrays over the cases
-        add((size_t) ncase * 4); add((size_t) (ncase + 1) * 8); add(k1_blk.size() * sizeof(int4));   // K1 launch order and blocks
+        add((size_t) ncase * 4); add((size_t) (ncase + 1) * 8); add(k1.blk.size() * sizeof(int4));   // K1 launch order and blocks
         add(gl_ns.size() * 4); add(gl_mo.size() * 8); add(gl_go.size() * 8); add(gl_pt.size() * 4);
         add(gl_pi.size() * 4); add(gl_guess.size() * 8); add(gl_jr.size() * 8);
         if (L.save_control == 2) {
@@ -1685,7 +1710,7 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
         for (int i = 0; i < p.n; ++i) h_rcase[r0 + i] = k;
     }, host_cores());
     int *h_k1ord = put(hp, ho, k1ord.data(), (size_t) ncase);
-    int4 *h_k1blk = put(hp, ho, k1_blk.data(), k1_blk.size());
+    int4 *h_k1blk = put(hp, ho, k1.blk.data(), k1.blk.size());
     long long *h_k1pre = put(hp, ho, k1pre.data(), (size_t) ncase + 1);
     long long *h_off = put(hp, ho, coff.data(), (size_t) R + 1);
     long long *h_ckoff = put(hp, ho, ckoff.data(), (size_t) R + 1);
@@ -1792,8 +1817,10 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
     B.rs_m = 1;
     B.rs_x = 1 + 2 * (int) hm;
     B.oz_wl = wl;
-    B.k1_nblk = (int) k1_blk.size();
-    B.k1_rows = k1_rows;
+    B.k1_nblk = (int) k1.blk.size();
+    B.k1_smem = k1.smem;
+    B.k1_rows = k1.rows;
+    B.k1_rows_dz = k1.rows_dz;
     B.k1_blk = (const int4 *) dptr(h_k1blk);
     B.pu_lp = L.pu_lp;
     B.ex_run = L.ex_run;

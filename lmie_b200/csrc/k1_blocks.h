@@ -15,12 +15,16 @@ template <class Rows, class Put>
 inline int k1_cut(int nr, int rows, int most, Rows &&rows_of, Put &&put) {
     int nb = 0;
     for (int i = 0; i < nr; ++nb) {
-        int n = 1, longest = rows_of(i);
-        while (n < most && i + n < nr) {
+        int longest = rows_of(i), fit = rows / longest, n = 1;
+        if (fit > most) fit = most;
+        if (fit > nr - i) fit = nr - i;
+        for (; n < fit; ++n) {
             const int next = rows_of(i + n);
-            if (next > longest) longest = next;
-            if ((n + 1) * longest > rows) break;
-            ++n;
+            if (next > longest) {
+                longest = next;
+                if (fit > rows / longest) fit = rows / longest;
+                if (n >= fit) break;
+            }
         }
         put(i, n);
         i += n;

@@ -196,7 +196,7 @@ __device__ __forceinline__ MieRadius<HX> radius_setup(const DevBatch &B, const D
 template <bool HM, bool HX, bool TC>
 __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck, double *__restrict__ coef,
                                             float *__restrict__ bop, double *__restrict__ rs) {
-    constexpr int CW = k1_ck_width(HX);              // D (2), u (2), exponent, u's tangent (2)
+    constexpr int CW = k1_ck_width(HM, HX);          // D (2), u (2), exponent, u's tangent (2), D's (2)
     const long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= B.R) return;
     const int r = radius_of(B, t);
@@ -204,27 +204,33 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     const DevCase &C = B.cs[B.rcase[r]];
     const int n1 = B.n1r[r], n2 = B.n2r[r];
     const MieRadius<HX> c = radius_setup<HX>(B, C, r);
+    const bool zr = HM ? mie_dz_chain(C.m, c.x) : HX && B.x_own && mie_dz_chain(C.m, c.x);   // D's tangent
     const int nb = n1 / MIE_B + 1;
     double *ckr = ck + (size_t) B.ckoff[r] * CW;     // nb blocks of CW doubles
     const double *fv4 = B.fv + 3 * (B.n1max + 2), *fv3 = fv4 - (B.n1max + 2);
 
+    auto d_step = [&](MieD &p, int n) {
+        if ((HM || HX) && zr) p.step<true>(n, c.zinv, c.zinv2);
+        else p.step(n, c.zinv);
+    };
     // ---- downward: D from n2, u from n1 (n2 > n1 + MIE_B), block by block ----
     double u0, ux0 = 0.;
     int eu = 0;
     {
         MieD p;
         p.start();                                   // D_{n2} = 0, n2 > n1 + MIE_B
-        for (int n = n2 - 1; n >= nb * MIE_B; --n) p.step(n, c.zinv);
+        for (int n = n2 - 1; n >= nb * MIE_B; --n) d_step(p, n);
         MieU<HX> q;
         q.start();
         for (int b = nb - 1; b >= 0; --b) {
             double *w = ckr + (size_t) b * CW;
             w[0] = p.cur.re; w[1] = p.cur.im; w[2] = q.hi; w[3] = q.cur; w[4] = (double) eu;
-            if (HX) { w[5] = q.xhi; w[CW - 1] = q.xcur; }
+            if (HX) { w[5] = q.xhi; w[HX ? 6 : 0] = q.xcur; }
+            if (HM || HX) { w[CW - 2] = p.dz.re; w[CW - 1] = p.dz.im; }
 #pragma unroll
             for (int i = MIE_B - 1; i >= 0; --i) {
                 const int k = b * MIE_B + i;
-                if (b > 0 || i > 0) p.step(k, c.zinv);
+                if (b > 0 || i > 0) d_step(p, k);
                 if (k <= n1 && (b > 0 || i > 0)) q.step(k, c.xinv);
             }
             if (b > 0) eu += q.rescale();
@@ -238,7 +244,8 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     sincos(c.x, &sinx, &cosx);
     const double spsi = sinx / u0, spsix = HX ? fma(-spsi, ux0, cosx) / u0 : 0.;
     double chi_p = cosx, chi_c = fma(c.xinv, cosx, sinx);       // chi_0, chi_1
-    double psi_p = spsi * u0, psix_p = HX ? c.xl * fma(spsix, u0, spsi * ux0) : 0.;
+    double psi_p = spsi * u0, px = HX ? fma(spsix, u0, spsi * ux0) : 0.;   // px: d psi / dx
+    double psix_p = c.xl * px;
     MieSums<HM, HX> sums;
     sums.zero();
     MieAB prev;
@@ -264,20 +271,21 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
         {
             MieD p;
             p.cur = mk(w[0], w[1]);
+            p.dz = HM || HX ? mk(w[CW - 2], w[CW - 1]) : mk(0., 0.);
             MieU<HX> q;
             q.hi = w[2];
             q.cur = w[3];
-            if (HX) { q.xhi = w[5]; q.xcur = w[CW - 1]; }
+            if (HX) { q.xhi = w[5]; q.xcur = w[HX ? 6 : 0]; }
 #pragma unroll
             for (int i = MIE_B - 1; i >= 0; --i) {
                 const int k = b * MIE_B + i;
                 ub[i] = q.cur;
                 if (HX) uxb[HX ? i : 0] = q.xcur;
                 if (k > 0) {
-                    p.step(k, c.zinv);
+                    d_step(p, k);
                     if (k <= n1) {
                         D[i] = p.cur;
-                        if (HM || HX) Dz[i] = mie_dz(c, k, p.cur);
+                        if (HM || HX) Dz[i] = zr ? p.dz : mie_dz(c, k, p.cur);
                         q.step(k, c.xinv);
                     }
                 }
@@ -287,7 +295,9 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
         for (int i = 0; i < MIE_B; ++i) {
             const int j = b * MIE_B + i;
             if (j < 1 || j > n1) continue;
-            const double psi = spsi * ub[i] * su, psix = HX ? c.xl * (fma(spsix, ub[i], spsi * uxb[HX ? i : 0]) * su) : 0.;
+            const double psi = spsi * ub[i] * su;
+            if (HX) px = fma(spsix, ub[i], spsi * uxb[HX ? i : 0]) * su;
+            const double psix = c.xl * px;
             const MieAB q = mie_ab<HM, HX>(c, j, D[i], Dz[i], psi, psi_p, chi_c, chi_p, psix, psix_p);
             sums.add(j, q, prev, fv3[j - 1], fv4[j - 1]);
             const double f4 = fv4[j];
@@ -344,7 +354,7 @@ __global__ void __launch_bounds__(MIE_BLOCK_T, HX ? 2 : 4) k_mie_block(DevBatch 
     constexpr int TS = TEAM == 32 ? 32 : MIE_BLOCK_T;
     const int tl = threadIdx.x % TS;
     mie_block<HM, HX, TEAM>(
-        smem, B.k1_rows, blk.y,
+        smem, (HM || HX) && blk.w ? B.k1_rows_dz : B.k1_rows, (HM || HX) && blk.w, blk.y,
         [&](MieRadius<HX> &c) {
             c.set_m(C.m, C.minv, HX && B.x_own ? B.m_l[C.ml_off + B.idx1[0]] : mk(0., 0.));
         },
@@ -414,7 +424,7 @@ int launch_block(cudaStream_t s, const DevBatch &B, double *coef, float *bop, do
                                             MIE_BLOCK_SMEM));
         attr = true;
     }
-    k_mie_block<HM, HX, TC, TEAM><<<B.k1_nblk, MIE_BLOCK_T, mie_block_smem(B.k1_rows, HX), s>>>(B, coef, bop, rs);
+    k_mie_block<HM, HX, TC, TEAM><<<B.k1_nblk, MIE_BLOCK_T, B.k1_smem, s>>>(B, coef, bop, rs);
     LMIEB_CUDA_TRY(cudaGetLastError());
     return 0;
 }

@@ -38,7 +38,7 @@ constexpr double NA_MAX_X = 900.;
 struct Trunc {
     int2 n[NA_MAX_RADII];
 };
-static_assert(mie_block_smem(mie_block_rows(NA_MAX_ORDER), false) <= 48 * 1024, "shared memory of a block");
+static_assert(mie_block_smem(mie_block_rows(NA_MAX_ORDER), false, false) <= 48 * 1024, "shared memory of a block");
 
 // Bound by FP64 latency: the three chains of the largest radius (n1 dependent
 // pairs of FMAs), then n1 / 128 rounds of orders.  1000 radii up to x = 880: 66 us, the
@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(MIE_BLOCK_T) k_cross_sections(int n, const dou
         return;
     }
     mie_block<false, false, MIE_BLOCK_T>(
-        smem, rows, 1,
+        smem, rows, false, 1,
         [&](MieRadius<false> &c) { c.set_m(m, minv, mk(0., 0.)); },
         [&](int, MieRadius<false> &c, int &n1, int &n2) {
             c.set_x(2. * LMIEB_PI * radius[i] / lambda, 0.);
@@ -120,7 +120,7 @@ extern "C" int lmie_cross_sections_noalloc(int n_radii, const double *radius, do
         n1max = n1 > n1max ? n1 : n1max;
     }
     const int rows = mie_block_rows(n1max);
-    k_cross_sections<<<n_radii, MIE_BLOCK_T, mie_block_smem(rows, false), s>>>(n_radii, radius, lambda, m, 1. / m, rows,
+    k_cross_sections<<<n_radii, MIE_BLOCK_T, mie_block_smem(rows, false, false), s>>>(n_radii, radius, lambda, m, 1. / m, rows,
                                                                                trunc, out);
     LMIEB_CUDA_TRY(cudaGetLastError());
     LMIEB_CUDA_TRY(cudaStreamSynchronize(s));

@@ -21,10 +21,12 @@
 // Im D, which is all of a small absorbing sphere's extinction (see MIE_P_MIN).
 //
 // Derivatives: dD/dz = n/z^2 - 1 + (n/z - D)(n/z + D), the Riccati equation with
-// its difference of large terms in factors, no recurrence of its own; chi' =
-// chi_{n-1} - n/x chi_n; psi' from the tangent of u's recurrence, since u is not
-// exactly psi (it starts from zero at n1) and the reference differentiates what
-// it computes.
+// its difference of large terms in factors, no recurrence of its own, for
+// radii through which light gets; of others D is near -i and the terms cancel, so
+// where they are wanted by m theirs is the tangent of D's recurrence (see
+// MIE_DZ_MIN).  chi' = chi_{n-1} - n/x chi_n.  psi' from the tangent of u's
+// recurrence, since u is not exactly psi (it starts from zero at n1) and the
+// reference differentiates what it computes.
 //
 // Every FMA is written out, and K1's and the cross sections' files are compiled
 // without FMA contraction, so with derivatives a radius' coefficients are the
@@ -55,12 +57,18 @@ constexpr int MIE_BLOCK_SMEM = 220 * 1024;            // what a block may take
 // x = 2 (15 orders) to 900 equal for Cext, Csca, Cbak, g and Cext - Csca.  A
 // chain of D from below 32 orders takes at most 3 us.
 constexpr int MIE_P_MIN = 32;
+// mi x from which dD/dz for a derivative by m is the tangent of D's recurrence.
+// Medians of d Cext/dmr of 400 spheres of x 100 .. 900 against 113-bit arithmetic,
+// tangent / Riccati: mi x 0.3 .. 1 9.2e-14 / 9.4e-14, 1 .. 3 8.9e-14 / 1.0e-13,
+// 3 .. 10 2.7e-13 / 4.1e-12, 30 .. 100 9.3e-15 / 7.2e-13; x 8 .. 96 alike.  By x the two
+// are equal everywhere.
+constexpr double MIE_DZ_MIN = 0.5;
 
-// rows of shared memory of a radius of n1 orders; bytes of a block of that many rows: D, u, chi (and u's
-// tangent), two exponents per MIE_B orders, reduction space, what the team needs to know of each radius
+// rows of shared memory of a radius of n1 orders; bytes of a block of that many rows: D, u, chi (hx: and u's
+// tangent; dz: and D's), two exponents per MIE_B orders, reduction space, what the team needs to know of each radius
 __host__ __device__ constexpr int mie_block_rows(int n1) { return (n1 + 2 * MIE_B) & ~(MIE_B - 1); }
-__host__ __device__ constexpr int mie_block_smem(int rows, bool hx) {
-    return rows * (16 + 8 + 8 + (hx ? 8 : 0)) + rows / MIE_B * 8 + (4 * 12 + 20 * 4) * 8 + MIE_BLOCK_MAX * 72;
+__host__ __device__ constexpr int mie_block_smem(int rows, bool hx, bool dz) {
+    return rows * (16 + 8 + 8 + (hx ? 8 : 0) + (dz ? 16 : 0)) + rows / MIE_B * 8 + (4 * 12 + 20 * 4) * 8 + MIE_BLOCK_MAX * 72;
 }
 
 #ifdef __CUDACC__
@@ -93,6 +101,9 @@ __device__ __forceinline__ cplx cmulc(cplx a, cplx b) {
 // Re(a conj(b)) + c
 __device__ __forceinline__ double rfmac(cplx a, cplx b, double c) { return fma(a.re, b.re, fma(a.im, b.im, c)); }
 __device__ __forceinline__ double rmulc(cplx a, cplx b) { return fma(a.re, b.re, a.im * b.im); }
+
+// whether a radius takes dD/dz from D's recurrence (where a derivative by m is wanted)
+__host__ __device__ __forceinline__ bool mie_dz_chain(cplx m, double x) { return fabs(m.im) * x > MIE_DZ_MIN; }
 
 // What every order of a radius needs.
 template <bool HX>
@@ -140,18 +151,25 @@ struct MieP {
     }
 };
 
-// The chain of D_n (cur), from D_{n2} = 0.
+// The chain of D_n (cur), from D_{n2} = 0, and its tangent dD/dz (dz).
 struct MieD {
-    cplx cur;
-    __device__ __forceinline__ void start() { cur = mk(0., 0.); }
-    // from D_{n + 1} to D_n
-    __device__ __forceinline__ void step(int n, cplx zinv) {
+    cplx cur, dz;
+    __device__ __forceinline__ void start() { cur = dz = mk(0., 0.); }
+    // from D_{n + 1} to D_n; DZ: the tangent too
+    template <bool DZ>
+    __device__ __forceinline__ void step(int n, cplx zinv, cplx zinv2) {
         const double s = n + 1.;
         const cplx g = mk(__dmul_rn(s, zinv.re), __dmul_rn(s, zinv.im));
         const cplx e = mk(__dadd_rn(cur.re, g.re), __dadd_rn(cur.im, g.im));
         const double d = 1. / fma(e.re, e.re, e.im * e.im);
-        cur = mk(__dsub_rn(g.re, __dmul_rn(e.re, d)), __dadd_rn(g.im, __dmul_rn(e.im, d)));
+        const cplx i = mk(__dmul_rn(e.re, d), -__dmul_rn(e.im, d));   // 1 / e
+        if (DZ) {
+            const cplx h = -s * zinv2;                                // dg/dz
+            dz = cfma(dz + h, i * i, h);
+        }
+        cur = mk(__dsub_rn(g.re, i.re), __dsub_rn(g.im, i.im));
     }
+    __device__ __forceinline__ void step(int n, cplx zinv) { step<false>(n, zinv, zinv); }
 };
 
 // The chain of u (and its tangent w.r.t. x): cur = u_n, hi = u_{n+1}.
@@ -186,7 +204,7 @@ struct MieU {
     }
 };
 
-// dD/dz of D_n
+// dD/dz of D_n from the Riccati equation
 template <bool HX>
 __device__ __forceinline__ cplx mie_dz(const MieRadius<HX> &c, int n, cplx D) {
     const cplx nz = (double) n * c.zinv;
@@ -290,15 +308,16 @@ struct MieSums {
 // shared memory laid out for `rows`.  common(c) sets up what the radii share,
 // radius(g, c, n1, n2) radius g; factors(n, f3, f4) gives MieSums::add's;
 // begin(g) is called by a radius' team, then store(n, ab) once per order, by one
-// thread each, and sum(sums) by all its threads.
+// thread each, and sum(sums) by all its threads.  dz: some of them take dD/dz from
+// D's recurrence.
 template <bool HM, bool HX, int TEAM, class Common, class Radius, class Factors, class Begin, class Store, class Sum>
-__device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, Common &&common, Radius &&radius,
+__device__ __forceinline__ void mie_block(unsigned char *smem, int rows, bool dz, int G, Common &&common, Radius &&radius,
                                           Factors &&factors, Begin &&begin, Store &&store, Sum &&sum) {
     constexpr int T = MIE_BLOCK_T, W = T / 32, NP = HX ? 12 : 8, NS = MieSums<HM, HX>::N;
     static_assert(TEAM == T || TEAM == 32, "the block or a warp");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    double2 *Ds = (double2 *) smem;
-    double *u = (double *) (Ds + rows), *chi = u + rows, *ux = chi + rows;
+    double2 *Ds = (double2 *) smem, *Dzs = Ds + rows;
+    double *u = (double *) (dz ? Dzs + rows : Dzs), *chi = u + rows, *ux = chi + rows;
     double *pass = chi + rows + (HX ? rows : 0);      // [W][12] last coefficients of a warp
     double *red = pass + W * 12;                      // [20][W]
     // psi_n = spsi u_n 2^(eU[n / MIE_B] - eu)
@@ -339,10 +358,20 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
             if (chain_d(n1)) {
                 MieD p;
                 p.start();
-                for (int n = n2 - 1; n > n1; --n) p.step(n, c.zinv);
-                for (int n = n1; n >= 1; --n) {       // n2 > n1
-                    p.step(n, c.zinv);
-                    Dr[n] = make_double2(p.cur.re, p.cur.im);
+                if (DER && dz) {
+                    double2 *Zr = Dzs + row;
+                    for (int n = n2 - 1; n > n1; --n) p.step<true>(n, c.zinv, c.zinv2);
+                    for (int n = n1; n >= 1; --n) {
+                        p.step<true>(n, c.zinv, c.zinv2);
+                        Dr[n] = make_double2(p.cur.re, p.cur.im);
+                        Zr[n] = make_double2(p.dz.re, p.dz.im);
+                    }
+                } else {
+                    for (int n = n2 - 1; n > n1; --n) p.step(n, c.zinv);
+                    for (int n = n1; n >= 1; --n) {   // n2 > n1
+                        p.step(n, c.zinv);
+                        Dr[n] = make_double2(p.cur.re, p.cur.im);
+                    }
                 }
             } else {
                 MieP p;
@@ -418,7 +447,8 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
         if (HX) c.xl = sh_xl[g];
         const double spsi = sh_psi[g], spsix = HX ? sh_psix[g] : 0.;
         const int eu0 = sh_eu[g], row = sh_row[g];
-        const double2 *Dr = Ds + row;
+        const double2 *Dr = Ds + row, *Zr = Dzs + row;
+        const bool zr = DER && dz && mie_dz_chain(c.m, c.x);
         const double *ur = u + row, *uxr = ux + row, *cr = chi + row;
         const int *eur = eU + row / MIE_B;
         MieSums<HM, HX> sums;
@@ -436,7 +466,12 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, int G, 
             if (on) {
                 const double2 dj = Dr[j];
                 cplx D = mk(dj.x, dj.y), Dz = mk(0., 0.);
-                if (DER) Dz = mie_dz(c, j, D);
+                if (zr) {
+                    const double2 zj = Zr[j];
+                    Dz = mk(zj.x, zj.y);
+                } else if (DER) {
+                    Dz = mie_dz(c, j, D);
+                }
                 if (!chain_d(n1)) {
                     const double2 lo = Dr[j - 1];
                     const int *er = eP + row / MIE_B;
