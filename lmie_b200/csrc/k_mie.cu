@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     const int n1 = B.n1r[r], n2 = B.n2r[r];
     const MieRadius<HX> c = radius_setup<HX>(B, C, r);
     const bool zr = HM ? mie_dz_chain(C.m, c.x) : HX && B.x_own && mie_dz_chain(C.m, c.x);   // D's tangent
+    const bool ratio = HX && n1 < MIE_P_MIN;         // q.cur, q.xcur: psi's ratio and its tangent
     const int nb = n1 / MIE_B + 1;
     double *ckr = ck + (size_t) B.ckoff[r] * CW;     // nb blocks of CW doubles
     const double *fv4 = B.fv + 3 * (B.n1max + 2), *fv3 = fv4 - (B.n1max + 2);
@@ -212,6 +213,14 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     auto d_step = [&](MieD &p, int n) {
         if ((HM || HX) && zr) p.step<true>(n, c.zinv, c.zinv2);
         else p.step(n, c.zinv);
+    };
+    // (the ratio of order n - 1; that of order 0 is not used)
+    auto u_step = [&](MieU<HX> &q, int n) {
+        if (HX && ratio) {
+            mie_ratio(n - 1, c.xinv, q.cur, q.xcur);
+        } else {
+            q.step(n, c.xinv);
+        }
     };
     // ---- downward: D from n2, u from n1 (n2 > n1 + MIE_B), block by block ----
     double u0, ux0 = 0.;
@@ -231,9 +240,9 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
             for (int i = MIE_B - 1; i >= 0; --i) {
                 const int k = b * MIE_B + i;
                 if (b > 0 || i > 0) d_step(p, k);
-                if (k <= n1 && (b > 0 || i > 0)) q.step(k, c.xinv);
+                if (k <= n1 && (b > 0 || i > 0)) u_step(q, k);
             }
-            if (b > 0) eu += q.rescale();
+            if (b > 0 && !ratio) eu += q.rescale();
         }
         u0 = q.cur;
         if (HX) ux0 = q.xcur;
@@ -245,6 +254,10 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     const double spsi = sinx / u0, spsix = HX ? fma(-spsi, ux0, cosx) / u0 : 0.;
     double chi_p = cosx, chi_c = fma(c.xinv, cosx, sinx);       // chi_0, chi_1
     double psi_p = spsi * u0, px = HX ? fma(spsix, u0, spsi * ux0) : 0.;   // px: d psi / dx
+    if (ratio) {
+        psi_p = sinx;
+        px = cosx;
+    }
     double psix_p = c.xl * px;
     MieSums<HM, HX> sums;
     sums.zero();
@@ -286,7 +299,7 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
                     if (k <= n1) {
                         D[i] = p.cur;
                         if (HM || HX) Dz[i] = zr ? p.dz : mie_dz(c, k, p.cur);
-                        q.step(k, c.xinv);
+                        u_step(q, k);
                     }
                 }
             }
@@ -295,8 +308,8 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
         for (int i = 0; i < MIE_B; ++i) {
             const int j = b * MIE_B + i;
             if (j < 1 || j > n1) continue;
-            const double psi = spsi * ub[i] * su;
-            if (HX) px = fma(spsix, ub[i], spsi * uxb[HX ? i : 0]) * su;
+            const double psi = ratio ? ub[i] * psi_p : spsi * ub[i] * su;
+            if (HX) px = ratio ? fma(uxb[HX ? i : 0], psi_p, ub[i] * px) : fma(spsix, ub[i], spsi * uxb[HX ? i : 0]) * su;
             const double psix = c.xl * px;
             const MieAB q = mie_ab<HM, HX>(c, j, D[i], Dz[i], psi, psi_p, chi_c, chi_p, psix, psix_p);
             sums.add(j, q, prev, fv3[j - 1], fv4[j - 1]);

@@ -26,7 +26,9 @@
 // where they are wanted by m theirs is the tangent of D's recurrence (see
 // MIE_DZ_MIN).  chi' = chi_{n-1} - n/x chi_n.  psi' from the tangent of u's
 // recurrence, since u is not exactly psi (it starts from zero at n1) and the
-// reference differentiates what it computes.
+// reference differentiates what it computes; for radii of fewer than MIE_P_MIN
+// orders, whose u grows by orders of magnitude between psi's few, from the tangent
+// of the reference's ratios.
 //
 // Every FMA is written out, and K1's and the cross sections' files are compiled
 // without FMA contraction, so with derivatives a radius' coefficients are the
@@ -56,6 +58,11 @@ constexpr int MIE_BLOCK_SMEM = 220 * 1024;            // what a block may take
 // 1.1e-15 / 1.2e-14, x 0.3 .. 1 2.4e-15 / 5.4e-15, x 1 .. 2 2.9e-15 / 3.7e-15; from
 // x = 2 (15 orders) to 900 equal for Cext, Csca, Cbak, g and Cext - Csca.  A
 // chain of D from below 32 orders takes at most 3 us.
+//
+// With the x column, psi and its tangent of smaller radii come from the ratios
+// psi_n / psi_{n-1}, as the reference's: medians of d Cext/dx at x 1 .. 2 5.5e-16 (from u
+// 7.7e-16), of dg/dx at 0.1 .. 0.3 2.3e-14 (1.0e-13); from x = 5 on u's are the better
+// ones (x 100 .. 900 1.2e-12, ratios 1.9e-12).
 constexpr int MIE_P_MIN = 32;
 // mi x from which dD/dz for a derivative by m is the tangent of D's recurrence.
 // Medians of d Cext/dmr of 400 spheres of x 100 .. 900 against 113-bit arithmetic,
@@ -203,6 +210,13 @@ struct MieU {
         return g;
     }
 };
+
+// One order of the ratio r_n = psi_n / psi_{n-1} and its tangent, from those of order n + 1 (zeros at n1).
+__device__ __forceinline__ void mie_ratio(int n, double xinv, double &r, double &rx) {
+    const double c = (2. * n + 1.) * xinv, q = 1. / (c - r);
+    rx = fma(c, xinv, rx) * (q * q);
+    r = q;
+}
 
 // dD/dz of D_n from the Riccati equation
 template <bool HX>
@@ -395,6 +409,30 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, bool dz
                     e += p.rescale();
                 }
             }
+        } else if (HX && warp == 1 && n1 < MIE_P_MIN) {
+            // psi and psi' themselves in the place of u and its tangent
+            double *ur = u + row, *uxr = ux + row, r = 0., rx = 0.;
+            int *er = eU + row / MIE_B;
+            ur[n1] = uxr[n1] = 0.;
+            for (int n = n1 - 1; n >= 1; --n) {
+                mie_ratio(n, c.xinv, r, rx);
+                ur[n] = r;
+                uxr[n] = rx;
+            }
+            double psi, px;
+            sincos(c.x, &psi, &px);
+            for (int n = 0; n <= n1; ++n) {
+                if (n > 0) {
+                    px = fma(uxr[n], psi, ur[n] * px);
+                    psi = ur[n] * psi;
+                }
+                ur[n] = psi;
+                uxr[n] = px;
+                er[n / MIE_B] = 0;
+            }
+            sh_psi[lane] = 1.;
+            sh_psix[lane] = 0.;
+            sh_eu[lane] = 0;
         } else if (warp == 1) {
             MieU<HX> q;
             q.start();

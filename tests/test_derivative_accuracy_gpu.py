@@ -8,6 +8,9 @@ Bounds, fixed before the first run, on the median over the spheres:
   tangent likewise.  d Cext, a difference of the orders' oscillating terms, may
   have all of it twice, 2e-13; d Csca sums terms of one sign: 1e-14.  (With
   dD/dz as a difference of terms of order 1: 1e-12 and 3e-14.)
+- small spheres (x from 0.02 to 0.5) by the wavelength.  g is a sum whose terms
+  cancel to x^2 of their size, so eight roundings of 2^-52 make 8 2^-52 / x^2.
+  (With psi' as a difference of two terms: 13 to 20.)
 """
 import numpy as np
 import pytest
@@ -20,6 +23,7 @@ from lmie_b200.abi import deriv_unit
 pytestmark = pytest.mark.gpu
 
 LAM = 0.7
+EPS = 2.**-52
 
 
 def solve(x, mr, mi, derivs, extra=()):
@@ -49,3 +53,12 @@ def test_absorbing_spheres_by_the_refractive_index(mr, mi, threads):
             w = want[name].d * (np.longdouble(LAM) * np.longdouble(LAM) / (2 * np.longdouble(np.pi)))
             err = np.abs(np.array([g.scalars_l[name][k] for g in got]).astype(np.longdouble) - w) / np.abs(w)
             assert np.median(err) <= bound, (name, k, float(np.median(err)))
+
+
+@pytest.mark.parametrize("mr, mi", [(1.4, 0.01), (1.33, 1e-6)])
+@pytest.mark.parametrize("threads", [False, True])
+def test_small_spheres_by_the_wavelength(mr, mi, threads):
+    x, got = solve(np.geomspace(0.02, 0.5, 300), mr, mi, ("lambda",), [long_radii(2600, ("lambda",))] if threads else ())
+    want = mie_extended.cross_sections(x, mr, mi, -x.astype(np.longdouble) / np.longdouble(LAM), 0.)["g"].d
+    err = np.abs(np.array([g.scalars_l["g"][0] for g in got]).astype(np.longdouble) - want) / np.abs(want)
+    assert np.median(err * x * x) <= 8 * EPS, float(np.median(err * x * x)) / EPS
