@@ -307,14 +307,18 @@ extern "C" void lmieb_host_parallel(int n, int n_threads, void (*fn)(void *, int
 // by blocks and 3.1 by threads, 8000 radii 4.7 and 3.8; with, 1000 radii about 2
 // and 3.7 ms, 8000 radii 24 and 4.2.
 struct K1Blocks {
-    std::vector<int4> blk;
+    const int4 *blk = nullptr;             // until the next call (calls are serialised)
+    int n = 0;
     int smem = 0, rows = 0, rows_dz = 0;   // of a block; its rows, without and with dD/dz
 };
+// pre[k]: radii of the cases before ord[k].  The pool's threads take 30 us to
+// start: cutting the radii one after the other is as fast up to K1_SERIAL of them.
 template <class Orders>
-bool k1_blocks(const std::vector<int> &ord, const std::vector<DevCase> &cs, const std::vector<int> &cn1max,
-               const std::vector<char> &dz, int R, bool hm, bool hx, int sms, K1Blocks &K, Orders &&n1) {
+bool k1_blocks(const std::vector<int> &ord, const std::vector<long long> &pre, const std::vector<DevCase> &cs,
+               const std::vector<int> &cn1max, const std::vector<char> &dz, int R, bool hm, bool hx, int sms,
+               K1Blocks &K, Orders &&n1) {
+    constexpr int K1_SERIAL = 16384;
     constexpr int K1_ROWS = 1500;
-    std::vector<int4> &blk = K.blk;
     const int ncase = (int) ord.size();
     int top = 0, top_dz = 0;               // orders of the longest radius, and of the cases with dD/dz
     for (int k = 0; k < ncase; ++k) {
@@ -329,23 +333,25 @@ bool k1_blocks(const std::vector<int> &ord, const std::vector<DevCase> &cs, cons
     const int per_sm = std::min(8, 227 * 1024 / (smem + 1024));
     const int most = R <= 4 * sms ? 1 : std::min(MIE_BLOCK_MAX, std::max(4, (R + 4 * sms - 1) / (4 * sms)));
     if (per_sm < 3 && R > (hm || hx ? 8 : 36) * per_sm * sms) return false;
-    // a case's blocks; counted first, but for a case alone
+    static std::vector<int4> blk;          // kept between calls
+    if ((int) blk.size() < R) blk.resize(R);
     auto cut = [&](int c, int4 *out) {
         return k1_cut(cs[c].nr, dz[c] ? rows_dz : rows, most, [&](int i) { return mie_block_rows(n1(c, i)); },
-                      [&](int i, int n) {
-                          if (out) *out++ = make_int4(cs[c].r0 + cs[c].nr - 1 - i, n, c, dz[c]);
-                      });
+                      [&](int i, int n) { *out++ = make_int4(cs[c].r0 + cs[c].nr - 1 - i, n, c, dz[c]); });
     };
-    if (ncase == 1) {
-        blk.resize(R);
-        blk.resize(cut(ord[0], blk.data()));
+    K.n = 0;
+    if (R <= K1_SERIAL) {
+        for (int c : ord) K.n += cut(c, blk.data() + K.n);
     } else {
-        std::vector<int> at(ncase + 1, 0);
-        parallel_for(ncase, 64, [&](int k) { at[k + 1] = cut(ord[k], nullptr); });
-        for (int k = 0; k < ncase; ++k) at[k + 1] += at[k];
-        blk.resize(at[ncase]);
-        parallel_for(ncase, 64, [&](int k) { cut(ord[k], blk.data() + at[k]); });
+        // every case's from where a block per radius would put them, then closed up
+        std::vector<int> nb(ncase);
+        parallel_for(ncase, 64, [&](int k) { nb[k] = cut(ord[k], blk.data() + pre[k]); });
+        for (int k = 0; k < ncase; ++k) {
+            if (pre[k] > K.n) std::copy_n(blk.data() + pre[k], nb[k], blk.data() + K.n);
+            K.n += nb[k];
+        }
     }
+    K.blk = blk.data();
     K.smem = smem;
     K.rows = rows;
     K.rows_dz = rows_dz;
@@ -1056,7 +1062,7 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
         for (int k = 0; k < ncase; ++k)   // (the radii ascend: the host layer refuses others)
             case_dz[k] = ps[k].n > 0 && mie_dz_chain(cs[k].m, ps[k].x[ps[k].n - 1]);
     K1Blocks k1;
-    const bool k1_block = !re_solve && k1_blocks(k1ord, cs, cn1max, case_dz, R, hm, hx, c.sms, k1, [&](int k, int i) {
+    const bool k1_block = !re_solve && k1_blocks(k1ord, k1pre, cs, cn1max, case_dz, R, hm, hx, c.sms, k1, [&](int k, int i) {
         return ps[k].n1r[ps[k].n - 1 - i];
     });
     // (K1's checkpoints are the thread-per-radius form's only)
@@ -1672,7 +1678,7 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
         add(tg_nk.size() * 4); add(tg_off.size() * 8); add(oz_f2.size() * 8);
         add(a_start.size() * 8);
         for (int q = 0; q < 6; ++q) add((size_t) (ncase + 1) * 8);   // prefix arrays over the cases
-        add((size_t) ncase * 4); add((size_t) (ncase + 1) * 8); add(k1.blk.size() * sizeof(int4));   // K1 launch order and blocks
+        add((size_t) ncase * 4); add((size_t) (ncase + 1) * 8); add((size_t) k1.n * sizeof(int4));   // K1 launch order and blocks
         add(gl_ns.size() * 4); add(gl_mo.size() * 8); add(gl_go.size() * 8); add(gl_pt.size() * 4);
         add(gl_pi.size() * 4); add(gl_guess.size() * 8); add(gl_jr.size() * 8);
         if (L.save_control == 2) {
@@ -1710,7 +1716,7 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
         for (int i = 0; i < p.n; ++i) h_rcase[r0 + i] = k;
     }, host_cores());
     int *h_k1ord = put(hp, ho, k1ord.data(), (size_t) ncase);
-    int4 *h_k1blk = put(hp, ho, k1.blk.data(), k1.blk.size());
+    int4 *h_k1blk = put(hp, ho, k1.blk, (size_t) k1.n);
     long long *h_k1pre = put(hp, ho, k1pre.data(), (size_t) ncase + 1);
     long long *h_off = put(hp, ho, coff.data(), (size_t) R + 1);
     long long *h_ckoff = put(hp, ho, ckoff.data(), (size_t) R + 1);
@@ -1817,7 +1823,7 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
     B.rs_m = 1;
     B.rs_x = 1 + 2 * (int) hm;
     B.oz_wl = wl;
-    B.k1_nblk = (int) k1.blk.size();
+    B.k1_nblk = k1.n;
     B.k1_smem = k1.smem;
     B.k1_rows = k1.rows;
     B.k1_rows_dz = k1.rows_dz;
