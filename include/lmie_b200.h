@@ -32,8 +32,14 @@ int lmie_solution_batch(int n_cases, lmie_in_data *in, lmie_out_data *out, int a
  * LMIEB_PRECISION_FP64: the reference's arithmetic (within 1e-10 of it);
  *   lmie_solution and lmie_solution_batch use it.  Every stage runs in FP64 but
  *   the angular S1/S2 sums of sub-batches with 2e6 products and more, which are
- *   formed as LMIEB_PRECISION_INT8 does with seven digits (2^-53 of the largest
+ *   formed as LMIEB_PRECISION_INT8 does with seven digits (2^-54 of the largest
  *   term of a row and column), closer to 64-bit truth than the FP64 kernel's.
+ *   n_coef is the FP64 kernel's (cases that could differ are solved again with
+ *   it).  Which sums a case takes, and how its radii's orders are summed, goes
+ *   by its whole sub-batch, so a case's results can differ in their last
+ *   digits from those of the same case in other company or alone; integrals
+ *   taken away (lmieb_solution_partial) and those of a group of processes are
+ *   always the FP64 kernel's.
  * LMIEB_PRECISION_TF32X3: the angular S1/S2 contraction runs on the tensor
  *   cores with each operand split into two TF32 terms (lo*hi + hi*lo + hi*hi):
  *   the hi*hi products accumulate in FP32 over segments of 32 orders
@@ -49,13 +55,14 @@ int lmie_solution_batch(int n_cases, lmie_in_data *in, lmie_out_data *out, int a
  *   cores as an exact fixed-point sum: each operand value is scaled by powers
  *   of two (per order, per angle row, per operand column) to 47 fractional
  *   bits and split into six signed 8-bit digits; the 21 digit products that
- *   carry the result are summed exactly in int32 and combined in FP64.  Each
+ *   carry the result are summed exactly in int32, combined in int64 and rounded
+ *   to FP64 once.  Each
  *   product carries about 2^-46 of the largest term of its row and column
- *   (FP64: 2^-53 of itself); everything else is the FP64 form's arithmetic.  A case
+ *   (FP64: 2^-53 of itself); everything else is in FP64.  A case
  *   whose truncation n_coef could depend on that difference -- some
  *   |beta_l| (l < n_coef) within the contraction's error bound of `accuracy`
- *   -- is solved again in FP64 within the same call, so n_coef is always the
- *   FP64 form's.  Problems this mode does not cover (save_control != 0, more
+ *   -- is solved again with the FP64 kernel within the same call, so n_coef is
+ *   always that kernel's.  Problems this mode does not cover (save_control != 0, more
  *   than 4 index1 or 3 index2 derivative slots) and cases of fewer than 16 or
  *   more than 5120 orders run in FP64. */
 #define LMIEB_PRECISION_INT8 2

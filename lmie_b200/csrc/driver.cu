@@ -84,7 +84,7 @@ struct Slot {
     // other slots too.
     cudaStream_t down = nullptr;
     cudaEvent_t kdone = nullptr;       // after the sub-batch's kernels (the downloads wait for it)
-    // int8 K3's A operand and row exponents depend on the angles only: they
+    // the fixed-point K3's A operand and row exponents depend on the angles only: they
     // run on this stream beside K1 (fork and join events)
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;

@@ -45,9 +45,9 @@ struct DevCase {
     long long pu_scr_off;       // K5 with more than one part: its [part][ncol][6][n_angles] partial sums
     int scal_off;               // [ncol][4] normalised cross sections and g
     int G;                      // angular radius groups
-    int nkx;                    // int8 K3: chunks of OZ_KC orders its row exponents cover
-    long long rx_off;           // int8 K3: its row exponents ([nh][2] bytes)
-    long long a_off;            // int8 K3: its A operand digits ([tile][nkx][AROW / 16 pieces][OZ_M rows][16 bytes])
+    int nkx;                    // fixed-point K3: chunks of OZ_KC orders its row exponents cover
+    long long rx_off;           // fixed-point K3: its row exponents ([nh][2] bytes)
+    long long a_off;            // fixed-point K3: its A operand digits ([tile][nkx][AROW / 16 pieces][OZ_M rows][16 bytes])
     double trunc_band;          // > 0: K4 records where |beta_l| comes within trunc_band (2l + 1)
                                 // of `accuracy` (band[2c], band[2c + 1]; see launch_expand)
 };
@@ -91,7 +91,7 @@ struct DevBatch {
                                 //     (-1: the radius' case keeps the FP64 angular stage)
     const long long *tc_roff;   // [R] float offset of the radius' group in the B operand
     const int *tg_r0, *tg_n, *tg_nk;   // per group: first radius, radii, chunks of TC_KC orders
-    const long long *tg_off;    // per group: float offset of its B operand block (int8 K3: byte offset)
+    const long long *tg_off;    // per group: float offset of its B operand block (fixed-point K3: byte offset)
     // int8 fixed-point K3 (oz_layout.cuh); null in the other forms
     int oz_wl;                  // some index1 derivative moves the weights (w rows 1 + idx1 not all zero)
     const double *oz_f2;        // [OZ_KC * max chunks + 2]: (k + 1) / k

@@ -47,8 +47,8 @@ constexpr int MIE_B = 4;                              // orders per block of the
 // after the other, and one of many is held by the latency of an order (some 1800
 // cycles with derivatives).  Here three warps run the three chains of the
 // block's radii, a lane each, into shared memory, and then the orders are formed
-// side by side: by all threads for one radius (TEAM 128), a warp per radius
-// (TEAM 32) for several.
+// side by side: by all threads, radius after radius (TEAM 128), or by a
+// warp per radius (TEAM 32).
 constexpr int MIE_BLOCK_T = 128;
 constexpr int MIE_BLOCK_MAX = 32;                     // radii of a block
 constexpr int MIE_BLOCK_SMEM = 220 * 1024;            // what a block may take
@@ -318,7 +318,7 @@ struct MieSums {
     }
 };
 
-// The block's radii, G of them (TEAM 128: one), of one refractive index, in
+// The block's radii, G of them, of one refractive index, in
 // shared memory laid out for `rows`.  common(c) sets up what the radii share,
 // radius(g, c, n1, n2) radius g; factors(n, f3, f4) gives MieSums::add's;
 // begin(g) is called by a radius' team, then store(n, ab) once per order, by one
