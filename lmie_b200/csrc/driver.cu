@@ -1026,7 +1026,7 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
         x_own = c.gather.x_own;
     }
     const int n_tan = (int) hm + (int) hx;                    // tangent columns of the coefficients
-    const int n_co = 1 + n_tan, n_rs = 1 + 2 * (int) hm + (int) hx, ck_w = k1_ck_width(hm, hx);
+    const int n_co = 1 + n_tan, n_rs = 1 + 2 * (int) hm + (int) hx;
     // an FP64 re-solve whose cases' K1 outputs are in an earlier sub-batch's
     // arena: their copy, in pieces of at most GATHER_PIECE doubles (one
     // block each), replaces K1
@@ -1065,8 +1065,9 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
     const bool k1_block = !re_solve && k1_blocks(k1ord, k1pre, cs, cn1max, case_dz, R, hm, hx, c.sms, k1, [&](int k, int i) {
         return ps[k].n1r[ps[k].n - 1 - i];
     });
+    const bool k1_dz = std::find(case_dz.begin(), case_dz.end(), 1) != case_dz.end();
     // (K1's checkpoints are the thread-per-radius form's only)
-    const size_t ck_used = k1_block ? 0 : (size_t) ckn * ck_w;
+    const size_t ck_used = k1_block ? 0 : (size_t) ckn * k1_ck_width(hx, k1_dz);
 
     // ---- order tables ----
     std::vector<double> fv((size_t) 4 * (n1max + 2), 0.);
@@ -1825,6 +1826,7 @@ int submit_sub_as(Slot &S, long long ticket, int ncase, const lmieb_problem *ps,
     B.oz_wl = wl;
     B.k1_nblk = k1.n;
     B.k1_smem = k1.smem;
+    B.k1_dz = k1_dz;
     B.k1_rows = k1.rows;
     B.k1_rows_dz = k1.rows_dz;
     B.k1_blk = (const int4 *) dptr(h_k1blk);

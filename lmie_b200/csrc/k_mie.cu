@@ -187,36 +187,34 @@ __device__ __forceinline__ MieRadius<HX> radius_setup(const DevBatch &B, const D
 // values), forms D_n and the orders' coefficients and tangents, writes the
 // coefficient columns and sums the per-radius cross sections in order.  HM, HX:
 // with the m, the x column; TC: the split-precision cases' derivatives go to the
-// tensor-core operand instead.  Bound by FP64 latency (a thread's chain) where
-// few radii are long, by the FP64 pipe where many fill the SMs.
+// tensor-core operand instead; DZ: some radii's dD/dz is the tangent of D's
+// recurrence; RATIO: psi of fewer than MIE_P_MIN orders.  (3000 radii up to x =
+// 5000, values and a derivative by lambda 5.0 ms, by mr with DZ 5.3; with both
+// decided order by order in one body 5.8 and 5.3.)  Bound by FP64 latency (a
+// thread's chain) where few radii are long, by the FP64 pipe where many fill the SMs.
 // Per-radius sums rs[(col 5 + q) R + r], q: se, ss, Re sb, Im sb, sg, of the
 // columns 0 value, B.rs_m d/dmr, B.rs_m + 1 d/dmi (both from the m column),
 // B.rs_x the x column.
 // ---------------------------------------------------------------------------
-template <bool HM, bool HX, bool TC>
-__global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck, double *__restrict__ coef,
-                                            float *__restrict__ bop, double *__restrict__ rs) {
-    constexpr int CW = k1_ck_width(HM, HX);          // D (2), u (2), exponent, u's tangent (2), D's (2)
-    const long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= B.R) return;
-    const int r = radius_of(B, t);
+template <bool HM, bool HX, bool TC, bool DZ, bool RATIO>
+__device__ __forceinline__ void mie_thread(const DevBatch &B, const DevCase &C, int r, int n1, int n2,
+                                           double *__restrict__ ck, double *__restrict__ coef,
+                                           float *__restrict__ bop, double *__restrict__ rs) {
+    constexpr int CW = k1_ck_width(HX, DZ);          // D (2), u (2), exponent, u's tangent (2), D's (2)
     const int R = B.R;
-    const DevCase &C = B.cs[B.rcase[r]];
-    const int n1 = B.n1r[r], n2 = B.n2r[r];
     const MieRadius<HX> c = radius_setup<HX>(B, C, r);
-    const bool zr = HM ? mie_dz_chain(C.m, c.x) : HX && B.x_own && mie_dz_chain(C.m, c.x);   // D's tangent
-    const bool ratio = HX && n1 < MIE_P_MIN;         // q.cur, q.xcur: psi's ratio and its tangent
+    const bool zr = DZ && mie_dz_chain(C.m, c.x);    // D's tangent
     const int nb = n1 / MIE_B + 1;
     double *ckr = ck + (size_t) B.ckoff[r] * CW;     // nb blocks of CW doubles
     const double *fv4 = B.fv + 3 * (B.n1max + 2), *fv3 = fv4 - (B.n1max + 2);
 
     auto d_step = [&](MieD &p, int n) {
-        if ((HM || HX) && zr) p.step<true>(n, c.zinv, c.zinv2);
+        if (DZ && zr) p.step<true>(n, c.zinv, c.zinv2);
         else p.step(n, c.zinv);
     };
     // (the ratio of order n - 1; that of order 0 is not used)
     auto u_step = [&](MieU<HX> &q, int n) {
-        if (HX && ratio) {
+        if (RATIO) {                                  // q.cur, q.xcur: psi's ratio and its tangent
             mie_ratio(n - 1, c.xinv, q.cur, q.xcur);
         } else {
             q.step(n, c.xinv);
@@ -235,14 +233,14 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
             double *w = ckr + (size_t) b * CW;
             w[0] = p.cur.re; w[1] = p.cur.im; w[2] = q.hi; w[3] = q.cur; w[4] = (double) eu;
             if (HX) { w[5] = q.xhi; w[HX ? 6 : 0] = q.xcur; }
-            if (HM || HX) { w[CW - 2] = p.dz.re; w[CW - 1] = p.dz.im; }
+            if (DZ) { w[CW - 2] = p.dz.re; w[CW - 1] = p.dz.im; }
 #pragma unroll
             for (int i = MIE_B - 1; i >= 0; --i) {
                 const int k = b * MIE_B + i;
                 if (b > 0 || i > 0) d_step(p, k);
                 if (k <= n1 && (b > 0 || i > 0)) u_step(q, k);
             }
-            if (b > 0 && !ratio) eu += q.rescale();
+            if (b > 0 && !RATIO) eu += q.rescale();
         }
         u0 = q.cur;
         if (HX) ux0 = q.xcur;
@@ -254,7 +252,7 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     const double spsi = sinx / u0, spsix = HX ? fma(-spsi, ux0, cosx) / u0 : 0.;
     double chi_p = cosx, chi_c = fma(c.xinv, cosx, sinx);       // chi_0, chi_1
     double psi_p = spsi * u0, px = HX ? fma(spsix, u0, spsi * ux0) : 0.;   // px: d psi / dx
-    if (ratio) {
+    if (RATIO) {
         psi_p = sinx;
         px = cosx;
     }
@@ -284,7 +282,7 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
         {
             MieD p;
             p.cur = mk(w[0], w[1]);
-            p.dz = HM || HX ? mk(w[CW - 2], w[CW - 1]) : mk(0., 0.);
+            p.dz = DZ ? mk(w[CW - 2], w[CW - 1]) : mk(0., 0.);
             MieU<HX> q;
             q.hi = w[2];
             q.cur = w[3];
@@ -298,7 +296,10 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
                     d_step(p, k);
                     if (k <= n1) {
                         D[i] = p.cur;
-                        if (HM || HX) Dz[i] = zr ? p.dz : mie_dz(c, k, p.cur);
+                        if (HM || HX) {
+                            Dz[i] = mie_dz(c, k, p.cur);
+                            if (DZ && zr) Dz[i] = mie_dz_add(Dz[i], mie_dz_corr(c, k, p.cur, p.dz));
+                        }
                         u_step(q, k);
                     }
                 }
@@ -308,8 +309,8 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
         for (int i = 0; i < MIE_B; ++i) {
             const int j = b * MIE_B + i;
             if (j < 1 || j > n1) continue;
-            const double psi = ratio ? ub[i] * psi_p : spsi * ub[i] * su;
-            if (HX) px = ratio ? fma(uxb[HX ? i : 0], psi_p, ub[i] * px) : fma(spsix, ub[i], spsi * uxb[HX ? i : 0]) * su;
+            const double psi = RATIO ? ub[i] * psi_p : spsi * ub[i] * su;
+            if (HX) px = RATIO ? fma(uxb[HX ? i : 0], psi_p, ub[i] * px) : fma(spsix, ub[i], spsi * uxb[HX ? i : 0]) * su;
             const double psix = c.xl * px;
             const MieAB q = mie_ab<HM, HX>(c, j, D[i], Dz[i], psi, psi_p, chi_c, chi_p, psix, psix_p);
             sums.add(j, q, prev, fv3[j - 1], fv4[j - 1]);
@@ -338,12 +339,24 @@ __global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck,
     }
 }
 
+template <bool HM, bool HX, bool TC, bool DZ>
+__global__ void __launch_bounds__(64) k_mie(DevBatch B, double *__restrict__ ck, double *__restrict__ coef,
+                                            float *__restrict__ bop, double *__restrict__ rs) {
+    const long long t = (long long) blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= B.R) return;
+    const int r = radius_of(B, t), n1 = B.n1r[r], n2 = B.n2r[r];
+    const DevCase &C = B.cs[B.rcase[r]];
+    if (HX && n1 < MIE_P_MIN) mie_thread<HM, HX, TC, DZ, HX>(B, C, r, n1, n2, ck, coef, bop, rs);
+    else mie_thread<HM, HX, TC, DZ, false>(B, C, r, n1, n2, ck, coef, bop, rs);
+}
+
 // ---------------------------------------------------------------------------
 // K1 by blocks: block i's B.k1_blk[i].y radii are of case .z, from radius .x
 // down.  Bound by instruction issue (half of it taken, a third of the FP64
 // pipe's) where the blocks are many, by the chains' latency where they are few.
 // 107 thousand radii, 777 cases, values only: 303 us (a thread per radius: 789);
-// 109 thousand, 766 cases, with the m column: 766 us (915); the cloud
+// 109 thousand, 766 cases, with the m column: 766 us (915), 4096 cases 3.43 ms,
+// 3.87 with D's tangent for the sixth of the orders that takes it; the cloud
 // droplet's 2000 radii up to x = 436: 69 us (a thread per radius 380).
 // ---------------------------------------------------------------------------
 template <bool HM, bool HX, bool TC, int TEAM>
@@ -442,6 +455,17 @@ int launch_block(cudaStream_t s, const DevBatch &B, double *coef, float *bop, do
     return 0;
 }
 
+template <bool HM, bool HX, bool DZ>
+int launch_threads(cudaStream_t s, const DevBatch &B, double *ck, double *coef, float *bop, double *rs) {
+    if (bop)
+        k_mie<HM, HX, true, DZ>
+            <<<ceil_div(B.R, 64), 64, 4 * 8 * (1 + B.nd1) * 64 * sizeof(float), s>>>(B, ck, coef, bop, rs);
+    else
+        k_mie<HM, HX, false, DZ><<<ceil_div(B.R, 64), 64, 0, s>>>(B, ck, coef, nullptr, rs);
+    LMIEB_CUDA_TRY(cudaGetLastError());
+    return 0;
+}
+
 template <bool HM, bool HX>
 int launch(cudaStream_t s, const DevBatch &B, double *ck, double *coef, float *bop, double *rs) {
     // the orders of a radius by the whole block where it has one, or where they
@@ -453,12 +477,9 @@ int launch(cudaStream_t s, const DevBatch &B, double *ck, double *coef, float *b
     if (B.k1_nblk)
         return bop ? launch_block<HM, HX, true, 32>(s, B, coef, bop, rs)
                    : launch_block<HM, HX, false, 32>(s, B, coef, bop, rs);
-    if (bop)
-        k_mie<HM, HX, true><<<ceil_div(B.R, 64), 64, 4 * 8 * (1 + B.nd1) * 64 * sizeof(float), s>>>(B, ck, coef, bop, rs);
-    else
-        k_mie<HM, HX, false><<<ceil_div(B.R, 64), 64, 0, s>>>(B, ck, coef, nullptr, rs);
-    LMIEB_CUDA_TRY(cudaGetLastError());
-    return 0;
+    if (HM || HX)
+        if (B.k1_dz) return launch_threads<HM, HX, HM || HX>(s, B, ck, coef, bop, rs);
+    return launch_threads<HM, HX, false>(s, B, ck, coef, bop, rs);
 }
 
 }  // namespace

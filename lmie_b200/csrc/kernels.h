@@ -20,9 +20,9 @@ struct GatherSeg {
     long long dst_off, n;
     int which;
 };
-// doubles per K1 checkpoint (k_mie.cu; one per MIE_B orders), hm, hx: with the m,
-// the x column of the tangent basis
-__host__ __device__ constexpr int k1_ck_width(bool hm, bool hx) { return (hx ? 7 : 5) + (hm || hx ? 2 : 0); }
+// doubles per K1 checkpoint (k_mie.cu; one per MIE_B orders), hx: with the x column of the tangent basis, dz: some
+// radius takes dD/dz from D's recurrence
+__host__ __device__ constexpr int k1_ck_width(bool hx, bool dz) { return (hx ? 7 : 5) + (dz ? 2 : 0); }
 
 // One case of a batch (device copy).  Offsets index the batch-wide arrays.
 struct DevCase {
@@ -75,6 +75,7 @@ struct DevBatch {
     // and rs_x.
     int t_m, t_x, x_own, rs_m, rs_x;
     int k1_nblk, k1_smem;       // K1: blocks (0: a thread per radius) and the shared memory of one
+    int k1_dz;                  // some radius takes dD/dz from D's recurrence (mie_radius.cuh)
     int k1_rows, k1_rows_dz;    // its rows, without and with dD/dz from D's recurrence
     const int4 *k1_blk;         // [k1_nblk] blocks (mie_radius.cuh): largest radius, radii, case, with dD/dz
     const double *w;            // [(1 + nd)][R] row 0: f = nr qw; row 1+kk: f_l (index1) or f_l2 (index2)

@@ -68,14 +68,16 @@ constexpr int MIE_P_MIN = 32;
 // Medians of d Cext/dmr of 400 spheres of x 100 .. 900 against 113-bit arithmetic,
 // tangent / Riccati: mi x 0.3 .. 1 9.2e-14 / 9.4e-14, 1 .. 3 8.9e-14 / 1.0e-13,
 // 3 .. 10 2.7e-13 / 4.1e-12, 30 .. 100 9.3e-15 / 7.2e-13; x 8 .. 96 alike.  By x the two
-// are equal everywhere.
-constexpr double MIE_DZ_MIN = 0.5;
+// are equal everywhere.  A block keeps the tangent as a correction of the Riccati
+// equation's in 8 bytes an order: with 16, four blocks no longer fit an SM (4096
+// uneven cases 4.66 ms, with 8 3.87, without the tangent 3.43).
+constexpr double MIE_DZ_MIN = 1.;
 
 // rows of shared memory of a radius of n1 orders; bytes of a block of that many rows: D, u, chi (hx: and u's
-// tangent; dz: and D's), two exponents per MIE_B orders, reduction space, what the team needs to know of each radius
+// tangent; dz: and D's, as a correction), two exponents per MIE_B orders, reduction space, what the team needs to know of each radius
 __host__ __device__ constexpr int mie_block_rows(int n1) { return (n1 + 2 * MIE_B) & ~(MIE_B - 1); }
 __host__ __device__ constexpr int mie_block_smem(int rows, bool hx, bool dz) {
-    return rows * (16 + 8 + 8 + (hx ? 8 : 0) + (dz ? 16 : 0)) + rows / MIE_B * 8 + (4 * 12 + 20 * 4) * 8 + MIE_BLOCK_MAX * 72;
+    return rows * (16 + 8 + 8 + (hx ? 8 : 0) + (dz ? 8 : 0)) + rows / MIE_B * 8 + (4 * 12 + 20 * 4) * 8 + MIE_BLOCK_MAX * 72;
 }
 
 #ifdef __CUDACC__
@@ -225,6 +227,16 @@ __device__ __forceinline__ cplx mie_dz(const MieRadius<HX> &c, int n, cplx D) {
     return cfma(nz - D, nz + D, cfma(c.zinv2, (double) n, mk(-1., 0.)));
 }
 
+// The tangent dz of D's recurrence as what it corrects the Riccati equation's
+// dD/dz by: that is a rounding of terms of order 1, and 24 bits of it are more
+// than the sum can hold.
+template <bool HX>
+__device__ __forceinline__ float2 mie_dz_corr(const MieRadius<HX> &c, int n, cplx D, cplx dz) {
+    const cplx e = dz - mie_dz(c, n, D);
+    return make_float2((float) e.re, (float) e.im);
+}
+__device__ __forceinline__ cplx mie_dz_add(cplx ric, float2 e) { return mk(ric.re + (double) e.x, ric.im + (double) e.y); }
+
 // The coefficients of order n and their tangents: a, b; am, bm w.r.t. m; ax, bx
 // in the x column's direction.
 struct MieAB {
@@ -330,7 +342,8 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, bool dz
     constexpr int T = MIE_BLOCK_T, W = T / 32, NP = HX ? 12 : 8, NS = MieSums<HM, HX>::N;
     static_assert(TEAM == T || TEAM == 32, "the block or a warp");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    double2 *Ds = (double2 *) smem, *Dzs = Ds + rows;
+    double2 *Ds = (double2 *) smem;
+    float2 *Dzs = (float2 *) (Ds + rows);
     double *u = (double *) (dz ? Dzs + rows : Dzs), *chi = u + rows, *ux = chi + rows;
     double *pass = chi + rows + (HX ? rows : 0);      // [W][12] last coefficients of a warp
     double *red = pass + W * 12;                      // [20][W]
@@ -373,12 +386,13 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, bool dz
                 MieD p;
                 p.start();
                 if (DER && dz) {
-                    double2 *Zr = Dzs + row;
+                    float2 *Zr = Dzs + row;
                     for (int n = n2 - 1; n > n1; --n) p.step<true>(n, c.zinv, c.zinv2);
+#pragma unroll 4
                     for (int n = n1; n >= 1; --n) {
                         p.step<true>(n, c.zinv, c.zinv2);
                         Dr[n] = make_double2(p.cur.re, p.cur.im);
-                        Zr[n] = make_double2(p.dz.re, p.dz.im);
+                        Zr[n] = mie_dz_corr(c, n, p.cur, p.dz);
                     }
                 } else {
                     for (int n = n2 - 1; n > n1; --n) p.step(n, c.zinv);
@@ -485,7 +499,8 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, bool dz
         if (HX) c.xl = sh_xl[g];
         const double spsi = sh_psi[g], spsix = HX ? sh_psix[g] : 0.;
         const int eu0 = sh_eu[g], row = sh_row[g];
-        const double2 *Dr = Ds + row, *Zr = Dzs + row;
+        const double2 *Dr = Ds + row;
+        const float2 *Zr = Dzs + row;
         const bool zr = DER && dz && mie_dz_chain(c.m, c.x);
         const double *ur = u + row, *uxr = ux + row, *cr = chi + row;
         const int *eur = eU + row / MIE_B;
@@ -504,11 +519,9 @@ __device__ __forceinline__ void mie_block(unsigned char *smem, int rows, bool dz
             if (on) {
                 const double2 dj = Dr[j];
                 cplx D = mk(dj.x, dj.y), Dz = mk(0., 0.);
-                if (zr) {
-                    const double2 zj = Zr[j];
-                    Dz = mk(zj.x, zj.y);
-                } else if (DER) {
+                if (DER) {
                     Dz = mie_dz(c, j, D);
+                    if (zr) Dz = mie_dz_add(Dz, Zr[j]);
                 }
                 if (!chain_d(n1)) {
                     const double2 lo = Dr[j - 1];
