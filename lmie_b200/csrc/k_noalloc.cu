@@ -41,8 +41,8 @@ struct Trunc {
 static_assert(mie_block_smem(mie_block_rows(NA_MAX_ORDER), false, false) <= 48 * 1024, "shared memory of a block");
 
 // Bound by FP64 latency: the three chains of the largest radius (n1 dependent
-// pairs of FMAs), then n1 / 128 rounds of orders.  1000 radii up to x = 880: 66 us, the
-// whole call: 130 us (a thread per radius with D and psi in device memory: 1795).
+// pairs of FMAs), then n1 / 128 rounds of orders.  1000 radii up to x = 880: 45 us, the
+// whole call: 110 us (a thread per radius with D and psi in device memory: 1770).
 __global__ void __launch_bounds__(MIE_BLOCK_T) k_cross_sections(int n, const double *__restrict__ radius,
                                                                 double lambda, cplx m, cplx minv, int rows,
                                                                 const __grid_constant__ Trunc trunc,

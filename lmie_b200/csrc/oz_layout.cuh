@@ -68,7 +68,7 @@ constexpr int OZ_M = 128;                            // product rows: 64 half-an
 constexpr int OZ_HALF = OZ_M / 2;
 constexpr int OZ_MAX_ND1 = 4;                        // index1 derivatives the kernel is built for
 constexpr int OZ_MAX_ND2 = 3;                        // index2 derivatives the kernel is built for
-constexpr int OZ_MAX_NK = 160;                       // chunks per group (5120 orders: int32 sums exact)
+constexpr int OZ_MAX_NK = 160;                       // chunks per group (5120 orders; int32 sums are exact to 18 thousand)
 constexpr int OZ_MIN_N1 = 16;                        // smaller cases keep the FP64 angular stage
 
 // whether the stage takes a case of truncation n1 whose radii reach n1max orders: at least OZ_MIN_N1, and
